@@ -324,6 +324,15 @@ ncclResult_t commCollective(ncclComm* c, int kind, const void* send, void* recv,
   if (kind == dfcclCollAllReduce || kind == dfcclCollReduce || kind == dfcclCollReduceScatter)
     DFCHECK(resolveRedOp(c, op, type, c->nranks, &devOp, &cs.scale, &cs.postDiv));
   cs.op = devOp;
+  if (c->nranks == 1 && c->backend == dfcclBackendCuda) {
+    l.unlock();
+    int prev = 0;
+    cudaGetDevice(&prev);
+    if (prev != c->device) cudaSetDevice(c->device);
+    ncclResult_t res = launchOneRankCuda(cs, send, recv, stream);
+    if (prev != c->device) cudaSetDevice(prev);
+    return res;
+  }
   const Topology* topo = nullptr;
   DFCHECK(topoGet(&topo));
   const size_t bytes = count * dtypeSize(type);

@@ -14,6 +14,9 @@ ncclResult_t launchDaemonCuda(RankDev** devRankTable, int nRanks, int blocksPerR
 ncclResult_t launchStandaloneCuda(RankDev* rd, const CollStatic& cs, uint64_t send, uint64_t recv, uint32_t epoch,
                                   uint32_t sqeFlags, int threads, cudaStream_t stream);
 
+// The same on a one-rank communicator: one streaming kernel, buffers used where they are.
+ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream);
+
 // Force the lazily loaded kernels of the runtime into the context (no launch).
 ncclResult_t warmRuntimeKernels();
 

@@ -1,0 +1,50 @@
+"""Collectives of a one-rank communicator run as one streaming kernel over the whole GPU (csrc/src/daemon/onerank.cu):
+sizes around its pack, block and grid boundaries, buffers off the 16-byte grid, every element size."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+PACKS_OF_FOUR = 148 * 256 * 4           # 16-byte packs from which a thread takes four (148 SMs)
+
+
+@pytest.fixture(scope="module")
+def comm():
+    from dfccl_b200 import native as nv
+    nv.set_backend("cuda")
+    torch.cuda.set_device(0)
+    (c,) = nv.Comm.init_loopback(1, 0)
+    yield c
+    c.destroy()
+
+
+@pytest.mark.parametrize("dt", ["float32", "bfloat16", "float16", "float64", "int32", "int8"])
+@pytest.mark.parametrize("nbytes", [8, 16, 4096 - 8, 256 * 16 + 8, PACKS_OF_FOUR * 16 - 24, PACKS_OF_FOUR * 16 + 40])
+@pytest.mark.parametrize("skew", [(0, 0), (1, 1), (1, 0)])
+def test_premultiplied_sum_and_copies_of_one_rank(comm, dt, nbytes, skew):
+    """A pre-multiplied sum is one multiplication in the accumulator type and one rounding: the result is exactly that
+    of the same multiplication in PyTorch.  Kinds that only copy, and a plain sum in place, leave the bytes as they are."""
+    from dfccl_b200 import native as nv
+    from dfccl_b200.ops import collectives
+    from dfccl_b200.utils import nccl_dtype
+    tdt = getattr(torch, dt)
+    n = nbytes // torch.empty((), dtype=tdt).element_size()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = (torch.randn(n + 8, device="cuda", generator=g) * 50).to(tdt)[skew[0]:skew[0] + n]
+    y = torch.zeros(n + 8, device="cuda", dtype=tdt)
+    out = y[skew[1]:skew[1] + n]
+    assert torch.equal(collectives.all_gather(comm, x, out), x)
+    assert torch.equal(y[skew[1] + n:], torch.zeros_like(y[skew[1] + n:]))          # nothing behind the end
+    z = x.clone()
+    assert torch.equal(collectives.all_reduce(comm, z, op="avg"), x)
+    if not tdt.is_floating_point:
+        return
+    L, op, s = nv.lib(), C.c_int(), C.c_float(0.3)
+    nv.check(L.ncclRedOpCreatePreMulSum(C.byref(op), C.byref(s), nv.FLOAT32, 1, comm.handle))
+    st = torch.cuda.current_stream().cuda_stream
+    nv.check(L.ncclReduceScatter(x.data_ptr(), out.data_ptr(), n, nccl_dtype(tdt), op.value, comm.handle, st))
+    nv.check(L.ncclRedOpDestroy(op.value, comm.handle))
+    acc = torch.float64 if tdt == torch.float64 else torch.float32
+    assert torch.equal(out, (x.to(acc) * torch.tensor(s.value, dtype=acc, device="cuda")).to(tdt))
