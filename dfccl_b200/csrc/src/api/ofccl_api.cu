@@ -189,7 +189,7 @@ static void observerMain(DaemonLauncher* L) {
     }
     bool work = false, dead = false;
     for (auto* m : members) {
-      if ((ctl_load(&m->ctl->hold) ? m->remaining.load() : m->remaining.load() - m->untriggered.load()) - m->netPending.load() > 0 && !ctl_load(&m->ctl->finalQuit)) work = true;
+      if ((ctl_load(&m->ctl->hold) ? m->remaining.load() : m->remaining.load() - m->untriggered.load()) - m->outside.load() > 0 && !ctl_load(&m->ctl->finalQuit)) work = true;
       if (ctl_load(&m->ctl->abortFlag)) dead = true;
     }
     if (work && !dead) {
@@ -202,7 +202,7 @@ static void observerMain(DaemonLauncher* L) {
         if (r != ncclSuccess) for (auto* m : members) m->asyncError = r;
       } else {
         runDaemonHost(L->devTable, L->expected, L->blocks);     // returns when every block has left
-        for (auto* m : members) if (m->remaining.load() - m->untriggered.load() - m->netPending.load() > 0 && !ctl_load(&m->ctl->finalQuit) && !ctl_load(&m->ctl->abortFlag)) { lk.lock(); L->wake = true; lk.unlock(); break; }
+        for (auto* m : members) if (m->remaining.load() - m->untriggered.load() - m->outside.load() > 0 && !ctl_load(&m->ctl->finalQuit) && !ctl_load(&m->ctl->abortFlag)) { lk.lock(); L->wake = true; lk.unlock(); break; }
       }
     }
     lk.lock();
@@ -227,8 +227,10 @@ static void deliver(ofcclRankCtx* ctx, uint64_t entry) {
   if (cb) { cb(coll, args); ctx->cbs++; }
   {
     std::lock_guard<std::mutex> l(ctx->mu);
-    { uint64_t* w = &ctx->byId[coll]->completed; __atomic_store_n(w, *w + 1, __ATOMIC_RELEASE); }   // also read lock-free by spinning waiters
+    CollEntry* e = ctx->byId[coll];
+    { uint64_t* w = &e->completed; __atomic_store_n(w, *w + 1, __ATOMIC_RELEASE); }   // also read lock-free by spinning waiters
     ctx->remaining--;
+    if (e->direct) { e->direct = false; ctx->outside--; }
     if (ctx->remaining.load() == 0) ctl_store(&ctx->ctl->hold, 0);
   }
   ctx->doneCv.notify_all();
@@ -294,7 +296,7 @@ static void pollerMain(ofcclRankCtx* ctx) {
     }
     // nothing new: if the daemon left while work is outstanding, have it launched again
     if (++empty % ctx->checkInterval == 0 || (empty & 63) == 0) {
-      const int64_t ready = (ctl_load(&ctx->ctl->hold) ? ctx->remaining.load() : ctx->remaining.load() - ctx->untriggered.load()) - ctx->netPending.load();
+      const int64_t ready = (ctl_load(&ctx->ctl->hold) ? ctx->remaining.load() : ctx->remaining.load() - ctx->untriggered.load()) - ctx->outside.load();
       if (!ctl_load(&ctx->ctl->alive) && ready > 0 && !ctl_load(&ctx->ctl->abortFlag)) wakeLauncher(ctx->launcher.get());
     }
     if (empty > 2000) std::this_thread::sleep_for(std::chrono::microseconds(20)); else sched_yield();
@@ -660,6 +662,52 @@ enum SubmitMode {
   SUBMIT_DEFERRED = 2,    // by a later dfcclTriggerOnStream (or by the replay of a graph that captured one)
 };
 
+static bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// A stream-ordered collective of a one-rank communicator waits for nobody, so no order of issue can make it part of a
+// deadlock and nothing is gained by handing it to the daemon: it runs in the stream itself, as one kernel over the
+// whole GPU that publishes the same device flag and completion entry.  (Through the daemon the release, the pass that
+// finds it and the stream's wait cost about 20 us a call, and a 25 MB gradient bucket moved on 8 daemon blocks took
+// about 250 us.)
+static bool runsDirect(const ofcclRankCtx* ctx, const CollEntry& e, cudaStream_t stream) {
+  return ctx->backend == dfcclBackendCuda && e.cs.nranks == 1 && ctx->fnWait64 && ctx->faultDrop == 0 && !capturing(stream);
+}
+
+// Called with ctx->mu held (`l`), after the previous submission of the id has completed.  The launch itself happens
+// without the lock: a launch can block while the GPU's queue is full, and the poller, which needs the lock, may have to
+// relaunch a parked daemon for other streams in the meantime.
+static ncclResult_t runDirect(ofcclRankCtx* ctx, CollEntry& e, int collId, const void* send, void* recv, CallbackFunc cb, void* cbArgs,
+                              cudaStream_t stream, std::unique_lock<std::mutex>& l) {
+  unsigned long long streamId = 0;
+  if (cudaStreamGetId(stream, &streamId) != cudaSuccess) { (void)cudaGetLastError(); DF_WARN("collective %d: not a stream of this context", collId); return ncclInvalidArgument; }
+  e.cb = cb; e.cbArgs = cbArgs;
+  e.submitted++;
+  e.direct = e.lastDirect = true;
+  e.directStream = streamId;
+  ctx->outside++;
+  ctx->remaining++;
+  ctx->sqes++;
+  const OneRankDone done{ctx->rdDev, collId, (uint32_t)e.submitted};
+  l.unlock();
+  int prev = 0;
+  cudaGetDevice(&prev);
+  if (prev != ctx->device) cudaSetDevice(ctx->device);
+  ncclResult_t r = launchOneRankCuda(e.cs, send, recv, stream, &done);
+  if (prev != ctx->device) cudaSetDevice(prev);
+  if (r != ncclSuccess) {                    // nothing was launched: undo the bookkeeping
+    std::lock_guard<std::mutex> g(ctx->mu);
+    e.submitted--;
+    e.direct = e.lastDirect = false;
+    ctx->remaining--; ctx->outside--; ctx->sqes--;
+  }
+  ctx->pollCv.notify_one();
+  return r;
+}
+
 static ncclResult_t submit(ofcclRankCtx* ctx, const void* send, void* recv, int collId, CallbackFunc cb, void* cbArgs,
                            SubmitMode mode, cudaStream_t stream) {
   if (!ctx || !ctx->finalized || ctx->destroyed) { DF_WARN("context is not ready for submissions"); return ncclInvalidUsage; }
@@ -708,24 +756,25 @@ static ncclResult_t submit(ofcclRankCtx* ctx, const void* send, void* recv, int 
       e.cb = cb; e.cbArgs = cbArgs;
       e.submitted++;
       ctx->remaining++;
-      ctx->netPending++;
+      ctx->outside++;
       ctx->sqes++;
       const bool posted = ctx->netWorkers.post([ctx, comm, ring, d, send, recv, collId] {
         logSetRank(ctx->rank);
         ncclResult_t r = netStagedCollective(comm, ring.get(), d, send, recv, nullptr);
         const uint32_t st = r == ncclSuccess ? ST_OK : r == dfcclAborted ? ST_ABORTED : r == dfcclTimeout ? ST_TIMEOUT : ST_BAD_ARG;
-        ctx->netPending--;
+        ctx->outside--;
         deliver(ctx, ((uint64_t)st << 24) | (uint64_t)(uint32_t)collId);
       });
       if (!posted) {                        // no thread to run it on: undo the bookkeeping, the caller may try again
         e.cb = prevCb; e.cbArgs = prevArgs;
-        e.submitted--; ctx->remaining--; ctx->netPending--; ctx->sqes--;
+        e.submitted--; ctx->remaining--; ctx->outside--; ctx->sqes--;
         DF_WARN("collective %d: no worker thread could be created for the network path", collId);
         return ncclSystemError;
       }
       ctx->pollCv.notify_one();
       return ncclSuccess;
     }
+    if (mode == SUBMIT_STREAM && runsDirect(ctx, e, stream)) return runDirect(ctx, e, collId, send, recv, cb, cbArgs, stream, l);
     Heap* heap = e.comm->heap;
     const size_t sB = sendBytes(&cs), rB = recvBytes(&cs);
     q.collId = collId;
@@ -756,7 +805,7 @@ static ncclResult_t submit(ofcclRankCtx* ctx, const void* send, void* recv, int 
       if (stageSend) { q.flags |= SQE_SEND_STAGED; q.send = (uint64_t)(uintptr_t)send; } else if (needSend) q.send = heap->offsetOf(send);
       if (stageRecv) { q.flags |= SQE_RECV_STAGED; q.recv = (uint64_t)(uintptr_t)recv; } else if (needRecv) q.recv = heap->offsetOf(recv);
     }
-    if (onStream) { q.flags |= SQE_TRIGGERED; q.trigger = trig = ++e.triggerSeq; }
+    if (onStream) { q.flags |= SQE_TRIGGERED; trig = ++e.triggerSeq; q.trigger = (uint32_t)trig; }
     // flow control: never overwrite an entry some block has not consumed yet
     while (ctx->sqTail - ctx->sqMinFrontier >= ctx->sqCap && (ctx->sqMinFrontier = minFrontier(ctx), ctx->sqTail - ctx->sqMinFrontier >= ctx->sqCap)) {
       ctx->sqFull++;
@@ -767,6 +816,8 @@ static ncclResult_t submit(ofcclRankCtx* ctx, const void* send, void* recv, int 
     }
     e.cb = cb; e.cbArgs = cbArgs;
     e.submitted++;
+    e.lastDirect = false;
+    q.epoch = (uint32_t)e.submitted;
     ctx->remaining++;
     ctx->sqes++;
     if (deferWake) {                   // the poller watches the trigger's host mirror and wakes a parked daemon
@@ -910,23 +961,26 @@ DF_API ncclResult_t dfcclSetHoldOnWait(ofcclRankCtx_t ctx, int on) {
 DF_API ncclResult_t dfcclStreamWait(int collId, cudaStream_t stream, ofcclRankCtx_t ctx) {
   if (!ctx || !ctx->finalized) return ncclInvalidUsage;
   uint64_t want;
+  bool direct = false;
   {
     std::lock_guard<std::mutex> l(ctx->mu);
-    auto it = ctx->colls.find(collId);
-    if (it == ctx->colls.end()) return ncclInvalidArgument;
-    want = it->second.submitted;
+    CollEntry* e = collId >= 0 && collId < (int)ctx->byId.size() ? ctx->byId[collId] : nullptr;
+    if (!e) return ncclInvalidArgument;
+    want = e->submitted;
+    direct = e->lastDirect;
+    unsigned long long id = 0;
+    // it ran in this very stream: everything enqueued from here on is behind it already
+    if (direct && cudaStreamGetId(stream, &id) == cudaSuccess && id == e->directStream) return ncclSuccess;
   }
   if (ctx->backend == dfcclBackendCuda && ctx->fnWait64) {
     // The stream is about to park on a word only the daemon sets.  Outside a capture, make sure an instance is
     // queued BEFORE the wait in host order and that it stays until the work is done: the release of the stream
     // then never depends on another host thread getting a launch through while this one may be blocked in the
     // driver (full launch queue, module load).  Captured steps keep the poller-driven wake-up.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) { (void)cudaGetLastError(); cap = cudaStreamCaptureStatusNone; }
     // (only where this context has the daemon launch to itself: ranks that share one launch - several ranks
     // of one process on one device - must keep leaving when stalled, or one rank's held blocks would keep the
     // shared kernel alive in front of the relaunch another rank is waiting for)
-    if (ctx->holdOnWait && cap == cudaStreamCaptureStatusNone && ctx->remaining.load() > 0 && ctx->launcher && ctx->launcher->expected == 1) {
+    if (!direct && ctx->holdOnWait && !capturing(stream) && ctx->remaining.load() > ctx->outside.load() && ctx->launcher && ctx->launcher->expected == 1) {
       ctl_store(&ctx->ctl->hold, 1);
       std::atomic_thread_fence(std::memory_order_seq_cst);
       if (!ctl_load(&ctx->ctl->alive)) DFCHECK(launchFromCaller(ctx));

@@ -38,6 +38,10 @@ struct CollEntry {
   uint64_t submitted = 0, completed = 0;     // guarded by ctx->mu
   uint64_t triggerSeq = 0;
   uint32_t lastStatus = 0;
+  // The last submission ran as a kernel of its own on a stream (one-rank communicators, see runDirect): `direct` until
+  // its completion is delivered, `directStream` (the runtime's unique id of a stream, never reused) for stream waits.
+  bool direct = false, lastDirect = false;
+  unsigned long long directStream = 0;
   std::shared_ptr<NetRing> ring;             // network-mode communicators: this collective's own ring of connections
   // fused tensor-parallel operator (dfcclPrepareFusedGemm): one heap block per member holds its rendezvous words,
   // counters and receive areas; the daemon never sees these ids
@@ -108,7 +112,8 @@ struct ofcclRankCtx {
   std::thread poller;
   dfccl::NetWorkers netWorkers;               // submissions on network-mode communicators run here
   std::vector<dfccl::CollEntry*> byId;        // collId -> entry (built at finalize: no tree walk on the hot path)
-  std::atomic<int64_t> netPending{0};         // submissions running on the host network path (not the daemon's business)
+  std::atomic<int64_t> outside{0};            // submissions that are not the daemon's business: on the host network path, or
+                                              // running as kernels of their own
   std::mutex mu;                      // submissions, callbacks table, counters
   std::condition_variable pollCv;     // poller sleeps here while nothing is outstanding
   std::condition_variable doneCv;     // dfcclWait

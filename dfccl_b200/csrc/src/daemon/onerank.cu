@@ -25,6 +25,7 @@ struct OneRankArgs {
   uint64_t nPacks;           // packs of 16 source bytes
   double scale;
   int postDiv;
+  OneRankDone done;          // registered collective: where the completion goes (rd null: a stream-ordered call, nowhere)
 };
 
 // One element of the head, the ragged tail, or of buffers that do not line up.
@@ -77,6 +78,17 @@ __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs 
     const uint64_t e = i < a.head ? i : tail0 + (i - a.head);
     if (COPY) a.dst[e] = a.src[e]; else oneElem<Tin, Tout>(a, e);
   }
+  if (a.done.rd == nullptr) return;
+  // the last block out publishes the completion, as the daemon's blocks do
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    fence_gpu();
+    uint32_t* count = &a.done.rd->doneCount[a.done.coll];
+    if (atomic_add_u32(count, 1u) + 1u == gridDim.x) {
+      atomic_exch_u32(count, 0u);
+      publishCompletion(a.done.rd, a.done.coll, ST_OK, a.done.epoch);
+    }
+  }
 }
 
 template <typename Tin, typename Tout, bool COPY>
@@ -113,16 +125,20 @@ int smCount() {
 
 }  // namespace
 
-ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream) {
+ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream, const OneRankDone* done) {
   OneRankArgs a;
   memset(&a, 0, sizeof(a));
+  if (done) a.done = *done;
   a.src = (const char*)send; a.dst = (char*)recv; a.n = cs.count; a.scale = cs.scale; a.postDiv = cs.postDiv;
   const bool reduces = cs.kind == dfcclCollAllReduce || cs.kind == dfcclCollReduce || cs.kind == dfcclCollReduceScatter;
   const bool plain = cs.inType == cs.outType && (!reduces || (cs.scale == 1.0 && cs.postDiv <= 1));
   const int sms = smCount();
   if (plain) {
-    if (send == recv) return ncclSuccess;                // in place: already where it belongs
     a.n = cs.count * (uint64_t)dtypeSize(cs.inType);
+    if (send == recv) {                                  // in place: already where it belongs
+      if (!done) return ncclSuccess;
+      a.n = 0;
+    }
     return launchTyped<uint8_t, uint8_t, true>(a, sms, stream);
   }
   if (cs.inType == cs.outType) {

@@ -62,11 +62,11 @@ DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b) {
     sh->stats.sqesSeen++;
     if (!mine) continue;
     d->send = q.send; d->recv = q.recv; d->trigger = q.trigger; d->cursor = 0;
-    d->epoch = d->epoch + 1; d->sqeFlags = q.flags; d->status = ST_OK; d->stallSinceNs = 0; d->patience = 0;
+    d->epoch = q.epoch; d->sqeFlags = q.flags; d->status = ST_OK; d->stallSinceNs = 0; d->patience = 0;
     trace(rd, b, TR_SQE, coll);
     if (q.flags & SQE_TRIGGERED) {
       d->phase = PH_TRIGGER;
-      sh->trigColl[sh->nTrig] = (uint16_t)coll; sh->trigVal[sh->nTrig] = (uint32_t)q.trigger; ++sh->nTrig;
+      sh->trigColl[sh->nTrig] = (uint16_t)coll; sh->trigVal[sh->nTrig] = q.trigger; ++sh->nTrig;
     } else {
       d->phase = PH_COPY_IN;          // runColl skips ahead to the first phase that has work
       sh->actWait[sh->nActive] = 0;

@@ -173,7 +173,7 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
     for (;;) {
       bool laneOk = true;
       if (which == 2) {
-        if (lane == 0) laneOk = ld_relaxed_sys_u64(&rd->trigger[sh->loadedColl]) >= sh->dyn.trigger;
+        if (lane == 0) laneOk = (int32_t)((uint32_t)ld_relaxed_sys_u64(&rd->trigger[sh->loadedColl]) - (uint32_t)sh->dyn.trigger) >= 0;
       } else {
         for (int j = lane; j < n; j += ws) {
           if (j == me) continue;

@@ -14,8 +14,10 @@ ncclResult_t launchDaemonCuda(RankDev** devRankTable, int nRanks, int blocksPerR
 ncclResult_t launchStandaloneCuda(RankDev* rd, const CollStatic& cs, uint64_t send, uint64_t recv, uint32_t epoch,
                                   uint32_t sqeFlags, int threads, cudaStream_t stream);
 
-// The same on a one-rank communicator: one streaming kernel, buffers used where they are.
-ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream);
+// The same on a one-rank communicator: one streaming kernel, buffers used where they are.  With `done` the kernel also
+// publishes the completion of a registered collective (device flag and completion entry).
+struct OneRankDone { RankDev* rd; int32_t coll; uint32_t epoch; };
+ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream, const OneRankDone* done = nullptr);
 
 // Force the lazily loaded kernels of the runtime into the context (no launch).
 ncclResult_t warmRuntimeKernels();

@@ -35,8 +35,11 @@ struct alignas(16) Sqe {
   uint32_t flags;
   uint64_t send;          // heap offset, or raw local address when SQE_SEND_STAGED
   uint64_t recv;          // heap offset, or raw local address when SQE_RECV_STAGED
-  uint64_t trigger;       // value trigger[collId] must reach (SQE_TRIGGERED)
+  uint32_t trigger;       // value the low half of trigger[collId] must reach (SQE_TRIGGERED)
+  uint32_t epoch;         // number of this submission of the collective, counted by the host from 1: not every submission
+                          // of an id has to pass through the daemon
 };
+static_assert(sizeof(Sqe) == 32, "an entry is written as four 64-bit words");
 
 // ---- completion entry: one 64-bit word, gen makes a slot self-validating
 //   [63:32] generation of the ring slot (index / capacity + 1)   [31:24] status   [23:0] collId
@@ -103,9 +106,9 @@ struct alignas(16) CollStatic {
 // ---- mutable per (block, collective) state; what a context switch saves and loads
 struct alignas(16) CollDyn {
   uint64_t send, recv;    // this submission's buffers (offset or raw address, see Sqe)
-  uint64_t trigger;
+  uint64_t trigger;       // low 32 bits count
   uint64_t cursor;        // progress inside PH_DATA / copies when sliced
-  uint32_t epoch;         // submissions of this collective seen so far
+  uint32_t epoch;         // number of the running submission (0 = none yet)
   int32_t phase;
   uint32_t sqeFlags;
   uint32_t status;

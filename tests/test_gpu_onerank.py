@@ -48,3 +48,48 @@ def test_premultiplied_sum_and_copies_of_one_rank(comm, dt, nbytes, skew):
     nv.check(L.ncclRedOpDestroy(op.value, comm.handle))
     acc = torch.float64 if tdt == torch.float64 else torch.float32
     assert torch.equal(out, (x.to(acc) * torch.tensor(s.value, dtype=acc, device="cuda")).to(tdt))
+
+
+@pytest.mark.parametrize("n", [1, 1000003])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_registered_collective_of_one_rank_in_the_stream_and_through_the_daemon(n, in_place):
+    """A stream-ordered submission of a one-rank collective runs in the stream itself; deferred and host submissions of
+    the same id go through the daemon.  Mixed, they must count alike: a wait on another stream sees the right one, and
+    every submission is delivered to the host."""
+    from dfccl_b200 import native as nv
+    from dfccl_b200.utils import tensor_from_ptr
+    nv.set_backend("cuda")
+    torch.cuda.set_device(0)
+    (c,) = nv.Comm.init_loopback(1, 0)
+    ctx = nv.RankCtx(0, 0)
+    scale = 1.0 if in_place else 3.0
+    ctx.prepare(0, c, nv.ALLREDUCE, n, nv.FLOAT32, scale=scale)
+    ctx.finalize()
+    p = c.alloc(4 * n)
+    q = p if in_place else c.alloc(4 * n)
+    x, y = tensor_from_ptr(p, (n,), torch.float32, "cuda:0"), tensor_from_ptr(q, (n,), torch.float32, "cuda:0")
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    for it in range(6):
+        how = ("stream", "deferred", "host")[it % 3]
+        with torch.cuda.stream(s1):
+            x.fill_(float(it + 1))
+            if how == "stream":
+                ctx.run_on_stream(0, p, q, s1.cuda_stream)
+            elif how == "deferred":
+                ctx.run_deferred(0, p, q)
+                ctx.trigger_on_stream(0, s1.cuda_stream)
+            else:
+                s1.synchronize()
+                ctx.run(0, p, q)
+            ctx.stream_wait(0, s1.cuda_stream)
+            a = y.sum(dtype=torch.float64)
+        with torch.cuda.stream(s2):
+            ctx.stream_wait(0, s2.cuda_stream)
+            b = y.sum(dtype=torch.float64)
+        torch.cuda.synchronize()
+        assert float(a) == float(b) == scale * (it + 1) * n, (it, how)
+    assert ctx.wait_all(10000) == nv.SUCCESS
+    st = ctx.stats()
+    assert st["sqesSubmitted"] == st["cqesDelivered"] == 6
+    ctx.destroy()
+    c.destroy()
