@@ -29,7 +29,7 @@ static_assert(kStageRecv + DFCCL_NOALLOC_MAX_BYTES == DFCCL_NOALLOC_SCRATCH_BYTE
 // the device address obtained there is what kernels receive.
 static __device__ __align__(256) unsigned char g_noallocScratch[DFCCL_NOALLOC_SCRATCH_BYTES];
 
-__global__ void __launch_bounds__(512, 1) dfcclNoAllocKernel(unsigned char* scratch, CollStatic cs, uint64_t send,
+__global__ void __launch_bounds__(DF_BLOCK_THREADS, 1) dfcclNoAllocKernel(unsigned char* scratch, CollStatic cs, uint64_t send,
                                                               uint64_t recv, uint32_t epoch, uint32_t sqeFlags) {
   __shared__ BlockShared sh;
   standaloneBlockMain((RankDev*)(scratch + kRdOff), blockIdx.x, &sh, &cs, send, recv, epoch, sqeFlags);
@@ -108,7 +108,7 @@ ncclResult_t dfcclAllReduceNoAlloc(const void* sendbuff, void* recvbuff, size_t 
   cs.peerFlags[0] = cs.myFlags;
   uint32_t epoch;
   { std::lock_guard<std::mutex> l(g_mu); epoch = ++g_epoch[dev]; }
-  dfcclNoAllocKernel<<<cs.nBlocks, 512, 0, stream>>>(base, cs, (uint64_t)(uintptr_t)sendbuff, (uint64_t)(uintptr_t)recvbuff,
+  dfcclNoAllocKernel<<<cs.nBlocks, DF_BLOCK_THREADS, 0, stream>>>(base, cs, (uint64_t)(uintptr_t)sendbuff, (uint64_t)(uintptr_t)recvbuff,
                                                      epoch, SQE_SEND_STAGED | SQE_RECV_STAGED);
   CUDACHECK(cudaGetLastError());
   return ncclSuccess;

@@ -44,51 +44,17 @@ __global__ void dfcclBumpWordKernel(volatile uint64_t* word, volatile uint64_t* 
   if (mirror) *mirror = v;
 }
 
-// Fallback of the ring fill when stream memory operations are unavailable: one thread writes the entry, then the tail.
-__global__ void dfcclPushSqeKernel(Sqe* slot, Sqe q, volatile uint64_t* tail, uint64_t newTail) {
-  *slot = q;
-  __threadfence_system();
-  *tail = newTail;
-}
-
-// Append one entry to the device-resident submission ring (caller holds ctx->mu).  The host writes the ring: four
-// 64-bit words of the entry and then the tail, as one batch of stream memory operations on a stream that carries
-// nothing else, so the daemon finds its work in device memory.  (The reference's daemon polls a ring in pinned host
-// memory, src/collectives_ofccl/device/enqueue_ofccl_dev.cu:85-173; here a load of host memory by a block costs a
-// PCIe round trip, and such loads from tens of blocks queue behind one another.)
+// Append one entry to the submission ring (caller holds ctx->mu): four tagged words with plain stores into pinned
+// memory, where the daemon's service warp finds them (device/daemon_impl.h: serviceMain); on the host backend into the
+// ring the blocks read.  Measured on one B200 (four ranks on one device, 1 KB all-reduce): written by the host through a
+// batch of five stream memory operations an entry cost 3.5-5 us of host time and was seen about 10 us later.
 static ncclResult_t pushSqe(ofcclRankCtx* ctx, const Sqe& q) {
-  const uint64_t tail = ctx->sqTail;
-  Sqe* slot = ctx->rdHost.devSq + (tail & (ctx->sqCap - 1));
-  volatile uint64_t* tailWord = (volatile uint64_t*)((char*)ctx->rdDev + offsetof(RankDev, devSqTail));
-  if (ctx->backend != dfcclBackendCuda) {
-    *slot = q;
-    __atomic_store_n((uint64_t*)tailWord, tail + 1, __ATOMIC_RELEASE);
-  } else if (ctx->fnBatch) {
-    typedef CUresult (*Fn)(CUstream, unsigned int, CUstreamBatchMemOpParams*, unsigned int);
-    uint64_t w[4];
-    memcpy(w, &q, sizeof(w));
-    CUstreamBatchMemOpParams ops[5];
-    memset(ops, 0, sizeof(ops));
-    for (int i = 0; i < 4; ++i) {
-      ops[i].writeValue.operation = CU_STREAM_MEM_OP_WRITE_VALUE_64;
-      ops[i].writeValue.address = (CUdeviceptr)(uintptr_t)((uint64_t*)slot + i);
-      ops[i].writeValue.value64 = w[i];
-    }
-    ops[4].writeValue.operation = CU_STREAM_MEM_OP_WRITE_VALUE_64;      // every write is preceded by a fence: the entry is there before the tail
-    ops[4].writeValue.address = (CUdeviceptr)(uintptr_t)tailWord;
-    ops[4].writeValue.value64 = tail + 1;
-    CUresult r = ((Fn)ctx->fnBatch)((CUstream)ctx->sqStream, 5, ops, 0);
-    if (r != CUDA_SUCCESS) { DF_WARN("cuStreamBatchMemOp failed (%d)", (int)r); return ncclUnhandledCudaError; }
-  } else {
-    int prev = 0;
-    cudaGetDevice(&prev);
-    if (prev != ctx->device) cudaSetDevice(ctx->device);
-    dfcclPushSqeKernel<<<1, 1, 0, ctx->sqStream>>>(slot, q, tailWord, tail + 1);
-    cudaError_t e = cudaGetLastError();
-    if (prev != ctx->device) cudaSetDevice(prev);
-    if (e != cudaSuccess) { DF_WARN("submission ring fill failed: %s", cudaGetErrorString(e)); return ncclUnhandledCudaError; }
-  }
-  ctx->sqTail = tail + 1;
+  const uint64_t index = ctx->sqTail;
+  const SqSlot s = sqEncode(q, sqTag(index, ctx->sqCap));
+  uint64_t* w = (uint64_t*)((ctx->backend == dfcclBackendCuda ? ctx->hostSq : ctx->rdHost.devSq) + (index & (ctx->sqCap - 1)));
+  for (int i = 3; i >= 0; --i) __atomic_store_n(w + i, s.w[i], __ATOMIC_RELEASE);
+  ctx->sqTail = index + 1;
+  std::atomic_thread_fence(std::memory_order_seq_cst);     // the entry before the look at the `alive` word
   return ncclSuccess;
 }
 
@@ -530,6 +496,7 @@ DF_API ncclResult_t ofcclFinalizeRankCtx7StartHostThrds(ofcclRankCtx_t ctx) {
   for (auto& kv : ctx->colls) ctx->byId[kv.first] = &kv.second;
   ctx->sqCap = pow2ceil(std::max<uint32_t>(64, 2 * (uint32_t)ctx->colls.size() + 2));
   ctx->cqCap = pow2ceil(std::max<uint32_t>(64, 2 * (uint32_t)ctx->colls.size() + 2));
+  if (be == dfcclBackendCuda) DFCHECK(pinnedAlloc(be, (void**)&ctx->hostSq, sizeof(SqSlot) * ctx->sqCap));
   DFCHECK(pinnedAlloc(be, (void**)&ctx->hostFrontier, sizeof(uint64_t) * ctx->nBlocks));
   DFCHECK(pinnedAlloc(be, (void**)&ctx->hostCq, sizeof(uint64_t) * ctx->cqCap));
   DFCHECK(pinnedAlloc(be, (void**)&ctx->ctl, sizeof(DaemonCtl)));
@@ -537,11 +504,12 @@ DF_API ncclResult_t ofcclFinalizeRankCtx7StartHostThrds(ofcclRankCtx_t ctx) {
   RankDev& rd = ctx->rdHost;
   memset(&rd, 0, sizeof(rd));
   rd.hostFrontier = ctx->hostFrontier;
+  rd.hostSq = ctx->hostSq;
   if (be == dfcclBackendCuda) { DFCHECK(devAlloc(be, (void**)&ctx->devAbort, 64)); rd.abortWord = ctx->devAbort; }
   else rd.abortWord = &ctx->ctl->abortFlag;
   rd.hostCq = ctx->hostCq; rd.ctl = ctx->ctl;
   rd.sqCap = ctx->sqCap; rd.cqCap = ctx->cqCap; rd.nBlocks = (uint32_t)ctx->nBlocks; rd.maxColls = maxColls;
-  DFCHECK(devAlloc(be, (void**)&rd.devSq, sizeof(Sqe) * ctx->sqCap));
+  DFCHECK(devAlloc(be, (void**)&rd.devSq, sizeof(SqSlot) * ctx->sqCap));
   DFCHECK(devAlloc(be, (void**)&rd.colls, sizeof(CollStatic) * maxColls));
   DFCHECK(devAlloc(be, (void**)&rd.dyn, sizeof(CollDyn) * (size_t)maxColls * ctx->nBlocks));
   DFCHECK(devAlloc(be, (void**)&rd.doneCount, sizeof(uint32_t) * maxColls));
@@ -571,6 +539,10 @@ DF_API ncclResult_t ofcclFinalizeRankCtx7StartHostThrds(ofcclRankCtx_t ctx) {
   memset(table.data(), 0, sizeof(CollStatic) * maxColls);
   for (auto& kv : ctx->colls) table[kv.first] = kv.second.cs;
   DFCHECK(devUpload(be, rd.colls, table.data(), sizeof(CollStatic) * maxColls));
+  std::vector<uint32_t> meta(maxColls);
+  for (uint32_t i = 0; i < maxColls; ++i) meta[i] = collMeta(table[i]);
+  DFCHECK(devAlloc(be, (void**)&rd.meta, sizeof(uint32_t) * maxColls));
+  DFCHECK(devUpload(be, rd.meta, meta.data(), sizeof(uint32_t) * maxColls));
   DFCHECK(devAlloc(be, (void**)&ctx->rdDev, sizeof(RankDev)));
   DFCHECK(devUpload(be, ctx->rdDev, &rd, sizeof(RankDev)));
   if (be == dfcclBackendCuda) {
@@ -998,7 +970,7 @@ DF_API ncclResult_t dfcclAbort(ofcclRankCtx_t ctx) {
   if (!ctx) return ncclInvalidArgument;
   if (ctx->ctl) ctl_store(&ctx->ctl->abortFlag, 1);
   if (ctx->devAbort && ctx->sqStream) {
-    // the daemon polls a word in device memory; the write goes through the stream that fills the ring (a stream
+    // the daemon polls a word in device memory; the write goes through a stream of its own (a stream
     // memory operation needs no SM, so it lands whatever the kernels are doing)
     std::lock_guard<std::mutex> l(ctx->mu);
     typedef CUresult (*Fn)(CUstream, CUdeviceptr, cuuint32_t, unsigned int);
@@ -1124,9 +1096,10 @@ static void releaseCtx(ofcclRankCtx* ctx) {
   if (ctx->wakeStream) { cudaStreamSynchronize(ctx->wakeStream); cudaStreamDestroy(ctx->wakeStream); }
   for (auto e : ctx->wakeEvents) cudaEventDestroy(e);
   RankDev& rd = ctx->rdHost;
-  devFree(be, rd.devSq); devFree(be, rd.colls); devFree(be, rd.dyn); devFree(be, rd.doneCount); devFree(be, rd.failCount);
+  devFree(be, (void*)rd.devSq); devFree(be, rd.colls); devFree(be, rd.meta); devFree(be, rd.dyn); devFree(be, rd.doneCount); devFree(be, rd.failCount);
   devFree(be, (void*)rd.doneEpoch); devFree(be, (void*)rd.trigger); devFree(be, rd.saved); devFree(be, rd.stats); devFree(be, rd.trace);
   devFree(be, ctx->rdDev);
+  if (ctx->hostSq) pinnedFree(be, (void*)ctx->hostSq);
   pinnedFree(be, (void*)ctx->hostFrontier);
   if (ctx->sqStream) { cudaStreamSynchronize(ctx->sqStream); cudaStreamDestroy(ctx->sqStream); }
   if (ctx->devAbort) devFree(be, ctx->devAbort);
@@ -1149,7 +1122,6 @@ DF_API ncclResult_t ofcclDestroy(ofcclRankCtx_t ctx) {
     q.collId = -1; q.flags = SQE_QUIT;
     (void)pushSqe(ctx, q);
   }
-  if (ctx->sqStream) cudaStreamSynchronize(ctx->sqStream);         // the quit entry is in the ring
   if (ctx->wakeStream) cudaStreamSynchronize(ctx->wakeStream);     // no wake-up callback may outlive the context
   ctx->stopPoller = true;
   ctx->pollCv.notify_all();

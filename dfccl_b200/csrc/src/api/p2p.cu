@@ -9,8 +9,9 @@
 
 namespace dfccl {
 
-__global__ void __launch_bounds__(512, 1) dfcclP2pKernel(RankDev* rd, const P2pList* lists) {
+__global__ void __launch_bounds__(DF_BLOCK_THREADS, 1) dfcclP2pKernel(RankDev* rd, const P2pList* lists) {
   __shared__ P2pShared sh;
+  if (df_is_service()) return;
   p2pBlockMain(rd, &lists[blockIdx.x / DF_P2P_CHANNELS], blockIdx.x % DF_P2P_CHANNELS, &sh);
 }
 
@@ -144,7 +145,7 @@ ncclResult_t launchFor(ncclComm* c, cudaStream_t stream, const std::vector<Pendi
     P2pList* dl = nullptr;
     CUDACHECK(cudaMallocAsync((void**)&dl, sizeof(P2pList) * lists.size(), stream));
     CUDACHECK(cudaMemcpyAsync(dl, lists.data(), sizeof(P2pList) * lists.size(), cudaMemcpyHostToDevice, stream));
-    dfcclP2pKernel<<<(unsigned)(lists.size() * DF_P2P_CHANNELS), 512, 0, stream>>>(c->saRd, dl);
+    dfcclP2pKernel<<<(unsigned)(lists.size() * DF_P2P_CHANNELS), DF_BLOCK_THREADS, 0, stream>>>(c->saRd, dl);
     CUDACHECK(cudaGetLastError());
     CUDACHECK(cudaFreeAsync(dl, stream));
     if (!temps.empty()) CUDACHECK(cudaLaunchHostFunc(stream, freeStaging, new FreeLater{c->heap, temps}));

@@ -91,10 +91,11 @@ struct ofcclRankCtx {
   std::map<int, dfccl::CollEntry> colls;
   int maxCollId = -1;
   // queues (pinned)
-  uint64_t sqTail = 0;                         // entries pushed into the device ring so far (guarded by mu)
+  uint64_t sqTail = 0;                         // entries pushed into the submission ring so far (guarded by mu)
+  volatile dfccl::SqSlot* hostSq = nullptr;    // pinned ring the daemon's service warp reads (cuda backend)
   uint64_t sqMinFrontier = 0;                  // lower bound of what every block has consumed (refreshed when the ring looks full)
   volatile uint64_t* hostFrontier = nullptr;   // pinned, [nBlocks]: written by the blocks
-  cudaStream_t sqStream = nullptr;             // carries nothing but the memory operations that fill the device ring
+  cudaStream_t sqStream = nullptr;             // carries nothing but the abort request
   uint32_t* devAbort = nullptr;                // device word the daemon polls for an abort request
   volatile uint64_t* hostCq = nullptr;
   dfccl::DaemonCtl* ctl = nullptr;

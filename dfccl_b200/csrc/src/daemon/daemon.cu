@@ -7,14 +7,14 @@
 
 namespace dfccl {
 
-__global__ void __launch_bounds__(512, 1) dfcclDaemonKernel(RankDev** ranks, int blocksPerRank) {
+__global__ void __launch_bounds__(DF_BLOCK_THREADS, 1) dfcclDaemonKernel(RankDev** ranks, int blocksPerRank) {
   __shared__ BlockShared sh;
   const int vr = blockIdx.x / blocksPerRank, b = blockIdx.x % blocksPerRank;
   daemonBlockMain(ranks[vr], b, &sh);
 }
 
 ncclResult_t launchDaemonCuda(RankDev** devRankTable, int nRanks, int blocksPerRank, int threads, cudaStream_t stream) {
-  dim3 grid(nRanks * blocksPerRank), block(threads);
+  dim3 grid(nRanks * blocksPerRank), block(df_block_threads(threads));
   if (nRanks > 1) {
     void* args[] = {&devRankTable, &blocksPerRank};
     CUDACHECK(cudaLaunchCooperativeKernel((void*)dfcclDaemonKernel, grid, block, args, 0, stream));
@@ -33,7 +33,7 @@ ncclResult_t warmDaemonKernel() {
 
 ncclResult_t daemonMaxResidentBlocks(int device, int threads, int* blocks) {
   int perSm = 0, sms = 0;
-  CUDACHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, dfcclDaemonKernel, threads, 0));
+  CUDACHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, dfcclDaemonKernel, df_block_threads(threads), 0));
   CUDACHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   *blocks = perSm * sms;
   return ncclSuccess;

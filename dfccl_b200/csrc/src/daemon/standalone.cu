@@ -7,7 +7,7 @@
 
 namespace dfccl {
 
-__global__ void __launch_bounds__(512, 1) dfcclCollKernel(RankDev* rd, CollStatic cs, uint64_t send, uint64_t recv,
+__global__ void __launch_bounds__(DF_BLOCK_THREADS, 1) dfcclCollKernel(RankDev* rd, CollStatic cs, uint64_t send, uint64_t recv,
                                                             uint32_t epoch, uint32_t sqeFlags) {
   __shared__ BlockShared sh;
   standaloneBlockMain(rd, blockIdx.x, &sh, &cs, send, recv, epoch, sqeFlags);
@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(512, 1) dfcclCollKernel(RankDev* rd, CollStati
 
 ncclResult_t launchStandaloneCuda(RankDev* rd, const CollStatic& cs, uint64_t send, uint64_t recv, uint32_t epoch,
                                   uint32_t sqeFlags, int threads, cudaStream_t stream) {
-  dfcclCollKernel<<<cs.nBlocks, threads, 0, stream>>>(rd, cs, send, recv, epoch, sqeFlags);
+  dfcclCollKernel<<<cs.nBlocks, df_block_threads(threads), 0, stream>>>(rd, cs, send, recv, epoch, sqeFlags);
   CUDACHECK(cudaGetLastError());
   return ncclSuccess;
 }

@@ -2,8 +2,8 @@
 //
 // Every block of a rank runs daemonBlockMain independently; nothing in here makes
 // one block of a GPU wait for another block of the same GPU.  Each block
-//   1. finds new submissions in the device-resident ring (the host writes entries
-//      and tail there with stream memory operations: no block reads host memory),
+//   1. finds new submissions in the device-resident ring (one warp per rank copies
+//      them there from the host's ring: no other warp reads host memory),
 //   2. consumes every entry of that ring in order (its own frontier), and
 //      appends the collectives it takes part in (relative block index < nBlocks of the
 //      collective) to its task queue,
@@ -24,57 +24,83 @@
 
 namespace dfccl {
 
+// The service warp of a rank's first block: copies new entries of the pinned ring into the device ring, up to eight at a
+// time (one lane per word), until the block leaves.  Runs beside the block's scheduler and data phases, so that the other
+// blocks of the rank find their work whatever this one is doing.
+DF_HD void serviceMain(BlockShared* sh, RankDev* rd) {
+#if DF_DEVICE_CODE
+  const int lane = df_lane();
+  uint64_t head = rd->svcHead;
+  const uint32_t cap = rd->sqCap;
+  for (;;) {
+    const uint64_t index = head + (lane >> 2);
+    const uint64_t at = (index & (cap - 1)) * 4 + (lane & 3);
+    const uint64_t w = ld_relaxed_sys_u64((const volatile uint64_t*)rd->hostSq + at);
+    const uint32_t bad = ~__ballot_sync(0xffffffffu, (w >> 57) == sqTag(index, cap));
+    const int whole = (bad ? __ffs(bad) - 1 : 32) >> 2;          // entries from `head` on of which every word is there
+    if (whole == 0) {
+      if (sh->svcStop) break;
+      continue;
+    }
+    // (no fence: the words say everything themselves, and what the addresses in them point to was complete before the
+    // host published the entry)
+    if (lane < 4 * whole) st_relaxed_sys_u64((volatile uint64_t*)rd->devSq + at, w);
+    head += whole;
+  }
+  if (lane == 0) rd->svcHead = head;
+#endif
+}
+
 // Consume new entries of the device ring.  Thread 0 only.  Returns the number consumed.
 // A submission that waits for its stream goes to the trigger list, everything else to the task queue.
 DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b) {
-  uint64_t tail = ld_relaxed_sys_u64(&rd->devSqTail);
-  if (tail == sh->frontier) return 0;
-  // The entries were written (by the host, through stream memory operations, each preceded by a fence) before the
-  // tail that announced them.  On this side the entry loads are issued after the branch on the tail's value, which
-  // the hardware does not speculate past; the fence keeps the compiler and the memory pipeline from hoisting them.
-  fence_gpu();
   int got = 0;
-  const uint32_t mask = rd->sqCap - 1;
-  while (sh->frontier < tail) {
-    const Sqe* e = &rd->devSq[sh->frontier & mask];
-    uint4 w0 = ld16(e), w1 = ld16((const char*)e + 16);
-    Sqe q;
-    __builtin_memcpy(&q, &w0, 16);
-    __builtin_memcpy((char*)&q + 16, &w1, 16);
+  SqSlot slot;
+  while (sqPeek(rd, sh->frontier, &slot)) {
+    const Sqe q = sqDecode(slot);
     if (q.flags & SQE_QUIT) { sh->quit = 2; break; }       // the frontier stays on the quit entry
     const int coll = q.collId;
-    const bool mine = coll >= 0 && (uint32_t)coll < rd->maxColls && rd->colls[coll].valid && relBlock(rd, &rd->colls[coll], b) < rd->colls[coll].nBlocks;
-    CollDyn* d = mine ? &rd->dyn[(uint64_t)b * rd->maxColls + coll] : nullptr;
+    bool mine = false;
+    if (coll >= 0 && (uint32_t)coll < rd->maxColls) {
+      const uint32_t m = sh->meta[coll];
+      int r = b - (int)((m >> 8) & 0xffu);
+      if (r < 0) r += (int)rd->nBlocks;
+      mine = (m & DF_META_VALID) && r < (int)(m & 0xffu);
+    }
     if (mine) {
       // A stream-ordered caller may publish the next submission of a collective while this block
       // still runs the previous one.  The entry is never dropped: consumption stops here and
       // resumes once the running submission has completed.
-      const CollDyn* cur = sh->loadedColl == coll ? &sh->dyn : d;
-      if (cur->epoch != 0 && cur->phase != PH_COMPLETE) break;
-      if (sh->loadedColl == coll) {                         // re-armed below in global memory: drop the cached copy
-        saveLoaded(sh, rd, b);
-        sh->loadedColl = -1;
-      }
+      if (sh->busy[coll >> 5] & (1u << (coll & 31))) break;
       if ((q.flags & SQE_TRIGGERED) ? sh->nTrig >= DF_MAX_ACTIVE : sh->nActive >= DF_MAX_ACTIVE) break;   // (cannot happen: one outstanding submission per id)
     }
     ++sh->frontier;
     ++got;
     sh->stats.sqesSeen++;
     if (!mine) continue;
-    d->send = q.send; d->recv = q.recv; d->trigger = q.trigger; d->cursor = 0;
-    d->epoch = q.epoch; d->sqeFlags = q.flags; d->status = ST_OK; d->stallSinceNs = 0; d->patience = 0;
+    sh->busy[coll >> 5] |= 1u << (coll & 31);
+    CollDyn d;
+    d.send = q.send; d.recv = q.recv; d.trigger = q.trigger; d.cursor = 0;
+    d.epoch = q.epoch; d.sqeFlags = q.flags; d.status = ST_OK; d.stallSinceNs = 0; d.patience = 0; d.pad = 0;
+    d.phase = (q.flags & SQE_TRIGGERED) ? PH_TRIGGER : PH_COPY_IN;          // runColl skips ahead to the first phase that has work
+    if (sh->loadedColl == coll && !(q.flags & SQE_TRIGGERED)) { sh->dyn = d; sh->dynDirty = 1; }      // its context is still here
+    else {
+      if (sh->loadedColl == coll) { sh->loadedColl = -1; sh->dynDirty = 0; }                          // re-armed in global memory: drop the cached copy
+      rd->dyn[(uint64_t)b * rd->maxColls + coll] = d;
+    }
     trace(rd, b, TR_SQE, coll);
     if (q.flags & SQE_TRIGGERED) {
-      d->phase = PH_TRIGGER;
       sh->trigColl[sh->nTrig] = (uint16_t)coll; sh->trigVal[sh->nTrig] = q.trigger; ++sh->nTrig;
     } else {
-      d->phase = PH_COPY_IN;          // runColl skips ahead to the first phase that has work
       sh->actWait[sh->nActive] = 0;
       sh->active[sh->nActive++] = (uint16_t)coll;
       trace(rd, b, TR_START, coll);
     }
   }
-  if (got) st_relaxed_sys_u64(&rd->hostFrontier[b], sh->frontier);   // posted store: the host reads it when its ring looks full
+  if (got) {
+    fence_gpu();                                           // the entries, before anything that is read because of them
+    st_relaxed_sys_u64(&rd->hostFrontier[b], sh->frontier);   // posted store: the host reads it when its ring looks full
+  }
   return got;
 }
 
@@ -148,14 +174,25 @@ DF_HD void blockRestore(BlockShared* sh, RankDev* rd, int b) {
     sh->stats = z;
     sv->exited = 0;
   }
+  for (uint32_t i = tid; i < rd->maxColls; i += nt) sh->meta[i] = rd->meta[i];
+  for (uint32_t i = tid; i < DF_MAX_COLLS / 32; i += nt) sh->busy[i] = 0;
   df_sync();
   for (uint32_t i = tid; i < sh->nActive; i += nt) { sh->active[i] = sv->active[i]; sh->actWait[i] = 0; }    // everything gets a visit first
   for (uint32_t i = tid; i < sh->nTrig; i += nt) { sh->trigColl[i] = sv->trigColl[i]; sh->trigVal[i] = sv->trigVal[i]; }
+  df_sync();
+  if (tid == 0) {                                        // what is queued is being worked on
+    for (uint32_t i = 0; i < sh->nActive; ++i) if (sh->active[i] != 0xffff) sh->busy[sh->active[i] >> 5] |= 1u << (sh->active[i] & 31);
+    for (uint32_t i = 0; i < sh->nTrig; ++i) sh->busy[sh->trigColl[i] >> 5] |= 1u << (sh->trigColl[i] & 31);
+  }
   df_sync();
 }
 
 DF_HD void blockPark(BlockShared* sh, RankDev* rd, int b) {
   const int tid = df_tid(), nt = df_nthreads();
+  if (b == 0 && rd->hostSq) {                              // what the service warp copied is in the ring, its position saved
+    if (tid == 0) sh->svcStop = 1;
+    df_sync_service();
+  }
   saveLoaded(sh, rd, b);
   BlockSaved* sv = &rd->saved[b];
   for (uint32_t i = tid; i < sh->nActive; i += nt) sv->active[i] = sh->active[i];
@@ -189,6 +226,14 @@ DF_HD void blockPark(BlockShared* sh, RankDev* rd, int b) {
 
 DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
   const int tid = df_tid();
+  if (df_is_service()) {
+    if (b == 0 && rd->hostSq) { df_sync_service(); serviceMain(sh, rd); df_sync_service(); }
+    return;
+  }
+  if (b == 0 && rd->hostSq) {
+    if (tid == 0) sh->svcStop = 0;
+    df_sync_service();
+  }
   blockRestore(sh, rd, b);
   if (tid == 0) trace(rd, b, TR_LAUNCH, 0);
   uint64_t lastUseful = df_now_ns();     // only thread 0's copies of these are ever consulted
@@ -223,7 +268,7 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
         if (rc == RC_DONE || rc == RC_YIELD || moved) progressed = true;
         if (tid == 0) {
           sh->stats.visits++;
-          if (rc == RC_DONE) sh->active[i] = 0xffff;
+          if (rc == RC_DONE) { sh->active[i] = 0xffff; sh->busy[coll >> 5] &= ~(1u << (coll & 31)); }
           sh->actWait[i] = rc == RC_STALLED ? (sh->dyn.phase == PH_WAIT_ARRIVE ? 1 : sh->dyn.phase == PH_WAIT_DONE ? 2 : 0) : 0;
         }
         // a collective released by its stream should not wait for a walk over a long queue
@@ -289,6 +334,7 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
 // same phases, but a wait that runs out is simply retried until the time limit.
 DF_HD void standaloneBlockMain(RankDev* rd, int b, BlockShared* sh, const CollStatic* cs, uint64_t send, uint64_t recv,
                                uint32_t epoch, uint32_t sqeFlags) {
+  if (df_is_service()) return;
   const int tid = df_tid(), nt = df_nthreads();
   {
     const uint4* s = (const uint4*)cs;

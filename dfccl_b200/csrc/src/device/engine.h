@@ -48,6 +48,7 @@ struct BlockShared {
   uint64_t frontier;
   uint32_t nActive;
   uint32_t quit;                 // 1 = voluntary, 2 = final, 3 = abort
+  volatile uint32_t svcStop;     // the block is leaving: so does its service warp
   uint32_t abortSeen;            // the host's abort flag as last read by thread 0 (the flag lives in host memory: one
                                  // read costs a PCIe round trip, so it is sampled once per scheduler pass, not per wait)
   // peers' buffer offsets of the running submission, fetched by one lane per peer (one memory round trip for all)
@@ -56,6 +57,10 @@ struct BlockShared {
   // without loading any context; a released one joins the task queue
   uint32_t nTrig;
   uint32_t trigFired;
+  // what consuming an entry needs to know of its collective, so that it costs no load of the tables: RankDev::meta, and
+  // whether this block still works on the previous submission
+  uint32_t meta[DF_MAX_COLLS];
+  uint32_t busy[DF_MAX_COLLS / 32];
   uint16_t active[DF_MAX_ACTIVE];
   // per task-queue entry: 0 = needs a visit, 1 = parked in the wait for the peers' arrival, 2 = parked in the wait for
   // their done flags.  Parked entries are not visited (a visit loads the context and polls for a while); their flag
@@ -72,6 +77,15 @@ DF_HD void trace(RankDev* rd, int b, uint16_t ev, int coll) {
   unsigned long long i = atomic_add_u64((unsigned long long*)&rd->traceHead, 1ull);
   TraceEvent* e = &rd->trace[i & (rd->traceCap - 1)];
   e->ns = df_now_ns(); e->block = (uint16_t)b; e->event = ev; e->collId = coll;
+}
+
+// Entry `index` of the device ring, if it is there.
+DF_HD bool sqPeek(const RankDev* rd, uint64_t index, SqSlot* out) {
+  const volatile uint64_t* w = rd->devSq[index & (rd->sqCap - 1)].w;
+  ld_relaxed_sys_2u64(w, &out->w[0], &out->w[1]);
+  ld_relaxed_sys_2u64(w + 2, &out->w[2], &out->w[3]);
+  const uint64_t tag = sqTag(index, rd->sqCap);
+  return (out->w[0] >> 57) == tag && (out->w[1] >> 57) == tag && (out->w[2] >> 57) == tag && (out->w[3] >> 57) == tag;
 }
 
 DF_HD uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
@@ -504,7 +518,8 @@ DF_HD bool dataPhase(BlockShared* sh, RankDev* rd, int b) {
       sh->dyn.cursor = sh->ctl64; sh->dynDirty = 1;
       // anything else for this block?  queued collectives, submissions waiting for their stream, or entries of the
       // device ring this block has not consumed yet
-      sh->ctl0 = (sh->nActive > 1 || sh->nTrig > 0 || ld_relaxed_sys_u64(&rd->devSqTail) != sh->frontier) ? 1 : 0;
+      SqSlot next;
+      sh->ctl0 = (sh->nActive > 1 || sh->nTrig > 0 || sqPeek(rd, sh->frontier, &next)) ? 1 : 0;
     }
   }
   df_sync();

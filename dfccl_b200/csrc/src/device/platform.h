@@ -25,6 +25,16 @@
 
 namespace dfccl {
 
+// One warp of every block of the kernels built on these shims takes no part in the work: the daemon's first block uses it
+// to watch the submission ring whatever the other warps are doing; elsewhere it leaves at once.  df_nthreads and
+// df_sync mean the working threads.  (15 + 1 warps and not 16 + 1: a seventeenth warp makes five on one of the SM's four
+// schedulers, which cuts the register limit from 128 to 96 a thread.)
+#define DF_SERVICE_THREADS 32
+#define DF_BLOCK_THREADS 512
+inline int df_block_threads(int threads) {          // of a block that is asked for `threads`
+  return threads + DF_SERVICE_THREADS < DF_BLOCK_THREADS ? threads + DF_SERVICE_THREADS : DF_BLOCK_THREADS;
+}
+
 DF_HD int df_tid() {
 #if DF_DEVICE_CODE
   return threadIdx.x;
@@ -34,7 +44,7 @@ DF_HD int df_tid() {
 }
 DF_HD int df_nthreads() {
 #if DF_DEVICE_CODE
-  return blockDim.x;
+  return blockDim.x - DF_SERVICE_THREADS;
 #else
   return 1;
 #endif
@@ -55,7 +65,20 @@ DF_HD int df_warpsize() {
 }
 DF_HD void df_sync() {
 #if DF_DEVICE_CODE
-  __syncthreads();
+  asm volatile("bar.sync 1, %0;" ::"r"(df_nthreads()) : "memory");
+#endif
+}
+// the service warp and the working threads meet (once, when the block leaves)
+DF_HD void df_sync_service() {
+#if DF_DEVICE_CODE
+  asm volatile("bar.sync 2, %0;" ::"r"(blockDim.x) : "memory");
+#endif
+}
+DF_HD bool df_is_service() {
+#if DF_DEVICE_CODE
+  return (int)threadIdx.x >= df_nthreads();
+#else
+  return false;
 #endif
 }
 // true on every lane iff pred holds on every lane of the calling warp
@@ -246,6 +269,15 @@ DF_HD void st16(void* p, uint4 v) {
   asm volatile("st.relaxed.sys.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 #else
   __builtin_memcpy(p, &v, 16);
+#endif
+}
+// two words whose tags the reader checks: each is read as a whole
+DF_HD void ld_relaxed_sys_2u64(const volatile uint64_t* p, uint64_t* a, uint64_t* b) {
+#if DF_DEVICE_CODE
+  asm volatile("ld.relaxed.sys.global.v2.u64 {%0,%1}, [%2];" : "=l"(*a), "=l"(*b) : "l"(p) : "memory");
+#else
+  *a = __atomic_load_n((const uint64_t*)p, __ATOMIC_ACQUIRE);
+  *b = __atomic_load_n((const uint64_t*)p + 1, __ATOMIC_ACQUIRE);
 #endif
 }
 }  // namespace dfccl

@@ -8,7 +8,7 @@
 //   CollDyn                 - DynamicCollCtx  include/collectives_ofccl.h:344-355
 //   BlockSaved / BlockShared- BlkStatus       include/collectives_ofccl.h:171-318
 // The differences are deliberate: queues have a device-resident mirror so that
-// only one block at a time polls host memory; a collective owns flag words in
+// only one warp polls host memory; a collective owns flag words in
 // every member's symmetric heap instead of a private communicator with FIFOs;
 // the saved cursor of a parked collective is (phase, cursor) because the data
 // movement between two waits never blocks.
@@ -23,23 +23,44 @@
 
 namespace dfccl {
 
-// ---- submission queue entry (32 bytes, copied as two 16-byte words)
+// ---- submission queue entry: four 64-bit words, each with a 7-bit tag in its top bits that changes with every turn of
+// the ring.  A word is read and written as a whole, so a reader that finds the expected tag in all four words has the
+// entry, in whatever order they arrived: one look at a slot both finds and fetches an entry, and no tail word, fence or
+// second round trip stands between the two.
 enum SqeFlags : uint32_t {
   SQE_QUIT = 1u,          // final quit: every block saves nothing and leaves for good
   SQE_TRIGGERED = 2u,     // do not start before trigger[collId] >= trigger value (stream-ordered submit)
   SQE_SEND_STAGED = 4u,   // sendbuff is outside the symmetric heap: copy it into the staging area first
   SQE_RECV_STAGED = 8u,   // recvbuff is outside the heap: peers write staging, copy out at the end
 };
-struct alignas(16) Sqe {
+struct Sqe {
   int32_t collId;
   uint32_t flags;
-  uint64_t send;          // heap offset, or raw local address when SQE_SEND_STAGED
-  uint64_t recv;          // heap offset, or raw local address when SQE_RECV_STAGED
+  uint64_t send;          // heap offset, or raw local address when SQE_SEND_STAGED (57 bits)
+  uint64_t recv;          // heap offset, or raw local address when SQE_RECV_STAGED (57 bits)
   uint32_t trigger;       // value the low half of trigger[collId] must reach (SQE_TRIGGERED)
   uint32_t epoch;         // number of this submission of the collective, counted by the host from 1: not every submission
                           // of an id has to pass through the daemon
 };
-static_assert(sizeof(Sqe) == 32, "an entry is written as four 64-bit words");
+struct alignas(32) SqSlot { uint64_t w[4]; };
+#define DF_SQ_PAYLOAD ((1ull << 57) - 1)
+// Tag of ring position `index`: 1..127, so that a slot never written to (all zero) matches nothing; the slot's previous
+// contents are exactly one turn old.
+static __host__ __device__ inline uint64_t sqTag(uint64_t index, uint32_t cap) { return (index / cap) % 127u + 1u; }
+static __host__ __device__ inline SqSlot sqEncode(const Sqe& q, uint64_t tag) {
+  SqSlot s;
+  s.w[0] = tag << 57 | (uint64_t)(q.flags & 0x1ffu) << 48 | (uint64_t)(q.collId & 0xffff) << 32 | q.epoch;
+  s.w[1] = tag << 57 | (q.send & DF_SQ_PAYLOAD);
+  s.w[2] = tag << 57 | (q.recv & DF_SQ_PAYLOAD);
+  s.w[3] = tag << 57 | q.trigger;
+  return s;
+}
+static __host__ __device__ inline Sqe sqDecode(const SqSlot& s) {
+  Sqe q;
+  q.epoch = (uint32_t)s.w[0]; q.collId = (int16_t)(uint16_t)(s.w[0] >> 32); q.flags = (uint32_t)(s.w[0] >> 48) & 0x1ffu;
+  q.send = s.w[1] & DF_SQ_PAYLOAD; q.recv = s.w[2] & DF_SQ_PAYLOAD; q.trigger = (uint32_t)s.w[3];
+  return q;
+}
 
 // ---- completion entry: one 64-bit word, gen makes a slot self-validating
 //   [63:32] generation of the ring slot (index / capacity + 1)   [31:24] status   [23:0] collId
@@ -102,6 +123,9 @@ struct alignas(16) CollStatic {
   char* peerPush[DF_MAX_RANKS];
   uint64_t pushSlotBytes;
 };
+
+#define DF_META_VALID (1u << 16)
+inline uint32_t collMeta(const CollStatic& c) { return c.valid ? DF_META_VALID | (uint32_t)c.nBlocks | (uint32_t)c.blockBase << 8 : 0u; }
 
 // ---- mutable per (block, collective) state; what a context switch saves and loads
 struct alignas(16) CollDyn {
@@ -167,12 +191,13 @@ struct BlockSaved {                // survives a voluntary quit (reference: Dyna
 
 // ---- everything the daemon needs for one rank; lives in device memory (host memory for the host backend)
 struct RankDev {
-  // submission path: the ring and its tail live in device memory and are written by the HOST (stream memory
-  // operations on a stream of its own: entry words first, then the tail), so that no block ever reads host
-  // memory to find work - a load of pinned host memory costs a PCIe round trip and such loads from many blocks
-  // queue behind one another
-  Sqe* devSq;
-  uint64_t devSqTail;
+  // Submission path: the host writes entries into a ring in pinned memory with plain stores; ONE warp per rank (the
+  // service warp of block 0) polls it and copies new entries into the ring in device memory that the blocks poll.
+  // (A load of pinned host memory is a PCIe round trip, and such loads from many blocks queue behind one another; a
+  // write by the host through stream memory operations costs it a driver call and the device a fence per word.)
+  const volatile SqSlot* hostSq;   // null: the host writes devSq itself (host backend)
+  volatile SqSlot* devSq;
+  uint64_t svcHead;                // entries the service warp has copied
   uint32_t sqCap;                  // power of two
   uint32_t pad0;
   volatile uint64_t* hostFrontier; // pinned, [nBlocks]: entries consumed by each block (posted stores; flow control for the host)
@@ -185,6 +210,8 @@ struct RankDev {
   uint32_t nBlocks;
   // tables
   CollStatic* colls;               // [maxColls]
+  uint32_t* meta;                  // [maxColls] what a block needs to know to take or skip an entry: nBlocks | blockBase << 8 |
+                                   // DF_META_VALID; never written after finalize
   CollDyn* dyn;                    // [nBlocks][maxColls]
   uint32_t* doneCount;             // [maxColls] blocks that finished the current submission
   uint32_t* failCount;             // [maxColls] of those, how many ended with an error
