@@ -39,13 +39,20 @@ struct FusedArgs {
 // stored with the contraction index slow (A as [K, M], B as [K, N], row-major) and read by the tensor cores as it is.
 ncclResult_t gemmLaunch(const void* A, const void* B, void* C, int M, int N, int K, const FusedArgs* f, cudaStream_t stream,
                         int aMn = 0, int bMn = 0);
-// The CTA-pair kernel (cta_group::2, tiles of 256 x 256) for plain GEMMs whose sizes allow it.
-bool gemmPairEligible(int M, int N, int K);
+// Plain GEMMs: what runs them.  tn = 0: the persistent CTA-pair kernel (cta_group::2, tiles of 256 x 256); otherwise one tile of
+// 128 or (pair) 256 rows x tn columns, or one of `split` slices of its contraction, per CTA or CTA pair.
+struct GemmTilePlan { bool pair; int tn, split; };
+GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs);
+ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream,
+                            int aMn, int bMn, uint32_t* errDev, uint32_t* errHost);
 int gemmPairResident();
 ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
                             uint32_t* errDev, uint32_t* errHost);
 // Cached tensor map of a row-major bf16 matrix [rows, cols] cut into boxes of boxRows x 64 columns, 128-byte swizzle.
 ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows);
+// The same for whole operands of a stage in one load: a K-major matrix [rows, k] as (64, rows, k / 64) with boxes of
+// 64 x boxRows x boxK / 64, an MN-major one ([k, rows] as stored) as (64, k, rows / 64) with boxes of 64 x boxK x boxRows / 64.
+ncclResult_t gemmMakeMap3(CUtensorMap* m, const void* base, uint64_t rows, uint64_t k, int mnMajor, uint32_t boxRows, uint32_t boxK);
 // True when a kernel of the current device gave up on a bounded wait (pinned word, no device access).
 bool gemmGaveUp();
 // SMs the fused launches leave to a co-resident persistent kernel: raised to at least `n`.

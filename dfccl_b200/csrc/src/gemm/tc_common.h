@@ -80,6 +80,12 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 
+// ---- programmatic dependent launch: a kernel launched with the attribute may start while the kernel in front of it in the
+// stream still runs.  It touches global memory only after the wait, which ends when that kernel has completed and its
+// writes are visible; the second call lets the next launch start in the same way.  (No early start without the attribute.)
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- tensor memory
 __device__ __forceinline__ void tmem_alloc(uint32_t* smemResult, uint32_t ncols) {      // one full warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smemResult)), "r"(ncols) : "memory");
@@ -182,8 +188,7 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmemD, uint64_t descA, u
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in both CTAs of the pair when the MMAs issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  const uint16_t mask = 3;
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask = 3) {     // mask: the pair's two CTAs of the cluster
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask) : "memory");
 }
 

@@ -1,6 +1,7 @@
 // bf16 GEMM on the 5th-generation tensor cores, hand-written for sm_100a:
 //     C[M,N] = A[M,K] * B[N,K]^T        (both operands K-major: y = x W^T of a linear layer)
-// and its two communication-fused forms for tensor parallelism over NVLink peer memory:
+// in two communication-fused forms for tensor parallelism over NVLink peer memory (plain products run on the kernels of
+// tcgen05_gemm_pair.cu and tcgen05_gemm_tile.cu):
 //   * all-gather -> GEMM : A is row-sharded over the ranks.  Extra warps of the SAME kernel pull
 //     the peers' row blocks into the local A buffer (plain peer loads) and publish one flag per
 //     128-row block; the TMA producer waits for the flag of the block it is about to load, so the
@@ -45,7 +46,6 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * EPI_WARP_BYTES + 1024 /*al
 struct GemmArgs {
   __nv_bfloat16* C;
   int M, N, K, ldc;
-  int groupM;                       // plain GEMM: row tiles per rasterisation group (0 = row-major tile order, the fused forms)
   int aMn, bMn;                     // operand stored with the contraction index slow: A as [K, M], B as [K, N] (row-major)
   uint32_t* err;                    // device word: non-zero = a bounded wait ran out (later launches return at once)
   uint64_t waitNs;                  // limit of every wait on a word another GPU or CTA writes
@@ -129,7 +129,6 @@ __device__ __forceinline__ int orderedMTile(const FusedArgs& f, int i, int mTile
 }
 
 __device__ __forceinline__ void tileCoord(const GemmArgs& g, int t, int mTiles, int nTiles, int& mt, int& nt) {
-  if (g.groupM > 0) { raster_tile(t, mTiles, nTiles, g.groupM, mt, nt); return; }
   mt = orderedMTile(g.f, t / nTiles, mTiles);
   nt = t % nTiles;
 }
@@ -428,39 +427,51 @@ EncodeTiled encodeFn() {
   return fn;
 }
 
-// rows x cols bf16, row-major (cols contiguous), tiles of boxRows x 64 columns, 128-byte swizzle
-ncclResult_t makeMapUncached(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows);
-
 // Encoding a tensor map costs microseconds of host time per call; layers call with the same few
 // (pointer, shape) pairs every step, so the encoded maps are kept.
-ncclResult_t makeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows) {
-  struct Key { const void* p; uint64_t r, c; uint32_t b; bool operator<(const Key& o) const { return std::tie(p, r, c, b) < std::tie(o.p, o.r, o.c, o.b); } };
-  static std::map<Key, CUtensorMap> cache;
+struct MapKey {
+  const void* base;
+  uint64_t d1, d2, s1;               // extents above the innermost one and the byte stride of the second dimension
+  uint32_t d0, b1, b2;               // innermost extent; box above the innermost 64 columns (b2 = 0: a 2-D map)
+  bool operator<(const MapKey& o) const {
+    return std::tie(base, d0, d1, d2, s1, b1, b2) < std::tie(o.base, o.d0, o.d1, o.d2, o.s1, o.b1, o.b2);
+  }
+};
+
+ncclResult_t encodeMap(CUtensorMap* m, const MapKey& k) {
+  EncodeTiled fn = encodeFn();
+  if (!fn) { DF_WARN("cuTensorMapEncodeTiled is not available"); return ncclSystemError; }
+  cuuint64_t dims[3] = {k.d0, k.d1, k.d2};
+  cuuint64_t strides[2] = {k.s1, 128};
+  cuuint32_t box[3] = {BK, k.b1, k.b2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k.b2 ? 3 : 2, (void*)k.base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    DF_WARN("cuTensorMapEncodeTiled failed (%d) for %llu x %llu at %p", (int)r, (unsigned long long)k.d1, (unsigned long long)(k.d2 ? k.d2 * 64 : k.d0), k.base);
+    return ncclInvalidArgument;
+  }
+  return ncclSuccess;
+}
+
+ncclResult_t cachedMap(CUtensorMap* m, const MapKey& k) {
+  static std::map<MapKey, CUtensorMap> cache;
   static std::mutex mu;
-  Key k{base, rows, cols, boxRows};
   {
     std::lock_guard<std::mutex> l(mu);
     auto it = cache.find(k);
     if (it != cache.end()) { *m = it->second; return ncclSuccess; }
   }
-  DFCHECK(makeMapUncached(m, base, rows, cols, boxRows));
+  DFCHECK(encodeMap(m, k));
   std::lock_guard<std::mutex> l(mu);
   if (cache.size() > 4096) cache.clear();
   cache[k] = *m;
   return ncclSuccess;
 }
 
-ncclResult_t makeMapUncached(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows) {
-  EncodeTiled fn = encodeFn();
-  if (!fn) { DF_WARN("cuTensorMapEncodeTiled is not available"); return ncclSystemError; }
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {BK, boxRows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { DF_WARN("cuTensorMapEncodeTiled failed (%d) for %llu x %llu at %p", (int)r, (unsigned long long)rows, (unsigned long long)cols, base); return ncclInvalidArgument; }
-  return ncclSuccess;
+// rows x cols bf16, row-major (cols contiguous), tiles of boxRows x 64 columns, 128-byte swizzle
+ncclResult_t makeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows) {
+  return cachedMap(m, MapKey{base, rows, 0, cols * 2, (uint32_t)cols, boxRows, 0});
 }
 
 std::atomic<int> g_reservedSms{0};
@@ -492,9 +503,14 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
   if (((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) return ncclInvalidArgument;
   const ErrWords ew = errWords();
   if (*ew.host) { DF_WARN("an earlier tensor-core kernel on this device gave up on a bounded wait; call dfcclGemmCheck to clear"); return dfcclTimeout; }
-  // plain products whose sizes allow it run on CTA pairs (tiles of 256 x 256, half the shared-memory traffic per FLOP)
-  if ((!f || f->mode == 0 || f->nranks <= 1) && gemmPairEligible(M, N, K) && paramI64("GEMM_PAIR", 1) != 0)
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!f || f->mode == 0 || f->nranks <= 1) {
+    const GemmTilePlan p = gemmTilePlan(M, N, K, sms, paramI64("GEMM_PAIR", 1) != 0);
+    if (p.tn) return gemmTileLaunch(p, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host);
     return gemmPairLaunch(A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host);
+  }
   CUtensorMap ma, mb;
   // K-major operand [rows, K]: boxes of [tile rows] x 64 K-columns; MN-major operand [K, cols]: boxes of 64 K-rows x 64 columns
   if (!aMn) DFCHECK(makeMap(&ma, A, (uint64_t)M, (uint64_t)K, BM)); else DFCHECK(makeMap(&ma, A, (uint64_t)K, (uint64_t)M, BK));
@@ -506,18 +522,12 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
   g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.ldc = N; g.err = ew.dev; g.errHost = (uint32_t*)ew.host;
   g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0;
   { int64_t ms = paramI64("WAIT_TIMEOUT_MS", 30000); g.waitNs = (uint64_t)(ms > 0 ? ms : 30000) * 1000000ull; }
-  if (f) g.f = *f; else { g.f.nranks = 1; g.f.mode = 0; }
-  if (g.f.mode == 0 || g.f.nranks <= 1) { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : 2 * gm); }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = (M / BM) * (N / BN);
+  g.f = *f;
   // The CTAs of a fused launch serve one another (gathered pieces, partial tiles), so all of them must be resident
   // at once: SMs that a co-running persistent kernel (the daemon) may occupy are left out of the grid.
   const int usable = std::max(1, sms - g_reservedSms.load());
-  // fused modes keep one CTA per usable SM even with few tiles: the communication warps of idle CTAs still work
-  const int grid = (g.f.mode == 0) ? (tiles < sms ? tiles : sms) : usable;
-  dfcclGemmKernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ma, mb, g);
+  // one CTA per usable SM even with few tiles: the communication warps of idle CTAs still work
+  dfcclGemmKernel<<<usable, NUM_THREADS, SMEM_BYTES, stream>>>(ma, mb, g);
   CUDACHECK(cudaGetLastError());
   return ncclSuccess;
 }
@@ -525,6 +535,9 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
 }  // namespace
 
 ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows) { return makeMap(m, base, rows, cols, boxRows); }
+ncclResult_t gemmMakeMap3(CUtensorMap* m, const void* base, uint64_t rows, uint64_t k, int mnMajor, uint32_t boxRows, uint32_t boxK) {
+  return cachedMap(m, mnMajor ? MapKey{base, k, rows / 64, rows * 2, 64, boxK, boxRows / 64} : MapKey{base, rows, k / 64, k * 2, 64, boxRows, boxK / 64});
+}
 ncclResult_t gemmLaunch(const void* A, const void* B, void* C, int M, int N, int K, const FusedArgs* f, cudaStream_t stream, int aMn, int bMn) {
   return launch(A, B, C, M, N, K, f, stream, aMn, bMn);
 }

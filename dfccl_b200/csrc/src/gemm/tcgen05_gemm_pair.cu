@@ -1,5 +1,6 @@
 // bf16 GEMM on CTA pairs (tcgen05 cta_group::2), hand-written for sm_100a:
-//     C[M,N] = A[M,K] * B[N,K]^T,  tiles of 256 x 256, one tile per pair of CTAs (a cluster of two SMs).
+//     C[M,N] = A[M,K] * B[N,K]^T,  tiles of 256 x 256, one tile per pair of CTAs (a cluster of two SMs).  Rows of the last
+//     row tile beyond M (M is a multiple of 128) are loaded as zeros and not stored.
 // Each CTA of a pair loads 128 rows of A and 128 rows of B per 64-wide K block (32 KB per stage instead of the 48 KB
 // of the one-CTA form, so six stages fit), the leader's single MMA thread issues 256 x 256 x 16 instructions that read
 // both CTAs' shared memory, and each CTA ends up with its 128 rows of the accumulator in its own tensor memory.
@@ -7,7 +8,7 @@
 // operand traffic per FLOP, which is what bounds the one-CTA kernel.
 //
 // Roles per CTA: warp 0 = TMA producer (one elected thread; completion of both CTAs' loads is counted on the
-// LEADER's barrier), warp 1 = tensor-memory owner, and in the leader the MMA issuer; warps 2-5 = epilogue over the
+// LEADER's barrier), warp 1 = tensor-memory owner, and in the leader the MMA issuer; warps 2-9 = epilogue over the
 // CTA's own accumulator half.  Stages are released and accumulators handed over with tcgen05.commit to both CTAs;
 // the epilogues of both CTAs arrive on the leader's accumulator-empty barrier.  No TMA load uses cluster multicast.
 // Every wait is bounded and ends in the error word of the device.
@@ -30,10 +31,11 @@ constexpr int PM = 256, PN = 256, BK = 64, HALF = 128, STAGES = 6, UMMA_K = 16;
 constexpr int A_BYTES = HALF * BK * 2, B_BYTES = HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;   // per CTA
 constexpr int MN_BLOCK_BYTES = 64 * BK * 2;
 constexpr int TMEM_COLS = 512;                       // two accumulators of 256 fp32 columns (128 lanes each, per CTA)
-constexpr int NUM_THREADS = 192;                     // 6 warps
-constexpr int EPI_ROW_BYTES = 64 * 2 + 16;
+constexpr int NUM_THREADS = 320;                     // 10 warps
+constexpr int EPI_WARPS = 8;                         // two per 32 accumulator rows: the last tile's epilogue is not overlapped with anything
+constexpr int EPI_ROW_BYTES = 32 * 2 + 16;           // 32 columns of a row at a time (64 would not leave room for six stages)
 constexpr int EPI_WARP_BYTES = 32 * EPI_ROW_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * EPI_WARP_BYTES + 1024 + 256;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * EPI_WARP_BYTES + 1024 + 256;
 constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on another GPU: seconds mean a lost partner
 
 struct PairArgs {
@@ -50,22 +52,22 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
   uint8_t* epiSmem = smem + STAGES * STAGE_BYTES;
-  uint64_t* fullBar = (uint64_t*)(epiSmem + 4 * EPI_WARP_BYTES);     // used in the leader only
+  uint64_t* fullBar = (uint64_t*)(epiSmem + EPI_WARPS * EPI_WARP_BYTES);     // used in the leader only
   uint64_t* emptyBar = fullBar + STAGES;                             // in both CTAs (commit to both)
   uint64_t* accFull = emptyBar + STAGES;                             // [2] in both CTAs
-  uint64_t* accEmpty = accFull + 2;                                  // [2] used in the leader only: 8 epilogue warps arrive
+  uint64_t* accEmpty = accFull + 2;                                  // [2] used in the leader only: the epilogue warps of both CTAs arrive
   uint32_t* tmemBaseSlot = (uint32_t*)(accEmpty + 2);
   volatile uint32_t* giveUp = tmemBaseSlot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cr = cluster_ctarank();             // 0 = leader
-  const int mTiles = g.M / PM, nTiles = g.N / PN, kBlocks = g.K / BK;
+  const int mTiles = (g.M + PM - 1) / PM, nTiles = g.N / PN, kBlocks = g.K / BK;
   const int numTiles = mTiles * nTiles;
   const int pair = blockIdx.x >> 1, numPairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&fullBar[s], 1); mbar_init(&emptyBar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&accFull[a], 1); mbar_init(&accEmpty[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&accFull[a], 1); mbar_init(&accEmpty[a], 2 * EPI_WARPS); }
     *giveUp = *(volatile uint32_t*)g.err;            // an earlier kernel gave up: do nothing (both CTAs read the same word)
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
@@ -78,6 +80,8 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   tc_fence_after();
   const uint32_t tmemBase = *tmemBaseSlot;
   const bool dead = *giveUp != 0;
+  grid_dependency_wait();                            // everything above may run beside the kernel in front of this one
+  grid_launch_dependents();
 
   if (dead) {
   } else if (warp == 0) {
@@ -135,7 +139,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     }
   } else {
     // ------------------------------------------------------------ epilogue: my 128 rows, TMEM -> bf16 -> global
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, colHalf = (warp - 2) >> 2;
     const uint32_t accEmptyLeader0 = mapa_u32(smem_u32(&accEmpty[0]), 0), accEmptyLeader1 = mapa_u32(smem_u32(&accEmpty[1]), 0);
     int it = 0;
     for (int t = pair; t < numTiles; t += numPairs, ++it) {
@@ -146,36 +150,34 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       tc_fence_after();
       uint8_t* stg = epiSmem + (warp - 2) * EPI_WARP_BYTES;
       __nv_bfloat16* cbase = g.C + (size_t)(mt * PM + (int)cr * HALF + quarter * 32) * g.ldc + nt * PN;   // row 0 of this warp's 32 rows
+      const bool mine = mt * PM + (int)cr * HALF < g.M;               // the last row tile may have only its upper half
 #pragma unroll 1
-      for (int c4 = 0; c4 < PN / 64; ++c4) {
+      for (int c = colHalf * (PN / 2); mine && c < (colHalf + 1) * (PN / 2); c += 32) {
+        uint32_t r[32];
+        tmem_ld32(tmemBase + ((uint32_t)(quarter * 32) << 16) + ab * PN + c, r);
+        tmem_ld_wait();
+        uint4* srow = (uint4*)(stg + lane * EPI_ROW_BYTES);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t r[32];
-          tmem_ld32(tmemBase + ((uint32_t)(quarter * 32) << 16) + ab * PN + c4 * 64 + h * 32, r);
-          tmem_ld_wait();
-          uint4* srow = (uint4*)(stg + lane * EPI_ROW_BYTES + h * 64);
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint4 o;
-            o.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
-            o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
-            o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
-            o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
-            srow[v] = o;
-          }
+        for (int v = 0; v < 4; ++v) {
+          uint4 o;
+          o.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
+          o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
+          o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
+          o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
+          srow[v] = o;
         }
         __syncwarp();
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {                 // 32 rows x 8 chunks of 16 bytes; 8 lanes cover one 128-byte row segment
-          const int chunk = q * 32 + lane, rr = chunk >> 3, cc = chunk & 7;
+        for (int q = 0; q < 4; ++q) {                 // 32 rows x 4 chunks of 16 bytes; 4 lanes cover one 64-byte row segment
+          const int chunk = q * 32 + lane, rr = chunk >> 2, cc = chunk & 3;
           const uint4 o = *(const uint4*)(stg + rr * EPI_ROW_BYTES + cc * 16);
-          *(uint4*)(cbase + (size_t)rr * g.ldc + c4 * 64 + cc * 8) = o;
+          *(uint4*)(cbase + (size_t)rr * g.ldc + c + cc * 8) = o;
         }
         __syncwarp();
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(ab ? accEmptyLeader1 : accEmptyLeader0);   // 8 epilogue warps of the pair release the accumulator
+      if (lane == 0) mbar_arrive_cluster(ab ? accEmptyLeader1 : accEmptyLeader0);   // the pair's epilogue warps release the accumulator
     }
   }
 
@@ -189,8 +191,6 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 }
 
 }  // namespace
-
-bool gemmPairEligible(int M, int N, int K) { return M > 0 && N > 0 && K > 0 && M % PM == 0 && N % PN == 0 && K % BK == 0; }
 
 namespace {
 int maxResidentPairs(int dev, int sms) {
@@ -232,10 +232,15 @@ ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N,
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = (M / PM) * (N / PN);
+  const int tiles = (M + PM - 1) / PM * (N / PN);
   const int pairs = std::min(tiles, maxResidentPairs(dev, sms));
-  dfcclGemmPairKernel<<<2 * pairs, NUM_THREADS, SMEM_BYTES, stream>>>(ma, mb, g);
-  CUDACHECK(cudaGetLastError());
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at; cfg.numAttrs = 1;
+  CUDACHECK(cudaLaunchKernelEx(&cfg, dfcclGemmPairKernel, ma, mb, g));
   return ncclSuccess;
 }
 

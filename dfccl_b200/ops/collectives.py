@@ -16,13 +16,13 @@ from typing import Optional
 import torch
 
 from .. import native as nv
-from ..utils.tensors import nccl_dtype
+from ..utils.tensors import nccl_dtype, raw_stream
 
 _OPS = {"sum": nv.SUM, "prod": nv.PROD, "max": nv.MAX, "min": nv.MIN, "avg": nv.AVG}
 
 
 def _stream(t: torch.Tensor):
-    return torch.cuda.current_stream(t.device).cuda_stream if t.device.type == "cuda" else None
+    return raw_stream(t.device) if t.device.type == "cuda" else None
 
 
 def _check(t: torch.Tensor, name: str) -> torch.Tensor:

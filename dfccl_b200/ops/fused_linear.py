@@ -24,7 +24,7 @@ import torch
 import torch.distributed as dist
 
 from .. import native as nv
-from ..utils.tensors import tensor_from_ptr
+from ..utils.tensors import raw_stream, tensor_from_ptr
 from .gemm import BM, BN, BK
 
 
@@ -136,7 +136,7 @@ class AllGatherGemm:
             out = torch.empty(self.m, self.n_out, dtype=torch.bfloat16, device=tp.device)
         if self.coll_id is not None:
             x_shard, w = x_shard.contiguous(), w.contiguous()
-            st = torch.cuda.current_stream(tp.device).cuda_stream if tp.device.type == "cuda" else 0
+            st = raw_stream(tp.device) if tp.device.type == "cuda" else 0
             tp.ctx.run_fused(self.coll_id, x_shard.data_ptr(), w.data_ptr(), out.data_ptr(), st, w_transposed)
             return out
         if w_transposed:
@@ -159,7 +159,7 @@ class AllGatherGemm:
         a.epoch = self.rv.epoch
         w = w.contiguous()
         nv.check(nv.lib().dfcclGemmFused(self.gathered.data_ptr(), w.data_ptr(), out.data_ptr(), self.m, self.n_out, self.k,
-                                         C.byref(a), C.sizeof(a), torch.cuda.current_stream(tp.device).cuda_stream), "dfcclGemmFused(ag)")
+                                         C.byref(a), C.sizeof(a), raw_stream(tp.device)), "dfcclGemmFused(ag)")
         return out
 
 
@@ -196,12 +196,12 @@ class GemmReduceScatter:
         if out is None:
             out = torch.empty(self.rows, self.n_out, dtype=torch.bfloat16, device=tp.device)
         if self.coll_id is not None:
-            st = torch.cuda.current_stream(tp.device).cuda_stream if tp.device.type == "cuda" else 0
+            st = raw_stream(tp.device) if tp.device.type == "cuda" else 0
             tp.ctx.run_fused(self.coll_id, x.data_ptr(), w.data_ptr(), out.data_ptr(), st, w_transposed)
             return out
         if tp.n == 1:
             nv.check(nv.lib().dfcclGemmBf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), self.m, self.n_out, self.k,
-                                            torch.cuda.current_stream(tp.device).cuda_stream), "dfcclGemmBf16")
+                                            raw_stream(tp.device)), "dfcclGemmBf16")
             return out
         self.rv.epoch += 1
         a = self._args
@@ -218,5 +218,5 @@ class GemmReduceScatter:
             a.epochCounter = self.rv.epoch_counter.data_ptr()
         a.epoch, a.reduced = self.rv.epoch, out.data_ptr()
         nv.check(nv.lib().dfcclGemmFused(x.data_ptr(), w.data_ptr(), self._dummy.data_ptr(), self.m, self.n_out, self.k,
-                                         C.byref(a), C.sizeof(a), torch.cuda.current_stream(tp.device).cuda_stream), "dfcclGemmFused(rs)")
+                                         C.byref(a), C.sizeof(a), raw_stream(tp.device)), "dfcclGemmFused(rs)")
         return out

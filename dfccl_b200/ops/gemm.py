@@ -1,4 +1,4 @@
-"""Python face of the hand-written tcgen05 GEMM (``csrc/src/gemm/tcgen05_gemm.cu``)."""
+"""Python face of the hand-written tcgen05 GEMMs (``csrc/src/gemm``)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -6,6 +6,7 @@ import ctypes as C
 import torch
 
 from .. import native as nv
+from ..utils.tensors import raw_stream
 
 BM, BN, BK = 128, 256, 64
 
@@ -28,7 +29,7 @@ def matmul_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None)
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     nv.check(nv.lib().dfcclGemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k,
-                                    torch.cuda.current_stream(a.device).cuda_stream), "dfcclGemmBf16")
+                                    raw_stream(a.device)), "dfcclGemmBf16")
     return out
 
 
@@ -48,7 +49,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *,
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     nv.check(nv.lib().dfcclGemmBf16Ex(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_transposed), int(b_transposed),
-                                      torch.cuda.current_stream(a.device).cuda_stream), "dfcclGemmBf16Ex")
+                                      raw_stream(a.device)), "dfcclGemmBf16Ex")
     return out
 
 

@@ -30,7 +30,7 @@ import torch
 import torch.nn as nn
 
 from .. import native as nv
-from ..utils.tensors import HeapTensorPool, nccl_dtype
+from ..utils.tensors import HeapTensorPool, nccl_dtype, raw_stream
 from .groups import Dist
 
 
@@ -243,7 +243,7 @@ class DaemonDDP:
 
     # ------------------------------------------------------------------ per step
     def _stream(self) -> int:
-        return torch.cuda.current_stream(self.device).cuda_stream if self.device.type == "cuda" else 0
+        return raw_stream(self.device) if self.device.type == "cuda" else 0
 
     def _bucket_ready(self, b: Bucket) -> None:
         self._ready.append(b)

@@ -21,11 +21,11 @@ import torch.nn as nn
 
 from .. import native as nv
 from ..ops.fused_linear import AllGatherGemm, GemmReduceScatter, TpGroup
-from ..utils.tensors import nccl_dtype
+from ..utils.tensors import nccl_dtype, raw_stream
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream if t.device.type == "cuda" else 0
+    return raw_stream(t.device) if t.device.type == "cuda" else 0
 
 
 _OPS: Dict[Tuple, object] = {}

@@ -22,6 +22,13 @@ def nccl_dtype(dt: torch.dtype) -> int:
         raise TypeError(f"{dt} has no collective datatype") from None
 
 
+def raw_stream(device: torch.device) -> int:
+    """Handle of the device's current stream: what ``torch.cuda.current_stream(device).cuda_stream`` gives, without making
+    a Stream object for every launch (2.2 us of host time)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
 class _CudaBlob:
     """Minimal ``__cuda_array_interface__`` provider for a raw device range."""
 

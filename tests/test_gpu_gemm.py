@@ -111,3 +111,63 @@ def test_gemm_throughput_report():
     print(f"tcgen05 gemm 8192^3: CTA pairs {ours:.3f} ms = {flops / ours / 1e9:.0f} TFLOP/s; one CTA per tile {one:.3f} ms = "
           f"{flops / one / 1e9:.0f} TFLOP/s; cuBLAS {cublas:.3f} ms = {flops / cublas / 1e9:.0f} TFLOP/s")
     assert gemm.check_kernels()
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (128, 512, 64), (128, 256, 192),                        # half a stage; a stage and a half
+    (128, 256, 8256), (384, 256, 4160),                     # four slices of a contraction, of unequal length
+    (256, 2048, 8192), (1024, 1024, 1024),                  # two slices; one narrow tile per SM
+    (640, 2048, 4096), (896, 2304, 3072),                   # pairs of 256 x 128, the last row tile half empty
+    (1280, 768, 1920), (1408, 2048, 1024),                  # pairs of 256 x 256, half empty
+    (1920, 1280, 768), (2048, 1024, 448),
+    (9600, 512, 1024), (9600, 1024, 192)])                  # persistent pairs, half empty
+def test_every_tile_form_at_its_edges(m, n, k):
+    """All storage orders give the same bits, and the error against 64 bits is that of one rounding to bf16: 2**-9 of a
+    value at most (uniform between 0 and that: 2**-9 / sqrt(3) in the mean) plus fp32 sums."""
+    from dfccl_b200.ops import gemm
+    torch.manual_seed(m + 3 * n + 5 * k)
+    a = torch.randn(m, k, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(n, k, device="cuda", dtype=torch.bfloat16)
+    out = torch.full((m + 128, n), 7.0, device="cuda", dtype=torch.bfloat16)       # rows behind the result stay as they are
+    gemm.matmul_nt(a, b, out[:m])
+    at, bt = a.t().contiguous(), b.t().contiguous()
+    torch.cuda.synchronize()
+    assert gemm.check_kernels()
+    ref = a.double() @ b.double().t()
+    assert ((out[:m].double() - ref).norm() / ref.norm()).item() < 2 ** -9
+    assert bool((out[m:] == 7.0).all())
+    for a_t, b_t in ((True, False), (False, True), (True, True)):
+        assert torch.equal(out[:m], gemm.matmul(at if a_t else a, bt if b_t else b, a_transposed=a_t, b_transposed=b_t))
+
+
+def test_chained_products_wait_for_one_another():
+    """Launches overlap the set-up of the next product with the end of the one before: a chain in which every product
+    reads the previous result (and overwrites what the one before it read) gives what separate launches give, in a
+    stream and in a captured graph."""
+    from dfccl_b200.ops import gemm
+    torch.manual_seed(5)
+    n = 512
+    w = [(torch.randn(n, n, device="cuda") * n ** -0.5).to(torch.bfloat16) for _ in range(3)]
+    x = torch.randn(256, n, device="cuda", dtype=torch.bfloat16)
+    big = (torch.randn(256, 8192, device="cuda") * 0.02).to(torch.bfloat16)         # a longer kernel in front: 4 slices
+    wb = (torch.randn(n, 8192, device="cuda") * 0.02).to(torch.bfloat16)
+    h = [torch.empty(256, n, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+
+    def chain(sync):
+        gemm.matmul_nt(big, wb, h[0])
+        h[0].add_(x)
+        for i in range(12):
+            gemm.matmul_nt(h[i % 2], w[i % 3], h[(i + 1) % 2])
+            if sync:
+                torch.cuda.synchronize()
+        return h[0].clone()
+
+    want = chain(True)
+    for _ in range(5):
+        assert torch.equal(chain(False), want)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        got = chain(False)
+    g.replay()
+    torch.cuda.synchronize()
+    assert gemm.check_kernels() and torch.equal(got, want)
