@@ -1158,6 +1158,9 @@ DF_API ncclResult_t ofcclDestroy(ofcclRankCtx_t ctx) {
 
 // ------------------------------------------------------------------ registered fused operators
 
+extern "C" ncclResult_t dfcclGemmBf16Epilogue(const void* A, const void* B, void* C, int M, int N, int K, int aTransposed, int bTransposed, int kind,
+                                              const void* bias, const void* aux, void* pre, cudaStream_t stream);
+
 static CollEntry* fusedEntry(ofcclRankCtx* ctx, int collId) {
   if (!ctx || !ctx->finalized || ctx->destroyed || collId < 0 || collId >= (int)ctx->byId.size()) return nullptr;
   CollEntry* e = ctx->byId[collId];
@@ -1195,6 +1198,25 @@ DF_API ncclResult_t dfcclRunFusedGemm(int collId, const void* x, const void* w, 
 // over W as it is stored (the tensor cores read it as an MN-major operand, no transposed copy).
 DF_API ncclResult_t dfcclRunFusedGemmT(int collId, const void* x, const void* wT, void* out, cudaStream_t stream, ofcclRankCtx_t ctx) {
   return runFused(collId, x, wT, out, 1, stream, ctx);
+}
+
+// One-rank communicators: the operator is its GEMM, with an epilogue (gemm/epilogue.h) and without a gathered copy of x.
+DF_API ncclResult_t dfcclRunFusedGemmLocal(int collId, const void* x, const void* w, void* out, int wT, int kind, const void* bias, const void* aux,
+                                           void* pre, cudaStream_t stream, ofcclRankCtx_t ctx) {
+  CollEntry* e = fusedEntry(ctx, collId);
+  if (!e) { DF_WARN("id %d is not a registered fused operator of a finalized context", collId); return ncclInvalidArgument; }
+  if (!x || !w || !out) return ncclInvalidArgument;
+  if (e->comm->nranks != 1 || ctx->backend != dfcclBackendCuda) { DF_WARN("id %d: only one-rank operators on a GPU take an epilogue", collId); return ncclInvalidUsage; }
+  if (ctl_load(&ctx->ctl->abortFlag)) return dfcclAborted;
+  if (gemmGaveUp()) { ctx->asyncError = dfcclTimeout; DF_WARN("an earlier fused operator on this device gave up on a bounded wait"); return dfcclTimeout; }
+  NvtxRange range(e->fused.kind == dfcclFusedAllGatherGemm ? "dfccl:AllGatherGemm" : "dfccl:GemmReduceScatter");
+  ctx->fusedLaunches++;
+  int prev = 0;
+  cudaGetDevice(&prev);
+  if (prev != e->comm->device) cudaSetDevice(e->comm->device);
+  const ncclResult_t res = dfcclGemmBf16Epilogue(x, w, out, e->fused.rowsPerRank, e->fused.n, e->fused.k, 0, wT, kind, bias, aux, pre, stream);
+  if (prev != e->comm->device) cudaSetDevice(prev);
+  return res;
 }
 
 static void hostTranspose(const uint16_t* src, uint16_t* dst, int rows, int cols) {        // dst[cols, rows] = src[rows, cols]^T

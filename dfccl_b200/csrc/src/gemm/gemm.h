@@ -46,8 +46,11 @@ GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs);
 ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream,
                             int aMn, int bMn, uint32_t* errDev, uint32_t* errHost);
 int gemmPairResident();
+struct GemmEpilogue;
 ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
-                            uint32_t* errDev, uint32_t* errHost);
+                            uint32_t* errDev, uint32_t* errHost, const GemmEpilogue* e);
+// The same pass over a finished bf16 product C [M, N], in place (csrc/src/ops/block.cu).
+ncclResult_t applyEpilogue(const GemmEpilogue& e, void* C, int M, int N, cudaStream_t stream);
 // Cached tensor map of a row-major bf16 matrix [rows, cols] cut into boxes of boxRows x 64 columns, 128-byte swizzle.
 ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows);
 // The same for whole operands of a stage in one load: a K-major matrix [rows, k] as (64, rows, k / 64) with boxes of

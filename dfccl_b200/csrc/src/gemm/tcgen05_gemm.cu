@@ -18,6 +18,7 @@
 // stages and to hand accumulators over.  Every wait is bounded and ends in an error word.
 #include "tc_common.h"
 #include "gemm.h"
+#include "epilogue.h"
 #include "../common/param.h"
 #include "dfccl.h"
 #include "../common/log.h"
@@ -495,7 +496,7 @@ ErrWords errWords() {                       // one pair per device, created on f
 }
 
 ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, const FusedArgs* f, cudaStream_t stream,
-                    int aMn = 0, int bMn = 0) {
+                    int aMn = 0, int bMn = 0, const GemmEpilogue* e = nullptr) {
   if (M <= 0 || N <= 0 || K <= 0 || M % BM || N % BN || K % BK) {
     DF_WARN("tcgen05 GEMM needs M %% %d == 0, N %% %d == 0, K %% %d == 0 (got %d x %d x %d)", BM, BN, BK, M, N, K);
     return ncclInvalidArgument;
@@ -508,8 +509,9 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!f || f->mode == 0 || f->nranks <= 1) {
     const GemmTilePlan p = gemmTilePlan(M, N, K, sms, paramI64("GEMM_PAIR", 1) != 0);
-    if (p.tn) return gemmTileLaunch(p, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host);
-    return gemmPairLaunch(A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host);
+    if (p.tn == 0) return gemmPairLaunch(A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host, e);
+    DFCHECK(gemmTileLaunch(p, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host));
+    return e && e->kind ? applyEpilogue(*e, C, M, N, stream) : ncclSuccess;
   }
   CUtensorMap ma, mb;
   // K-major operand [rows, K]: boxes of [tile rows] x 64 K-columns; MN-major operand [K, cols]: boxes of 64 K-rows x 64 columns
@@ -562,6 +564,27 @@ DF_API ncclResult_t dfcclGemmBf16(const void* A, const void* B, void* C, int M, 
 // (B) then need no transposed copy: the tensor cores read MN-major operands as they are.
 DF_API ncclResult_t dfcclGemmBf16Ex(const void* A, const void* B, void* C, int M, int N, int K, int aTransposed, int bTransposed, cudaStream_t stream) {
   return launch(A, B, C, M, N, K, nullptr, stream, aTransposed, bTransposed);
+}
+
+// The same followed by an epilogue (epilogue.h): bias, residual, GELU or its gradient; arrays 16-byte aligned.
+static bool epilogueOk(const GemmEpilogue& e) {
+  if (e.kind < EPI_NONE || e.kind > EPI_GELU_GRAD) return false;
+  if ((e.kind == EPI_BIAS || e.kind == EPI_BIAS_RES || e.kind == EPI_BIAS_GELU) && !e.bias) return false;
+  if ((e.kind == EPI_BIAS_RES || e.kind == EPI_GELU_GRAD) && !e.aux) return false;
+  return (((uintptr_t)e.bias | (uintptr_t)e.aux | (uintptr_t)e.pre) & 15) == 0;
+}
+DF_API ncclResult_t dfcclGemmBf16Epilogue(const void* A, const void* B, void* C, int M, int N, int K, int aTransposed, int bTransposed, int kind,
+                                          const void* bias, const void* aux, void* pre, cudaStream_t stream) {
+  const GemmEpilogue e{kind, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux, (__nv_bfloat16*)pre};
+  if (!epilogueOk(e)) return ncclInvalidArgument;
+  return launch(A, B, C, M, N, K, nullptr, stream, aTransposed, bTransposed, &e);
+}
+
+// An epilogue over a finished product C [M, N], in place.
+DF_API ncclResult_t dfcclApplyEpilogue(void* C, int M, int N, int kind, const void* bias, const void* aux, void* pre, cudaStream_t stream) {
+  const GemmEpilogue e{kind, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux, (__nv_bfloat16*)pre};
+  if (!epilogueOk(e) || M <= 0 || N <= 0 || N % 8 || !C || ((uintptr_t)C & 15)) return ncclInvalidArgument;
+  return applyEpilogue(e, C, M, N, stream);
 }
 
 // CTA pairs of the cta_group::2 kernel that can be resident together on the current device.

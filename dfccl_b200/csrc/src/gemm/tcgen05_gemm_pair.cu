@@ -17,6 +17,7 @@
 // workloads' plain GEMMs (weight and data gradients, unfused forwards).
 #include "tc_common.h"
 #include "gemm.h"
+#include "epilogue.h"
 #include "../common/param.h"
 #include "../common/log.h"
 #include <algorithm>
@@ -45,8 +46,10 @@ struct PairArgs {
   int groupM;                       // row tiles per rasterisation group
   uint32_t* err;
   uint32_t* errHost;
+  GemmEpilogue e;
 };
 
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const PairArgs g) {
   extern __shared__ uint8_t smemRaw[];
@@ -149,31 +152,90 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       if (!mbar_wait(&accFull[ab], (it >> 1) & 1, giveUp, WAIT_NS)) break;
       tc_fence_after();
       uint8_t* stg = epiSmem + (warp - 2) * EPI_WARP_BYTES;
-      __nv_bfloat16* cbase = g.C + (size_t)(mt * PM + (int)cr * HALF + quarter * 32) * g.ldc + nt * PN;   // row 0 of this warp's 32 rows
       const bool mine = mt * PM + (int)cr * HALF < g.M;               // the last row tile may have only its upper half
+      const size_t tileOff = (size_t)(mt * PM + (int)cr * HALF + quarter * 32) * g.ldc + nt * PN;   // row 0 of this warp's 32 rows
+      const int beg = colHalf * (PN / 2), end = beg + PN / 2;
+      // 32 columns at a time.  Global memory is touched in chunks of 16 bytes, 4 lanes to a 64-byte row segment; a lane's own
+      // row passes through this warp's staging rows.  `aux` is fetched one step ahead.
+      const int rr0 = lane >> 2, cc = lane & 3;
+      uint4 ax[4];
+      auto fetch = [&](int c) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ax[q] = *(const uint4*)(g.e.aux + tileOff + (size_t)(q * 8 + rr0) * g.ldc + c + cc * 8);
+      };
+      auto flush = [&](__nv_bfloat16* to, int c) {
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *(uint4*)(to + tileOff + (size_t)(q * 8 + rr0) * g.ldc + c + cc * 8) = *(const uint4*)(stg + (q * 8 + rr0) * EPI_ROW_BYTES + cc * 16);
+        __syncwarp();
+      };
+      constexpr bool AUX = EPI == EPI_BIAS_RES || EPI == EPI_GELU_GRAD;
+      if (AUX && mine) fetch(beg);
 #pragma unroll 1
-      for (int c = colHalf * (PN / 2); mine && c < (colHalf + 1) * (PN / 2); c += 32) {
+      for (int c = beg; mine && c < end; c += 32) {
         uint32_t r[32];
         tmem_ld32(tmemBase + ((uint32_t)(quarter * 32) << 16) + ab * PN + c, r);
-        tmem_ld_wait();
         uint4* srow = (uint4*)(stg + lane * EPI_ROW_BYTES);
+        uint4 own[4];
+        if (AUX) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) *(uint4*)(stg + (q * 8 + rr0) * EPI_ROW_BYTES + cc * 16) = ax[q];
+          __syncwarp();
+#pragma unroll
+          for (int v = 0; v < 4; ++v) own[v] = srow[v];
+          if (c + 32 < end) fetch(c + 32);
+        }
+        tmem_ld_wait();
+        if (EPI == EPI_BIAS || EPI == EPI_BIAS_RES || EPI == EPI_BIAS_GELU) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const uint4 bv = ((const uint4*)(g.e.bias + nt * PN + c))[v];
+            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              r[8 * v + 2 * w] = __float_as_uint(__uint_as_float(r[8 * v + 2 * w]) + bf16Lo(bw[w]));
+              r[8 * v + 2 * w + 1] = __float_as_uint(__uint_as_float(r[8 * v + 2 * w + 1]) + bf16Hi(bw[w]));
+            }
+          }
+        }
+        if (AUX) {
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const uint32_t xw[4] = {own[v].x, own[v].y, own[v].z, own[v].w};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              float lo = __uint_as_float(r[8 * v + 2 * w]), hi = __uint_as_float(r[8 * v + 2 * w + 1]);
+              if (EPI == EPI_BIAS_RES) { lo += bf16Lo(xw[w]); hi += bf16Hi(xw[w]); }
+              else { lo *= geluTanhGrad(bf16Lo(xw[w])); hi *= geluTanhGrad(bf16Hi(xw[w])); }
+              r[8 * v + 2 * w] = __float_as_uint(lo); r[8 * v + 2 * w + 1] = __float_as_uint(hi);
+            }
+          }
+        }
+        uint4 o[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          uint4 o;
-          o.x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
-          o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
-          o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
-          o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
-          srow[v] = o;
+          o[v].x = pack_bf16x2(__uint_as_float(r[8 * v + 0]), __uint_as_float(r[8 * v + 1]));
+          o[v].y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
+          o[v].z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
+          o[v].w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
         }
-        __syncwarp();
+        if (EPI == EPI_BIAS_GELU) {
+          if (g.e.pre) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {                 // 32 rows x 4 chunks of 16 bytes; 4 lanes cover one 64-byte row segment
-          const int chunk = q * 32 + lane, rr = chunk >> 2, cc = chunk & 3;
-          const uint4 o = *(const uint4*)(stg + rr * EPI_ROW_BYTES + cc * 16);
-          *(uint4*)(cbase + (size_t)rr * g.ldc + c + cc * 8) = o;
+            for (int v = 0; v < 4; ++v) srow[v] = o[v];
+            flush(g.e.pre, c);
+          }
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {                // of the rounded value: what the backward pass differentiates at
+            uint32_t* ow = (uint32_t*)&o[v];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) ow[w] = pack_bf16x2(geluTanh(bf16Lo(ow[w])), geluTanh(bf16Hi(ow[w])));
+          }
         }
-        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) srow[v] = o[v];
+        flush(g.C, c);
       }
       tc_fence_before();
       __syncwarp();
@@ -193,6 +255,12 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 }  // namespace
 
 namespace {
+typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const PairArgs);
+PairKernel pairKernel(int epi) {
+  static const PairKernel k[] = {dfcclGemmPairKernel<EPI_NONE>, dfcclGemmPairKernel<EPI_BIAS>, dfcclGemmPairKernel<EPI_BIAS_RES>,
+                                 dfcclGemmPairKernel<EPI_BIAS_GELU>, dfcclGemmPairKernel<EPI_GELU_GRAD>};
+  return k[epi];
+}
 int maxResidentPairs(int dev, int sms) {
   // pairs that can be resident together (a GPC with an odd number of free SMs leaves one unpaired)
   static int maxPairs[64];
@@ -200,12 +268,12 @@ int maxResidentPairs(int dev, int sms) {
   std::lock_guard<std::mutex> l(mu);
   if (!maxPairs[dev & 63]) {
     static std::once_flag once;
-    std::call_once(once, [] { cudaFuncSetAttribute(dfcclGemmPairKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+    std::call_once(once, [] { for (int e = EPI_NONE; e <= EPI_GELU_GRAD; ++e) cudaFuncSetAttribute(pairKernel(e), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(sms & ~1); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = SMEM_BYTES;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, dfcclGemmPairKernel, &cfg) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = sms / 2; }
+    if (cudaOccupancyMaxActiveClusters(&n, pairKernel(EPI_NONE), &cfg) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = sms / 2; }
     maxPairs[dev & 63] = std::min(n, sms / 2);
   }
   return maxPairs[dev & 63];
@@ -220,7 +288,7 @@ int gemmPairResident() {
 }
 
 ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
-                            uint32_t* errDev, uint32_t* errHost) {
+                            uint32_t* errDev, uint32_t* errHost, const GemmEpilogue* e) {
   CUtensorMap ma, mb;
   if (!aMn) DFCHECK(gemmMakeMap(&ma, A, (uint64_t)M, (uint64_t)K, HALF)); else DFCHECK(gemmMakeMap(&ma, A, (uint64_t)K, (uint64_t)M, BK));
   if (!bMn) DFCHECK(gemmMakeMap(&mb, B, (uint64_t)N, (uint64_t)K, HALF)); else DFCHECK(gemmMakeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
@@ -228,6 +296,7 @@ ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N,
   memset(&g, 0, sizeof(g));
   g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.ldc = N; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0;
   g.err = errDev; g.errHost = errHost;
+  if (e) g.e = *e;
   { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -240,7 +309,7 @@ ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N,
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
-  CUDACHECK(cudaLaunchKernelEx(&cfg, dfcclGemmPairKernel, ma, mb, g));
+  CUDACHECK(cudaLaunchKernelEx(&cfg, pairKernel(g.e.kind), ma, mb, g));
   return ncclSuccess;
 }
 

@@ -1,0 +1,306 @@
+// Elementwise and row / column work of a transformer block around its GEMMs, bf16 in and out, fp32 inside: layer norm
+// forward and backward, column sums (bias gradients), and the GEMM epilogues as passes of their own.
+// All of it streams activations once, so HBM (or L2) bounds it: 16 bytes per load, every row in registers between its two
+// passes, and enough warps to keep 148 SMs loading.  The figures stand at the kernels.
+// The reference has no counterpart (it is a collective library); the GPT-2 workload uses these.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <algorithm>
+#include "dfccl.h"
+#include "../gemm/epilogue.h"
+#include "../gemm/gemm.h"
+
+namespace dfccl {
+namespace {
+
+constexpr int MAX_D = 2048;            // widest row a warp keeps in registers (8 packs of 8 elements per lane)
+
+__device__ __forceinline__ float warpSum(float v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ void unpack8(const uint4& p, float (&f)[8]) {
+  const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { f[2 * i] = bf16Lo(w[i]); f[2 * i + 1] = bf16Hi(w[i]); }
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+}
+
+// One warp per row; NV packs of 8 elements per lane (d <= 256 NV, a multiple of 8).
+template <int NV>
+__global__ void __launch_bounds__(128) lnForwardKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
+                                                       const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
+                                                       float* __restrict__ mean, float* __restrict__ rstd, int rows, int d, float eps) {
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const uint4* src = (const uint4*)(x + (size_t)row * d);
+  uint4 p[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) { const int i = v * 32 + lane; p[v] = i * 8 < d ? src[i] : make_uint4(0u, 0u, 0u, 0u); }
+  float s = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    float f[8];
+    unpack8(p[v], f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s += f[e];
+  }
+  const float m = warpSum(s) / d;
+  float q = 0.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    if ((v * 32 + lane) * 8 >= d) continue;
+    float f[8];
+    unpack8(p[v], f);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q += (f[e] - m) * (f[e] - m);
+  }
+  const float r = rsqrtf(warpSum(q) / d + eps);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int i = v * 32 + lane;
+    if (i * 8 >= d) continue;
+    float f[8], g[8], b[8], o[8];
+    unpack8(p[v], f); unpack8(__ldg((const uint4*)gamma + i), g); unpack8(__ldg((const uint4*)beta + i), b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = (f[e] - m) * r * g[e] + b[e];
+    ((uint4*)(y + (size_t)row * d))[i] = pack8(o);
+  }
+  if (lane == 0) { mean[row] = m; rstd[row] = r; }
+}
+
+// gx = rstd (gy gamma - mean(gy gamma) - xhat mean(gy gamma xhat)) [+ pass]; every warp keeps its rows' sums of gy xhat and gy
+// in registers, a block adds its warps' and writes one line of `work`, [blocks][2][d].
+template <int NV>
+__global__ void __launch_bounds__(256, 1) lnBackwardKernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ x,
+                                                           const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean,
+                                                           const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ pass,
+                                                           __nv_bfloat16* __restrict__ gx, float* __restrict__ work, int rows, int d) {
+  extern __shared__ float sums[];                        // [2][d]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float dg[NV][8], db[NV][8];
+#pragma unroll
+  for (int v = 0; v < NV; ++v)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { dg[v][e] = 0.f; db[v][e] = 0.f; }
+  for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
+    const size_t off = (size_t)row * d;
+    uint4 pg[NV], px[NV], pp[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int i = v * 32 + lane;
+      const bool in = i * 8 < d;
+      pg[v] = in ? ((const uint4*)(gy + off))[i] : make_uint4(0u, 0u, 0u, 0u);
+      px[v] = in ? ((const uint4*)(x + off))[i] : make_uint4(0u, 0u, 0u, 0u);
+      pp[v] = in && pass ? ((const uint4*)(pass + off))[i] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const float m = mean[row], r = rstd[row];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int i = v * 32 + lane;
+      if (i * 8 >= d) continue;
+      float g[8], f[8], w[8];
+      unpack8(pg[v], g); unpack8(px[v], f); unpack8(__ldg((const uint4*)gamma + i), w);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float xh = (f[e] - m) * r, gw = g[e] * w[e];
+        s1 += gw; s2 += gw * xh;
+        dg[v][e] += g[e] * xh; db[v][e] += g[e];
+      }
+    }
+    s1 = warpSum(s1) / d; s2 = warpSum(s2) / d;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const int i = v * 32 + lane;
+      if (i * 8 >= d) continue;
+      float g[8], f[8], w[8], p[8], o[8];
+      unpack8(pg[v], g); unpack8(px[v], f); unpack8(__ldg((const uint4*)gamma + i), w); unpack8(pp[v], p);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) o[e] = r * (g[e] * w[e] - s1 - (f[e] - m) * r * s2) + p[e];
+      ((uint4*)(gx + off))[i] = pack8(o);
+    }
+  }
+  for (int w = 0; w < 8; ++w) {                          // the warps in turn: always the same order
+    if (warp == w) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const int i = (v * 32 + lane) * 8;
+        if (i >= d) continue;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          sums[i + e] = w ? sums[i + e] + dg[v][e] : dg[v][e];
+          sums[d + i + e] = w ? sums[d + i + e] + db[v][e] : db[v][e];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  float* line = work + (size_t)blockIdx.x * 2 * d;
+  for (int i = threadIdx.x; i < 2 * d; i += 256) line[i] = sums[i];
+}
+
+// out[c] = sum over lines of work[line][c], 32 columns per block, 8 lines at a time; columns from `split` on go to out2.
+__global__ void __launch_bounds__(256) sumLinesKernel(const float* __restrict__ work, int lines, int n, __nv_bfloat16* __restrict__ out,
+                                                      __nv_bfloat16* __restrict__ out2, int split) {
+  __shared__ float part[8][33];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (c < n) {
+#pragma unroll 4
+    for (int l = g; l < lines; l += 8) s += work[(size_t)l * n + c];
+  }
+  part[g][lane] = s;
+  __syncthreads();
+  if (g == 0 && c < n) {
+    for (int k = 1; k < 8; ++k) s += part[k][lane];
+    if (c < split) out[c] = __float2bfloat16_rn(s); else out2[c - split] = __float2bfloat16_rn(s);
+  }
+}
+
+// Column sums: a block takes 256 columns (8 per lane) and one of gridDim.y stretches of rows, its 8 warps interleaved.
+__global__ void __launch_bounds__(256) columnSumKernel(const __nv_bfloat16* __restrict__ g, float* __restrict__ work, int rows, int n) {
+  __shared__ float part[8][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 256 + lane * 8;
+  const int per = (rows + gridDim.y - 1) / gridDim.y, beg = blockIdx.y * per, end = min(rows, beg + per);
+  float a[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) a[e] = 0.f;
+  if (c < n) {
+#pragma unroll 4
+    for (int r = beg + warp; r < end; r += 8) {
+      float f[8];
+      unpack8(*(const uint4*)(g + (size_t)r * n + c), f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) a[e] += f[e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) part[warp][lane * 8 + e] = a[e];
+  __syncthreads();
+  const int col = blockIdx.x * 256 + threadIdx.x;
+  if (col < n) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += part[w][threadIdx.x];
+    work[(size_t)blockIdx.y * n + col] = s;
+  }
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(256) epilogueKernel(GemmEpilogue e, __nv_bfloat16* __restrict__ C, size_t packs, int packsPerRow) {
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < packs; i += (size_t)gridDim.x * 256) {
+    float v[8], b[8], x[8];
+    unpack8(((const uint4*)C)[i], v);
+    if (EPI == EPI_BIAS || EPI == EPI_BIAS_RES || EPI == EPI_BIAS_GELU) {
+      unpack8(__ldg((const uint4*)e.bias + i % packsPerRow), b);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += b[k];
+    }
+    if (EPI == EPI_BIAS_RES || EPI == EPI_GELU_GRAD) {
+      unpack8(((const uint4*)e.aux)[i], x);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = EPI == EPI_BIAS_RES ? v[k] + x[k] : v[k] * geluTanhGrad(x[k]);
+    }
+    if (EPI == EPI_BIAS_GELU) {
+      const uint4 p = pack8(v);
+      if (e.pre) ((uint4*)e.pre)[i] = p;
+      unpack8(p, v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = geluTanh(v[k]);
+    }
+    ((uint4*)C)[i] = pack8(v);
+  }
+}
+
+int smCount() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+ncclResult_t launched() { return cudaGetLastError() == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError; }
+bool aligned(const void* a, const void* b = nullptr, const void* c = nullptr, const void* d = nullptr, const void* e = nullptr) {
+  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 15) == 0;
+}
+int lnBlocks(int rows, int sms) { return std::max(1, std::min((rows + 7) / 8, sms)); }
+// stretches of rows of a column sum: about four blocks per SM, at least 32 rows (four per warp) each
+int sumStretches(int rows, int n, int sms) { return std::max(1, std::min(4 * sms / ((n + 255) / 256), rows / 32)); }
+
+template <int NV>
+void lnBackward(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* pass, void* gx, float* work,
+                int rows, int d, int blocks, cudaStream_t stream) {
+  lnBackwardKernel<NV><<<blocks, 256, 2 * d * sizeof(float), stream>>>((const __nv_bfloat16*)gy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma,
+                                                                       mean, rstd, (const __nv_bfloat16*)pass, (__nv_bfloat16*)gx, work, rows, d);
+}
+
+}  // namespace
+
+ncclResult_t applyEpilogue(const GemmEpilogue& e, void* C, int M, int N, cudaStream_t stream) {
+  const size_t packs = (size_t)M * N / 8;
+  const unsigned grid = (unsigned)std::min<size_t>((packs + 255) / 256, (size_t)smCount() * 8);
+  switch (e.kind) {
+    case EPI_BIAS: epilogueKernel<EPI_BIAS><<<grid, 256, 0, stream>>>(e, (__nv_bfloat16*)C, packs, N / 8); break;
+    case EPI_BIAS_RES: epilogueKernel<EPI_BIAS_RES><<<grid, 256, 0, stream>>>(e, (__nv_bfloat16*)C, packs, N / 8); break;
+    case EPI_BIAS_GELU: epilogueKernel<EPI_BIAS_GELU><<<grid, 256, 0, stream>>>(e, (__nv_bfloat16*)C, packs, N / 8); break;
+    case EPI_GELU_GRAD: epilogueKernel<EPI_GELU_GRAD><<<grid, 256, 0, stream>>>(e, (__nv_bfloat16*)C, packs, N / 8); break;
+    default: return ncclSuccess;
+  }
+  return launched();
+}
+
+}  // namespace dfccl
+
+using namespace dfccl;
+#define DF_API extern "C" __attribute__((visibility("default")))
+
+// Widest row of the layer norm kernels (a multiple of 8 elements).
+DF_API int dfcclLayerNormMaxWidth(void) { return MAX_D; }
+
+// y = (x - mean) rstd gamma + beta per row of d elements; mean and rstd [rows] fp32 for the backward pass.
+DF_API ncclResult_t dfcclLayerNormForward(const void* x, const void* gamma, const void* beta, void* y, void* mean, void* rstd, int rows, int d, float eps, cudaStream_t stream) {
+  if (rows <= 0 || d <= 0 || d % 8 || d > MAX_D || !x || !gamma || !beta || !y || !mean || !rstd || !aligned(x, gamma, beta, y)) return ncclInvalidArgument;
+  const int grid = (rows + 3) / 4;
+  auto go = [&](auto kernel) {
+    kernel<<<grid, 128, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, (float*)mean, (float*)rstd, rows, d, eps);
+  };
+  if (d <= 256) go(lnForwardKernel<1>);
+  else if (d <= 512) go(lnForwardKernel<2>);
+  else if (d <= 1024) go(lnForwardKernel<4>);
+  else go(lnForwardKernel<8>);
+  return launched();
+}
+
+// fp32 words of scratch memory a backward pass / a column sum needs on the current device.
+DF_API size_t dfcclLayerNormWork(int rows, int d) { return (size_t)lnBlocks(rows, smCount()) * 2 * d; }
+DF_API size_t dfcclColumnSumWork(int rows, int n) { return (size_t)sumStretches(rows, n, smCount()) * n; }
+
+// Gradients of x (plus `pass`, the gradient that reaches x by another way, where given), gamma and beta.
+DF_API ncclResult_t dfcclLayerNormBackward(const void* gy, const void* x, const void* gamma, const void* mean, const void* rstd, const void* pass,
+                                           void* gx, void* ggamma, void* gbeta, void* work, int rows, int d, cudaStream_t stream) {
+  if (rows <= 0 || d <= 0 || d % 8 || d > MAX_D || !gy || !x || !gamma || !mean || !rstd || !gx || !ggamma || !gbeta || !work) return ncclInvalidArgument;
+  if (!aligned(gy, x, gamma, pass, gx)) return ncclInvalidArgument;
+  const int blocks = lnBlocks(rows, smCount());
+  auto* fn = d <= 256 ? lnBackward<1> : d <= 512 ? lnBackward<2> : d <= 1024 ? lnBackward<4> : lnBackward<8>;
+  fn(gy, x, gamma, (const float*)mean, (const float*)rstd, pass, gx, (float*)work, rows, d, blocks, stream);
+  sumLinesKernel<<<(2 * d + 31) / 32, 256, 0, stream>>>((const float*)work, blocks, 2 * d, (__nv_bfloat16*)ggamma, (__nv_bfloat16*)gbeta, d);
+  return launched();
+}
+
+// out[n] = sum over rows of g [rows, n], added up in fp32.
+DF_API ncclResult_t dfcclColumnSum(const void* g, void* out, void* work, int rows, int n, cudaStream_t stream) {
+  if (rows <= 0 || n <= 0 || n % 8 || !g || !out || !work || !aligned(g)) return ncclInvalidArgument;
+  const int stretches = sumStretches(rows, n, smCount());
+  columnSumKernel<<<dim3((n + 255) / 256, stretches), 256, 0, stream>>>((const __nv_bfloat16*)g, (float*)work, rows, n);
+  sumLinesKernel<<<(n + 31) / 32, 256, 0, stream>>>((const float*)work, stretches, n, (__nv_bfloat16*)out, (__nv_bfloat16*)out, n);
+  return launched();
+}

@@ -23,8 +23,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops.block import norm_residual, unhooked
 from ..ops.fused_linear import TpGroup
-from ..parallel.tp import ColumnParallelLinear, RowParallelLinear
+from ..parallel.tp import ColumnParallelLinear, RowParallelLinear, gelu_mlp
 
 
 @dataclass
@@ -81,11 +82,14 @@ class ParallelBlock(nn.Module):
         cfg = self.cfg
         hd = cfg.d_model // cfg.n_head
         b = self.tokens // cfg.seq_len
-        qkv = self.qkv(self.ln1(h)).view(b, cfg.seq_len, 3, self.heads_local, hd)
+        h, x = norm_residual(self.ln1, h)
+        qkv = self.qkv(x).view(b, cfg.seq_len, 3, self.heads_local, hd)
         q, k, v = (t.transpose(1, 2) for t in qkv.unbind(2))     # [b, heads, seq, hd]
         a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
-        h = h + self.proj(a.transpose(1, 2).reshape(self.tokens, self.heads_local * hd))
-        return h + self.down(F.gelu(self.up(self.ln2(h)), approximate="tanh"))
+        a = a.transpose(1, 2).reshape(self.tokens, self.heads_local * hd)
+        h = self.proj(a, h) if unhooked(self.proj, RowParallelLinear) else h + self.proj(a)
+        h, x = norm_residual(self.ln2, h)
+        return gelu_mlp(self.up, self.down, x, h)
 
 
 class GPT2Stage(nn.Module):
@@ -133,5 +137,5 @@ class GPT2Stage(nn.Module):
             h = blk(h)
         if not self.is_last:
             return h
-        logits = self.ln_f(h) @ self.head.t()
+        logits = norm_residual(self.ln_f, h)[1] @ self.head.t()
         return F.cross_entropy(logits.float(), self.my_rows(targets.reshape(-1)), reduction="sum") / self.tokens

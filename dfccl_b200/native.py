@@ -126,6 +126,12 @@ def lib() -> C.CDLL:
             "dfcclOpsWarm": [],
             "dfcclGemmBf16": [vp, vp, vp, i, i, i, vp],
             "dfcclGemmBf16Ex": [vp, vp, vp, i, i, i, i, i, vp],
+            "dfcclGemmBf16Epilogue": [vp, vp, vp, i, i, i, i, i, i, vp, vp, vp, vp],
+            "dfcclRunFusedGemmLocal": [i, vp, vp, vp, i, i, vp, vp, vp, vp, vp],
+            "dfcclApplyEpilogue": [vp, i, i, i, vp, vp, vp, vp],
+            "dfcclColumnSum": [vp, vp, vp, i, i, vp], "dfcclColumnSumWork": [i, i],
+            "dfcclLayerNormForward": [vp, vp, vp, vp, vp, vp, i, i, C.c_float, vp],
+            "dfcclLayerNormBackward": [vp] * 10 + [i, i, vp], "dfcclLayerNormWork": [i, i], "dfcclLayerNormMaxWidth": [],
             "dfcclGemmCheck": [C.POINTER(i)],
             "dfcclGemmPairResident": [C.POINTER(i)],
             "dfcclGemmFused": [vp, vp, vp, i, i, i, vp, sz, vp],
@@ -151,6 +157,7 @@ def lib() -> C.CDLL:
         L.ncclGetErrorString.restype = C.c_char_p
         L.dfcclTunerPredictUs.restype = C.c_double
         L.dfcclTopoReset.restype = None
+        L.dfcclLayerNormWork.restype = L.dfcclColumnSumWork.restype = sz
         L.dfcclParam.argtypes = [C.c_char_p, C.c_longlong]
         L.dfcclParam.restype = C.c_longlong
         L.dfcclLogReset.argtypes = []

@@ -25,6 +25,7 @@ import torch.distributed as dist
 
 from .. import native as nv
 from ..utils.tensors import raw_stream, tensor_from_ptr
+from .block import Epilogue, NO_EPILOGUE
 from .gemm import BM, BN, BK
 
 
@@ -89,7 +90,22 @@ class _Rendezvous:
         self.epoch = 0
 
 
-class AllGatherGemm:
+class _Local:
+    """One-rank groups: the operator is its GEMM, with an epilogue (``ops.block``)."""
+
+    def local(self, x: torch.Tensor, w: torch.Tensor, w_transposed: bool = False, epi: Epilogue = NO_EPILOGUE) -> torch.Tensor:
+        assert self.tp.n == 1
+        x, w = x.contiguous(), w.contiguous()
+        out = torch.empty(self.m, self.n_out, dtype=torch.bfloat16, device=self.tp.device)
+        ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), raw_stream(self.tp.device)
+        if self.coll_id is not None:
+            nv.check(nv.lib().dfcclRunFusedGemmLocal(self.coll_id, *ptrs, int(w_transposed), *epi.args(), st, self.tp.ctx.handle), "dfcclRunFusedGemmLocal")
+        else:
+            nv.check(nv.lib().dfcclGemmBf16Epilogue(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epi.args(), st), "dfcclGemmBf16Epilogue")
+        return out
+
+
+class AllGatherGemm(_Local):
     """y[M, N] = concat_over_ranks(x_shard)[M, K] @ w[N, K]^T with the all-gather inside the GEMM."""
 
     def __init__(self, tp: TpGroup, rows_per_rank: int, k: int, n_out: int):
@@ -163,7 +179,7 @@ class AllGatherGemm:
         return out
 
 
-class GemmReduceScatter:
+class GemmReduceScatter(_Local):
     """y_shard[M/n, N] = sum_over_ranks(x[M, K_local] @ w[N, K_local]^T)[my rows] with the reduce-scatter
     inside the GEMM: the epilogue stores partial tiles into their owner's memory, the owner sums them."""
 

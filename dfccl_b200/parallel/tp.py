@@ -4,8 +4,8 @@ Forward passes run the fused kernels: the column-parallel layer is an all-gather
 row-parallel layer a GEMM -> reduce-scatter, both one tcgen05 kernel each with the collective
 inside (``dfccl_b200.ops.fused_linear``).  The data-gradient GEMMs of the backward passes are the same
 two kernels with the roles swapped (the column-parallel layer's is a GEMM -> reduce-scatter, the
-row-parallel layer's an all-gather -> GEMM, each on the transposed weight); the weight-gradient
-GEMMs contract over the token dimension and stay on cuBLAS.  On the host backend (tests) the layers
+row-parallel layer's an all-gather -> GEMM, each on the transposed weight).  Biases, residuals and the GELU of an MLP ride in the products' epilogues
+(on one rank; a pass over the operator's output on several).  On the host backend (tests) the layers
 fall back to this library's stream-ordered collectives around plain GEMMs.
 
 The reference has no tensor-parallel code; its simulator only generates the group structure of
@@ -18,8 +18,10 @@ from typing import Dict, Tuple
 import torch
 import torch.distributed as dist
 import torch.nn as nn
+from torch.autograd.function import once_differentiable
 
 from .. import native as nv
+from ..ops.block import BIAS, BIAS_GELU, BIAS_RES, GELU_GRAD, Epilogue, NO_EPILOGUE, apply_epilogue_, column_sum, unhooked
 from ..ops.fused_linear import AllGatherGemm, GemmReduceScatter, TpGroup
 from ..utils.tensors import nccl_dtype, raw_stream
 
@@ -86,60 +88,146 @@ def tp_reduce_scatter(tp: TpGroup, x: torch.Tensor) -> torch.Tensor:
 
 
 class _ColumnFn(torch.autograd.Function):
-    """y = all_gather(x_shard) W^T.  Backward: gW = gy^T x_full, gx_shard = reduce_scatter(gy W)."""
+    """y = all_gather(x_shard) W^T with plain GEMMs around this library's collectives (host backend, comparison arm).
+    Backward: gW = gy^T x_full, gx_shard = reduce_scatter(gy W)."""
 
     @staticmethod
     def forward(ctx, x_shard, weight, layer):
         ctx.layer = layer
-        if layer.op is None:                                # host backend (tests) / comparison arm: collective + plain GEMM
-            ctx.save_for_backward(x_shard, weight)
-            return tp_all_gather(layer.tp, x_shard) @ weight.t()
-        y = layer.op(x_shard, weight)
-        # the gathered activations are needed again for the weight gradient: keep a copy (the operator's buffer
-        # is shared by every layer of this shape) instead of gathering a second time in the backward pass
-        ctx.save_for_backward(layer.op.gathered.clone(), weight)
-        return y
+        ctx.save_for_backward(x_shard, weight)
+        return tp_all_gather(layer.tp, x_shard) @ weight.t()
 
     @staticmethod
     def backward(ctx, gy):
-        saved, weight = ctx.saved_tensors
-        layer = ctx.layer
-        tp = layer.tp
+        x_shard, weight = ctx.saved_tensors
+        tp = ctx.layer.tp
         gy = gy.contiguous()
-        if layer.op is None:
-            x_full = tp_all_gather(tp, saved)
-            return tp_reduce_scatter(tp, gy @ weight), gy.t() @ x_full, None
-        gw = _wgrad(gy, saved)
-        # data gradient with the reduce-scatter inside the GEMM: gx = RS(gy [M, N/n] @ W [N/n, K]); the B operand is W^T,
-        # handed over as W itself (stored [contraction, output]: read in place as an MN-major operand)
-        gx = layer.bwd_op(gy, weight, w_transposed=True)
-        return gx, gw, None
+        x_full = tp_all_gather(tp, x_shard)
+        return tp_reduce_scatter(tp, gy @ weight), gy.t() @ x_full, None
 
 
 class _RowFn(torch.autograd.Function):
-    """y_shard = reduce_scatter(x W^T).  Backward: gy = all_gather(gy_shard), gx = gy W, gW = gy^T x."""
+    """y_shard = reduce_scatter(x W^T), the same way.  Backward: gy = all_gather(gy_shard), gx = gy W, gW = gy^T x."""
 
     @staticmethod
     def forward(ctx, x, weight, layer):
         ctx.layer = layer
         ctx.save_for_backward(x, weight)
-        if layer.op is None:
-            return tp_reduce_scatter(layer.tp, x @ weight.t())
-        return layer.op(x, weight)
+        return tp_reduce_scatter(layer.tp, x @ weight.t())
 
     @staticmethod
     def backward(ctx, gy_shard):
         x, weight = ctx.saved_tensors
-        layer = ctx.layer
-        gy_shard = gy_shard.contiguous()
-        if layer.op is None:
-            gy = tp_all_gather(layer.tp, gy_shard)
-            return gy @ weight, gy.t() @ x, None
-        # data gradient with the all-gather inside the GEMM: gx = AG(gy_shard) [M, N] @ W [N, K/n], B operand = W^T;
-        # the operator's gathered buffer then holds the full output gradient for the weight gradient
-        gx = layer.bwd_op(gy_shard, weight, w_transposed=True)
-        gw = _wgrad(layer.bwd_op.gathered, x)
-        return gx, gw, None
+        gy = tp_all_gather(ctx.layer.tp, gy_shard.contiguous())
+        return gy @ weight, gy.t() @ x, None
+
+
+# ---- on the fused kernels: bias, residual and GELU belong to the product.  One rank: in the GEMM's epilogue, and no
+# ---- gathered copies; several ranks: one pass over the operator's output.
+def _product(op, x: torch.Tensor, w: torch.Tensor, epi: Epilogue = NO_EPILOGUE, w_transposed: bool = False) -> torch.Tensor:
+    if op.tp.n == 1:
+        return op.local(x, w, w_transposed, epi)
+    y = op(x, w, w_transposed=w_transposed)
+    return apply_epilogue_(y, epi) if epi.kind else y
+
+
+def _column(layer, x_shard: torch.Tensor, weight: torch.Tensor, epi: Epilogue):
+    """(y, the gathered activations: what the weight gradient needs).  The operator's own buffer is shared by every layer
+    of this shape, so several ranks keep a copy of it instead of gathering a second time in the backward pass."""
+    x_shard = x_shard.contiguous()
+    y = _product(layer.op, x_shard, weight, epi)
+    return y, x_shard if layer.tp.n == 1 else layer.op.gathered.clone()
+
+
+def _column_backward(layer, gy: torch.Tensor, x_full: torch.Tensor, weight: torch.Tensor):
+    """gW, and the data gradient with the reduce-scatter inside the GEMM: gx = RS(gy [M, N/n] @ W [N/n, K]); the B operand is
+    W^T, handed over as W itself (stored [contraction, output]: read in place as an MN-major operand)."""
+    return _wgrad(gy, x_full), _product(layer.bwd_op, gy, weight, w_transposed=True)
+
+
+def _row_backward(layer, gy_shard: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, epi: Epilogue = NO_EPILOGUE):
+    """gW, and the data gradient with the all-gather inside the GEMM, gx = AG(gy_shard) [M, N] @ W [N, K/n]; the operator's
+    gathered buffer then holds the full output gradient, which gW needs."""
+    gx = _product(layer.bwd_op, gy_shard, weight, epi, w_transposed=True)
+    return _wgrad(gy_shard if layer.tp.n == 1 else layer.bwd_op.gathered, x), gx
+
+
+def _bias_epilogue(bias, aux=None) -> Epilogue:
+    if bias is None:
+        return NO_EPILOGUE
+    return Epilogue(BIAS, bias) if aux is None else Epilogue(BIAS_RES, bias, aux=aux)
+
+
+class _ColumnFusedFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x_shard, weight, bias, layer):
+        y, x_full = _column(layer, x_shard, weight, _bias_epilogue(bias))
+        ctx.layer, ctx.has_bias = layer, bias is not None
+        ctx.save_for_backward(x_full, weight)
+        return y
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, gy):
+        x_full, weight = ctx.saved_tensors
+        gy = gy.contiguous()
+        gb = column_sum(gy) if ctx.has_bias else None
+        gw, gx = _column_backward(ctx.layer, gy, x_full, weight)
+        return gx, gw, gb, None
+
+
+class _RowFusedFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, bias, residual, layer):
+        x = x.contiguous()
+        ctx.layer, ctx.has_bias, ctx.has_residual = layer, bias is not None, residual is not None
+        ctx.save_for_backward(x, weight)
+        return _product(layer.op, x, weight, _bias_epilogue(bias, None if residual is None else residual.contiguous()))
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, gy_shard):
+        x, weight = ctx.saved_tensors
+        gy = gy_shard.contiguous()
+        gb = column_sum(gy) if ctx.has_bias else None
+        gw, gx = _row_backward(ctx.layer, gy, x, weight)
+        return gx, gw, gb, gy_shard if ctx.has_residual else None, None
+
+
+class _MlpFn(torch.autograd.Function):
+    """residual + down(gelu(up(x))): GELU in the up product's epilogue, its gradient in the epilogue of down's data gradient."""
+
+    @staticmethod
+    def forward(ctx, x, up_weight, up_bias, down_weight, down_bias, residual, up, down):
+        pre = torch.empty(up.op.m, up.op.n_out, dtype=torch.bfloat16, device=x.device) if any(ctx.needs_input_grad) else None
+        act, x_full = _column(up, x, up_weight, Epilogue(BIAS_GELU, up_bias, pre=pre))
+        ctx.up, ctx.down = up, down
+        ctx.save_for_backward(x_full, pre, act, up_weight, down_weight)
+        return _product(down.op, act, down_weight, Epilogue(BIAS_RES, down_bias, aux=residual.contiguous()))
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, gy_shard):
+        x_full, pre, act, up_weight, down_weight = ctx.saved_tensors
+        gy = gy_shard.contiguous()
+        gb_down = column_sum(gy)
+        gw_down, gpre = _row_backward(ctx.down, gy, act, down_weight, Epilogue(GELU_GRAD, aux=pre))
+        gb_up = column_sum(gpre)
+        gw_up, gx = _column_backward(ctx.up, gpre, x_full, up_weight)
+        return gx, gw_up, gb_up, gw_down, gb_down, gy_shard, None, None
+
+
+def _fused_bias(layer, x: torch.Tensor) -> bool:
+    """The epilogues take bf16 activations, weights and biases."""
+    return x.dtype == layer.weight.dtype == layer.bias.dtype == torch.bfloat16
+
+
+def gelu_mlp(up: "ColumnParallelLinear", down: "RowParallelLinear", x: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:
+    """``residual + down(gelu(up(x)))`` with the tanh form of GELU."""
+    if (up.op is not None and down.op is not None and unhooked(up, ColumnParallelLinear) and unhooked(down, RowParallelLinear)
+            and _fused_bias(up, x) and _fused_bias(down, residual)):
+        return _MlpFn.apply(x, up.weight, up.bias, down.weight, down.bias, residual, up, down)
+    return residual + down(nn.functional.gelu(up(x), approximate="tanh"))
 
 
 class ColumnParallelLinear(nn.Module):
@@ -161,7 +249,11 @@ class ColumnParallelLinear(nn.Module):
         self.bwd_op = shared_op(GemmReduceScatter, tp, rows_per_rank * tp.n, nl, in_features) if _fused(tp) else None
 
     def forward(self, x_shard):
-        return _ColumnFn.apply(x_shard, self.weight, self) + self.bias
+        if self.op is None:
+            return _ColumnFn.apply(x_shard, self.weight, self) + self.bias
+        if _fused_bias(self, x_shard):
+            return _ColumnFusedFn.apply(x_shard, self.weight, self.bias, self)
+        return _ColumnFusedFn.apply(x_shard, self.weight, None, self) + self.bias
 
 
 class RowParallelLinear(nn.Module):
@@ -180,5 +272,9 @@ class RowParallelLinear(nn.Module):
         self.op = shared_op(GemmReduceScatter, tp, m, kl, out_features) if _fused(tp) else None
         self.bwd_op = shared_op(AllGatherGemm, tp, m // tp.n, out_features, kl) if _fused(tp) else None
 
-    def forward(self, x):
-        return _RowFn.apply(x, self.weight, self) + self.bias
+    def forward(self, x, residual=None):
+        """``residual`` (sharded like the output) is added in the same pass as the bias."""
+        if self.op is not None and _fused_bias(self, x) and (residual is None or residual.dtype == torch.bfloat16):
+            return _RowFusedFn.apply(x, self.weight, self.bias, residual, self)
+        y = (_RowFn.apply(x, self.weight, self) if self.op is None else _RowFusedFn.apply(x, self.weight, None, None, self)) + self.bias
+        return y if residual is None else residual + y

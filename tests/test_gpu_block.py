@@ -1,0 +1,135 @@
+"""The kernels around a transformer block's GEMMs against 64-bit torch: epilogues, layer norm, column sums, and a whole
+block against the same block on torch's own operators."""
+import pytest
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+HALF_ULP = 2.0 ** -8                     # one rounding to bf16 (8 significant bits), relative, at most
+
+
+def _rel(got, want):
+    return ((got.double() - want).norm() / want.norm().clamp_min(1e-300)).item()
+
+
+# 8192 x 1024 x 1024 runs on the persistent kernel (epilogue inside), as does 9600 rows (last row tile half empty); the
+# others on tile forms followed by a pass of its own
+@pytest.mark.parametrize("m,n,k", [(128, 256, 64), (256, 768, 256), (8192, 1024, 1024), (9600, 512, 1024)])
+def test_epilogues(native, m, n, k):
+    from dfccl_b200.ops import block, gemm
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)              # noqa: E731
+    a, b, bias, aux = rnd(m, k), (rnd(n, k) * k ** -0.5).to(torch.bfloat16), rnd(n), rnd(m, n)
+    acc = a.double() @ b.double().t()
+    pre, out = torch.empty_like(aux), torch.empty_like(aux)
+
+    def run(epi):
+        native.check(native.lib().dfcclGemmBf16Epilogue(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, 0, 0, *epi.args(),
+                                                        torch.cuda.current_stream().cuda_stream), "epilogue")
+        return out.clone()
+
+    gelu = lambda x: F.gelu(x, approximate="tanh")                                               # noqa: E731
+    # a product rounded before its epilogue (a pass of its own) has one rounding more
+    assert _rel(run(block.Epilogue(block.BIAS, bias)), acc + bias.double()) < 2 * HALF_ULP
+    assert _rel(run(block.Epilogue(block.BIAS_RES, bias, aux=aux)), acc + bias.double() + aux.double()) < 2 * HALF_ULP
+    y = run(block.Epilogue(block.BIAS_GELU, bias, pre=pre))
+    assert _rel(pre, acc + bias.double()) < 2 * HALF_ULP
+    assert _rel(y, gelu(pre.double())) < HALF_ULP
+    assert torch.equal(run(block.Epilogue(block.BIAS_GELU, bias)), y)
+    x = aux.double().requires_grad_(True)
+    gelu(x).backward(acc)
+    assert _rel(run(block.Epilogue(block.GELU_GRAD, aux=aux)), x.grad) < 2 * HALF_ULP
+    torch.cuda.synchronize()
+    assert gemm.check_kernels()
+
+
+def test_gelu_far_from_zero(native):
+    from dfccl_b200.ops import block
+    v = torch.tensor([0.0, -0.0, 1e-30, 5.0, -5.0, 9.0, -9.0, -20.0, 3e4, -3e4, 1e12, -1e12, 3e38, -3e38, float("inf"), float("nan")],
+                     device="cuda", dtype=torch.bfloat16).view(1, 16)
+    y = block.apply_epilogue_(v.clone(), block.Epilogue(block.BIAS_GELU, torch.zeros(16, device="cuda", dtype=torch.bfloat16)))
+    want = F.gelu(v.double(), approximate="tanh")
+    # the reference's 1 + tanh is only good to 2**-53: times 20, the largest |x| at which the result is not 0
+    assert torch.allclose(y.double()[:, :14], want[:, :14], rtol=2 * HALF_ULP, atol=20 * 2.0 ** -53)
+    assert y[0, 14] == float("inf") and torch.isnan(y[0, 15])
+    d = block.apply_epilogue_(torch.ones_like(v), block.Epilogue(block.GELU_GRAD, aux=v.clone()))
+    x = v.double()[:, :12].clone().requires_grad_(True)
+    F.gelu(x, approximate="tanh").sum().backward()
+    assert torch.allclose(d.double()[:, :12], x.grad, rtol=2 * HALF_ULP, atol=1e-6)
+    assert d[0, 12] == 1 and d[0, 13] == 0 and torch.isnan(d[0, 15])
+
+
+@pytest.mark.parametrize("rows,d", [(1, 8), (3, 248), (37, 256), (130, 264), (1000, 768), (8192, 1024), (515, 1600), (64, 2048)])
+def test_layer_norm_with_the_residuals_gradient(native, rows, d):
+    from dfccl_b200.ops import block
+    torch.manual_seed(rows + d)
+    ln = nn.LayerNorm(d, dtype=torch.bfloat16, device="cuda")
+    with torch.no_grad():
+        ln.weight.add_(torch.randn_like(ln.weight) * 0.1)
+        ln.bias.add_(torch.randn_like(ln.bias) * 0.1)
+    x = (torch.randn(rows, d, device="cuda") * 2 + 1).to(torch.bfloat16).requires_grad_(True)
+    g1, g2 = (torch.randn(rows, d, device="cuda").to(torch.bfloat16) for _ in range(2))
+    h, y = block.norm_residual(ln, x)
+    torch.autograd.backward([h, y], [g1, g2])
+    x64 = x.detach().double().requires_grad_(True)
+    w64, b64 = ln.weight.detach().double().requires_grad_(True), ln.bias.detach().double().requires_grad_(True)
+    y64 = F.layer_norm(x64, (d,), w64, b64, ln.eps)
+    torch.autograd.backward([x64 * 1, y64], [g1.double(), g2.double()])
+    assert torch.equal(h, x)
+    # fp32 arithmetic (sums of up to 8192 terms), one rounding
+    for got, want in ((y, y64), (x.grad, x64.grad), (ln.weight.grad, w64.grad), (ln.bias.grad, b64.grad)):
+        assert _rel(got.detach(), want.detach()) < HALF_ULP
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8), (31, 64), (33, 264), (1000, 1024), (8192, 3072), (4100, 4096)])
+def test_column_sum(native, rows, n):
+    from dfccl_b200.ops import block
+    torch.manual_seed(rows + n)
+    g = torch.randn(rows, n, device="cuda").to(torch.bfloat16)
+    assert _rel(block.column_sum(g), g.double().sum(0)) < HALF_ULP
+
+
+@pytest.mark.parametrize("tokens,d,hooked", [(256, 256, False), (8192, 512, False), (256, 256, True)])
+def test_block_against_torch_operators(native, tokens, d, hooked):
+    """Output and every gradient of a one-rank block; modules with hooks are called as modules."""
+    from dfccl_b200.models.gpt2 import GPT2Config, ParallelBlock
+    from dfccl_b200.ops.fused_linear import TpGroup
+    native.set_backend("cuda")
+    (comm,) = native.Comm.init_loopback(1, 0)
+    dev = torch.device("cuda", 0)
+    cfg = GPT2Config(n_layer=1, d_model=d, n_head=d // 64, seq_len=128)
+    blk = ParallelBlock(cfg, TpGroup(comm, None, dev), tokens, 0, 11)
+    torch.manual_seed(3)
+    with torch.no_grad():
+        for p in blk.parameters():
+            if p.dim() == 1:
+                p.add_((torch.randn(p.shape, device=dev) * 0.1).to(p.dtype))
+    calls = []
+    if hooked:
+        for m in (blk.ln1, blk.qkv, blk.proj, blk.ln2, blk.up, blk.down):
+            m.register_forward_hook(lambda *_: calls.append(1))
+    x = torch.randn(tokens, d, device=dev).to(torch.bfloat16).requires_grad_(True)
+    gy = torch.randn(tokens, d, device=dev).to(torch.bfloat16)
+    y = blk(x)
+    y.backward(gy)
+    assert len(calls) == (6 if hooked else 0)
+
+    p = {k: v.detach().double().requires_grad_(True) for k, v in blk.named_parameters()}
+    x64 = x.detach().double().requires_grad_(True)
+    ln = lambda t, n: F.layer_norm(t, (d,), p[n + ".weight"], p[n + ".bias"])                     # noqa: E731
+    lin = lambda t, n: t @ p[n + ".weight"].t() + p[n + ".bias"]                                  # noqa: E731
+    q, k, v = (t.transpose(1, 2) for t in lin(ln(x64, "ln1"), "qkv").view(tokens // 128, 128, 3, d // 64, 64).unbind(2))
+    a = F.scaled_dot_product_attention(q, k, v, is_causal=True).transpose(1, 2).reshape(tokens, d)
+    h = x64 + lin(a, "proj")
+    y64 = h + lin(F.gelu(lin(ln(h, "ln2"), "up"), approximate="tanh"), "down")
+    y64.backward(gy.double())
+    # bf16 activations through a whole block: a few roundings of 2**-8 at most each on the way to the output and back
+    assert _rel(y.detach(), y64.detach()) < 1e-2 and _rel(x.grad, x64.grad) < 1e-2
+    for name, q in blk.named_parameters():
+        if name == "qkv.bias":                     # the key bias has no gradient but rounding noise (softmax is shift-invariant)
+            keep = torch.cat([torch.arange(0, d), torch.arange(2 * d, 3 * d)]).to(dev)
+            assert _rel(q.grad[keep], p[name].grad[keep]) < 2e-2, name
+        else:
+            assert _rel(q.grad, p[name].grad) < 2e-2, name
+    comm.destroy()

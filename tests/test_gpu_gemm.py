@@ -122,8 +122,8 @@ def test_gemm_throughput_report():
     (1920, 1280, 768), (2048, 1024, 448),
     (9600, 512, 1024), (9600, 1024, 192)])                  # persistent pairs, half empty
 def test_every_tile_form_at_its_edges(m, n, k):
-    """All storage orders give the same bits, and the error against 64 bits is that of one rounding to bf16: 2**-9 of a
-    value at most (uniform between 0 and that: 2**-9 / sqrt(3) in the mean) plus fp32 sums."""
+    """All storage orders give the same bits, and the error against 64 bits is that of one rounding to bf16: 2**-8 of a
+    value at most, half of that in the 2-norm over many values (0.41 x 2**-8 = 2**-8 / sqrt(3) averaged over a binade)."""
     from dfccl_b200.ops import gemm
     torch.manual_seed(m + 3 * n + 5 * k)
     a = torch.randn(m, k, device="cuda", dtype=torch.bfloat16)
