@@ -219,6 +219,18 @@ __device__ __forceinline__ void raster_tile(int t, int mTiles, int nTiles, int g
   nt = r / gsz;
 }
 
+// 32 bytes (two packs of 16) of global memory: one access of a whole sector where the address allows it (`wide`).
+__device__ __forceinline__ void st_global32(void* p, const uint4* v, bool wide) {
+  if (!wide) { ((uint4*)p)[0] = v[0]; ((uint4*)p)[1] = v[1]; return; }
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w),
+               "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w) : "memory");
+}
+__device__ __forceinline__ void ld_global32(const void* p, uint4* v, bool wide) {
+  if (!wide) { v[0] = ((const uint4*)p)[0]; v[1] = ((const uint4*)p)[1]; return; }
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w),
+               "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w) : "l"(p) : "memory");
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);

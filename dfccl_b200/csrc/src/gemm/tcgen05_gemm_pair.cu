@@ -34,9 +34,7 @@ constexpr int MN_BLOCK_BYTES = 64 * BK * 2;
 constexpr int TMEM_COLS = 512;                       // two accumulators of 256 fp32 columns (128 lanes each, per CTA)
 constexpr int NUM_THREADS = 320;                     // 10 warps
 constexpr int EPI_WARPS = 8;                         // two per 32 accumulator rows: the last tile's epilogue is not overlapped with anything
-constexpr int EPI_ROW_BYTES = 32 * 2 + 16;           // 32 columns of a row at a time (64 would not leave room for six stages)
-constexpr int EPI_WARP_BYTES = 32 * EPI_ROW_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * EPI_WARP_BYTES + 1024 + 256;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on another GPU: seconds mean a lost partner
 
 struct PairArgs {
@@ -47,6 +45,7 @@ struct PairArgs {
   uint32_t* err;
   uint32_t* errHost;
   GemmEpilogue e;
+  bool wide;                        // C, aux and pre start on 32-byte boundaries
 };
 
 template <int EPI>
@@ -54,8 +53,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const PairArgs g) {
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  uint8_t* epiSmem = smem + STAGES * STAGE_BYTES;
-  uint64_t* fullBar = (uint64_t*)(epiSmem + EPI_WARPS * EPI_WARP_BYTES);     // used in the leader only
+  uint64_t* fullBar = (uint64_t*)(smem + STAGES * STAGE_BYTES);     // used in the leader only
   uint64_t* emptyBar = fullBar + STAGES;                             // in both CTAs (commit to both)
   uint64_t* accFull = emptyBar + STAGES;                             // [2] in both CTAs
   uint64_t* accEmpty = accFull + 2;                                  // [2] used in the leader only: the epilogue warps of both CTAs arrive
@@ -149,42 +147,26 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       int mt, nt;
       raster_tile(t, mTiles, nTiles, g.groupM, mt, nt);
       const int ab = it & 1;
-      if (!mbar_wait(&accFull[ab], (it >> 1) & 1, giveUp, WAIT_NS)) break;
-      tc_fence_after();
-      uint8_t* stg = epiSmem + (warp - 2) * EPI_WARP_BYTES;
       const bool mine = mt * PM + (int)cr * HALF < g.M;               // the last row tile may have only its upper half
       const size_t tileOff = (size_t)(mt * PM + (int)cr * HALF + quarter * 32) * g.ldc + nt * PN;   // row 0 of this warp's 32 rows
-      const int beg = colHalf * (PN / 2), end = beg + PN / 2;
-      // 32 columns at a time.  Global memory is touched in chunks of 16 bytes, 4 lanes to a 64-byte row segment; a lane's own
-      // row passes through this warp's staging rows.  `aux` is fetched one step ahead.
-      const int rr0 = lane >> 2, cc = lane & 3;
-      uint4 ax[4];
-      auto fetch = [&](int c) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) ax[q] = *(const uint4*)(g.e.aux + tileOff + (size_t)(q * 8 + rr0) * g.ldc + c + cc * 8);
-      };
-      auto flush = [&](__nv_bfloat16* to, int c) {
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *(uint4*)(to + tileOff + (size_t)(q * 8 + rr0) * g.ldc + c + cc * 8) = *(const uint4*)(stg + (q * 8 + rr0) * EPI_ROW_BYTES + cc * 16);
-        __syncwarp();
-      };
+      const int beg = colHalf * (PN / 2);
+      // 32 columns of its row per lane and step, 32 bytes (a whole sector) per access: no staging rows, whose way through
+      // shared memory the operands need (8192 x 4096 x 1024 with GELU's gradient: 105 -> 76 us)
       constexpr bool AUX = EPI == EPI_BIAS_RES || EPI == EPI_GELU_GRAD;
-      if (AUX && mine) fetch(beg);
+      constexpr int STEPS = PN / 2 / 32;
+      const size_t mineOff = tileOff + (size_t)lane * g.ldc + beg;
+      if (!mbar_wait(&accFull[ab], (it >> 1) & 1, giveUp, WAIT_NS)) break;
+      tc_fence_after();
 #pragma unroll 1
-      for (int c = beg; mine && c < end; c += 32) {
+      for (int i = 0; i < STEPS; ++i) {
+        if (!mine) break;
+        const int c = beg + i * 32;
         uint32_t r[32];
         tmem_ld32(tmemBase + ((uint32_t)(quarter * 32) << 16) + ab * PN + c, r);
-        uint4* srow = (uint4*)(stg + lane * EPI_ROW_BYTES);
         uint4 own[4];
         if (AUX) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) *(uint4*)(stg + (q * 8 + rr0) * EPI_ROW_BYTES + cc * 16) = ax[q];
-          __syncwarp();
-#pragma unroll
-          for (int v = 0; v < 4; ++v) own[v] = srow[v];
-          if (c + 32 < end) fetch(c + 32);
+          ld_global32(g.e.aux + mineOff + i * 32, own, g.wide);
+          ld_global32(g.e.aux + mineOff + i * 32 + 16, own + 2, g.wide);
         }
         tmem_ld_wait();
         if (EPI == EPI_BIAS || EPI == EPI_BIAS_RES || EPI == EPI_BIAS_GELU) {
@@ -222,9 +204,8 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
         }
         if (EPI == EPI_BIAS_GELU) {
           if (g.e.pre) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) srow[v] = o[v];
-            flush(g.e.pre, c);
+            st_global32(g.e.pre + mineOff + i * 32, o, g.wide);
+            st_global32(g.e.pre + mineOff + i * 32 + 16, o + 2, g.wide);
           }
 #pragma unroll
           for (int v = 0; v < 4; ++v) {                // of the rounded value: what the backward pass differentiates at
@@ -233,9 +214,8 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             for (int w = 0; w < 4; ++w) ow[w] = pack_bf16x2(geluTanh(bf16Lo(ow[w])), geluTanh(bf16Hi(ow[w])));
           }
         }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) srow[v] = o[v];
-        flush(g.C, c);
+        st_global32(g.C + mineOff + i * 32, o, g.wide);
+        st_global32(g.C + mineOff + i * 32 + 16, o + 2, g.wide);
       }
       tc_fence_before();
       __syncwarp();
@@ -297,6 +277,7 @@ ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N,
   g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.ldc = N; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0;
   g.err = errDev; g.errHost = errHost;
   if (e) g.e = *e;
+  g.wide = (((uintptr_t)C | (uintptr_t)g.e.aux | (uintptr_t)g.e.pre) & 31) == 0;
   { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
