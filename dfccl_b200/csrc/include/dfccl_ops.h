@@ -41,6 +41,17 @@ ncclResult_t dfcclFusedSgdStep(void* master, const void* grad, void* momentum, v
 /* AdamW (decoupled weight decay) over the same flat arrays; `step` counts from 1, both moment arrays start at zero. */
 ncclResult_t dfcclFusedAdamWStep(void* master, const void* grad, void* moment1, void* moment2, void* param, size_t n, int paramType,
                                  float lr, float beta1, float beta2, float eps, float wd, int step, cudaStream_t stream);
+/* The same for all buckets of a step in one launch (16 to a launch).  `clear`, where given, is an array of n elements of the
+ * parameters' type that is set to zero on the way (the gradients before their reduction). */
+#define DFCCL_OPTIM_MAX_BUCKETS 16
+typedef struct {
+  void* master; const void* grad32; void* momentum; void* moment2 /* AdamW */; void* param; void* clear;
+  size_t n;
+  int paramType;
+} dfcclOptimBucket;
+ncclResult_t dfcclFusedSgdSteps(const dfcclOptimBucket* buckets, int n, float lr, float mu, float wd, int firstStep, cudaStream_t stream);
+ncclResult_t dfcclFusedAdamWSteps(const dfcclOptimBucket* buckets, int n, float lr, float beta1, float beta2, float eps, float wd, int step,
+                                  cudaStream_t stream);
 ncclResult_t dfcclOpsWarm(void);   /* load these kernels now (before any stream can block) */
 
 /* ---- fabric probes (roofline inputs): mean device time in microseconds */

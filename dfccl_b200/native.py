@@ -38,6 +38,11 @@ class CollInfo(C.Structure):
                 ("op", C.c_int), ("root", C.c_int), ("scale", C.c_float), ("algo", C.c_int), ("nBlocks", C.c_int), ("flags", C.c_int)]
 
 
+class OptimBucket(C.Structure):
+    _fields_ = [("master", C.c_void_p), ("grad32", C.c_void_p), ("momentum", C.c_void_p), ("moment2", C.c_void_p),
+                ("param", C.c_void_p), ("clear", C.c_void_p), ("n", C.c_size_t), ("param_type", C.c_int)]
+
+
 class FusedInfo(C.Structure):
     _fields_ = [("kind", C.c_int), ("rowsPerRank", C.c_int), ("k", C.c_int), ("n", C.c_int)]
 
@@ -123,6 +128,8 @@ def lib() -> C.CDLL:
             "dfcclInjectFault": [vp, i, C.c_int64],
             "dfcclFusedSgdStep": [vp, vp, vp, vp, sz, i, C.c_float, C.c_float, C.c_float, i, vp],
             "dfcclFusedAdamWStep": [vp, vp, vp, vp, vp, sz, i, C.c_float, C.c_float, C.c_float, C.c_float, C.c_float, i, vp],
+            "dfcclFusedSgdSteps": [C.POINTER(OptimBucket), i, C.c_float, C.c_float, C.c_float, i, vp],
+            "dfcclFusedAdamWSteps": [C.POINTER(OptimBucket), i, C.c_float, C.c_float, C.c_float, C.c_float, C.c_float, i, vp],
             "dfcclOpsWarm": [],
             "dfcclGemmBf16": [vp, vp, vp, i, i, i, vp],
             "dfcclGemmBf16Ex": [vp, vp, vp, i, i, i, i, i, vp],

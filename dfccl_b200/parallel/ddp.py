@@ -21,7 +21,6 @@ src/include/collectives_ofccl.h:63,78-100).
 """
 from __future__ import annotations
 
-import ctypes as C
 import random
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence
@@ -119,6 +118,7 @@ class DaemonDDP:
         self._pool = HeapTensorPool(self.comm, self.device)
         self._ready: List[Bucket] = []
         self._submitted: List[Bucket] = []
+        self._step_order: List[Bucket] = []     # the last step's buckets, the one submitted last first
         self._first_step = True
         self._capturing = False                 # gradient hooks record bucket releases into a stream capture (see graph.GraphedStep)
         self._captured: List[Bucket] = []
@@ -308,30 +308,34 @@ class DaemonDDP:
         s = self._stream()
         for b in self._submitted:
             self.ctx.stream_wait(b.coll_id, s)
-        self._submitted = []
+        self._step_order, self._submitted = self._submitted[::-1], []
         for b in self.buckets:
             b.pending = len(b.params)
 
     def step(self, lr: Optional[float] = None) -> None:
-        """One fused optimizer kernel per flat bucket (SGD with momentum, or AdamW), then clear the gradients."""
+        """One fused optimizer kernel over all flat buckets (SGD with momentum, or AdamW); clears the gradients."""
         lr = self.lr if lr is None else lr
-        s = self._stream()
         self._t += 1
         b1, b2 = self.betas
+        if self.device.type == "cuda":
+            # the bucket reduced last first: part of its reduced gradient is still in L2
+            last = self._step_order + [b for b in self.buckets if b not in self._step_order]
+            arr = (nv.OptimBucket * max(1, len(last)))()
+            for k, b in zip(arr, last):
+                k.master, k.grad32, k.momentum, k.param = b.master.data_ptr(), b.grad32.data_ptr(), b.momentum.data_ptr(), b.flat_param.data_ptr()
+                k.moment2 = None if b.moment2 is None else b.moment2.data_ptr()
+                k.clear, k.n, k.param_type = b.grad.data_ptr(), b.numel, nccl_dtype(b.dtype)
+            s = self._stream()
+            if self.optimizer == "adamw":
+                nv.check(self._lib.dfcclFusedAdamWSteps(arr, len(last), lr, b1, b2, self.eps, self.wd, self._t, s), "dfcclFusedAdamWSteps")
+            else:
+                nv.check(self._lib.dfcclFusedSgdSteps(arr, len(last), lr, self.mu, self.wd, 1 if self._first_step else 0, s), "dfcclFusedSgdSteps")
+            self.launches += (len(last) + 15) // 16
+            torch.autograd.graph.increment_version([b.grad for b in last])
+            self._first_step = False
+            return
         for b in self.buckets:
-            if self.device.type == "cuda":
-                if self.optimizer == "adamw":
-                    nv.check(self._lib.dfcclFusedAdamWStep(
-                        C.c_void_p(b.master.data_ptr()), C.c_void_p(b.grad32.data_ptr()), C.c_void_p(b.momentum.data_ptr()),
-                        C.c_void_p(b.moment2.data_ptr()), C.c_void_p(b.flat_param.data_ptr()), b.numel, nccl_dtype(b.dtype),
-                        lr, b1, b2, self.eps, self.wd, self._t, C.c_void_p(s)), "dfcclFusedAdamWStep")
-                else:
-                    nv.check(self._lib.dfcclFusedSgdStep(
-                        C.c_void_p(b.master.data_ptr()), C.c_void_p(b.grad32.data_ptr()), C.c_void_p(b.momentum.data_ptr()),
-                        C.c_void_p(b.flat_param.data_ptr()), b.numel, nccl_dtype(b.dtype), lr, self.mu, self.wd,
-                        1 if self._first_step else 0, C.c_void_p(s)), "dfcclFusedSgdStep")
-                self.launches += 1
-            elif self.optimizer == "adamw":        # host backend (tests): the same arithmetic in PyTorch
+            if self.optimizer == "adamw":          # host backend (tests): the same arithmetic in PyTorch
                 g = b.grad32
                 b.momentum.mul_(b1).add_(g, alpha=1 - b1)
                 b.moment2.mul_(b2).addcmul_(g, g, value=1 - b2)

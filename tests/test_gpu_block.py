@@ -133,3 +133,39 @@ def test_block_against_torch_operators(native, tokens, d, hooked):
         else:
             assert _rel(q.grad, p[name].grad) < 2e-2, name
     comm.destroy()
+
+
+@pytest.mark.parametrize("adamw", [False, True])
+def test_one_optimizer_launch_over_many_buckets(native, adamw):
+    """More buckets than a launch holds, of both parameter types and odd lengths, against one call per bucket: the same
+    bits, gradients cleared, nothing behind a bucket's end touched."""
+    native.set_backend("cuda")
+    L, st = native.lib(), torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    sizes = [1, 3, 4, 7, 2047, 2048, 2049, 100003, 0, 8, 4096, 5, 6, 1 << 20, 12, 16, 20, 2050]
+    pad = 8
+    rows, want = [], []
+    for i, n in enumerate(sizes):
+        ptype = torch.bfloat16 if i % 3 else torch.float32
+        f = [torch.rand(n + pad, device="cuda", generator=gen) for _ in range(4)]
+        p, c = torch.full((n + pad,), 3.0, device="cuda", dtype=ptype), torch.full((n + pad,), 5.0, device="cuda", dtype=ptype)
+        rows.append((n, *f, p, c))
+        want.append([t.clone() for t in (f[0], f[2], f[3], p)])
+    for (n, _, g, *_, p, _), (w, m, v, q) in zip(rows, want):
+        a = (w.data_ptr(), g.data_ptr(), m.data_ptr())
+        t = native.BFLOAT16 if p.dtype == torch.bfloat16 else native.FLOAT32
+        if adamw:
+            native.check(L.dfcclFusedAdamWStep(*a, v.data_ptr(), q.data_ptr(), n, t, 0.01, 0.9, 0.99, 1e-8, 0.1, 2, st), "one")
+        else:
+            native.check(L.dfcclFusedSgdStep(*a, q.data_ptr(), n, t, 0.1, 0.9, 0.01, 0, st), "one")
+    arr = (native.OptimBucket * len(rows))()
+    for k, (n, w, g, m, v, p, c) in zip(arr, rows):
+        k.master, k.grad32, k.momentum, k.moment2, k.param, k.clear = (t.data_ptr() for t in (w, g, m, v, p, c))
+        k.n, k.param_type = n, native.BFLOAT16 if p.dtype == torch.bfloat16 else native.FLOAT32
+    if adamw:
+        native.check(L.dfcclFusedAdamWSteps(arr, len(rows), 0.01, 0.9, 0.99, 1e-8, 0.1, 2, st), "all")
+    else:
+        native.check(L.dfcclFusedSgdSteps(arr, len(rows), 0.1, 0.9, 0.01, 0, st), "all")
+    for (n, w, g, m, v, p, c), ref in zip(rows, want):
+        assert all(torch.equal(x, y) for x, y in zip((w, m, v, p), ref))
+        assert bool((p[n:] == 3).all()) and bool((c[:n] == 0).all()) and bool((c[n:] == 5).all())
