@@ -278,10 +278,12 @@ DF_HD void reduceTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t 
   }
   for (int d = 0; d < ndst; ++d) {
     char* o = a->dst[d] + dstOff + p0 * OUTB;
+    const bool wide = OUTB == 32 && ((uintptr_t)o & 31) == 0;      // the same for every thread of the block
 #pragma unroll
     for (int u = 0; u < U; ++u) if (FULL || p0 + (uint64_t)u * stride < nPacks) {
       char* ou = o + (uint64_t)u * stride * OUTB;
       if (OUTB == 8) st8(ou, make_uint2(ow[u][0].x, ow[u][0].y));
+      else if (OUTB == 32) st32(ou, ow[u][0], ow[u][NW - 1], wide);
       else {
 #pragma unroll
         for (int w = 0; w < OUTB / 16; ++w) st16(ou + 16 * w, ow[u][w]);

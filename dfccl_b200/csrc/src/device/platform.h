@@ -271,6 +271,19 @@ DF_HD void st16(void* p, uint4 v) {
   __builtin_memcpy(p, &v, 16);
 #endif
 }
+// 32 consecutive bytes from one thread: a whole sector in one access where the address allows it (`wide`: 32-byte aligned).
+// Two 16-byte stores leave every store instruction of the warp with half sectors 32 bytes apart.
+DF_HD void st32(void* p, uint4 a, uint4 b, bool wide) {
+#if DF_DEVICE_CODE
+  if (wide) {
+    asm volatile("st.relaxed.sys.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+    return;
+  }
+#endif
+  st16(p, a);
+  st16((char*)p + 16, b);
+}
 // two words whose tags the reader checks: each is read as a whole
 DF_HD void ld_relaxed_sys_2u64(const volatile uint64_t* p, uint64_t* a, uint64_t* b) {
 #if DF_DEVICE_CODE

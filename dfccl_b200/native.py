@@ -27,6 +27,7 @@ FAULT_NONE, FAULT_DROP_SQE, FAULT_DELAY_SQE_US, FAULT_FREEZE_POLLER = range(4)
 DTYPE_SIZE = {INT8: 1, UINT8: 1, INT32: 4, UINT32: 4, INT64: 8, UINT64: 8, FLOAT16: 2, FLOAT32: 4, FLOAT64: 8, BFLOAT16: 2}
 
 CALLBACK = C.CFUNCTYPE(C.c_int, C.c_int, C.c_void_p)
+NO_CALLBACK = CALLBACK(0)
 
 
 class UniqueId(C.Structure):
@@ -400,18 +401,21 @@ class RankCtx:
         check(lib().ofcclFinalizeRankCtx7StartHostThrds(self.handle), "ofcclFinalizeRankCtx7StartHostThrds")
 
     def run(self, coll_id: int, send: int, recv: int, callback: Optional[Callable[[int], None]] = None) -> None:
-        cb = CALLBACK(0)
+        cb = NO_CALLBACK
         if callback is not None:
             def tramp(cid, _args, _f=callback):
                 _f(cid)
                 return 0
             cb = CALLBACK(tramp)
             self._callbacks[coll_id] = cb          # keep the trampoline alive until the next submit of this id
-        check(lib().dfcclRun(C.c_void_p(send), C.c_void_p(recv), coll_id, cb, None, self.handle), f"dfcclRun({coll_id})")
+        r = _lib.dfcclRun(send, recv, coll_id, cb, None, self.handle)
+        if r != SUCCESS:
+            raise DfcclError(r, f"dfcclRun({coll_id})")
 
     def run_on_stream(self, coll_id: int, send: int, recv: int, stream: int) -> None:
-        check(lib().dfcclRunOnStream(C.c_void_p(send), C.c_void_p(recv), coll_id, C.c_void_p(stream), CALLBACK(0), None,
-                                     self.handle), f"dfcclRunOnStream({coll_id})")
+        r = _lib.dfcclRunOnStream(send, recv, coll_id, stream, NO_CALLBACK, None, self.handle)
+        if r != SUCCESS:
+            raise DfcclError(r, f"dfcclRunOnStream({coll_id})")
 
     def run_deferred(self, coll_id: int, send: int, recv: int) -> None:
         """Publish a submission that ``trigger_on_stream`` (or the replay of a graph that captured it) releases."""
@@ -422,7 +426,9 @@ class RankCtx:
         check(lib().dfcclTriggerOnStream(coll_id, C.c_void_p(stream), self.handle), f"dfcclTriggerOnStream({coll_id})")
 
     def stream_wait(self, coll_id: int, stream: int) -> None:
-        check(lib().dfcclStreamWait(coll_id, C.c_void_p(stream), self.handle), f"dfcclStreamWait({coll_id})")
+        r = _lib.dfcclStreamWait(coll_id, stream, self.handle)
+        if r != SUCCESS:
+            raise DfcclError(r, f"dfcclStreamWait({coll_id})")
 
     def wait(self, coll_id: int, timeout_ms: int = -1) -> int:
         return lib().dfcclWait(coll_id, timeout_ms, self.handle)
