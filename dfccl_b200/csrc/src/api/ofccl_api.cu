@@ -423,6 +423,7 @@ DF_API ncclResult_t ofcclFinalizeRankCtx7StartHostThrds(ofcclRankCtx_t ctx) {
       }
     }
     e.cs.algo = ch.algo; e.cs.nBlocks = ch.nBlocks;
+    e.cs.oneDevice = e.comm->loop && e.comm->backend == dfcclBackendCuda && !e.comm->shmMode && !e.comm->netMode && ch.algo != dfcclAlgoNvls ? 1 : 0;
     // collectives too small for every block start at different blocks, so that their fixed costs (flag round trips,
     // completion) spread over the daemon instead of queueing on its first blocks
     e.cs.blockBase = ch.nBlocks < ctx->nBlocks ? (int32_t)((((uint32_t)kv.first * 0x9E3779B1u) >> 16) % (uint32_t)ctx->nBlocks) : 0;

@@ -223,6 +223,14 @@ DF_HD void loadPacks(uint4* out, const char* s, uint32_t strideB, uint32_t shift
   }
 }
 
+// First loose element of thread `tid`: the warps that the last, partly filled trip over `nPacks` leaves idle come first, so
+// that the ragged end is on its way while that trip still waits for memory.
+DF_HD uint64_t looseStart(int tid, int nt, uint64_t nPacks) {
+  int used = (int)(nPacks % (uint64_t)nt + 31) & ~31;
+  if (used >= nt) used = 0;
+  return (uint64_t)(tid >= used ? tid - used : tid + nt - used);
+}
+
 // One noinline body per (input type, output type, operator): the daemon's register
 // budget is the maximum over what it inlines, so the variants stay out of line.
 // The hot loop is written for instruction count (it was issue-bound at 150 warp instructions
@@ -241,6 +249,24 @@ DF_HD void reduceTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t 
   const uint64_t off = srcOff + p0 * 16;
   A acc[U][V];
   uint4 cur[U], nxt[U];
+  if (U == 1) {
+    // a small call is one such trip: four sources at a time, or it would wait for memory once per source (509 bf16 of four
+    // ranks: 8.5 us from the arrival to the end of the sum, a round trip each and another four for the ragged end)
+    for (int j0 = 0; j0 < nsrc; j0 += 4) {
+      uint4 in[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) if (j0 + q < nsrc) loadPacks<FULL, SHIFT, 1>(&in[q], a->src[j0 + q] + off, strideB, shift, p0, stride, nPacks);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (j0 + q >= nsrc) break;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const A e = (A)Lane<Tin>::get(in[q], k);
+          acc[0][k] = j0 + q == 0 ? e : red<OP>(acc[0][k], e);
+        }
+      }
+    }
+  } else {
   loadPacks<FULL, SHIFT, U>(cur, a->src[0] + off, strideB, shift, p0, stride, nPacks);
   for (int j = 1; j <= nsrc; ++j) {
     if (j < nsrc) loadPacks<FULL, SHIFT, U>(nxt, a->src[j] + off, strideB, shift, p0, stride, nPacks);
@@ -256,6 +282,7 @@ DF_HD void reduceTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t 
 #pragma unroll
       for (int u = 0; u < U; ++u) cur[u] = nxt[u];
     }
+  }
   }
   uint4 ow[U][NW];
 #pragma unroll
@@ -344,10 +371,19 @@ DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   }
   // the head, the ragged tail, or everything when the pointers do not line up: element by element
   const uint64_t tail0 = head + nPacks * V;
-  for (uint64_t i = tid; i < head + (n - tail0); i += nt) {
+  for (uint64_t i = looseStart(tid, nt, nPacks); i < head + (n - tail0); i += nt) {
     const uint64_t e = i < head ? i : tail0 + (i - head);
-    A acc = Elem<Tin>::up(ld_elem((const Tin*)a->src[0] + e));
-    for (int j = 1; j < nsrc; ++j) acc = red<OP>(acc, Elem<Tin>::up(ld_elem((const Tin*)a->src[j] + e)));
+    A acc = A();
+    for (int j0 = 0; j0 < nsrc; j0 += 4) {
+      Tin in[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) if (j0 + q < nsrc) in[q] = ld_elem((const Tin*)a->src[j0 + q] + e);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (j0 + q >= nsrc) break;
+        acc = j0 + q == 0 ? Elem<Tin>::up(in[q]) : red<OP>(acc, Elem<Tin>::up(in[q]));
+      }
+    }
     Tout o = Elem<Tout>::down(finish<Tin, Tout>(acc, scale, postDiv));
     for (int d = 0; d < ndst; ++d) st_elem((Tout*)a->dst[d] + e, o);
   }
@@ -396,7 +432,7 @@ __host__ __device__ void copy_multi(const DataArgs* a) {
     else copyTrips<true>(a, nPacks, ndst, head, shift);
   }
   const uint64_t tail0 = head + nPacks * 16;
-  for (uint64_t i = tid; i < head + (nbytes - tail0); i += nt) {
+  for (uint64_t i = looseStart(tid, nt, nPacks); i < head + (nbytes - tail0); i += nt) {
     const uint64_t e = i < head ? i : tail0 + (i - head);
     uint8_t b = ld_elem((const uint8_t*)a->src[0] + e);
     for (int d = 0; d < ndst; ++d) st_elem((uint8_t*)a->dst[d] + e, b);

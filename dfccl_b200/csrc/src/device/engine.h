@@ -88,6 +88,11 @@ DF_HD bool sqPeek(const RankDev* rd, uint64_t index, SqSlot* out) {
   return (out->w[0] >> 57) == tag && (out->w[1] >> 57) == tag && (out->w[2] >> 57) == tag && (out->w[3] >> 57) == tag;
 }
 
+// Orders this rank's accesses with those of the members it exchanges flags with.
+DF_HD void fence_members(const CollStatic* c) {
+  if (c->oneDevice) fence_gpu(); else fence_sys();
+}
+
 DF_HD uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 
 DF_HD bool abortRequested(const RankDev* rd) {
@@ -204,7 +209,7 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
     }
     // polls are relaxed loads (an acquire at system scope per poll costs a fence each time); the one
     // fence that orders the payload accesses after the flags is paid when the wait succeeds
-    if (ok && lane == 0) fence_sys();
+    if (ok && lane == 0) { if (which == 2) fence_sys(); else fence_members(&sh->cs); }
     if (lane == 0) { sh->waitOk = ok ? 1 : 0; sh->waitSpins = spins; sh->stats.waitPolls += spins; }
   }
   df_sync();
@@ -669,7 +674,7 @@ DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget
         if ((sh->dyn.sqeFlags & SQE_SEND_STAGED) && !rawSend(&sh->cs)) {
           bool needed = !(sh->cs.kind == dfcclCollBroadcast && me != sh->cs.root);
           if (needed) stageCopy(sh, rb, true);
-          if (tid == 0) fence_sys();
+          if (tid == 0) fence_members(&sh->cs);
         }
         setPhase(sh, nextPhase(sh, PH_POST_ARRIVE));
         break;
@@ -677,7 +682,7 @@ DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget
         if (sh->cs.algo == dfcclAlgoPush && n > 1) {
           // the payload travels with the arrival flag: stores to a peer, one fence, then the flag
           pushOut(sh, rb);
-          if (tid == 0) fence_sys();
+          if (tid == 0) fence_members(&sh->cs);
           df_sync();
         }
         const uint64_t so = mySendOff(sh), ro = myRecvOff(sh), epoch = sh->dyn.epoch;
@@ -691,7 +696,7 @@ DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget
           if (pushed) { st_relaxed_sys_u64(&s->arrive, epoch); continue; }
           st_relaxed_sys_u64(&s->sendOff, so);
           st_relaxed_sys_u64(&s->recvOff, ro);
-          st_release_sys_u64(&s->arrive, epoch);
+          if (sh->cs.oneDevice) st_release_gpu_u64(&s->arrive, epoch); else st_release_sys_u64(&s->arrive, epoch);
         }
         setPhase(sh, PH_WAIT_ARRIVE);
         break;
@@ -725,10 +730,10 @@ DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget
       case PH_POST_DONE: {
         if (n > 1) {
           // all payload stores of this block were issued before the barrier inside setPhase; one fence
-          // by the posting thread makes them visible system-wide before any done flag is
+          // by the posting thread makes them visible to the members before any done flag is
           const uint64_t epoch = sh->dyn.epoch;
           if (tid == 0) {
-            fence_sys();
+            fence_members(&sh->cs);
             for (int j = 0; j < n; ++j)
               if (j != me) st_relaxed_sys_u64(&(sh->cs.peerFlags[j] + (uint64_t)rb * n + me)->done, epoch);
           }

@@ -108,6 +108,9 @@ struct alignas(16) CollStatic {
                           // blockBase, blockBase + 1, ... (mod the daemon's block count), so that collectives too small
                           // for every block do not all land on the first blocks.  A per-rank choice: ranks meet by
                           // relative index only.
+  int32_t oneDevice;      // all members are ranks on this GPU, their heaps in its memory: what orders one member's
+                          // accesses for another is a fence of GPU scope (0.24 - 0.45 us against 1.4 - 1.8 us)
+  int32_t pad0;
   double scale;           // multiplies the reduced value (1.0 = off)
   uint64_t count;         // elements, NCCL convention of the kind
   uint64_t stagingSendOff, stagingRecvOff;      // my heap offsets of staging areas (0 = none)
