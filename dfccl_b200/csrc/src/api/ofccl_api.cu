@@ -770,10 +770,12 @@ static ncclResult_t submit(ofcclRankCtx* ctx, const void* send, void* recv, int 
     if (needSend && cs.kind == dfcclCollAllReduce && cs.algo == dfcclAlgoOneShot && send == recv && cs.nranks > 1) stageSend = true;
     bool stageRecv = !viaArena && needRecv && !heap->contains(recv, rB);
     // staging areas are created on first need; the static table on the device learns their offsets
-    bool tableDirty = false;
-    if (stageSend && e.stagingBytes[0] < sB) { if (e.stagingBytes[0]) heap->free(e.stagingOff[0]); DFCHECK(heap->alloc(sB, &e.stagingOff[0], false)); e.stagingBytes[0] = sB; e.cs.stagingSendOff = e.stagingOff[0]; tableDirty = true; }
-    if (stageRecv && e.stagingBytes[1] < rB) { if (e.stagingBytes[1]) heap->free(e.stagingOff[1]); DFCHECK(heap->alloc(rB, &e.stagingOff[1], false)); e.stagingBytes[1] = rB; e.cs.stagingRecvOff = e.stagingOff[1]; tableDirty = true; }
-    if (tableDirty) DFCHECK(devUpload(ctx->backend, &ctx->rdHost.colls[collId], &e.cs, sizeof(CollStatic)));
+    if (stageSend && e.stagingBytes[0] < sB) { if (e.stagingBytes[0]) heap->free(e.stagingOff[0]); DFCHECK(heap->alloc(sB, &e.stagingOff[0], false)); e.stagingBytes[0] = sB; e.cs.stagingSendOff = e.stagingOff[0]; e.staticDirty = true; }
+    if (stageRecv && e.stagingBytes[1] < rB) { if (e.stagingBytes[1]) heap->free(e.stagingOff[1]); DFCHECK(heap->alloc(rB, &e.stagingOff[1], false)); e.stagingBytes[1] = rB; e.cs.stagingRecvOff = e.stagingOff[1]; e.staticDirty = true; }
+    if (e.staticDirty) {
+      DFCHECK(devUpload(ctx->backend, &ctx->rdHost.colls[collId], &e.cs, sizeof(CollStatic)));
+      q.flags |= SQE_NEW_STATIC;
+    }
     if (!viaArena) {
       if (stageSend) { q.flags |= SQE_SEND_STAGED; q.send = (uint64_t)(uintptr_t)send; } else if (needSend) q.send = heap->offsetOf(send);
       if (stageRecv) { q.flags |= SQE_RECV_STAGED; q.recv = (uint64_t)(uintptr_t)recv; } else if (needRecv) q.recv = heap->offsetOf(recv);
@@ -801,6 +803,7 @@ static ncclResult_t submit(ofcclRankCtx* ctx, const void* send, void* recv, int 
       --ctx->faultDrop;
     } else {
       DFCHECK(pushSqe(ctx, q));
+      e.staticDirty = false;
     }
   }
   ctx->pollCv.notify_one();

@@ -38,6 +38,7 @@ struct CollEntry {
   uint64_t submitted = 0, completed = 0;     // guarded by ctx->mu
   uint64_t triggerSeq = 0;
   uint32_t lastStatus = 0;
+  bool staticDirty = false;                  // cs has changed since the last entry the blocks were given
   // The last submission ran as a kernel of its own on a stream (one-rank communicators, see runDirect): `direct` until
   // its completion is delivered, `directStream` (the runtime's unique id of a stream, never reused) for stream waits.
   bool direct = false, lastDirect = false;

@@ -83,7 +83,7 @@ DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b) {
     d.send = q.send; d.recv = q.recv; d.trigger = q.trigger; d.cursor = 0;
     d.epoch = q.epoch; d.sqeFlags = q.flags; d.status = ST_OK; d.stallSinceNs = 0; d.patience = 0; d.pad = 0;
     d.phase = (q.flags & SQE_TRIGGERED) ? PH_TRIGGER : PH_COPY_IN;          // runColl skips ahead to the first phase that has work
-    if (sh->loadedColl == coll && !(q.flags & SQE_TRIGGERED)) { sh->dyn = d; sh->dynDirty = 1; }      // its context is still here
+    if (sh->loadedColl == coll && !(q.flags & (SQE_TRIGGERED | SQE_NEW_STATIC))) { sh->dyn = d; sh->dynDirty = 1; }   // its context is still here
     else {
       if (sh->loadedColl == coll) { sh->loadedColl = -1; sh->dynDirty = 0; }                          // re-armed in global memory: drop the cached copy
       rd->dyn[(uint64_t)b * rd->maxColls + coll] = d;

@@ -32,6 +32,7 @@ enum SqeFlags : uint32_t {
   SQE_TRIGGERED = 2u,     // do not start before trigger[collId] >= trigger value (stream-ordered submit)
   SQE_SEND_STAGED = 4u,   // sendbuff is outside the symmetric heap: copy it into the staging area first
   SQE_RECV_STAGED = 8u,   // recvbuff is outside the heap: peers write staging, copy out at the end
+  SQE_NEW_STATIC = 16u,   // the host has changed the collective's CollStatic (new staging areas): a copy kept by a block is stale
 };
 struct Sqe {
   int32_t collId;
