@@ -152,7 +152,8 @@ DF_HD uint32_t scanParked(BlockShared* sh, RankDev* rd, int b) {
     const CollStatic* c = &rd->colls[coll];
     const int n = c->nranks, me = c->rank;
     const FlagSlot* f = c->myFlags + (uint64_t)relBlock(rd, c, b) * n;
-    const uint64_t epoch = rd->dyn[(uint64_t)b * rd->maxColls + coll].epoch;
+    // (the collective whose context is loaded may have been submitted again since that was last saved)
+    const uint64_t epoch = sh->loadedColl == coll ? sh->dyn.epoch : rd->dyn[(uint64_t)b * rd->maxColls + coll].epoch;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
       if (j == me) continue;

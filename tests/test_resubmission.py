@@ -1,5 +1,8 @@
 """A collective whose context a block still holds from its previous submission (csrc/src/device/daemon_impl.h:
 consumeSubmissions) is submitted again.  Host backend; the scheduler is the same source as the device's."""
+import threading
+import time
+
 import numpy as np
 import pytest
 
@@ -49,3 +52,42 @@ def test_resubmission_that_needs_staging_areas(host_backend, algo, then):
     for c in comms:
         c.destroy()
     assert all(n < 4096 for n in changed.values()), changed          # flag words
+
+
+@pytest.mark.parametrize("count", [1000, COUNT])          # push and read schedules: the waits differ
+def test_resubmission_that_stalls_lets_the_daemon_leave(host_backend, count):
+    """One rank submits the id again and its peer comes 0.2 s late.  Stalled on the new epoch's flags (the previous epoch's are
+    all there), the block must leave after the stall limit of 5 ms - again and again, since the work stays outstanding - and
+    the peer's blocks, which share the launch, get in with the next one: not only after the lifetime limit, which is off."""
+    nv = host_backend
+    comms = nv.Comm.init_loopback(2)
+    met = threading.Barrier(2)
+    took, quits = {}, {}
+
+    def body(r):
+        c = comms[r]
+        p, q = c.alloc(4 * count), c.alloc(4 * count)
+        ctx = nv.RankCtx(r)
+        ctx.prepare(0, c, nv.ALLREDUCE, count, nv.FLOAT32)
+        ctx.finalize()
+        host_array(p, count, np.float32)[:] = r + 1.0
+        for _ in range(2):
+            ctx.run(0, p, q)
+            assert ctx.wait(0, 30000) == nv.SUCCESS
+        met.wait()
+        before = ctx.stats()["daemonVoluntaryQuits"]
+        if r == 1:
+            time.sleep(0.2)
+        t = time.perf_counter()
+        ctx.run(0, p, q)
+        assert ctx.wait(0, 10000) == nv.SUCCESS
+        took[r] = time.perf_counter() - t
+        quits[r] = ctx.stats()["daemonVoluntaryQuits"] - before
+        assert np.all(host_array(q, count, np.float32) == 3.0)
+        ctx.destroy()
+
+    with _env(DFCCL_DAEMON_BLOCKS=1, DFCCL_IDLE_QUIT_US=1000, DFCCL_STALL_QUIT_US=5000, DFCCL_MAX_LIFETIME_MS=0):
+        run_ranks(2, body)
+    for c in comms:
+        c.destroy()
+    assert quits[0] >= 2 and took[1] < 2.0, (quits, took)
