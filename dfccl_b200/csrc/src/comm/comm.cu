@@ -324,8 +324,7 @@ ncclResult_t commCollective(ncclComm* c, int kind, const void* send, void* recv,
   if (kind == dfcclCollAllReduce || kind == dfcclCollReduce || kind == dfcclCollReduceScatter)
     DFCHECK(resolveRedOp(c, op, type, c->nranks, &devOp, &cs.scale, &cs.postDiv));
   cs.op = devOp;
-  if (c->nranks == 1 && c->backend == dfcclBackendCuda) {
-    l.unlock();
+  if (c->nranks == 1 && c->backend == dfcclBackendCuda) {      // (under the lock, like every launch here: an abort waits for it)
     int prev = 0;
     cudaGetDevice(&prev);
     if (prev != c->device) cudaSetDevice(c->device);

@@ -1,6 +1,8 @@
 """Collectives of a one-rank communicator run as one streaming kernel over the whole GPU (csrc/src/daemon/onerank.cu):
 sizes around its pack, block and grid boundaries, buffers off the 16-byte grid, every element size."""
 import ctypes as C
+import threading
+import time
 
 import pytest
 import torch
@@ -93,3 +95,45 @@ def test_registered_collective_of_one_rank_in_the_stream_and_through_the_daemon(
     assert st["sqesSubmitted"] == st["cqesDelivered"] == 6
     ctx.destroy()
     c.destroy()
+
+
+def test_abort_waits_for_a_collective_that_is_being_launched():
+    """The launch queue of a stream holds about a thousand kernels: a thread that goes on calling behind a long kernel ends up
+    waiting inside a call.  An abort by another thread returns only after that call has left the communicator."""
+    from dfccl_b200 import native as nv
+    nv.set_backend("cuda")
+    torch.cuda.set_device(0)
+    (c,) = nv.Comm.init_loopback(1, 0)
+    x, y = torch.ones(64, device="cuda"), torch.empty(64, device="cuda")
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(2_000_000_000)                       # about a second
+    state = {"inside": 0.0, "stop": False, "left": 0.0}
+
+    def caller():
+        torch.cuda.set_device(0)
+        while not state["stop"]:
+            state["inside"] = time.perf_counter()
+            assert nv.lib().ncclAllReduce(x.data_ptr(), y.data_ptr(), 64, nv.FLOAT32, nv.SUM, c.handle, s.cuda_stream) == nv.SUCCESS
+            state["inside"] = 0.0
+        state["left"] = time.perf_counter()
+
+    t = threading.Thread(target=caller)
+    t.start()
+    deadline = time.perf_counter() + 5
+    while time.perf_counter() < deadline and not (state["inside"] and time.perf_counter() - state["inside"] > 0.1):
+        time.sleep(0.001)
+    stuck = bool(state["inside"])
+    state["stop"] = True
+    if not stuck:                                              # (a deeper queue: nothing to see)
+        t.join()
+        c.destroy()
+        pytest.skip("no call came to wait for the launch queue")
+    c._live = False
+    r = nv.lib().ncclCommAbort(c.handle)
+    after = time.perf_counter()
+    t.join(30)
+    assert r == nv.SUCCESS and state["left"] and state["left"] - after < 0.05
+    torch.cuda.synchronize()
+    assert torch.equal(x, y)
