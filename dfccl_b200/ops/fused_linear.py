@@ -93,9 +93,17 @@ class _Rendezvous:
 class _Local:
     """One-rank groups: the operator is its GEMM, with an epilogue (``ops.block``)."""
 
+    def operand(self, x: torch.Tensor) -> torch.Tensor:
+        """``x`` as the GEMM reads it, [M, K] bf16: cast, and spread over the rows, as copying it into an operand does."""
+        if x.shape != (self.m, self.k):
+            x = x.reshape(self.m, self.k) if x.numel() == self.m * self.k and x.shape[-1] == self.k else x.expand(self.m, self.k)
+        return x.to(self.tp.device, torch.bfloat16).contiguous()
+
     def local(self, x: torch.Tensor, w: torch.Tensor, w_transposed: bool = False, epi: Epilogue = NO_EPILOGUE) -> torch.Tensor:
         assert self.tp.n == 1
-        x, w = x.contiguous(), w.contiguous()
+        x, w = self.operand(x), w.to(self.tp.device, torch.bfloat16).contiguous()
+        if w.shape != ((self.k, self.n_out) if w_transposed else (self.n_out, self.k)):
+            raise ValueError(f"weight of {tuple(w.shape)} for an operator of {self.n_out} outputs and {self.k} inputs")
         out = torch.empty(self.m, self.n_out, dtype=torch.bfloat16, device=self.tp.device)
         ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), raw_stream(self.tp.device)
         if self.coll_id is not None:

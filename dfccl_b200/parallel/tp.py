@@ -134,7 +134,7 @@ def _product(op, x: torch.Tensor, w: torch.Tensor, epi: Epilogue = NO_EPILOGUE, 
 def _column(layer, x_shard: torch.Tensor, weight: torch.Tensor, epi: Epilogue):
     """(y, the gathered activations: what the weight gradient needs).  The operator's own buffer is shared by every layer
     of this shape, so several ranks keep a copy of it instead of gathering a second time in the backward pass."""
-    x_shard = x_shard.contiguous()
+    x_shard = layer.op.operand(x_shard) if layer.tp.n == 1 else x_shard.contiguous()
     y = _product(layer.op, x_shard, weight, epi)
     return y, x_shard if layer.tp.n == 1 else layer.op.gathered.clone()
 
@@ -179,7 +179,7 @@ class _ColumnFusedFn(torch.autograd.Function):
 class _RowFusedFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, residual, layer):
-        x = x.contiguous()
+        x = layer.op.operand(x) if layer.tp.n == 1 else x.contiguous()
         ctx.layer, ctx.has_bias, ctx.has_residual = layer, bias is not None, residual is not None
         ctx.save_for_backward(x, weight)
         return _product(layer.op, x, weight, _bias_epilogue(bias, None if residual is None else residual.contiguous()))

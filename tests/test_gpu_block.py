@@ -135,6 +135,29 @@ def test_block_against_torch_operators(native, tokens, d, hooked):
     comm.destroy()
 
 
+@pytest.mark.parametrize("kind", ["ColumnParallelLinear", "RowParallelLinear"])
+def test_layers_take_fp32_activations(native, kind):
+    """An operator that is not registered with a context has always taken its input through a copy, which casts."""
+    from dfccl_b200.ops.fused_linear import TpGroup
+    from dfccl_b200.parallel import tp as tp_mod
+    native.set_backend("cuda")
+    (comm,) = native.Comm.init_loopback(1, 0)
+    torch.manual_seed(5)
+    w = torch.randn(512, 256, device="cuda") * 256 ** -0.5
+    layer = getattr(tp_mod, kind)(TpGroup(comm, None, torch.device("cuda", 0)), 384, w)
+    x = torch.randn(384, 256, device="cuda", requires_grad=True)
+    gy = torch.randn(384, 512, device="cuda").to(torch.bfloat16)
+    y = layer(x)
+    y.backward(gy)
+    x64, w64 = x.detach().to(torch.bfloat16).double().requires_grad_(True), layer.weight.detach().double().requires_grad_(True)
+    (x64 @ w64.t()).backward(gy.double())
+    # products of bf16 operands, summed in fp32, one rounding (the bias is zero: adding it rounds nothing)
+    for got, want in ((y, x64 @ w64.t()), (x.grad, x64.grad), (layer.weight.grad, w64.grad)):
+        assert _rel(got.detach(), want.detach()) < HALF_ULP
+    assert x.grad.dtype == torch.float32
+    comm.destroy()
+
+
 @pytest.mark.parametrize("adamw", [False, True])
 def test_one_optimizer_launch_over_many_buckets(native, adamw):
     """More buckets than a launch holds, of both parameter types and odd lengths, against one call per bucket: the same

@@ -1,0 +1,59 @@
+"""What a one-rank fused operator (ops/fused_linear.py) hands to its GEMM, which takes bare pointers: operands of the
+declared size and type whatever it was called with.  The library is a recorder here."""
+import ctypes as C
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from dfccl_b200.ops import fused_linear
+
+M, K, N = 128, 64, 256
+
+
+class Recorder:
+    """Stands for the library: notes the product's operands as the kernel would read them."""
+
+    def __init__(self):
+        self.calls = []
+
+    def dfcclGemmBf16Epilogue(self, x, w, out, m, n, k, *rest):
+        read = lambda p, rows, cols: torch.frombuffer((C.c_char * (2 * rows * cols)).from_address(p), dtype=torch.bfloat16).view(rows, cols).clone()   # noqa: E731
+        self.calls.append((read(x, m, k), read(w, n, k), rest))
+        return 0
+
+
+@pytest.fixture()
+def op(monkeypatch):
+    rec = Recorder()
+    monkeypatch.setattr(fused_linear.nv, "lib", lambda: rec)
+    monkeypatch.setattr(fused_linear, "raw_stream", lambda _d: 0)
+    o = fused_linear.AllGatherGemm.__new__(fused_linear.AllGatherGemm)
+    o.tp, o.m, o.rows, o.k, o.n_out, o.coll_id = SimpleNamespace(n=1, device=torch.device("cpu")), M, M, K, N, None
+    o.rec = rec
+    return o
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("form", ["rows", "strided", "flat", "row", "vector"])
+def test_operand_is_cast_and_spread_like_a_copy(op, dtype, form):
+    x = torch.randn(M, K).to(dtype)
+    want = x
+    if form == "strided":
+        x = x.t().contiguous().t()
+    elif form == "flat":
+        x = x.view(2, M // 2, K)
+    elif form in ("row", "vector"):
+        x = x[:1] if form == "row" else x[0]
+        want = x.expand(M, K)
+    w = torch.randn(N, K).to(dtype)
+    op.local(x, w)
+    (got_x, got_w, _), = op.rec.calls
+    assert torch.equal(got_x, want.to(torch.bfloat16)) and torch.equal(got_w, w.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("xs,ws", [((M - 1, K), (N, K)), ((M, K // 2), (N, K)), ((M // 2, 2 * K), (N, K)), ((M, K), (N - 1, K)), ((M, K), (K, N))])
+def test_operands_of_another_size_do_not_reach_the_kernel(op, xs, ws):
+    with pytest.raises((ValueError, RuntimeError)):
+        op.local(torch.zeros(xs, dtype=torch.bfloat16), torch.zeros(ws, dtype=torch.bfloat16))
+    assert not op.rec.calls
