@@ -29,6 +29,19 @@ class Epilogue:
             assert t is None or (t.dtype == torch.bfloat16 and t.is_cuda and t.is_contiguous())
         return (self.kind, _ptr(self.bias), _ptr(self.aux), _ptr(self.pre))
 
+    def args_for(self, m: int, n: int):
+        """The same for a product of [m, n]; the kernels read and write by address alone."""
+        for t, shape in ((self.bias, (n,)), (self.aux, (m, n)), (self.pre, (m, n))):
+            if t is not None and t.shape != shape:
+                raise ValueError(f"operand of {tuple(t.shape)} in the epilogue of a product of {m} x {n}")
+        return self.args()
+
+
+def epilogue_operand(t: Optional[torch.Tensor], shape, device: torch.device) -> bool:
+    """True if a bias or residual can ride in an epilogue: bf16 of just this shape, on this device, 16-byte aligned."""
+    return (t is not None and t.dtype == torch.bfloat16 and tuple(t.shape) == tuple(shape) and t.device == device
+            and (not t.is_contiguous() or t.data_ptr() % 16 == 0))
+
 
 NO_EPILOGUE = Epilogue()
 
@@ -41,7 +54,8 @@ def apply_epilogue_(product: torch.Tensor, epi: Epilogue) -> torch.Tensor:
     """In place, for products whose kernel has no epilogue."""
     assert product.dtype == torch.bfloat16 and product.dim() == 2 and product.is_contiguous()
     m, n = product.shape
-    nv.check(nv.lib().dfcclApplyEpilogue(product.data_ptr(), m, n, *epi.args(), raw_stream(product.device)), "dfcclApplyEpilogue")
+    args = epi.args_for(m, n)
+    nv.check(nv.lib().dfcclApplyEpilogue(product.data_ptr(), m, n, *args, raw_stream(product.device)), "dfcclApplyEpilogue")
     return product
 
 

@@ -105,11 +105,12 @@ class _Local:
         if w.shape != ((self.k, self.n_out) if w_transposed else (self.n_out, self.k)):
             raise ValueError(f"weight of {tuple(w.shape)} for an operator of {self.n_out} outputs and {self.k} inputs")
         out = torch.empty(self.m, self.n_out, dtype=torch.bfloat16, device=self.tp.device)
+        epilogue = epi.args_for(self.m, self.n_out)
         ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), raw_stream(self.tp.device)
         if self.coll_id is not None:
-            nv.check(nv.lib().dfcclRunFusedGemmLocal(self.coll_id, *ptrs, int(w_transposed), *epi.args(), st, self.tp.ctx.handle), "dfcclRunFusedGemmLocal")
+            nv.check(nv.lib().dfcclRunFusedGemmLocal(self.coll_id, *ptrs, int(w_transposed), *epilogue, st, self.tp.ctx.handle), "dfcclRunFusedGemmLocal")
         else:
-            nv.check(nv.lib().dfcclGemmBf16Epilogue(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epi.args(), st), "dfcclGemmBf16Epilogue")
+            nv.check(nv.lib().dfcclGemmBf16Epilogue(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epilogue, st), "dfcclGemmBf16Epilogue")
         return out
 
 

@@ -21,7 +21,7 @@ import torch.nn as nn
 from torch.autograd.function import once_differentiable
 
 from .. import native as nv
-from ..ops.block import BIAS, BIAS_GELU, BIAS_RES, GELU_GRAD, Epilogue, NO_EPILOGUE, apply_epilogue_, column_sum, unhooked
+from ..ops.block import BIAS, BIAS_GELU, BIAS_RES, GELU_GRAD, Epilogue, NO_EPILOGUE, apply_epilogue_, column_sum, epilogue_operand, unhooked
 from ..ops.fused_linear import AllGatherGemm, GemmReduceScatter, TpGroup
 from ..utils.tensors import nccl_dtype, raw_stream
 
@@ -218,14 +218,20 @@ class _MlpFn(torch.autograd.Function):
 
 
 def _fused_bias(layer, x: torch.Tensor) -> bool:
-    """The epilogues take bf16 activations, weights and biases."""
-    return x.dtype == layer.weight.dtype == layer.bias.dtype == torch.bfloat16
+    """The epilogues take bf16 activations and weights, and one bias per output feature."""
+    return (x.dtype == layer.weight.dtype == torch.bfloat16 and layer.bias.is_contiguous()
+            and epilogue_operand(layer.bias, (layer.op.n_out,), layer.weight.device))
+
+
+def _fused_residual(layer, residual: torch.Tensor) -> bool:
+    """And a residual of the output's own shape; anything that has to be cast or spread is added by torch."""
+    return epilogue_operand(residual, (layer.op.rows, layer.op.n_out), layer.weight.device)
 
 
 def gelu_mlp(up: "ColumnParallelLinear", down: "RowParallelLinear", x: torch.Tensor, residual: torch.Tensor) -> torch.Tensor:
     """``residual + down(gelu(up(x)))`` with the tanh form of GELU."""
     if (up.op is not None and down.op is not None and unhooked(up, ColumnParallelLinear) and unhooked(down, RowParallelLinear)
-            and _fused_bias(up, x) and _fused_bias(down, residual)):
+            and _fused_bias(up, x) and _fused_bias(down, x) and _fused_residual(down, residual)):
         return _MlpFn.apply(x, up.weight, up.bias, down.weight, down.bias, residual, up, down)
     return residual + down(nn.functional.gelu(up(x), approximate="tanh"))
 
@@ -274,7 +280,7 @@ class RowParallelLinear(nn.Module):
 
     def forward(self, x, residual=None):
         """``residual`` (sharded like the output) is added in the same pass as the bias."""
-        if self.op is not None and _fused_bias(self, x) and (residual is None or residual.dtype == torch.bfloat16):
+        if self.op is not None and _fused_bias(self, x) and (residual is None or _fused_residual(self, residual)):
             return _RowFusedFn.apply(x, self.weight, self.bias, residual, self)
         y = (_RowFn.apply(x, self.weight, self) if self.op is None else _RowFusedFn.apply(x, self.weight, None, None, self)) + self.bias
         return y if residual is None else residual + y

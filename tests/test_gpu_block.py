@@ -158,6 +158,34 @@ def test_layers_take_fp32_activations(native, kind):
     comm.destroy()
 
 
+@pytest.mark.parametrize("residual", ["same", "strided", "row", "vector", "column", "misaligned", "fp32"])
+@pytest.mark.parametrize("bias", ["full", "misaligned", "one"])
+def test_residuals_and_biases_of_any_form(native, residual, bias):
+    """What the epilogue takes as it is and what is added by torch, with gradients."""
+    from dfccl_b200.ops.fused_linear import TpGroup
+    from dfccl_b200.parallel.tp import RowParallelLinear
+    native.set_backend("cuda")
+    (comm,) = native.Comm.init_loopback(1, 0)
+    torch.manual_seed(6)
+    m, n, k = 256, 512, 256
+    rnd = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)                           # noqa: E731
+    layer = RowParallelLinear(TpGroup(comm, None, torch.device("cuda", 0)), m, torch.randn(n, k, device="cuda") * k ** -0.5)
+    layer.bias = nn.Parameter({"full": lambda: rnd(n), "misaligned": lambda: rnd(n + 1)[1:], "one": lambda: rnd(1)}[bias]())
+    r = {"same": lambda: rnd(m, n), "strided": lambda: rnd(n, m).t(), "row": lambda: rnd(1, n), "vector": lambda: rnd(n), "column": lambda: rnd(m, 1),
+         "misaligned": lambda: rnd(m * n + 1)[1:].view(m, n), "fp32": lambda: torch.randn(m, n, device="cuda")}[residual]().requires_grad_(True)
+    x, gy = rnd(m, k).requires_grad_(True), rnd(m, n)
+    y = layer(x, r)
+    y.backward(gy.to(y.dtype))
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, layer.weight, layer.bias, r)]
+    y64 = leaves[0] @ leaves[1].t() + leaves[2] + leaves[3]
+    y64.backward(gy.double())
+    # three roundings to bf16 where bias and residual are added one by one; gradients are sums rounded once
+    assert y.dtype == (r.dtype if residual == "fp32" else torch.bfloat16) and _rel(y.detach(), y64.detach()) < 3 * HALF_ULP
+    for got, want in zip((x, layer.weight, layer.bias, r), leaves):
+        assert _rel(got.grad, want.grad) < 2 * HALF_ULP
+    comm.destroy()
+
+
 @pytest.mark.parametrize("adamw", [False, True])
 def test_one_optimizer_launch_over_many_buckets(native, adamw):
     """More buckets than a launch holds, of both parameter types and odd lengths, against one call per bucket: the same

@@ -6,7 +6,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-from dfccl_b200.ops import fused_linear
+from dfccl_b200.ops import block, fused_linear
 
 M, K, N = 128, 64, 256
 
@@ -56,4 +56,25 @@ def test_operand_is_cast_and_spread_like_a_copy(op, dtype, form):
 def test_operands_of_another_size_do_not_reach_the_kernel(op, xs, ws):
     with pytest.raises((ValueError, RuntimeError)):
         op.local(torch.zeros(xs, dtype=torch.bfloat16), torch.zeros(ws, dtype=torch.bfloat16))
+    assert not op.rec.calls
+
+
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("t,ok", [(torch.zeros(M, N, dtype=BF), True), (torch.zeros(N, M, dtype=BF).t(), True), (torch.zeros(M, N), False),
+                                  (torch.zeros(1, N, dtype=BF), False), (torch.zeros(N, dtype=BF), False), (torch.zeros(M, 1, dtype=BF), False),
+                                  (torch.zeros(M + 1, N, dtype=BF), False), (torch.zeros(M * N + 1, dtype=BF)[1:].view(M, N), False), (None, False)])
+def test_which_residuals_ride_in_an_epilogue(t, ok):
+    assert block.epilogue_operand(t, (M, N), torch.device("cpu")) == ok
+
+
+@pytest.mark.parametrize("kw", [dict(bias=torch.zeros(1, dtype=BF)), dict(bias=torch.zeros(N, dtype=BF), aux=torch.zeros(1, N, dtype=BF)),
+                                dict(bias=torch.zeros(N, dtype=BF), aux=torch.zeros(M - 1, N, dtype=BF)),
+                                dict(bias=torch.zeros(N, dtype=BF), pre=torch.zeros(M, N - 8, dtype=BF))])
+def test_epilogue_operands_of_another_shape_do_not_reach_the_kernel(op, kw):
+    with pytest.raises(ValueError):
+        op.local(torch.zeros(M, K, dtype=BF), torch.zeros(N, K, dtype=BF), epi=block.Epilogue(block.BIAS_RES, **kw))
+    with pytest.raises(ValueError):
+        block.apply_epilogue_(torch.zeros(M, N, dtype=BF), block.Epilogue(block.BIAS_RES, **kw))
     assert not op.rec.calls
