@@ -137,3 +137,37 @@ def test_abort_waits_for_a_collective_that_is_being_launched():
     assert r == nv.SUCCESS and state["left"] and state["left"] - after < 0.05
     torch.cuda.synchronize()
     assert torch.equal(x, y)
+
+
+def test_a_captured_wait_orders_its_graph_behind_an_earlier_collective():
+    """The collective ran in the stream that is then captured; the graph is replayed on another one."""
+    from dfccl_b200 import native as nv
+    from dfccl_b200.utils import tensor_from_ptr
+    nv.set_backend("cuda")
+    torch.cuda.set_device(0)
+    (c,) = nv.Comm.init_loopback(1, 0)
+    n = 1 << 20
+    ctx = nv.RankCtx(0, 0)
+    ctx.prepare(0, c, nv.ALLREDUCE, n, nv.FLOAT32, scale=2.0)
+    ctx.finalize()
+    p, q = c.alloc(4 * n), c.alloc(4 * n)
+    x, y = tensor_from_ptr(p, (n,), torch.float32, "cuda:0"), tensor_from_ptr(q, (n,), torch.float32, "cuda:0")
+    seen = torch.zeros(n, device="cuda")
+    x.fill_(1.0)
+    y.zero_()
+    torch.cuda.synchronize()
+    s, other, g = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(400_000_000)                          # about 0.2 s: the capture is over and replayed before the collective
+        ctx.run_on_stream(0, p, q, s.cuda_stream)
+        g.capture_begin()
+        ctx.stream_wait(0, s.cuda_stream)
+        seen.copy_(y)
+        g.capture_end()
+    with torch.cuda.stream(other):
+        g.replay()
+    torch.cuda.synchronize()
+    assert bool((seen == 2.0).all())
+    assert ctx.wait_all(10000) == nv.SUCCESS
+    ctx.destroy()
+    c.destroy()
