@@ -946,8 +946,8 @@ DF_API ncclResult_t dfcclStreamWait(int collId, cudaStream_t stream, ofcclRankCt
     direct = e->lastDirect;
     unsigned long long id = 0;
     // it ran in this very stream: everything enqueued from here on is behind it already (what a capture records is not
-    // enqueued here, and may be replayed anywhere)
-    if (direct && cudaStreamGetId(stream, &id) == cudaSuccess && id == e->directStream && !capturing(stream)) return ncclSuccess;
+    // enqueued here, and may be replayed anywhere; asking a capturing stream for its id ends the capture)
+    if (direct && !capturing(stream) && cudaStreamGetId(stream, &id) == cudaSuccess && id == e->directStream) return ncclSuccess;
   }
   if (ctx->backend == dfcclBackendCuda && ctx->fnWait64) {
     // The stream is about to park on a word only the daemon sets.  Outside a capture, make sure an instance is

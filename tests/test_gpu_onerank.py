@@ -160,10 +160,12 @@ def test_a_captured_wait_orders_its_graph_behind_an_earlier_collective():
     with torch.cuda.stream(s):
         torch.cuda._sleep(400_000_000)                          # about 0.2 s: the capture is over and replayed before the collective
         ctx.run_on_stream(0, p, q, s.cuda_stream)
-        g.capture_begin()
-        ctx.stream_wait(0, s.cuda_stream)
-        seen.copy_(y)
-        g.capture_end()
+        g.capture_begin(capture_error_mode="thread_local")      # (the library's own threads go on calling the runtime)
+        try:
+            ctx.stream_wait(0, s.cuda_stream)
+            seen.copy_(y)
+        finally:
+            g.capture_end()
     with torch.cuda.stream(other):
         g.replay()
     torch.cuda.synchronize()
