@@ -19,6 +19,7 @@
 #include "tc_common.h"
 #include "gemm.h"
 #include "epilogue.h"
+#include "../common/device_once.h"
 #include "../common/param.h"
 #include "dfccl.h"
 #include "../common/log.h"
@@ -517,8 +518,7 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
   // K-major operand [rows, K]: boxes of [tile rows] x 64 K-columns; MN-major operand [K, cols]: boxes of 64 K-rows x 64 columns
   if (!aMn) DFCHECK(makeMap(&ma, A, (uint64_t)M, (uint64_t)K, BM)); else DFCHECK(makeMap(&ma, A, (uint64_t)K, (uint64_t)M, BK));
   if (!bMn) DFCHECK(makeMap(&mb, B, (uint64_t)N, (uint64_t)K, BN)); else DFCHECK(makeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
-  static std::once_flag once;
-  std::call_once(once, [] { cudaFuncSetAttribute(dfcclGemmKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+  CUDACHECK(oncePerDevice([] { return allowSharedMemory(dfcclGemmKernel, SMEM_BYTES); }));
   GemmArgs g;
   memset(&g, 0, sizeof(g));
   g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.ldc = N; g.err = ew.dev; g.errHost = (uint32_t*)ew.host;

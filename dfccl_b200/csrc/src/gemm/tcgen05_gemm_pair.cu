@@ -18,6 +18,7 @@
 #include "tc_common.h"
 #include "gemm.h"
 #include "epilogue.h"
+#include "../common/device_once.h"
 #include "../common/param.h"
 #include "../common/log.h"
 #include <algorithm>
@@ -241,14 +242,20 @@ PairKernel pairKernel(int epi) {
                                  dfcclGemmPairKernel<EPI_BIAS_GELU>, dfcclGemmPairKernel<EPI_GELU_GRAD>};
   return k[epi];
 }
+cudaError_t allowPairs() {
+  return oncePerDevice([] {
+    cudaError_t r = cudaSuccess;
+    for (int e = EPI_NONE; e <= EPI_GELU_GRAD && r == cudaSuccess; ++e) r = allowSharedMemory(pairKernel(e), SMEM_BYTES);
+    return r;
+  });
+}
 int maxResidentPairs(int dev, int sms) {
   // pairs that can be resident together (a GPC with an odd number of free SMs leaves one unpaired)
   static int maxPairs[64];
   static std::mutex mu;
   std::lock_guard<std::mutex> l(mu);
   if (!maxPairs[dev & 63]) {
-    static std::once_flag once;
-    std::call_once(once, [] { for (int e = EPI_NONE; e <= EPI_GELU_GRAD; ++e) cudaFuncSetAttribute(pairKernel(e), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); });
+    (void)allowPairs();                                // (the launch reports it)
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(sms & ~1); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = SMEM_BYTES;
@@ -272,6 +279,7 @@ ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N,
   CUtensorMap ma, mb;
   if (!aMn) DFCHECK(gemmMakeMap(&ma, A, (uint64_t)M, (uint64_t)K, HALF)); else DFCHECK(gemmMakeMap(&ma, A, (uint64_t)K, (uint64_t)M, BK));
   if (!bMn) DFCHECK(gemmMakeMap(&mb, B, (uint64_t)N, (uint64_t)K, HALF)); else DFCHECK(gemmMakeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
+  CUDACHECK(allowPairs());
   PairArgs g;
   memset(&g, 0, sizeof(g));
   g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.ldc = N; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0;

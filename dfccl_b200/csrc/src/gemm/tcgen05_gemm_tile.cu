@@ -19,9 +19,9 @@
 // epilogue, two warps per 32 accumulator rows.  No TMA load uses cluster multicast; every wait is bounded.
 #include "tc_common.h"
 #include "gemm.h"
+#include "../common/device_once.h"
 #include "../common/log.h"
 #include <algorithm>
-#include <mutex>
 
 namespace dfccl {
 namespace {
@@ -329,10 +329,11 @@ ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B,
   CUtensorMap ma, mb;
   DFCHECK(gemmMakeMap3(&ma, A, (uint64_t)M, (uint64_t)K, aMn, TM, BK));
   DFCHECK(gemmMakeMap3(&mb, B, (uint64_t)N, (uint64_t)K, bMn, bRows(p.pair, p.tn), BK));
-  static std::once_flag once;
-  std::call_once(once, [] {
-    for (const Form& f : FORMS) cudaFuncSetAttribute(kernelOf(f.pair, f.tn), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-  });
+  CUDACHECK(oncePerDevice([] {
+    cudaError_t r = cudaSuccess;
+    for (const Form& f : FORMS) if (r == cudaSuccess) r = allowSharedMemory(kernelOf(f.pair, f.tn), SMEM_LIMIT);
+    return r;
+  }));
   TileArgs g;
   memset(&g, 0, sizeof(g));
   g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0;

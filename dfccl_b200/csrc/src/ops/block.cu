@@ -7,8 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
-#include <mutex>
 #include "dfccl.h"
+#include "../common/device_once.h"
 #include "../gemm/epilogue.h"
 #include "../gemm/gemm.h"
 
@@ -257,13 +257,15 @@ int lnBlocks(int rows, int sms) { return std::max(1, std::min((rows + 7) / 8, sm
 int sumStretches(int rows, int n, int sms) { return std::max(1, std::min(4 * sms / ((n + 255) / 256), rows / 32)); }
 
 template <int NV>
-void lnBackward(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* pass, void* gx, float* work,
+cudaError_t lnBackward(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* pass, void* gx, float* work,
                 int rows, int d, int blocks, cudaStream_t stream) {
   const int smem = 8 * 2 * d * (int)sizeof(float);
-  static std::once_flag once;                            // (up to 128 KB for the widest rows)
-  std::call_once(once, [] { cudaFuncSetAttribute(lnBackwardKernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 2 * 256 * NV * (int)sizeof(float)); });
+  // (up to 128 KB for the widest rows)
+  const cudaError_t e = oncePerDevice([] { return allowSharedMemory(lnBackwardKernel<NV>, 8 * 2 * 256 * NV * (int)sizeof(float)); });
+  if (e != cudaSuccess) return e;
   lnBackwardKernel<NV><<<blocks, 256, smem, stream>>>((const __nv_bfloat16*)gy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gamma,
                                                                        mean, rstd, (const __nv_bfloat16*)pass, (__nv_bfloat16*)gx, work, rows, d);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -314,7 +316,7 @@ DF_API ncclResult_t dfcclLayerNormBackward(const void* gy, const void* x, const 
   if (!aligned(gy, x, gamma, pass, gx)) return ncclInvalidArgument;
   const int blocks = lnBlocks(rows, smCount());
   auto* fn = d <= 256 ? lnBackward<1> : d <= 512 ? lnBackward<2> : d <= 1024 ? lnBackward<4> : lnBackward<8>;
-  fn(gy, x, gamma, (const float*)mean, (const float*)rstd, pass, gx, (float*)work, rows, d, blocks, stream);
+  if (fn(gy, x, gamma, (const float*)mean, (const float*)rstd, pass, gx, (float*)work, rows, d, blocks, stream) != cudaSuccess) return ncclUnhandledCudaError;
   sumLinesKernel<<<(2 * d + 31) / 32, 1024, 0, stream>>>((const float*)work, blocks, 2 * d, (__nv_bfloat16*)ggamma, (__nv_bfloat16*)gbeta, d);
   return launched();
 }
@@ -324,6 +326,7 @@ DF_API ncclResult_t dfcclColumnSum(const void* g, void* out, void* work, int row
   if (rows <= 0 || n <= 0 || n % 8 || !g || !out || !work || !aligned(g)) return ncclInvalidArgument;
   const int stretches = sumStretches(rows, n, smCount());
   columnSumKernel<<<dim3((n + 255) / 256, stretches), 256, 0, stream>>>((const __nv_bfloat16*)g, (float*)work, rows, n);
+  if (cudaGetLastError() != cudaSuccess) return ncclUnhandledCudaError;
   sumLinesKernel<<<(n + 31) / 32, 1024, 0, stream>>>((const float*)work, stretches, n, (__nv_bfloat16*)out, (__nv_bfloat16*)out, n);
   return launched();
 }

@@ -186,6 +186,22 @@ def test_residuals_and_biases_of_any_form(native, residual, bias):
     comm.destroy()
 
 
+@pytest.mark.multigpu
+def test_a_second_device_of_the_process(native):
+    """Shared-memory limits are set on every device a kernel is launched on: widths above 768 (layer norm backward), tile
+    forms and the persistent kernel, on device 1 after device 0."""
+    from dfccl_b200.ops import block, gemm
+    for dev in (0, 1):
+        with torch.cuda.device(dev):
+            ln = nn.LayerNorm(1024, dtype=torch.bfloat16, device=f"cuda:{dev}")
+            x = torch.randn(512, 1024, device=f"cuda:{dev}").to(torch.bfloat16).requires_grad_(True)
+            block.norm_residual(ln, x)[1].sum().backward()
+            assert bool(torch.isfinite(x.grad).all())
+            for m in (128, 8192):
+                a = torch.ones(m, 1024, device=f"cuda:{dev}", dtype=torch.bfloat16)
+                assert bool((gemm.matmul_nt(a, torch.ones_like(a[0]).expand(1024, 1024).contiguous()) == 1024).all())
+
+
 @pytest.mark.parametrize("adamw", [False, True])
 def test_one_optimizer_launch_over_many_buckets(native, adamw):
     """More buckets than a launch holds, of both parameter types and odd lengths, against one call per bucket: the same
