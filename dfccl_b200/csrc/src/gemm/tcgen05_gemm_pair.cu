@@ -70,7 +70,9 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&fullBar[s], 1); mbar_init(&emptyBar[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&accFull[a], 1); mbar_init(&accEmpty[a], 2 * EPI_WARPS); }
-    *giveUp = *(volatile uint32_t*)g.err;            // an earlier kernel gave up: do nothing (both CTAs read the same word)
+    // (not the device's error word: read here, beside the kernel in front, it could differ between the two CTAs, and one would
+    // wait for a partner that does nothing.  After a kernel has given up the host refuses launches.)
+    *giveUp = 0;
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
     tma_prefetch_desc(&mapB);
@@ -81,12 +83,10 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   cluster_sync_all();                                // the partner's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmemBase = *tmemBaseSlot;
-  const bool dead = *giveUp != 0;
   grid_dependency_wait();                            // everything above may run beside the kernel in front of this one
   grid_launch_dependents();
 
-  if (dead) {
-  } else if (warp == 0) {
+  if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs; bytes counted in the leader)
     if (elect_one()) {
       int stage = 0;
@@ -230,7 +230,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   cluster_sync_all();
   tc_fence_after();
   if (warp == 1) tmem_dealloc_pair(tmemBase, TMEM_COLS);
-  if (threadIdx.x == 0 && *giveUp && !dead) { atomicExch(g.err, 1u); *(volatile uint32_t*)g.errHost = 1u; __threadfence_system(); }
+  if (threadIdx.x == 0 && *giveUp) { atomicExch(g.err, 1u); *(volatile uint32_t*)g.errHost = 1u; __threadfence_system(); }
 }
 
 }  // namespace
