@@ -39,7 +39,7 @@ DF_HD void serviceMain(BlockShared* sh, RankDev* rd) {
     const uint32_t bad = ~__ballot_sync(0xffffffffu, (w >> 57) == sqTag(index, cap));
     const int whole = (bad ? __ffs(bad) - 1 : 32) >> 2;          // entries from `head` on of which every word is there
     if (whole == 0) {
-      if (sh->svcStop) break;
+      if (__any_sync(0xffffffffu, sh->svcStop != 0)) break;        // one decision for the warp: the lanes meet in the vote above
       continue;
     }
     // (no fence: the words say everything themselves, and what the addresses in them point to was complete before the
