@@ -194,6 +194,14 @@ DF_HD void fence_sys() {
   __atomic_thread_fence(__ATOMIC_SEQ_CST);
 #endif
 }
+// what this thread has read, before what it writes
+DF_HD void fence_acq_rel_sys() {
+#if DF_DEVICE_CODE
+  asm volatile("fence.acq_rel.sys;" ::: "memory");
+#else
+  __atomic_thread_fence(__ATOMIC_ACQ_REL);
+#endif
+}
 DF_HD void fence_gpu() {
 #if DF_DEVICE_CODE
   __threadfence();
