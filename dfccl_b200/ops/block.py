@@ -10,7 +10,7 @@ import torch.nn as nn
 from torch.autograd.function import once_differentiable
 
 from .. import native as nv
-from ..utils.tensors import raw_stream
+from ..utils.tensors import on_device, raw_stream
 
 NONE, BIAS, BIAS_RES, BIAS_GELU, GELU_GRAD = range(5)
 
@@ -55,16 +55,18 @@ def apply_epilogue_(product: torch.Tensor, epi: Epilogue) -> torch.Tensor:
     assert product.dtype == torch.bfloat16 and product.dim() == 2 and product.is_contiguous()
     m, n = product.shape
     args = epi.args_for(m, n)
-    nv.check(nv.lib().dfcclApplyEpilogue(product.data_ptr(), m, n, *args, raw_stream(product.device)), "dfcclApplyEpilogue")
+    with on_device(product.device):
+        nv.check(nv.lib().dfcclApplyEpilogue(product.data_ptr(), m, n, *args, raw_stream(product.device)), "dfcclApplyEpilogue")
     return product
 
 
 def column_sum(g: torch.Tensor) -> torch.Tensor:
     """Sum over the rows of a contiguous bf16 matrix, in fp32, rounded once."""
     rows, n = g.shape
-    work = torch.empty(nv.lib().dfcclColumnSumWork(rows, n), dtype=torch.float32, device=g.device)
     out = torch.empty(n, dtype=torch.bfloat16, device=g.device)
-    nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), work.data_ptr(), rows, n, raw_stream(g.device)), "dfcclColumnSum")
+    with on_device(g.device):
+        work = torch.empty(nv.lib().dfcclColumnSumWork(rows, n), dtype=torch.float32, device=g.device)
+        nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), work.data_ptr(), rows, n, raw_stream(g.device)), "dfcclColumnSum")
     return out
 
 
@@ -77,8 +79,9 @@ class _NormFn(torch.autograd.Function):
         rows, d = x.shape
         y = torch.empty_like(x)
         stats = torch.empty(2, rows, dtype=torch.float32, device=x.device)
-        nv.check(nv.lib().dfcclLayerNormForward(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), stats.data_ptr(), stats[1].data_ptr(),
-                                                rows, d, eps, raw_stream(x.device)), "dfcclLayerNormForward")
+        with on_device(x.device):
+            nv.check(nv.lib().dfcclLayerNormForward(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), stats.data_ptr(), stats[1].data_ptr(),
+                                                    rows, d, eps, raw_stream(x.device)), "dfcclLayerNormForward")
         ctx.save_for_backward(x, gamma, stats)
         ctx.set_materialize_grads(False)
         return x, y
@@ -93,10 +96,11 @@ class _NormFn(torch.autograd.Function):
         gy = gy.contiguous()
         gpass = None if gpass is None else gpass.contiguous()
         gx, gg, gb = torch.empty_like(x), torch.empty_like(gamma), torch.empty_like(gamma)
-        work = torch.empty(nv.lib().dfcclLayerNormWork(rows, d), dtype=torch.float32, device=x.device)
-        nv.check(nv.lib().dfcclLayerNormBackward(gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), stats.data_ptr(), stats[1].data_ptr(), _ptr(gpass),
-                                                 gx.data_ptr(), gg.data_ptr(), gb.data_ptr(), work.data_ptr(), rows, d, raw_stream(x.device)),
-                 "dfcclLayerNormBackward")
+        with on_device(x.device):
+            work = torch.empty(nv.lib().dfcclLayerNormWork(rows, d), dtype=torch.float32, device=x.device)
+            nv.check(nv.lib().dfcclLayerNormBackward(gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), stats.data_ptr(), stats[1].data_ptr(), _ptr(gpass),
+                                                     gx.data_ptr(), gg.data_ptr(), gb.data_ptr(), work.data_ptr(), rows, d, raw_stream(x.device)),
+                     "dfcclLayerNormBackward")
         return gx, gg, gb, None
 
 

@@ -1,6 +1,7 @@
 """Views of symmetric-heap memory as torch tensors (no copy, no ownership)."""
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from typing import Sequence
 
@@ -27,6 +28,15 @@ def raw_stream(device: torch.device) -> int:
     a Stream object for every launch (2.2 us of host time)."""
     index = device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+_HERE = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """Makes ``device`` the current one for a launch on its stream, where it is not already (a launch on another device's
+    stream is refused by the runtime)."""
+    return _HERE if device.index is None or device.index == torch.cuda.current_device() else torch.cuda.device(device.index)
 
 
 class _CudaBlob:

@@ -202,6 +202,21 @@ def test_a_second_device_of_the_process(native):
                 assert bool((gemm.matmul_nt(a, torch.ones_like(a[0]).expand(1024, 1024).contiguous()) == 1024).all())
 
 
+@pytest.mark.multigpu
+def test_tensors_of_a_device_that_is_not_current(native):
+    from dfccl_b200.ops import block
+    with torch.cuda.device(0):
+        ln = nn.LayerNorm(256, dtype=torch.bfloat16, device="cuda:1")
+        x = torch.randn(64, 256, device="cuda:1").to(torch.bfloat16).requires_grad_(True)
+        h, y = block.norm_residual(ln, x)
+        (h + y).float().square().sum().backward()
+        assert bool(torch.isfinite(x.grad).all())
+        assert _rel(block.column_sum(x.detach()), x.detach().double().sum(0)) < HALF_ULP
+        block.apply_epilogue_(torch.zeros_like(x.detach()), block.Epilogue(block.BIAS, ln.weight.detach()))
+        torch.cuda.synchronize(1)
+        assert torch.cuda.current_device() == 0
+
+
 @pytest.mark.parametrize("adamw", [False, True])
 def test_one_optimizer_launch_over_many_buckets(native, adamw):
     """More buckets than a launch holds, of both parameter types and odd lengths, against one call per bucket: the same

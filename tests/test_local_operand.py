@@ -78,3 +78,12 @@ def test_epilogue_operands_of_another_shape_do_not_reach_the_kernel(op, kw):
     with pytest.raises(ValueError):
         block.apply_epilogue_(torch.zeros(M, N, dtype=BF), block.Epilogue(block.BIAS_RES, **kw))
     assert not op.rec.calls
+
+
+def test_launches_on_a_device_that_is_not_current(monkeypatch):
+    import contextlib
+    from dfccl_b200.utils.tensors import on_device
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    assert isinstance(on_device(torch.device("cuda", 1)), torch.cuda.device)
+    assert isinstance(on_device(torch.device("cuda", 0)), contextlib.nullcontext)
+    assert isinstance(on_device(torch.device("cuda")), contextlib.nullcontext)
