@@ -205,7 +205,8 @@ ncclResult_t dfcclNvlsAlloc(void** ptr, size_t bytes, ncclComm_t comm);
 ncclResult_t dfcclNvlsInfo(ncclComm_t comm, void** unicastBase, void** multicastBase, size_t* bytes, size_t* used);
 
 ncclResult_t dfcclInitRankCtxOnDevice(ofcclRankCtx_t* rankCtx, int rank, int device);
-/* Daemon grid of this context: thread blocks per rank and threads per block (multiple of 32, <= 512);
+/* Daemon grid of this context: thread blocks per rank and working threads per block (multiple of 32, <= 512, of which
+ * 480 at most are used: a warp of the block serves the submission ring);
  * 0 keeps the default (DFCCL_DAEMON_BLOCKS / DFCCL_DAEMON_THREADS).  Call before finalizing.  All ranks
  * of a collective must use the same number of blocks. */
 ncclResult_t dfcclSetDaemonGeometry(ofcclRankCtx_t rankCtx, int blocks, int threads);

@@ -31,8 +31,10 @@ namespace dfccl {
 // schedulers, which cuts the register limit from 128 to 96 a thread.)
 #define DF_SERVICE_THREADS 32
 #define DF_BLOCK_THREADS 512
-inline int df_block_threads(int threads) {          // of a block that is asked for `threads`
-  return threads + DF_SERVICE_THREADS < DF_BLOCK_THREADS ? threads + DF_SERVICE_THREADS : DF_BLOCK_THREADS;
+// Of a block that is asked for `threads` working ones: whole warps, since the working threads' barrier counts by warps.
+inline int df_block_threads(int threads) {
+  const int whole = (threads > 32 ? (threads + 31) / 32 * 32 : 32) + DF_SERVICE_THREADS;
+  return whole < DF_BLOCK_THREADS ? whole : DF_BLOCK_THREADS;
 }
 
 DF_HD int df_tid() {
@@ -68,7 +70,7 @@ DF_HD void df_sync() {
   asm volatile("bar.sync 1, %0;" ::"r"(df_nthreads()) : "memory");
 #endif
 }
-// the service warp and the working threads meet (once, when the block leaves)
+// the service warp and the working threads meet (when the block starts, and when the warp has stopped)
 DF_HD void df_sync_service() {
 #if DF_DEVICE_CODE
   asm volatile("bar.sync 2, %0;" ::"r"(blockDim.x) : "memory");
