@@ -664,7 +664,7 @@ static ncclResult_t runDirect(ofcclRankCtx* ctx, CollEntry& e, int collId, const
   ctx->outside++;
   ctx->remaining++;
   ctx->sqes++;
-  const OneRankDone done{ctx->rdDev, collId, (uint32_t)e.submitted};
+  const OneRankDone done{ctx->rdDev, collId, (uint32_t)e.submitted, ctx->rdHost.trace != nullptr};
   l.unlock();
   int prev = 0;
   cudaGetDevice(&prev);
@@ -676,6 +676,9 @@ static ncclResult_t runDirect(ofcclRankCtx* ctx, CollEntry& e, int collId, const
     e.submitted--;
     e.direct = e.lastDirect = false;
     ctx->remaining--; ctx->outside--; ctx->sqes--;
+  } else {                                   // counted like the daemon's data phases: one source, or one destination elsewhere
+    const bool reduces = e.cs.kind == dfcclCollAllReduce || e.cs.kind == dfcclCollReduce || e.cs.kind == dfcclCollReduceScatter;
+    if (reduces) ctx->directReduced += sendBytes(&e.cs); else if (send != recv) ctx->directCopied += sendBytes(&e.cs);
   }
   ctx->pollCv.notify_one();
   return r;
@@ -1013,6 +1016,7 @@ DF_API ncclResult_t dfcclGetStats(ofcclRankCtx_t ctx, dfcclStats* s) {
   memset(s, 0, sizeof(*s));
   s->sqesSubmitted = ctx->sqes; s->cqesDelivered = ctx->cqes; s->callbacksRun = ctx->cbs; s->sqFullRetries = ctx->sqFull;
   s->fusedLaunches = ctx->fusedLaunches;
+  s->bytesReduced = ctx->directReduced; s->bytesCopied = ctx->directCopied;
   if (!ctx->finalized) return ncclSuccess;
   s->daemonLaunches = ctx->ctl->launches; s->daemonVoluntaryQuits = ctx->ctl->voluntaryQuits;
   std::vector<DevStats> d(ctx->nBlocks);

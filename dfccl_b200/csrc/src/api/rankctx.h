@@ -125,6 +125,7 @@ struct ofcclRankCtx {
   int64_t checkInterval = 10000;      // CHECK_REMAINING_SQE_INTERVAL
   // stats / faults
   std::atomic<uint64_t> sqes{0}, cqes{0}, cbs{0}, sqFull{0}, fusedLaunches{0};
+  std::atomic<uint64_t> directReduced{0}, directCopied{0};     // bytes of submissions that ran as kernels of their own
   int64_t faultDrop = 0, faultDelayUs = 0, faultFreezeMs = 0;
   ncclResult_t asyncError = ncclSuccess;
   // stream memory operations (cuda backend)

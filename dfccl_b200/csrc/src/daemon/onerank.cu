@@ -42,6 +42,11 @@ __device__ __forceinline__ void oneElem(const OneRankArgs& a, uint64_t e) {
 template <typename Tin, typename Tout, bool COPY, int U>
 __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs a) {
   typedef typename Elem<Tin>::Acc A;
+  if (a.done.traced && blockIdx.x == 0 && threadIdx.x == 0) {
+    trace(a.done.rd, 0, TR_SQE, a.done.coll);
+    trace(a.done.rd, 0, TR_START, a.done.coll);
+    trace(a.done.rd, 0, TR_DATA_BEGIN, a.done.coll);
+  }
   constexpr int V = 16 / (int)sizeof(Tin);
   constexpr int OUTB = V * (int)sizeof(Tout);
   constexpr int NW = (OUTB + 15) / 16;
@@ -93,6 +98,10 @@ __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs 
       uint32_t* count = &rd->doneCount[a.done.coll];
       if (atomic_add_u32(count, 1u) + 1u != gridDim.x) return;
       *(volatile uint32_t*)count = 0u;
+    }
+    if (a.done.traced) {
+      trace(rd, 0, TR_DATA_END, a.done.coll);
+      trace(rd, 0, TR_DONE, a.done.coll);
     }
     const unsigned long long idx = atomic_add_u64((unsigned long long*)&rd->devCqTail, 1ull);
     fence_sys();

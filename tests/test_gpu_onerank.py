@@ -173,3 +173,34 @@ def test_a_captured_wait_orders_its_graph_behind_an_earlier_collective():
     assert ctx.wait_all(10000) == nv.SUCCESS
     ctx.destroy()
     c.destroy()
+
+
+@pytest.mark.parametrize("kind,reduced,copied", [("ALLREDUCE", 1, 0), ("REDUCESCATTER", 1, 0), ("ALLGATHER", 0, 1), ("BROADCAST", 0, 1)])
+def test_collectives_in_the_stream_are_counted_and_traced(kind, reduced, copied, tmp_path, monkeypatch):
+    """As the daemon's are: bytes in the statistics, the events of a collective's life in the trace."""
+    import json
+    from dfccl_b200 import native as nv
+    nv.set_backend("cuda")
+    torch.cuda.set_device(0)
+    monkeypatch.setenv("DFCCL_TRACE", "1")
+    (c,) = nv.Comm.init_loopback(1, 0)
+    n, calls = 3001, 3
+    ctx = nv.RankCtx(0, 0)
+    ctx.prepare(7, c, getattr(nv, kind), n, nv.FLOAT32)
+    ctx.finalize()
+    x, y = torch.randn(n, device="cuda"), torch.zeros(n, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    for _ in range(calls):
+        ctx.run_on_stream(7, x.data_ptr(), y.data_ptr(), s)
+        ctx.stream_wait(7, s)
+    assert ctx.wait_all(10000) == nv.SUCCESS
+    torch.cuda.synchronize()
+    assert torch.equal(x, y)
+    st = ctx.stats()
+    assert (st["bytesReduced"], st["bytesCopied"]) == (4 * n * calls * reduced, 4 * n * calls * copied)
+    assert st["deviceEvents"] >= 5 * calls
+    ctx.trace_dump(str(tmp_path / "t.json"))
+    names = [e["name"] for e in json.loads((tmp_path / "t.json").read_text())["traceEvents"] if e.get("args", {}).get("coll", 7) == 7]
+    assert (names.count("sqe"), names.count("data"), names.count("done")) == (calls, 2 * calls, calls), names      # data: begin and end
+    ctx.destroy()
+    c.destroy()
