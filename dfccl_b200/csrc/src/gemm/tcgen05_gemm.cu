@@ -124,7 +124,6 @@ __device__ __forceinline__ bool wait_flag32(const uint32_t* p, uint32_t want, vo
 // m-tile visiting order: own row blocks first, then the peers' in ring order, so that the
 // tensor cores start on data that is already here while the rest is in flight.
 __device__ __forceinline__ int orderedMTile(const FusedArgs& f, int i, int mTiles) {
-  if (f.nranks <= 1 || f.mode == 0) return i;
   const int per = mTiles / f.nranks;
   const int owner = (f.rank + (f.mode == 2 ? 1 : 0) + i / per) % f.nranks;   // reduce-scatter: other ranks' rows first, mine last
   return owner * per + i % per;
@@ -169,7 +168,7 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   const uint32_t tmemBase = *tmemBaseSlot;
   const bool dead = *giveUp != 0;
   const uint64_t epoch = *epochSlot;
-  if (!dead && f.mode == 2 && f.nranks > 1) {
+  if (!dead && f.mode == 2) {
     // the owners must have finished reducing the previous call before this one overwrites their slots
     if (warp == 2 && lane < f.nranks && lane != f.rank) wait_flag64(&f.done[lane], epoch - 1, giveUp, g.waitNs);
     __syncthreads();
@@ -185,7 +184,7 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       for (int t = blockIdx.x; t < numTiles && ok; t += gridDim.x) {
         int mt, nt;
         tileCoord(g, t, mTiles, nTiles, mt, nt);
-        if (f.mode == 1 && f.nranks > 1 && mt / (f.rowsPerRank / BM) != f.rank) {
+        if (f.mode == 1 && mt / (f.rowsPerRank / BM) != f.rank) {
           // this row block comes from a peer: wait until the communication warps have placed it
           ok = wait_flag32(&f.blockReady[mt], (uint32_t)epoch * GATHER_PIECES, giveUp, false, g.waitNs);
           asm volatile("fence.proxy.async.global;" ::: "memory");   // their generic-proxy stores before my async-proxy loads
@@ -253,7 +252,7 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       const int row = mt * BM + quarter * 32 + lane;
       __nv_bfloat16* crow;
       int owner = 0, tileInOwner = 0;
-      if (f.mode == 2 && f.nranks > 1) {
+      if (f.mode == 2) {
         owner = row / f.rowsPerRank;
         tileInOwner = ((mt * BM - owner * f.rowsPerRank) / BM) * nTiles + nt;
         crow = f.slot[owner] + (size_t)(row - owner * f.rowsPerRank) * g.N + nt * BN;
@@ -264,8 +263,8 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       // every store instruction writes whole 128-byte row segments (what NVLink and DRAM both want)
       // instead of 32 scattered 16-byte pieces
       uint8_t* stage = epiSmem + (warp - 2) * EPI_WARP_BYTES;
-      __nv_bfloat16* cbase = crow - (size_t)lane * (f.mode == 2 && f.nranks > 1 ? g.N : g.ldc);    // row 0 of this warp's 32 rows
-      const size_t rowStride = (f.mode == 2 && f.nranks > 1) ? (size_t)g.N : (size_t)g.ldc;
+      __nv_bfloat16* cbase = crow - (size_t)lane * (f.mode == 2 ? g.N : g.ldc);    // row 0 of this warp's 32 rows
+      const size_t rowStride = f.mode == 2 ? (size_t)g.N : (size_t)g.ldc;
 #pragma unroll 1
       for (int c4 = 0; c4 < BN / 64; ++c4) {
 #pragma unroll
@@ -296,7 +295,7 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&accEmpty[ab]);      // 4 epilogue warps release the accumulator
-      if (f.mode == 2 && f.nranks > 1) {
+      if (f.mode == 2) {
         // publish the tile in its owner's memory once all four warps have stored their rows
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (warp == 2 && lane == 0) {
@@ -308,7 +307,7 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
   } else {
     // ------------------------------------------------------------ communication warps (6..9)
     const int ct = threadIdx.x - 6 * 32;              // 0..127
-    if (f.mode == 1 && f.nranks > 1) {
+    if (f.mode == 1) {
       const int blocksPerRank = f.rowsPerRank / BM;
       const size_t blockBytes = (size_t)BM * g.K * 2;
       if (blockIdx.x == 0 && ct < f.nranks && ct != f.rank) st_rel_sys(f.peerArrive[ct], epoch);   // my shard is ready
@@ -351,7 +350,7 @@ dfcclGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         }
       }
       if (blockIdx.x == 0 && ct < f.nranks && ct != f.rank) wait_flag64(&f.done[ct], epoch, giveUp, g.waitNs);   // my shard stays put until read
-    } else if (f.mode == 2 && f.nranks > 1) {
+    } else if (f.mode == 2) {
       // reduce the tiles I own as their n partial copies arrive: slot[j] written by rank j's epilogue
       const int tilesMine = (f.rowsPerRank / BM) * nTiles;
       for (int i = blockIdx.x; i < tilesMine; i += gridDim.x) {
