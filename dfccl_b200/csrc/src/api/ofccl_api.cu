@@ -664,12 +664,12 @@ static ncclResult_t runDirect(ofcclRankCtx* ctx, CollEntry& e, int collId, const
   ctx->outside++;
   ctx->remaining++;
   ctx->sqes++;
-  const OneRankDone done{ctx->rdDev, collId, (uint32_t)e.submitted, ctx->rdHost.trace != nullptr};
+  const OneRankDone done{ctx->rdDev, collId, (uint32_t)e.submitted};
   l.unlock();
   int prev = 0;
   cudaGetDevice(&prev);
   if (prev != ctx->device) cudaSetDevice(ctx->device);
-  ncclResult_t r = launchOneRankCuda(e.cs, send, recv, stream, &done);
+  ncclResult_t r = launchOneRankCuda(e.cs, send, recv, stream, &done, ctx->rdHost.trace != nullptr);
   if (prev != ctx->device) cudaSetDevice(prev);
   if (r != ncclSuccess) {                    // nothing was launched: undo the bookkeeping
     std::lock_guard<std::mutex> g(ctx->mu);

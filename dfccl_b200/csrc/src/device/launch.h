@@ -15,9 +15,11 @@ ncclResult_t launchStandaloneCuda(RankDev* rd, const CollStatic& cs, uint64_t se
                                   uint32_t sqeFlags, int threads, cudaStream_t stream);
 
 // The same on a one-rank communicator: one streaming kernel, buffers used where they are.  With `done` the kernel also
-// publishes the completion of a registered collective (device flag and completion entry).
-struct OneRankDone { RankDev* rd; int32_t coll; uint32_t epoch; bool traced; };      // traced: leaves the daemon's events, as of block 0
-ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream, const OneRankDone* done = nullptr);
+// publishes the completion of a registered collective (device flag and completion entry); `traced`: and the daemon's events
+// for it, as block 0's.
+struct OneRankDone { RankDev* rd; int32_t coll; uint32_t epoch; };
+ncclResult_t launchOneRankCuda(const CollStatic& cs, const void* send, void* recv, cudaStream_t stream, const OneRankDone* done = nullptr,
+                               bool traced = false);
 
 // Force the lazily loaded kernels of the runtime into the context (no launch).
 ncclResult_t warmRuntimeKernels();
