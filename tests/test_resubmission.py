@@ -1,5 +1,5 @@
 """A collective whose context a block still holds from its previous submission (csrc/src/device/daemon_impl.h:
-consumeSubmissions) is submitted again.  Host backend; the scheduler is the same source as the device's."""
+consumeSubmissions) is submitted again.  Most of it on the host backend: the scheduler is the same source as the device's."""
 import threading
 import time
 
@@ -91,3 +91,79 @@ def test_resubmission_that_stalls_lets_the_daemon_leave(host_backend, count):
     for c in comms:
         c.destroy()
     assert quits[0] >= 2 and took[1] < 2.0, (quits, took)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("then", ["xy", "pp"])
+def test_resubmission_that_needs_staging_areas_gpu(native, then):
+    """One-shot; the daemon stays for 0.2 s, far longer than the four submissions take."""
+    import torch
+    from dfccl_b200.utils import tensor_from_ptr
+    native.set_backend("cuda")
+    torch.cuda.set_device(0)
+    comms = native.Comm.init_loopback(2, 0)
+    buf = [{n: tensor_from_ptr(comms[r].alloc(4 * COUNT), (COUNT,), torch.float32, "cuda:0") for n in "pq"} |
+           {n: torch.zeros(COUNT, device="cuda") for n in "xy"} for r in range(2)]
+    torch.cuda.synchronize()
+
+    def body(r):
+        torch.cuda.set_device(0)
+        ctx = native.RankCtx(r, 0)
+        ctx.set_daemon_geometry(2, 0)
+        ctx.prepare(0, comms[r], native.ALLREDUCE, COUNT, native.FLOAT32, algo=native.ALGO_ONESHOT)
+        ctx.finalize()
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            for it, (s, d) in enumerate(["pq"] * 3 + [then]):
+                buf[r][s].fill_(10.0 * (r + 1) + it)
+                st.synchronize()
+                ctx.run(0, buf[r][s].data_ptr(), buf[r][d].data_ptr())
+                assert ctx.wait(0, 30000) == native.SUCCESS
+                assert bool((buf[r][d] == 30.0 + 2 * it).all()), it
+        ctx.destroy()
+
+    with _env(DFCCL_IDLE_QUIT_US=200000, DFCCL_STALL_QUIT_US=200000):
+        run_ranks(2, body)
+    for c in comms:
+        c.destroy()
+
+
+@pytest.mark.gpu
+def test_resubmission_with_a_late_peer_gpu(native):
+    """With the default limits (a stalled block leaves after 5 ms, any daemon after 2 s)."""
+    import torch
+    from dfccl_b200.utils import tensor_from_ptr
+    native.set_backend("cuda")
+    torch.cuda.set_device(0)
+    comms = native.Comm.init_loopback(2, 0)
+    met = threading.Barrier(2)
+    took = {}
+
+    def body(r):
+        torch.cuda.set_device(0)
+        c = comms[r]
+        p, q = c.alloc(4 * COUNT), c.alloc(4 * COUNT)
+        x, y = (tensor_from_ptr(a, (COUNT,), torch.float32, "cuda:0") for a in (p, q))
+        ctx = native.RankCtx(r, 0)
+        ctx.set_daemon_geometry(2, 0)
+        ctx.prepare(0, c, native.ALLREDUCE, COUNT, native.FLOAT32)
+        ctx.finalize()
+        x.fill_(r + 1.0)
+        torch.cuda.current_stream().synchronize()
+        for _ in range(2):
+            ctx.run(0, p, q)
+            assert ctx.wait(0, 30000) == native.SUCCESS
+        met.wait()
+        if r == 1:
+            time.sleep(0.1)
+        t = time.perf_counter()
+        ctx.run(0, p, q)
+        assert ctx.wait(0, 30000) == native.SUCCESS
+        took[r] = time.perf_counter() - t
+        assert bool((y == 3.0).all())
+        ctx.destroy()
+
+    run_ranks(2, body)
+    for c in comms:
+        c.destroy()
+    assert took[1] < 0.5, took
