@@ -152,7 +152,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       const size_t tileOff = (size_t)(mt * PM + (int)cr * HALF + quarter * 32) * g.ldc + nt * PN;   // row 0 of this warp's 32 rows
       const int beg = colHalf * (PN / 2);
       // 32 columns of its row per lane and step, 32 bytes (a whole sector) per access: no staging rows, whose way through
-      // shared memory the operands need (8192 x 4096 x 1024 with GELU's gradient: 105 -> 76 us)
+      // shared memory the operands need (8192 x 4096 x 1024 with GELU's gradient: 105 -> 70 - 79 us, by run)
       constexpr bool AUX = EPI == EPI_BIAS_RES || EPI == EPI_GELU_GRAD;
       constexpr int STEPS = PN / 2 / 32;
       const size_t mineOff = tileOff + (size_t)lane * g.ldc + beg;

@@ -49,9 +49,9 @@ def test_gemm_reads_transposed_operands_in_place(m, n, k, a_t, b_t):
 @pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 768, 448), (2048, 1024, 4096), (9728, 512, 1024)])
 def test_cta_pair_kernel_agrees_with_the_one_cta_kernel(m, n, k, a_t, b_t, monkeypatch):
-    """Sizes that tile by 256 x 256 run on CTA pairs (cta_group::2) by default; DFCCL_GEMM_PAIR=0 keeps the one-CTA
-    kernel.  Both accumulate the same products in the same order, so the results are bit-identical; 9728 rows = 38 row
-    tiles x 2 column tiles make more tiles than resident pairs."""
+    """DFCCL_GEMM_PAIR=0 keeps products that would run on CTA pairs (cta_group::2) on a one-CTA form: here the last two (the
+    first two run on one all the same).  Both accumulate the same products in the same order, so the results are
+    bit-identical; 9728 rows = 38 row tiles x 2 column tiles make more tiles than resident pairs."""
     from dfccl_b200.ops import gemm
     torch.manual_seed(m + 7 * n + k)
     a = torch.randn(m, k, device="cuda", dtype=torch.bfloat16)
