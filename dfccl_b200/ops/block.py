@@ -50,6 +50,14 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+def packed(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """Contiguous and 16-byte aligned (a gradient may be a slice of anything)."""
+    if t is None:
+        return None
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def apply_epilogue_(product: torch.Tensor, epi: Epilogue) -> torch.Tensor:
     """In place, for products whose kernel has no epilogue."""
     assert product.dtype == torch.bfloat16 and product.dim() == 2 and product.is_contiguous()
@@ -93,8 +101,7 @@ class _NormFn(torch.autograd.Function):
         if gy is None:
             return gpass, None, None, None
         rows, d = x.shape
-        gy = gy.contiguous()
-        gpass = None if gpass is None else gpass.contiguous()
+        gy, gpass = packed(gy), packed(gpass)
         gx, gg, gb = torch.empty_like(x), torch.empty_like(gamma), torch.empty_like(gamma)
         with on_device(x.device):
             work = torch.empty(nv.lib().dfcclLayerNormWork(rows, d), dtype=torch.float32, device=x.device)

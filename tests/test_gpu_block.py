@@ -82,6 +82,22 @@ def test_layer_norm_with_the_residuals_gradient(native, rows, d):
         assert _rel(got.detach(), want.detach()) < HALF_ULP
 
 
+def test_layer_norm_with_gradients_off_the_grid(native):
+    """Both gradients arrive as slices of a flat array, one element from its start."""
+    from dfccl_b200.ops import block
+    torch.manual_seed(8)
+    ln = nn.LayerNorm(256, dtype=torch.bfloat16, device="cuda")
+    x = torch.randn(37, 256, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    one = torch.zeros(1, device="cuda", dtype=torch.bfloat16)
+    g1, g2 = (torch.randn(1 + x.numel(), device="cuda").to(torch.bfloat16) for _ in range(2))
+    h, y = block.norm_residual(ln, x)
+    torch.autograd.backward([torch.cat([one, h.reshape(-1)]), torch.cat([one, y.reshape(-1)])], [g1, g2])
+    x64, w64, b64 = (t.detach().double().requires_grad_(True) for t in (x, ln.weight, ln.bias))
+    torch.autograd.backward([x64 * 1, F.layer_norm(x64, (256,), w64, b64, ln.eps)], [g[1:].view(37, 256).double() for g in (g1, g2)])
+    for got, want in ((x.grad, x64.grad), (ln.weight.grad, w64.grad), (ln.bias.grad, b64.grad)):
+        assert _rel(got, want) < HALF_ULP
+
+
 @pytest.mark.parametrize("rows,n", [(1, 8), (31, 64), (33, 264), (1000, 1024), (8192, 3072), (4100, 4096)])
 def test_column_sum(native, rows, n):
     from dfccl_b200.ops import block

@@ -87,3 +87,13 @@ def test_launches_on_a_device_that_is_not_current(monkeypatch):
     assert isinstance(on_device(torch.device("cuda", 1)), torch.cuda.device)
     assert isinstance(on_device(torch.device("cuda", 0)), contextlib.nullcontext)
     assert isinstance(on_device(torch.device("cuda")), contextlib.nullcontext)
+
+
+def test_gradients_of_the_norm_kernel_are_brought_to_the_grid():
+    flat = torch.randn(1 + 8 * 16).to(BF)
+    g = flat[1:].view(8, 16)
+    assert g.data_ptr() % 16 and block.packed(None) is None
+    p = block.packed(g)
+    assert p.data_ptr() % 16 == 0 and p.is_contiguous() and torch.equal(p, g)
+    t = torch.randn(16, 8).to(BF)
+    assert block.packed(t) is t and torch.equal(block.packed(t.t()), t.t()) and block.packed(t.t()).is_contiguous()
