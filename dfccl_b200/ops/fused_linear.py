@@ -25,7 +25,7 @@ import torch.distributed as dist
 
 from .. import native as nv
 from ..utils.tensors import raw_stream, tensor_from_ptr
-from .block import Epilogue, NO_EPILOGUE
+from .block import Epilogue, NO_EPILOGUE, packed
 from .gemm import BM, BN, BK
 
 
@@ -94,10 +94,11 @@ class _Local:
     """One-rank groups: the operator is its GEMM, with an epilogue (``ops.block``)."""
 
     def operand(self, x: torch.Tensor) -> torch.Tensor:
-        """``x`` as the GEMM reads it, [M, K] bf16: cast, and spread over the rows, as copying it into an operand does."""
+        """``x`` as the GEMM reads it, [M, K] bf16 on the 16-byte grid: cast, and spread over the rows, as copying it into an
+        operand does."""
         if x.shape != (self.m, self.k):
             x = x.reshape(self.m, self.k) if x.numel() == self.m * self.k and x.shape[-1] == self.k else x.expand(self.m, self.k)
-        return x.to(self.tp.device, torch.bfloat16).contiguous()
+        return packed(x.to(self.tp.device, torch.bfloat16))
 
     def local(self, x: torch.Tensor, w: torch.Tensor, w_transposed: bool = False, epi: Epilogue = NO_EPILOGUE) -> torch.Tensor:
         assert self.tp.n == 1

@@ -21,7 +21,7 @@ import torch.nn as nn
 from torch.autograd.function import once_differentiable
 
 from .. import native as nv
-from ..ops.block import BIAS, BIAS_GELU, BIAS_RES, GELU_GRAD, Epilogue, NO_EPILOGUE, apply_epilogue_, column_sum, epilogue_operand, unhooked
+from ..ops.block import BIAS, BIAS_GELU, BIAS_RES, GELU_GRAD, Epilogue, NO_EPILOGUE, apply_epilogue_, column_sum, epilogue_operand, packed, unhooked
 from ..ops.fused_linear import AllGatherGemm, GemmReduceScatter, TpGroup
 from ..utils.tensors import nccl_dtype, raw_stream
 
@@ -170,7 +170,7 @@ class _ColumnFusedFn(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, gy):
         x_full, weight = ctx.saved_tensors
-        gy = gy.contiguous()
+        gy = packed(gy)
         gb = column_sum(gy) if ctx.has_bias else None
         gw, gx = _column_backward(ctx.layer, gy, x_full, weight)
         return gx, gw, gb, None
@@ -188,7 +188,7 @@ class _RowFusedFn(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, gy_shard):
         x, weight = ctx.saved_tensors
-        gy = gy_shard.contiguous()
+        gy = packed(gy_shard)
         gb = column_sum(gy) if ctx.has_bias else None
         gw, gx = _row_backward(ctx.layer, gy, x, weight)
         return gx, gw, gb, gy_shard if ctx.has_residual else None, None
@@ -209,7 +209,7 @@ class _MlpFn(torch.autograd.Function):
     @once_differentiable
     def backward(ctx, gy_shard):
         x_full, pre, act, up_weight, down_weight = ctx.saved_tensors
-        gy = gy_shard.contiguous()
+        gy = packed(gy_shard)
         gb_down = column_sum(gy)
         gw_down, gpre = _row_backward(ctx.down, gy, act, down_weight, Epilogue(GELU_GRAD, aux=pre))
         gb_up = column_sum(gpre)

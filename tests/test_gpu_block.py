@@ -174,6 +174,27 @@ def test_layers_take_fp32_activations(native, kind):
     comm.destroy()
 
 
+@pytest.mark.parametrize("kind", ["ColumnParallelLinear", "RowParallelLinear"])
+def test_layers_with_inputs_and_gradients_off_the_grid(native, kind):
+    """Slices one element from the start of a flat array; the copy into an operand used to take them."""
+    from dfccl_b200.ops.fused_linear import TpGroup
+    from dfccl_b200.parallel import tp as tp_mod
+    native.set_backend("cuda")
+    (comm,) = native.Comm.init_loopback(1, 0)
+    torch.manual_seed(9)
+    layer = getattr(tp_mod, kind)(TpGroup(comm, None, torch.device("cuda", 0)), 256, torch.randn(512, 256, device="cuda") * 256 ** -0.5)
+    flat = torch.randn(1 + 256 * 256, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    g = torch.randn(1 + 256 * 512, device="cuda").to(torch.bfloat16)
+    y = layer(flat[1:].view(256, 256))
+    torch.cat([g[:1], y.reshape(-1)]).backward(g)
+    f64, w64, b64 = (t.detach().double().requires_grad_(True) for t in (flat, layer.weight, layer.bias))
+    y64 = f64[1:].view(256, 256) @ w64.t() + b64
+    y64.backward(g[1:].view(256, 512).double())
+    for got, want in ((y, y64), (flat.grad, f64.grad), (layer.weight.grad, w64.grad), (layer.bias.grad, b64.grad)):
+        assert _rel(got.detach(), want.detach()) < HALF_ULP
+    comm.destroy()
+
+
 @pytest.mark.parametrize("residual", ["same", "strided", "row", "vector", "column", "misaligned", "fp32"])
 @pytest.mark.parametrize("bias", ["full", "misaligned", "one"])
 def test_residuals_and_biases_of_any_form(native, residual, bias):

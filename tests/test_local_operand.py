@@ -18,6 +18,7 @@ class Recorder:
         self.calls = []
 
     def dfcclGemmBf16Epilogue(self, x, w, out, m, n, k, *rest):
+        assert (x | w | out) % 16 == 0
         read = lambda p, rows, cols: torch.frombuffer((C.c_char * (2 * rows * cols)).from_address(p), dtype=torch.bfloat16).view(rows, cols).clone()   # noqa: E731
         self.calls.append((read(x, m, k), read(w, n, k), rest))
         return 0
@@ -35,12 +36,14 @@ def op(monkeypatch):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
-@pytest.mark.parametrize("form", ["rows", "strided", "flat", "row", "vector"])
+@pytest.mark.parametrize("form", ["rows", "strided", "flat", "row", "vector", "off"])
 def test_operand_is_cast_and_spread_like_a_copy(op, dtype, form):
     x = torch.randn(M, K).to(dtype)
     want = x
     if form == "strided":
         x = x.t().contiguous().t()
+    elif form == "off":                                    # one element behind the 16-byte grid
+        x = torch.cat([x.reshape(-1)[:1], x.reshape(-1)])[1:].view(M, K)
     elif form == "flat":
         x = x.view(2, M // 2, K)
     elif form in ("row", "vector"):
