@@ -26,7 +26,7 @@ SOURCES = [
     "src/common/log.cc", "src/common/param.cc", "src/common/socket.cc",
     "src/bootstrap/bootstrap.cc",
     "src/mem/heap.cu", "src/mem/mcast.cu", "src/topo/topo.cu", "src/net/net_socket.cc", "src/net/net_ring.cu",
-    "src/device/datapath.cu", "src/daemon/daemon.cu", "src/daemon/standalone.cu", "src/daemon/onerank.cu", "src/daemon/daemon_host.cu",
+    "src/device/datapath.cu", "src/device/datapath_small.cu", "src/daemon/daemon.cu", "src/daemon/standalone.cu", "src/daemon/onerank.cu", "src/daemon/daemon_host.cu",
     "src/comm/comm.cu",
     "src/api/nccl_api.cu", "src/api/p2p.cu", "src/api/ofccl_api.cu", "src/api/debug_api.cu",
     "src/ops/optim.cu", "src/ops/block.cu", "src/api/noalloc.cu", "src/api/probe.cu", "src/gemm/tcgen05_gemm.cu", "src/gemm/tcgen05_gemm_pair.cu", "src/gemm/tcgen05_gemm_tile.cu",
@@ -66,6 +66,8 @@ def _compile(src: str, verbose: bool, hdr_time: float, sanitize: str = "") -> Pa
         # out-of-line device functions do not inherit a kernel's launch bounds: cap them at what
         # a 512-thread block leaves per thread (the reference caps its device code the same way)
         extra = ["-maxrregcount=128"]
+    if src.endswith("device/datapath_small.cu"):
+        extra = ["-maxrregcount=80"]                 # what a function uses of the caller's registers it has to save
     if sanitize:                                     # host code only: the device code is the same as in the plain build
         extra += ["-Xcompiler", f"-fsanitize={sanitize},-fno-omit-frame-pointer,-g", "-DDF_FAST_BUILD"]
     cmd = [nvcc()] + _flags(verbose) + extra + ["-c", str(s), "-o", str(o)]

@@ -106,6 +106,7 @@ ncclResult_t dfcclAllReduceNoAlloc(const void* sendbuff, void* recvbuff, size_t 
   cs.peerHeap[0] = (char*)base;
   cs.myFlags = (FlagSlot*)(base + kFlagsOff);
   cs.peerFlags[0] = cs.myFlags;
+  planColl(&cs, 0);
   uint32_t epoch;
   { std::lock_guard<std::mutex> l(g_mu); epoch = ++g_epoch[dev]; }
   dfcclNoAllocKernel<<<cs.nBlocks, DF_BLOCK_THREADS, 0, stream>>>(base, cs, (uint64_t)(uintptr_t)sendbuff, (uint64_t)(uintptr_t)recvbuff,

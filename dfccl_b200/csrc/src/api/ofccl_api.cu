@@ -536,6 +536,7 @@ DF_API ncclResult_t ofcclFinalizeRankCtx7StartHostThrds(ofcclRankCtx_t ctx) {
   // a block's data phase is left after this many bytes when other work is queued (the reference parks a
   // collective at its 1 MiB slices: src/include/collectives.h:112-113)
   rd.sliceBytes = (uint64_t)std::max<int64_t>(0, paramI64("SLICE_BYTES", 1 << 20));
+  for (auto& kv : ctx->colls) if (!kv.second.comm->netMode && !kv.second.fused.kind) planColl(&kv.second.cs, rd.sliceBytes);
   std::vector<CollStatic> table(maxColls);
   memset(table.data(), 0, sizeof(CollStatic) * maxColls);
   for (auto& kv : ctx->colls) table[kv.first] = kv.second.cs;

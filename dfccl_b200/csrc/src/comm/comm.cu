@@ -389,6 +389,7 @@ ncclResult_t commCollective(ncclComm* c, int kind, const void* send, void* recv,
   if (viaArena) {
   } else if (needRecv && !c->heap->contains(recv, rBytes)) { DFCHECK(ensureScratch(c, 1, rBytes, stream)); flags |= SQE_RECV_STAGED; r = (uint64_t)(uintptr_t)recv; cs.stagingRecvOff = c->scratchOff[1]; }
   else if (needRecv) r = c->heap->offsetOf(recv);
+  planColl(&cs, 0);
   ++c->opCount;
   const uint32_t epoch = 0;            // the kernel reads the communicator's device-side count: works under graph replay too
   if (c->backend == dfcclBackendCuda) {

@@ -56,18 +56,18 @@ DF_HD void serviceMain(BlockShared* sh, RankDev* rd) {
 
 // Consume new entries of the device ring.  Thread 0 only.  Returns the number consumed.
 // A submission that waits for its stream goes to the trigger list, everything else to the task queue.
-DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b) {
+// `slot` and `next`: the first two entries, looked at together (a lone entry then costs no second round trip).
+DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b, SqSlot slot, SqSlot next, bool haveNext) {
   int got = 0;
-  SqSlot slot;
-  while (sqPeek(rd, sh->frontier, &slot)) {
+  for (bool have = true; have; slot = next, have = haveNext, haveNext = have && sqPeek(&sh->k, sh->frontier + 1, &next)) {
     const Sqe q = sqDecode(slot);
     if (q.flags & SQE_QUIT) { sh->quit = 2; break; }       // the frontier stays on the quit entry
     const int coll = q.collId;
     bool mine = false;
-    if (coll >= 0 && (uint32_t)coll < rd->maxColls) {
+    if (coll >= 0 && (uint32_t)coll < sh->k.maxColls) {
       const uint32_t m = sh->meta[coll];
       int r = b - (int)((m >> 8) & 0xffu);
-      if (r < 0) r += (int)rd->nBlocks;
+      if (r < 0) r += (int)sh->k.nBlocks;
       mine = (m & DF_META_VALID) && r < (int)(m & 0xffu);
     }
     if (mine) {
@@ -89,22 +89,27 @@ DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b) {
     if (sh->loadedColl == coll && !(q.flags & (SQE_TRIGGERED | SQE_NEW_STATIC))) { sh->dyn = d; sh->dynDirty = 1; }   // its context is still here
     else {
       if (sh->loadedColl == coll) { sh->loadedColl = -1; sh->dynDirty = 0; }                          // re-armed in global memory: drop the cached copy
-      rd->dyn[(uint64_t)b * rd->maxColls + coll] = d;
+      sh->k.dyn[(uint64_t)b * sh->k.maxColls + coll] = d;
     }
-    trace(rd, b, TR_SQE, coll);
+    trace(sh, rd, b, TR_SQE, coll);
     if (q.flags & SQE_TRIGGERED) {
       sh->trigColl[sh->nTrig] = (uint16_t)coll; sh->trigVal[sh->nTrig] = q.trigger; ++sh->nTrig;
     } else {
       sh->actWait[sh->nActive] = 0;
       sh->active[sh->nActive++] = (uint16_t)coll;
-      trace(rd, b, TR_START, coll);
+      trace(sh, rd, b, TR_START, coll);
     }
   }
-  if (got) {
-    fence_gpu();                                           // the entries, before anything that is read because of them
-    st_relaxed_sys_u64(&rd->hostFrontier[b], sh->frontier);   // posted store: the host reads it when its ring looks full
-  }
+  if (got) fence_acq_rel_gpu();                            // the entries, before anything that is read because of them
   return got;
+}
+
+// How far this block has come, for the host's flow control (it reads this when its ring looks full).  A store across PCIe that
+// the next fence of system scope would wait for, so it goes out when the block has nothing to do, or a quarter of the ring behind.
+DF_HD void reportFrontier(BlockShared* sh, int b, bool idle) {
+  if (sh->frontier == sh->frontierSeen || !(idle || sh->frontier - sh->frontierSeen >= sh->k.sqCap / 4)) return;
+  st_relaxed_sys_u64(&sh->k.hostFrontier[b], sh->frontier);
+  sh->frontierSeen = sh->frontier;
 }
 
 // Look at the trigger words of every submission that waits for its stream: one thread per entry, no context is
@@ -115,7 +120,7 @@ DF_HD uint32_t pollTriggers(BlockShared* sh, RankDev* rd, int b) {
   if (tid == 0) sh->trigFired = 0;
   df_sync();
   for (uint32_t i = tid; i < nTrig; i += nt) {
-    const uint32_t have = (uint32_t)ld_relaxed_sys_u64(&rd->trigger[sh->trigColl[i]]);
+    const uint32_t have = (uint32_t)ld_relaxed_sys_u64(&sh->k.trigger[sh->trigColl[i]]);
     if ((int32_t)(have - sh->trigVal[i]) >= 0) { sh->trigColl[i] |= 0x8000u; atomic_add_u32(&sh->trigFired, 1u); }
   }
   df_sync();
@@ -127,9 +132,9 @@ DF_HD uint32_t pollTriggers(BlockShared* sh, RankDev* rd, int b) {
       const uint16_t e = sh->trigColl[i];
       if (e & 0x8000u) {
         const int coll = e & 0x7fff;
-        rd->dyn[(uint64_t)b * rd->maxColls + coll].phase = PH_COPY_IN;
+        sh->k.dyn[(uint64_t)b * sh->k.maxColls + coll].phase = PH_COPY_IN;
         if (sh->nActive < DF_MAX_ACTIVE) { sh->actWait[sh->nActive] = 0; sh->active[sh->nActive++] = (uint16_t)coll; }
-        trace(rd, b, TR_START, coll);
+        trace(sh, rd, b, TR_START, coll);
       } else { sh->trigColl[w] = e; sh->trigVal[w] = sh->trigVal[i]; ++w; }
     }
     sh->nTrig = w;
@@ -144,19 +149,17 @@ DF_HD uint32_t pollTriggers(BlockShared* sh, RankDev* rd, int b) {
 // context switch and a polling budget each.  Everybody calls it; returns the number of entries that became ready.
 DF_HD uint32_t scanParked(BlockShared* sh, RankDev* rd, int b) {
   const int tid = df_tid(), nt = df_nthreads();
-  const uint32_t nAct = sh->nActive;
-  if (tid == 0) sh->nReady = 0;
-  df_sync();
+  const uint32_t nAct = sh->nActive;                       // (nReady: cleared at the end of the last pass)
   for (uint32_t i = tid; i < nAct; i += nt) {
     const uint32_t w = sh->actWait[i];
     if (w == 0) continue;
     const int coll = sh->active[i];
     if (coll == 0xffff) continue;
-    const CollStatic* c = &rd->colls[coll];
+    const CollStatic* c = &sh->k.colls[coll];
     const int n = c->nranks, me = c->rank;
-    const FlagSlot* f = c->myFlags + (uint64_t)relBlock(rd, c, b) * n;
+    const FlagSlot* f = c->myFlags + (uint64_t)relBlock((int)sh->k.nBlocks, c, b) * n;
     // (the collective whose context is loaded may have been submitted again since that was last saved)
-    const uint64_t epoch = sh->loadedColl == coll ? sh->dyn.epoch : rd->dyn[(uint64_t)b * rd->maxColls + coll].epoch;
+    const uint64_t epoch = sh->loadedColl == coll ? sh->dyn.epoch : sh->k.dyn[(uint64_t)b * sh->k.maxColls + coll].epoch;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
       if (j == me) continue;
@@ -172,6 +175,8 @@ DF_HD void blockRestore(BlockShared* sh, RankDev* rd, int b) {
   const int tid = df_tid(), nt = df_nthreads();
   BlockSaved* sv = &rd->saved[b];
   if (tid == 0) {
+    sh->k = *rd;
+    sh->nParked = 0; sh->nReady = 0; sh->frontierSeen = sv->frontier;
     sh->loadedColl = -1; sh->standalone = 0; sh->dynDirty = 0; sh->quit = 0; sh->abortSeen = 0; sh->ctl1Full = 0;
     sh->frontier = sv->frontier; sh->nActive = sv->nActive; sh->nTrig = sv->nTrig;
     DevStats z = {};
@@ -203,6 +208,7 @@ DF_HD void blockPark(BlockShared* sh, RankDev* rd, int b) {
   for (uint32_t i = tid; i < sh->nTrig; i += nt) { sv->trigColl[i] = sh->trigColl[i]; sv->trigVal[i] = sh->trigVal[i]; }
   df_sync();
   if (tid == 0) {
+    reportFrontier(sh, b, true);
     sv->frontier = sh->frontier; sv->nActive = sh->nActive; sv->nTrig = sh->nTrig;
     // fold this launch's counters into the totals the host reads
     DevStats* g = &rd->stats[b];
@@ -213,7 +219,7 @@ DF_HD void blockPark(BlockShared* sh, RankDev* rd, int b) {
     g->visits += sh->stats.visits; g->yields += sh->stats.yields; g->passes += sh->stats.passes;
     g->nsTriggers += sh->stats.nsTriggers; g->nsWalk += sh->stats.nsWalk; g->nsQueues += sh->stats.nsQueues;
     if (sh->stats.maxSwitchNs > g->maxSwitchNs) g->maxSwitchNs = sh->stats.maxSwitchNs;
-    trace(rd, b, TR_QUIT, (int)sh->quit);
+    trace(sh, rd, b, TR_QUIT, (int)sh->quit);
     fence_sys();
     sv->exited = 1;
     uint32_t prev = atomic_add_u32(&rd->exitedBlocks, 1u);
@@ -239,24 +245,26 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
     df_sync_service();
   }
   blockRestore(sh, rd, b);
-  if (tid == 0) trace(rd, b, TR_LAUNCH, 0);
+  if (tid == 0) trace(sh, rd, b, TR_LAUNCH, 0);
   uint64_t lastUseful = df_now_ns();     // only thread 0's copies of these are ever consulted
   const uint64_t bornNs = lastUseful;
   uint64_t lastSlowCheck = 0, lastFullPass = 0;
   uint32_t winding = 0;
   uint32_t idleBackoff = 32;
+  uint64_t tPass = lastUseful;           // when this pass began
 
   for (;;) {
     // ---- 0. submissions waiting for their stream (every value steering control flow here is block-uniform)
     bool progressed = false;
-    const uint64_t tPass = tid == 0 ? df_now_ns() : 0;
-    if (sh->nTrig && pollTriggers(sh, rd, b)) progressed = true;
-    const uint64_t tWalk = tid == 0 ? df_now_ns() : 0;
+    if (sh->nTrig) {
+      if (pollTriggers(sh, rd, b)) progressed = true;
+      if (tid == 0) { const uint64_t t = df_now_ns(); sh->stats.nsTriggers += t - tPass; tPass = t; }
+    }
     // ---- 1. task queue traversal: parked entries are skipped unless the scan found their flags ready; now and then
     // every entry is visited all the same, so that a wait that will never succeed reaches its time limit
     const uint32_t nAct = sh->nActive;
     if (nAct) {
-      if (scanParked(sh, rd, b)) progressed = true;
+      if (sh->nParked && scanParked(sh, rd, b)) progressed = true;
       const bool fullPass = sh->ctl1Full != 0;
       for (uint32_t i = 0; i < nAct; ++i) {
         const int coll = sh->active[i];
@@ -265,8 +273,8 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
         // With other collectives queued a wait gives up after a few polls: the scan brings the block back when
         // the flags are there.  The oldest submission (head of the queue) gets more patience, and with nothing
         // else queued there is nothing to switch to: polling longer is free.
-        const uint32_t base = nAct == 1 ? rd->spinBudget : (rd->spinBudget + 7u) / 8u;
-        const uint32_t budget = base * ((i == 0 || nAct == 1) ? rd->headTries : 1u);
+        const uint32_t base = nAct == 1 ? sh->k.spinBudget : (sh->k.spinBudget + 7u) / 8u;
+        const uint32_t budget = base * ((i == 0 || nAct == 1) ? sh->k.headTries : 1u);
         bool moved = false;
         int rc = runColl(sh, rd, b, coll, budget, &moved);
         if (rc == RC_DONE || rc == RC_YIELD || moved) progressed = true;
@@ -283,26 +291,30 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
     // ---- 2. compaction, new submissions, idle decision: thread 0 decides, everybody obeys
     if (tid == 0) {
       sh->stats.passes++;
-      uint32_t w = 0;
-      for (uint32_t i = 0; i < sh->nActive; ++i) if (sh->active[i] != 0xffff) { sh->active[w] = sh->active[i]; sh->actWait[w] = sh->actWait[i]; ++w; }
-      sh->nActive = w;
+      // the words of global memory this section looks at: on their way together
+      const uint32_t left = ld_relaxed_sys_u32(&rd->quitting);
+      SqSlot slot, next;
+      const bool haveNext = sqPeek(&sh->k, sh->frontier + 1, &next), have = sqPeek(&sh->k, sh->frontier, &slot);
+      uint32_t w = 0, parked = 0;
+      for (uint32_t i = 0; i < sh->nActive; ++i) if (sh->active[i] != 0xffff) { sh->active[w] = sh->active[i]; sh->actWait[w] = sh->actWait[i]; parked += sh->actWait[i] != 0; ++w; }
+      sh->nActive = w; sh->nParked = parked; sh->nReady = 0;
       const uint64_t now = df_now_ns();
       sh->ctl1Full = 0;
       if (now - lastFullPass > 2000000) { sh->ctl1Full = 1; lastFullPass = now; }     // every 2 ms: visit parked entries too
-      sh->stats.nsTriggers += tWalk - tPass; sh->stats.nsWalk += now - tWalk;
-      // Words that change rarely are sampled rarely: the abort request and the "somebody left" word.  Every
-      // 20 us, or right away when this pass achieved nothing.
+      sh->stats.nsWalk += now - tPass;
+      // The abort request is sampled every 20 us.
       const bool slow = now - lastSlowCheck > 20000;
       if (slow) {
-        sh->abortSeen = abortRequested(rd) ? 1u : 0u;
+        sh->abortSeen = abortRequested(&sh->k) ? 1u : 0u;
         lastSlowCheck = now;
       }
-      if (slow || !progressed || winding) winding = ld_relaxed_sys_u32(&rd->quitting);
       // once one block of this rank has left voluntarily the others take no new work and follow as
       // soon as they cannot progress: a collective needs all its blocks, so the relaunch comes sooner
-      if (!winding && consumeSubmissions(sh, rd, b) > 0) progressed = true;
+      winding = left;
+      if (!winding && have && consumeSubmissions(sh, rd, b, slot, next, haveNext) > 0) progressed = true;
+      reportFrontier(sh, b, !progressed);
       if (sh->abortSeen) sh->quit = 3;
-      else if (rd->maxLifetimeNs && now - bornNs > rd->maxLifetimeNs && !sh->quit) {
+      else if (sh->k.maxLifetimeNs && now - bornNs > sh->k.maxLifetimeNs && !sh->quit) {
         // safety net: no instance of the daemon outlives this, whatever its state; the host relaunches it
         sh->quit = 1;
         st_release_sys_u32(&rd->quitting, 1u);
@@ -311,24 +323,25 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
       // only waiting for streams to release submissions: the host relaunches the daemon when a trigger fires, so by
       // default it leaves as quickly as when idle; a caller whose releases come in quick succession (the buckets
       // of a captured backward pass) can ask it to stay for longer and save the relaunches
-      else if (!sh->quit && (winding || now - lastUseful > (sh->nActive ? rd->stallQuitNs : sh->nTrig ? rd->trigQuitNs : rd->idleQuitNs))) {
+      else if (!sh->quit && (winding || now - lastUseful > (sh->nActive ? sh->k.stallQuitNs : sh->nTrig ? sh->k.trigQuitNs : sh->k.idleQuitNs))) {
         // a stream parked on one of this context's completion words must not depend on a host thread's
         // relaunch: while the host holds the instance it only leaves by age (or with the others)
-        if (!winding && ctl_load(&rd->ctl->hold)) lastUseful = now;
+        if (!winding && ctl_load(&sh->k.ctl->hold)) lastUseful = now;
         else {
           sh->quit = 1;
           st_release_sys_u32(&rd->quitting, 1u);
         }
       }
       sh->ctl0 = progressed ? 1 : 0;
-      sh->stats.nsQueues += df_now_ns() - now;
+      tPass = df_now_ns();
+      sh->stats.nsQueues += tPass - now;
     }
     df_sync();
     if (sh->quit) break;
     if (sh->ctl0) idleBackoff = 32;
     else if (sh->nActive == 0 && sh->nTrig == 0) {            // nothing to do: poll gently
       df_backoff(idleBackoff);
-      if (idleBackoff < 1024) idleBackoff *= 2;
+      if (idleBackoff < 128) idleBackoff *= 2;             // (what it waits for longer, a new submission is seen later)
     }
   }
   blockPark(sh, rd, b);
@@ -346,6 +359,7 @@ DF_HD void standaloneBlockMain(RankDev* rd, int b, BlockShared* sh, const CollSt
     for (int i = tid; i < (int)(sizeof(CollStatic) / 16); i += nt) d[i] = s[i];
   }
   if (tid == 0) {
+    sh->k = *rd;
     sh->loadedColl = 0; sh->standalone = 1; sh->dynDirty = 0; sh->quit = 0; sh->abortSeen = 0;
     DevStats z = {};
     sh->stats = z;
@@ -358,6 +372,7 @@ DF_HD void standaloneBlockMain(RankDev* rd, int b, BlockShared* sh, const CollSt
   for (;;) {
     bool moved = false;
     if (runColl(sh, rd, b, 0, 4096u, &moved) == RC_DONE) break;
+    df_sync();                            // the phase it left is read again
   }
   if (epoch == 0) {                       // the last block out publishes the new count (every block has read the old one by now)
     df_sync();

@@ -339,12 +339,122 @@ DF_HD void reduceTrips(const DataArgs* a, uint64_t nPacks, int nsrc, int ndst, t
     reduceTrip<Tin, Tout, OP, false, SHIFT, 1>(a, base + tid, nPacks, strideB, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
 }
 
+// How a call's pointers line up.  The vector path needs all sources at one misalignment and all destinations at one
+// misalignment (true for equal offsets into symmetric buffers): `head` elements bring the destinations to their alignment, from
+// there on the sources are read as packs shifted by `shift` bytes.  Anything else goes element by element (no packs).
+struct Lineup { uint64_t head, nPacks; uint32_t shift; };
+DF_HD Lineup lineUp(const DataArgs* a, int nsrc, int ndst, uint64_t n, int esIn, int esOut) {
+  const int V = 16 / esIn, outB = V * esOut, DA = outB >= 16 ? 16 : outB;          // alignment the vector stores need
+  const uint32_t sphase = (uint32_t)((uintptr_t)a->src[0] & 15), dphase = (uint32_t)((uintptr_t)a->dst[0] & (DA - 1));
+  bool vec = (dphase & (esOut - 1)) == 0 && (sphase & (esIn - 1)) == 0;
+  for (int j = 1; j < nsrc; ++j) vec &= ((uintptr_t)a->src[j] & 15) == sphase;
+  for (int j = 1; j < ndst; ++j) vec &= ((uintptr_t)a->dst[j] & (DA - 1)) == dphase;
+  Lineup l;
+  l.head = vec ? (uint32_t)((DA - dphase) & (DA - 1)) / (uint32_t)esOut : 0;
+  if (l.head > n) l.head = n;
+  l.shift = (uint32_t)((sphase + l.head * esIn) & 15);
+  l.nPacks = vec ? (n - l.head) / (uint32_t)V : 0;
+  return l;
+}
+
+// Small calls: a pack per thread and trip, four sources at a time, the operator looked at per pack, in as few registers as
+// that takes (device/datapath_small.cu): what a call saves of the caller's registers goes to local memory and comes back after
+// fences that emptied L1.  509 bf16 of four ranks took 9000 clocks in the bodies for long calls, of which 2500 were the sum.
+// False (and nothing done) where the sources straddle packs: shifting them takes registers.
+template <typename Tin, typename Tout>
+DF_HD_NOINLINE bool reduceSmall(const DataArgs* a, int op) {
+  typedef typename Elem<Tin>::Acc A;
+  constexpr int V = 16 / (int)sizeof(Tin), OUTB = V * (int)sizeof(Tout), NW = (OUTB + 15) / 16;
+  const int tid = df_tid(), nt = df_nthreads(), nsrc = a->nsrc, ndst = a->ndst, postDiv = a->postDiv;
+  const uint64_t n = a->n;
+  const double scale = a->scale;
+  const bool doMul = scale != 1.0;
+  const Lineup l = lineUp(a, nsrc, ndst, n, (int)sizeof(Tin), (int)sizeof(Tout));
+  if (l.shift && l.nPacks) return false;
+  const uint32_t nPacks = (uint32_t)l.nPacks;
+  const uint64_t srcOff = l.head * sizeof(Tin), dstOff = l.head * sizeof(Tout);
+#pragma unroll 1
+  for (uint32_t p = (uint32_t)tid; p < nPacks; p += (uint32_t)nt) {
+    A acc[V];
+#pragma unroll 1
+    for (int j0 = 0; j0 < nsrc; j0 += 4) {
+      uint4 in[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) if (j0 + q < nsrc) in[q] = ld16(a->src[j0 + q] + srcOff + p * 16u);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (j0 + q >= nsrc) break;
+        if (j0 + q == 0) {
+#pragma unroll
+          for (int k = 0; k < V; ++k) acc[k] = (A)Lane<Tin>::get(in[q], k);
+        } else if (op == OP_SUM) {
+#pragma unroll
+          for (int k = 0; k < V; ++k) acc[k] = red<OP_SUM>(acc[k], (A)Lane<Tin>::get(in[q], k));
+        } else if (sizeof(Tin) == sizeof(Tout)) {        // (casts exist for sums only)
+          const bool mx = op == OP_MAX, pr = op == OP_PROD;
+#pragma unroll
+          for (int k = 0; k < V; ++k) {
+            const A e = (A)Lane<Tin>::get(in[q], k);
+            acc[k] = pr ? red<OP_PROD>(acc[k], e) : mx ? red<OP_MAX>(acc[k], e) : red<OP_MIN>(acc[k], e);
+          }
+        }
+      }
+    }
+    if (Elem<Tin>::isFloat) {
+      if (doMul) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[k] = acc[k] * (A)scale;
+      }
+    } else if (postDiv) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) acc[k] = acc[k] / (A)postDiv;
+    } else if (doMul) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) acc[k] = (A)((double)acc[k] * scale);
+    }
+    uint4 ow[NW];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) ow[w] = make_uint4(0u, 0u, 0u, 0u);
+    packAll<Tout, A, V>(ow, acc);
+#pragma unroll 1
+    for (int d = 0; d < ndst; ++d) {
+      char* o = a->dst[d] + dstOff + (uint64_t)p * OUTB;
+      if (OUTB == 8) st8(o, make_uint2(ow[0].x, ow[0].y));
+      else if (OUTB == 32) st32(o, ow[0], ow[NW - 1], ((uintptr_t)o & 31) == 0);
+      else {
+#pragma unroll
+        for (int w = 0; w < OUTB / 16; ++w) st16(o + 16 * w, ow[w]);
+      }
+    }
+  }
+  // the head, the ragged tail, or everything when the pointers do not line up: the last warps first, which had no pack
+  const uint64_t tail0 = l.head + (uint64_t)nPacks * V;
+#pragma unroll 1
+  for (uint64_t i = (uint64_t)(nt - 1 - tid); i < l.head + (n - tail0); i += nt) {
+    const uint64_t e = i < l.head ? i : tail0 + (i - l.head);
+    A acc = A();
+#pragma unroll 1
+    for (int j0 = 0; j0 < nsrc; j0 += 4) {
+      Tin in[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) if (j0 + q < nsrc) in[q] = ld_elem((const Tin*)a->src[j0 + q] + e);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (j0 + q >= nsrc) break;
+        const A v = Elem<Tin>::up(in[q]);
+        acc = j0 + q == 0 ? v : op == OP_SUM ? red<OP_SUM>(acc, v) : op == OP_PROD ? red<OP_PROD>(acc, v) : op == OP_MAX ? red<OP_MAX>(acc, v) : red<OP_MIN>(acc, v);
+      }
+    }
+    const Tout o = Elem<Tout>::down(finish<Tin, Tout>(acc, scale, postDiv));
+    for (int d = 0; d < ndst; ++d) st_elem((Tout*)a->dst[d] + e, o);
+  }
+  return true;
+}
+
 template <typename Tin, typename Tout, int OP>
 DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   typedef typename Elem<Tin>::Acc A;
   constexpr int V = 16 / (int)sizeof(Tin);
-  constexpr int OUTB = V * (int)sizeof(Tout);
-  constexpr int DA = OUTB >= 16 ? 16 : OUTB;          // alignment the vector stores need
   const int tid = df_tid(), nt = df_nthreads();
   const int nsrc = a->nsrc, ndst = a->ndst;
   const uint64_t n = a->n;
@@ -352,18 +462,9 @@ DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   const int postDiv = a->postDiv;
   const bool doMul = scale != 1.0;
   const A mul = (A)scale;
-
-  // The vector path needs all sources at one misalignment and all destinations at one misalignment (true for equal
-  // offsets into symmetric buffers): `head` elements bring the destinations to their alignment, from there on the
-  // sources are read as packs shifted by `shift` bytes.  Anything else goes element by element.
-  const uint32_t sphase = (uint32_t)((uintptr_t)a->src[0] & 15), dphase = (uint32_t)((uintptr_t)a->dst[0] & (DA - 1));
-  bool vec = (dphase % sizeof(Tout)) == 0 && (sphase % sizeof(Tin)) == 0;
-  for (int j = 1; j < nsrc; ++j) vec &= ((uintptr_t)a->src[j] & 15) == sphase;
-  for (int j = 1; j < ndst; ++j) vec &= ((uintptr_t)a->dst[j] & (DA - 1)) == dphase;
-  uint64_t head = vec ? ((DA - dphase) % DA) / sizeof(Tout) : 0;
-  if (head > n) head = n;
-  const uint32_t shift = (uint32_t)((sphase + head * sizeof(Tin)) & 15);
-  const uint64_t nPacks = vec ? (n - head) / V : 0;
+  const Lineup l = lineUp(a, nsrc, ndst, n, (int)sizeof(Tin), (int)sizeof(Tout));
+  const uint64_t head = l.head, nPacks = l.nPacks;
+  const uint32_t shift = l.shift;
   const uint64_t srcOff = head * sizeof(Tin), dstOff = head * sizeof(Tout);
   if (nPacks) {
     if (shift == 0) reduceTrips<Tin, Tout, OP, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
@@ -412,6 +513,29 @@ DF_HD void copyTrips(const DataArgs* a, uint64_t nPacks, int ndst, uint64_t off,
   for (; base + step <= nPacks; base += step) copyTrip<true, SHIFT, U>(a, base + tid, nPacks, strideB, ndst, off, shift);
   for (; base + nt <= nPacks; base += nt) copyTrip<true, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);
   if (base + tid < nPacks) copyTrip<false, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);
+}
+
+// Small copies, in the body of the kernel.
+DF_HD void copySmall(const DataArgs* a) {
+  const int tid = df_tid(), nt = df_nthreads(), ndst = a->ndst;
+  const uint64_t n = a->n;
+  const Lineup l = lineUp(a, 1, ndst, n, 1, 1);
+  const uint32_t nPacks = (uint32_t)l.nPacks;
+  const char* src = a->src[0] + l.head - l.shift;
+#pragma unroll 1
+  for (uint32_t p = (uint32_t)tid; p < nPacks; p += (uint32_t)nt) {
+    uint4 v = ld16(src + p * 16u);
+    if (l.shift) v = shiftPack(v, ld16(src + p * 16u + 16), l.shift);
+#pragma unroll 1
+    for (int d = 0; d < ndst; ++d) st16(a->dst[d] + l.head + p * 16u, v);
+  }
+  const uint64_t tail0 = l.head + (uint64_t)nPacks * 16;
+#pragma unroll 1
+  for (uint64_t i = (uint64_t)(nt - 1 - tid); i < l.head + (n - tail0); i += nt) {
+    const uint64_t e = i < l.head ? i : tail0 + (i - l.head);
+    const uint8_t b = ld_elem((const uint8_t*)a->src[0] + e);
+    for (int d = 0; d < ndst; ++d) st_elem((uint8_t*)a->dst[d] + e, b);
+  }
 }
 
 #ifdef DF_DATAPATH_IMPL
@@ -496,6 +620,47 @@ __host__ __device__ bool reduce_dispatch(int inType, int outType, int op, const 
 // Returns false when the (in, out, op) combination is not instantiated.
 __host__ __device__ bool reduce_dispatch(int inType, int outType, int op, const DataArgs* a);
 #endif
+
+#ifdef DF_DATAPATH_SMALL_IMPL
+__host__ __device__ bool reduce_small(int inType, int outType, int op, const DataArgs* a) {
+  if (inType == outType) {
+    switch (inType) {
+#ifndef DF_FAST_BUILD
+      case ncclInt8: return reduceSmall<int8_t, int8_t>(a, op);
+      case ncclUint8: return reduceSmall<uint8_t, uint8_t>(a, op);
+      case ncclInt32: return reduceSmall<int32_t, int32_t>(a, op);
+      case ncclUint32: return reduceSmall<uint32_t, uint32_t>(a, op);
+      case ncclInt64: return reduceSmall<int64_t, int64_t>(a, op);
+      case ncclUint64: return reduceSmall<uint64_t, uint64_t>(a, op);
+      case ncclFloat16: return reduceSmall<__half, __half>(a, op);
+      case ncclFloat64: return reduceSmall<double, double>(a, op);
+#endif
+      case ncclFloat32: return reduceSmall<float, float>(a, op);
+      case ncclBfloat16: return reduceSmall<__nv_bfloat16, __nv_bfloat16>(a, op);
+      default: return false;
+    }
+  }
+  if (op != OP_SUM) return false;
+  if (inType == ncclBfloat16 && outType == ncclFloat32) return reduceSmall<__nv_bfloat16, float>(a, op);
+  if (inType == ncclFloat16 && outType == ncclFloat32) return reduceSmall<__half, float>(a, op);
+  if (inType == ncclFloat32 && outType == ncclBfloat16) return reduceSmall<float, __nv_bfloat16>(a, op);
+  if (inType == ncclFloat32 && outType == ncclFloat16) return reduceSmall<float, __half>(a, op);
+  return false;
+}
+#else
+__host__ __device__ bool reduce_small(int inType, int outType, int op, const DataArgs* a);
+#endif
+
+#define DF_SMALL_TRIPS 4       // calls of at most this many packs per thread and source go through the small bodies
+// What the step engine calls.
+DF_HD bool reduce_block(int inType, int outType, int op, const DataArgs* a) {
+  const bool small = a->n * (uint64_t)dtypeSize(inType) <= (uint64_t)df_nthreads() * 16u * DF_SMALL_TRIPS;
+  if (small && reduce_small(inType, outType, op, a)) return true;
+  return reduce_dispatch(inType, outType, op, a);
+}
+DF_HD void copy_block(const DataArgs* a) {
+  if (a->n <= (uint64_t)df_nthreads() * 16u * DF_SMALL_TRIPS) copySmall(a); else copy_multi(a);
+}
 
 // Host-callable check used at prepare time.
 inline bool reduceSupported(int inType, int outType, int op) {

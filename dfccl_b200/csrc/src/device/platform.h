@@ -204,6 +204,14 @@ DF_HD void fence_acq_rel_sys() {
   __atomic_thread_fence(__ATOMIC_ACQ_REL);
 #endif
 }
+// the same among blocks of this GPU
+DF_HD void fence_acq_rel_gpu() {
+#if DF_DEVICE_CODE
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+#else
+  __atomic_thread_fence(__ATOMIC_ACQ_REL);
+#endif
+}
 DF_HD void fence_gpu() {
 #if DF_DEVICE_CODE
   __threadfence();

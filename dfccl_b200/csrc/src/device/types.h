@@ -15,6 +15,7 @@
 #pragma once
 #include <stdint.h>
 #include <cuda_runtime.h>
+#include "dfccl.h"
 
 #define DF_MAX_RANKS 64        // ranks of one communicator the direct-access engine serves (one NVLink domain: 8 per node, up to 72 in a rack)
 #define DF_MAX_BLOCKS 64       // daemon thread blocks per rank
@@ -47,7 +48,14 @@ struct alignas(32) SqSlot { uint64_t w[4]; };
 #define DF_SQ_PAYLOAD ((1ull << 57) - 1)
 // Tag of ring position `index`: 1..127, so that a slot never written to (all zero) matches nothing; the slot's previous
 // contents are exactly one turn old.
-static __host__ __device__ inline uint64_t sqTag(uint64_t index, uint32_t cap) { return (index / cap) % 127u + 1u; }
+static __host__ __device__ inline int log2Of(uint32_t powerOfTwo) {
+#if defined(__CUDA_ARCH__)
+  return 31 - __clz((int)powerOfTwo);
+#else
+  return __builtin_ctz(powerOfTwo);
+#endif
+}
+static __host__ __device__ inline uint64_t sqTag(uint64_t index, uint32_t cap) { return (uint32_t)(index >> log2Of(cap)) % 127u + 1u; }
 static __host__ __device__ inline SqSlot sqEncode(const Sqe& q, uint64_t tag) {
   SqSlot s;
   s.w[0] = tag << 57 | (uint64_t)(q.flags & 0x1ffu) << 48 | (uint64_t)(q.collId & 0xffff) << 32 | q.epoch;
@@ -75,12 +83,20 @@ static __host__ __device__ inline uint32_t cqeColl(uint64_t e) { return (uint32_
 // ---- per (collective, block, source rank) flag words, written by the source rank
 struct alignas(32) FlagSlot {
   uint64_t arrive;        // epoch of the submission whose offsets are valid
-  uint64_t sendOff;       // source rank's send buffer, offset in its heap
-  uint64_t recvOff;       // source rank's recv buffer, offset in its heap
+  uint64_t sendOff;       // source rank's send buffer, offset in its heap; in the engine's slots under the epoch's tag (offTagged)
+  uint64_t recvOff;       // source rank's recv buffer, offset in its heap, likewise
   uint64_t done;          // epoch whose data movement the source rank finished
 };
 
 // ---- phases of a collective on one block (the saved cursor)
+// An offset carries the low 16 bits of its epoch: whoever finds the tag in the slot of a registered collective has the offset
+// of that submission (what stood there before is exactly one epoch old), in whatever order the words of a slot arrive, so that
+// posting them takes no release among ranks of one device.
+#define DF_OFF_BITS 48
+static __host__ __device__ inline uint64_t offTagged(uint64_t off, uint32_t epoch) { return (off & ((1ull << DF_OFF_BITS) - 1)) | (uint64_t)(epoch & 0xffffu) << DF_OFF_BITS; }
+static __host__ __device__ inline bool offCurrent(uint64_t w, uint32_t epoch) { return (uint32_t)(w >> DF_OFF_BITS) == (epoch & 0xffffu); }
+static __host__ __device__ inline uint64_t offValue(uint64_t w) { return w & ((1ull << DF_OFF_BITS) - 1); }
+
 enum Phase : int32_t {
   PH_TRIGGER = 0,         // bounded wait: local trigger word
   PH_COPY_IN = 1,         // local copy user send buffer -> staging (unregistered buffers)
@@ -111,7 +127,13 @@ struct alignas(16) CollStatic {
                           // relative index only.
   int32_t oneDevice;      // all members are ranks on this GPU, their heaps in its memory: what orders one member's
                           // accesses for another is a fence of GPU scope (0.24 - 0.45 us against 1.4 - 1.8 us)
-  int32_t pad0;
+  int32_t esIn, esOut;    // bytes of an element
+  int32_t reduces;        // the unit of the partition below: elements (reducing kinds) or bytes (copying kinds)
+  // partition, so that no block divides (planColl): block b moves units [per b, per (b + 1)) of `total`, and of such a range
+  // member r owns [perShard r, perShard (r + 1)) in the two-shot schedules; the one range that is neither whole nor empty
+  // is cut at multiples of perShardLast
+  uint64_t total, per, perShard, perShardLast;
+  uint64_t sliceUnits;    // a visit moves at most this many (0: no limit)
   double scale;           // multiplies the reduced value (1.0 = off)
   uint64_t count;         // elements, NCCL convention of the kind
   uint64_t stagingSendOff, stagingRecvOff;      // my heap offsets of staging areas (0 = none)
@@ -127,6 +149,20 @@ struct alignas(16) CollStatic {
   char* peerPush[DF_MAX_RANKS];
   uint64_t pushSlotBytes;
 };
+
+// Fills the fields above from kind, types, count, nranks and nBlocks; sliceBytes as in RankConst.
+inline void planColl(CollStatic* c, uint64_t sliceBytes) {
+  auto size = [](int t) { return t == ncclInt8 || t == ncclUint8 ? 1 : t == ncclFloat16 || t == ncclBfloat16 ? 2 : t == ncclInt32 || t == ncclUint32 || t == ncclFloat32 ? 4 : 8; };
+  c->esIn = size(c->inType); c->esOut = size(c->outType);
+  c->reduces = c->kind == dfcclCollAllReduce || c->kind == dfcclCollReduce || c->kind == dfcclCollReduceScatter;
+  c->total = c->reduces ? c->count : c->count * (uint64_t)c->esIn;
+  auto cut = [](uint64_t total, int parts) { return ((total + parts - 1) / parts + 15) & ~(uint64_t)15; };
+  c->per = cut(c->total, c->nBlocks);
+  c->perShard = cut(c->per, c->nranks);
+  c->perShardLast = c->per ? cut(c->total % c->per, c->nranks) : 0;
+  const uint64_t unit = c->reduces ? (uint64_t)c->esIn : 1, slice = sliceBytes / unit & ~(uint64_t)15;
+  c->sliceUnits = sliceBytes == 0 ? 0 : slice < 16 ? 16 : slice;
+}
 
 #define DF_META_VALID (1u << 16)
 inline uint32_t collMeta(const CollStatic& c) { return c.valid ? DF_META_VALID | (uint32_t)c.nBlocks | (uint32_t)c.blockBase << 8 : 0u; }
@@ -194,14 +230,14 @@ struct BlockSaved {                // survives a voluntary quit (reference: Dyna
 };
 
 // ---- everything the daemon needs for one rank; lives in device memory (host memory for the host backend)
-struct RankDev {
+// What does not change after finalize: every block keeps a copy (BlockShared::k).
+struct RankConst {
   // Submission path: the host writes entries into a ring in pinned memory with plain stores; ONE warp per rank (the
   // service warp of block 0) polls it and copies new entries into the ring in device memory that the blocks poll.
   // (A load of pinned host memory is a PCIe round trip, and such loads from many blocks queue behind one another; a
   // write by the host through stream memory operations costs it a driver call and the device a fence per word.)
   const volatile SqSlot* hostSq;   // null: the host writes devSq itself (host backend)
   volatile SqSlot* devSq;
-  uint64_t svcHead;                // entries the service warp has copied
   uint32_t sqCap;                  // power of two
   uint32_t pad0;
   volatile uint64_t* hostFrontier; // pinned, [nBlocks]: entries consumed by each block (posted stores; flow control for the host)
@@ -209,7 +245,6 @@ struct RankDev {
                                    // writes it with a stream memory operation), the pinned control block otherwise
   // completion path
   volatile uint64_t* hostCq;       // pinned ring read by the poller
-  uint64_t devCqTail;
   uint32_t cqCap;                  // power of two
   uint32_t nBlocks;
   // tables
@@ -224,7 +259,6 @@ struct RankDev {
   BlockSaved* saved;               // [nBlocks]
   DevStats* stats;                 // [nBlocks]
   TraceEvent* trace;               // ring, or null
-  uint64_t traceHead;
   uint32_t traceCap;
   uint32_t maxColls;
   DaemonCtl* ctl;                  // pinned
@@ -232,16 +266,21 @@ struct RankDev {
   uint32_t spinBudget;             // BASE_CTX_SWITCH_THRESHOLD
   uint32_t headTries;              // NUM_TRY_TASKQ_HEAD
   uint32_t recvSuccessFactor;      // RECV_SUCCESS_FACTOR
-  uint32_t exitedBlocks;
-  volatile uint32_t quitting;      // a block left voluntarily during this launch
-  uint32_t saEpoch;                // stream-ordered kernels: number of collectives this communicator has finished (their epoch
-                                   // lives on the device so that a captured launch finds the right one at every replay)
   uint64_t idleQuitNs;             // leave after this long with an empty task queue and no new entry
   uint64_t stallQuitNs;            // leave after this long with only stalled collectives
   uint64_t trigQuitNs;             // leave after this long with nothing but submissions that wait for their stream
   uint64_t waitTimeoutNs;          // a single wait older than this fails with ST_TIMEOUT (0 = never)
   uint64_t maxLifetimeNs;          // one launch of the daemon leaves after this long regardless of its state (0 = never)
   uint64_t sliceBytes;             // PH_DATA yields after this many bytes when others are queued (0 = never)
+};
+struct RankDev : RankConst {
+  uint64_t svcHead;                // entries the service warp has copied
+  uint64_t devCqTail;
+  uint64_t traceHead;
+  uint32_t exitedBlocks;
+  volatile uint32_t quitting;      // a block left voluntarily during this launch
+  uint32_t saEpoch;                // stream-ordered kernels: number of collectives this communicator has finished (their epoch
+                                   // lives on the device so that a captured launch finds the right one at every replay)
 };
 
 }  // namespace dfccl
