@@ -6,11 +6,14 @@
 // thread and all four loads before the first store, so that 5 resident blocks (48 registers a thread) keep 80 KB per SM in
 // flight; calls too small to give every SM such a block take one pack per thread instead (more blocks, shorter chains).
 // Measured: all-reduce of 8388611 fp32 values in ordinary tensors 13.4 us = 5.0 TB/s read + write; the collective kernel
-// that stages such buffers into the heap and out again on 64 blocks took 64.7 us.  bf16 -> fp32 packs are stored as whole
+// that stages such buffers into the heap and out again on 64 blocks took 64.7 us; 11.3 with blocks that come up behind the
+// kernel in front (below).  Eight calls of 64 KB one behind the other in a stream, submitted and awaited: 61.0 us, with one
+// cluster a call and early blocks 41.6.  bf16 -> fp32 packs are stored as whole
 // 32-byte sectors: with that (and the shorter publication) three gradient buckets of 51 MB and their SGD step went from 186
 // to 172 us, 25 MiB among four ranks through the daemon's data path, which stores alike, from 112 to 106.
 #include "../device/engine.h"
 #include "../device/launch.h"
+#include "../gemm/tc_common.h"
 #include "../common/log.h"
 #include <algorithm>
 
@@ -18,6 +21,7 @@ namespace dfccl {
 namespace {
 
 constexpr int THREADS = 256;
+constexpr int CLUSTER = 8;                 // blocks of a short registered collective: one cluster
 
 struct OneRankArgs {
   const char* src;
@@ -47,22 +51,29 @@ __device__ __forceinline__ void publishDone(const OneRankDone& done) {
   st_relaxed_sys_u64(&rd->hostCq[idx & (rd->cqCap - 1)], cqeEncode((uint32_t)(idx / rd->cqCap) + 1u, ST_OK, (uint32_t)done.coll));
 }
 
-template <typename Tin, typename Tout, bool COPY, int U>
+// SHORT: the whole call is one cluster of blocks, which meet at the cluster's barrier before one thread publishes, instead of
+// counting themselves in global memory (a fence and an atomic, two round trips to L2 at the end of a kernel that moves 64 KB).
+// The blocks may come up while the kernel in front of them in the stream still runs, and wait for its end before they read.
+template <typename Tin, typename Tout, bool COPY, int U, bool SHORT>
 __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs a) {
   typedef typename Elem<Tin>::Acc A;
   constexpr int V = 16 / (int)sizeof(Tin);
   constexpr int OUTB = V * (int)sizeof(Tout);
   constexpr int NW = (OUTB + 15) / 16;
-  const uint64_t p0 = (uint64_t)blockIdx.x * (THREADS * U) + threadIdx.x;
+  // (a cluster shares out every THREADS packs, so that all of its SMs load)
+  constexpr int STEP = SHORT ? CLUSTER * THREADS : THREADS;
+  const uint64_t p0 = (uint64_t)blockIdx.x * (SHORT ? THREADS : THREADS * U) + threadIdx.x;
   const uint4* s = (const uint4*)(a.src + a.head * sizeof(Tin));
   char* d = a.dst + a.head * sizeof(Tout);
+  tc::grid_dependency_wait();
+  tc::grid_launch_dependents();
   uint4 v[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) if (p0 + u * THREADS < a.nPacks) v[u] = s[p0 + u * THREADS];
+  for (int u = 0; u < U; ++u) if (p0 + u * STEP < a.nPacks) v[u] = s[p0 + u * STEP];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    if (p0 + u * THREADS >= a.nPacks) continue;
-    char* o = d + (p0 + u * THREADS) * OUTB;
+    if (p0 + u * STEP >= a.nPacks) continue;
+    char* o = d + (p0 + u * STEP) * OUTB;
     if (COPY) { *(uint4*)o = v[u]; continue; }
     A r[V];
 #pragma unroll
@@ -88,6 +99,11 @@ __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs 
   for (uint64_t i = (uint64_t)blockIdx.x * THREADS + threadIdx.x; i < rest; i += (uint64_t)gridDim.x * THREADS) {
     const uint64_t e = i < a.head ? i : tail0 + (i - a.head);
     if (COPY) a.dst[e] = a.src[e]; else oneElem<Tin, Tout>(a, e);
+  }
+  if (SHORT) {
+    tc::cluster_sync_all();
+    if (blockIdx.x == 0 && threadIdx.x == 0) publishDone(a.done);
+    return;
   }
   if (a.done.rd == nullptr) return;
   // The last block out publishes the completion, as the daemon's blocks do, but with one system-wide fence for the device
@@ -134,14 +150,23 @@ ncclResult_t launchTyped(OneRankArgs a, int sms, cudaStream_t stream) {
   a.nPacks = vec ? (a.n - head) / V : 0;
   const uint64_t loose = a.n - a.nPacks * V;
   const uint64_t looseBlocks = std::min<uint64_t>((loose + THREADS - 1) / THREADS, (uint64_t)sms * 8);
-  if (a.nPacks >= (uint64_t)sms * THREADS * 4) {
-    const uint64_t grid = std::max((a.nPacks + THREADS * 4 - 1) / (THREADS * 4), looseBlocks);
-    dfcclOneRankKernel<Tin, Tout, COPY, 4><<<(unsigned)grid, THREADS, 0, stream>>>(a);
-  } else {
-    const uint64_t grid = std::max<uint64_t>(1, std::max((a.nPacks + THREADS - 1) / THREADS, looseBlocks));
-    dfcclOneRankKernel<Tin, Tout, COPY, 1><<<(unsigned)grid, THREADS, 0, stream>>>(a);
+  void (*kernel)(const OneRankArgs) = dfcclOneRankKernel<Tin, Tout, COPY, 1, false>;
+  uint64_t grid = std::max<uint64_t>(1, std::max((a.nPacks + THREADS - 1) / THREADS, looseBlocks));
+  int cluster = 1;
+  if (a.done.rd && a.nPacks <= CLUSTER * THREADS * 4 && looseBlocks <= CLUSTER) {
+    kernel = dfcclOneRankKernel<Tin, Tout, COPY, 4, true>;
+    grid = cluster = CLUSTER;
+  } else if (a.nPacks >= (uint64_t)sms * THREADS * 4) {
+    kernel = dfcclOneRankKernel<Tin, Tout, COPY, 4, false>;
+    grid = std::max((a.nPacks + THREADS * 4 - 1) / (THREADS * 4), looseBlocks);
   }
-  CUDACHECK(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(THREADS); cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
+  CUDACHECK(cudaLaunchKernelEx(&cfg, kernel, a));
   return ncclSuccess;
 }
 
