@@ -73,8 +73,7 @@ def column_sum(g: torch.Tensor) -> torch.Tensor:
     rows, n = g.shape
     out = torch.empty(n, dtype=torch.bfloat16, device=g.device)
     with on_device(g.device):
-        work = torch.empty(nv.lib().dfcclColumnSumWork(rows, n), dtype=torch.float32, device=g.device)
-        nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), work.data_ptr(), rows, n, raw_stream(g.device)), "dfcclColumnSum")
+        nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), None, rows, n, raw_stream(g.device)), "dfcclColumnSum")
     return out
 
 
