@@ -514,7 +514,6 @@ DF_API ncclResult_t ofcclFinalizeRankCtx7StartHostThrds(ofcclRankCtx_t ctx) {
   DFCHECK(devAlloc(be, (void**)&rd.colls, sizeof(CollStatic) * maxColls));
   DFCHECK(devAlloc(be, (void**)&rd.dyn, sizeof(CollDyn) * (size_t)maxColls * ctx->nBlocks));
   DFCHECK(devAlloc(be, (void**)&rd.doneCount, sizeof(uint32_t) * maxColls));
-  DFCHECK(devAlloc(be, (void**)&rd.failCount, sizeof(uint32_t) * maxColls));
   DFCHECK(devAlloc(be, (void**)&rd.doneEpoch, sizeof(uint64_t) * maxColls));
   DFCHECK(devAlloc(be, (void**)&rd.trigger, sizeof(uint64_t) * maxColls));
   DFCHECK(devAlloc(be, (void**)&rd.saved, sizeof(BlockSaved) * ctx->nBlocks));
@@ -1106,7 +1105,7 @@ static void releaseCtx(ofcclRankCtx* ctx) {
   if (ctx->wakeStream) { cudaStreamSynchronize(ctx->wakeStream); cudaStreamDestroy(ctx->wakeStream); }
   for (auto e : ctx->wakeEvents) cudaEventDestroy(e);
   RankDev& rd = ctx->rdHost;
-  devFree(be, (void*)rd.devSq); devFree(be, rd.colls); devFree(be, rd.meta); devFree(be, rd.dyn); devFree(be, rd.doneCount); devFree(be, rd.failCount);
+  devFree(be, (void*)rd.devSq); devFree(be, rd.colls); devFree(be, rd.meta); devFree(be, rd.dyn); devFree(be, rd.doneCount);
   devFree(be, (void*)rd.doneEpoch); devFree(be, (void*)rd.trigger); devFree(be, rd.saved); devFree(be, rd.stats); devFree(be, rd.trace);
   devFree(be, ctx->rdDev);
   if (ctx->hostSq) pinnedFree(be, (void*)ctx->hostSq);

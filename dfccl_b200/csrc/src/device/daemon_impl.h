@@ -294,7 +294,10 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
       // the words of global memory this section looks at: on their way together
       const uint32_t left = ld_relaxed_sys_u32(&rd->quitting);
       SqSlot slot, next;
-      const bool haveNext = sqPeek(&sh->k, sh->frontier + 1, &next), have = sqPeek(&sh->k, sh->frontier, &slot);
+      bool haveNext = sqPeek(&sh->k, sh->frontier + 1, &next), have = sqPeek(&sh->k, sh->frontier, &slot);
+      // with nothing else to do a look at the ring costs a round trip to L2, a pass several
+      if (!progressed && sh->nActive == 0 && sh->nTrig == 0)
+        for (int i = 0; i < 8 && !have; ++i) have = sqPeek(&sh->k, sh->frontier, &slot);
       uint32_t w = 0, parked = 0;
       for (uint32_t i = 0; i < sh->nActive; ++i) if (sh->active[i] != 0xffff) { sh->active[w] = sh->active[i]; sh->actWait[w] = sh->actWait[i]; parked += sh->actWait[i] != 0; ++w; }
       sh->nActive = w; sh->nParked = parked; sh->nReady = 0;

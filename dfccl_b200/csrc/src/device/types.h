@@ -252,8 +252,9 @@ struct RankConst {
   uint32_t* meta;                  // [maxColls] what a block needs to know to take or skip an entry: nBlocks | blockBase << 8 |
                                    // DF_META_VALID; never written after finalize
   CollDyn* dyn;                    // [nBlocks][maxColls]
-  uint32_t* doneCount;             // [maxColls] blocks that finished the current submission
-  uint32_t* failCount;             // [maxColls] of those, how many ended with an error
+  uint32_t* doneCount;             // [maxColls] blocks that finished the current submission: [7:0] how many, [15:8] of those, how many
+                                   // with an error, [31:16] the sum of their statuses (a collective that runs in its stream
+                                   // counts its kernel's blocks here)
   volatile uint64_t* doneEpoch;    // [maxColls] device flag: epoch of the last finished submission
   volatile uint64_t* trigger;      // [maxColls] device flag written by stream memory operations
   BlockSaved* saved;               // [nBlocks]
