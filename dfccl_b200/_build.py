@@ -21,6 +21,7 @@ CSRC = ROOT / "csrc"
 OBJ = CSRC / "build"
 LIBDIR = ROOT / "lib"
 LIB = LIBDIR / "libdfccl.so"
+HOSTCALL = LIBDIR / "dfccl_hostcall.so"          # Python extension: calls of the hot entry points without ctypes
 
 SOURCES = [
     "src/common/log.cc", "src/common/param.cc", "src/common/socket.cc",
@@ -79,6 +80,21 @@ def _compile(src: str, verbose: bool, hdr_time: float, sanitize: str = "") -> Pa
     return o
 
 
+def build_hostcall() -> Path:
+    """Compile the extension module of ``native.entry`` for the running interpreter's headers (stable ABI)."""
+    import sysconfig
+    src = CSRC / "src" / "python" / "hostcall.c"
+    if not HOSTCALL.exists() or HOSTCALL.stat().st_mtime < src.stat().st_mtime:
+        LIBDIR.mkdir(parents=True, exist_ok=True)
+        tmp = LIBDIR / f".hostcall.{os.getpid()}.so"             # several processes may find it missing: each makes its own
+        cmd = ["gcc", "-O2", "-shared", "-fPIC", "-Wall", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(tmp)]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"gcc failed for {src}:\n{r.stdout}\n{r.stderr}")
+        os.replace(tmp, HOSTCALL)
+    return HOSTCALL
+
+
 def build(verbose: bool = False, force: bool = False, extra_sources=(), sanitize: str = "") -> Path:
     """Compile what is stale and link ``libdfccl.so``; returns its path.
 
@@ -94,6 +110,7 @@ def build(verbose: bool = False, force: bool = False, extra_sources=(), sanitize
     srcs = [s for s in list(SOURCES) + list(extra_sources) if (CSRC / s).exists()]
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
         objs = list(ex.map(lambda s: _compile(s, verbose, hdr, sanitize), srcs))
+    build_hostcall()
     lib = LIBDIR / f"libdfccl_{sanitize}.so" if sanitize else LIB
     if lib.exists() and all(lib.stat().st_mtime > o.stat().st_mtime for o in objs):
         return lib

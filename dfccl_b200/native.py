@@ -8,6 +8,9 @@ unloadable library is an error, never a silent fallback to Python code.
 from __future__ import annotations
 
 import ctypes as C
+import functools
+import importlib.machinery
+import importlib.util
 import os
 import threading
 from typing import Callable, Dict, List, Optional, Sequence
@@ -70,11 +73,31 @@ class DfcclError(RuntimeError):
 
 _lib = None
 _lock = threading.Lock()
+_entries: Dict[str, Callable[..., int]] = {}
+
+
+def _load_hostcall():
+    path = _build.HOSTCALL if _build.HOSTCALL.exists() else _build.build_hostcall()
+    loader = importlib.machinery.ExtensionFileLoader("dfccl_hostcall", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("dfccl_hostcall", loader))
+    loader.exec_module(module)
+    return module
+
+
+def entry(name: str) -> Callable[..., int]:
+    """The entry point ``name`` as a callable of integers, addresses and ``None`` (for all of its arguments), without the cost of
+    a ctypes call.  Other argument types are a ``TypeError``; ``lib()`` still takes them."""
+    f = _entries.get(name)
+    if f is None:
+        f = _entries[name] = functools.partial(_load_hostcall().call, C.cast(getattr(lib(), name), C.c_void_p).value)
+    return f
 
 
 def lib() -> C.CDLL:
     """Load (building first if necessary) and return the native library."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -368,6 +391,9 @@ class RankCtx:
         h = C.c_void_p()
         check(lib().dfcclInitRankCtxOnDevice(C.byref(h), rank, device), "ofcclInitRankCtx")
         self.handle = h
+        self._h = h.value
+        self._run, self._run_on_stream, self._stream_wait = entry("dfcclRun"), entry("dfcclRunOnStream"), entry("dfcclStreamWait")
+        self._wait = entry("dfcclWait")
         self._callbacks: Dict[int, object] = {}
         self._live = True
 
@@ -401,19 +427,26 @@ class RankCtx:
         check(lib().ofcclFinalizeRankCtx7StartHostThrds(self.handle), "ofcclFinalizeRankCtx7StartHostThrds")
 
     def run(self, coll_id: int, send: int, recv: int, callback: Optional[Callable[[int], None]] = None) -> None:
-        cb = NO_CALLBACK
-        if callback is not None:
+        if callback is None:
+            try:
+                r = self._run(send, recv, coll_id, None, None, self._h)
+            except TypeError:                      # an argument that only ctypes converts
+                r = _lib.dfcclRun(send, recv, coll_id, NO_CALLBACK, None, self.handle)
+        else:
             def tramp(cid, _args, _f=callback):
                 _f(cid)
                 return 0
             cb = CALLBACK(tramp)
             self._callbacks[coll_id] = cb          # keep the trampoline alive until the next submit of this id
-        r = _lib.dfcclRun(send, recv, coll_id, cb, None, self.handle)
+            r = _lib.dfcclRun(send, recv, coll_id, cb, None, self.handle)
         if r != SUCCESS:
             raise DfcclError(r, f"dfcclRun({coll_id})")
 
     def run_on_stream(self, coll_id: int, send: int, recv: int, stream: int) -> None:
-        r = _lib.dfcclRunOnStream(send, recv, coll_id, stream, NO_CALLBACK, None, self.handle)
+        try:
+            r = self._run_on_stream(send, recv, coll_id, stream, None, None, self._h)
+        except TypeError:
+            r = _lib.dfcclRunOnStream(send, recv, coll_id, stream, NO_CALLBACK, None, self.handle)
         if r != SUCCESS:
             raise DfcclError(r, f"dfcclRunOnStream({coll_id})")
 
@@ -426,12 +459,18 @@ class RankCtx:
         check(lib().dfcclTriggerOnStream(coll_id, C.c_void_p(stream), self.handle), f"dfcclTriggerOnStream({coll_id})")
 
     def stream_wait(self, coll_id: int, stream: int) -> None:
-        r = _lib.dfcclStreamWait(coll_id, stream, self.handle)
+        try:
+            r = self._stream_wait(coll_id, stream, self._h)
+        except TypeError:
+            r = _lib.dfcclStreamWait(coll_id, stream, self.handle)
         if r != SUCCESS:
             raise DfcclError(r, f"dfcclStreamWait({coll_id})")
 
     def wait(self, coll_id: int, timeout_ms: int = -1) -> int:
-        return lib().dfcclWait(coll_id, timeout_ms, self.handle)
+        try:
+            return self._wait(coll_id, timeout_ms, self._h)
+        except TypeError:
+            return lib().dfcclWait(coll_id, timeout_ms, self.handle)
 
     def wait_all(self, timeout_ms: int = -1) -> int:
         return lib().dfcclWaitAll(timeout_ms, self.handle)

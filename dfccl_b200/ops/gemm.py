@@ -28,8 +28,9 @@ def matmul_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None)
         raise ValueError(f"tcgen05 GEMM needs M % {BM} == 0, N % {BN} == 0, K % {BK} == 0, got {m} x {n} x {k}")
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
-    nv.check(nv.lib().dfcclGemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k,
-                                    raw_stream(a.device)), "dfcclGemmBf16")
+    r = nv.entry("dfcclGemmBf16")(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, raw_stream(a.device))
+    if r:
+        nv.check(r, "dfcclGemmBf16")
     return out
 
 
@@ -48,8 +49,10 @@ def matmul(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *,
         raise ValueError(f"tcgen05 GEMM needs M % {BM} == 0, N % {BN} == 0, K % {BK} == 0, got {m} x {n} x {k}")
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
-    nv.check(nv.lib().dfcclGemmBf16Ex(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_transposed), int(b_transposed),
-                                      raw_stream(a.device)), "dfcclGemmBf16Ex")
+    r = nv.entry("dfcclGemmBf16Ex")(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_transposed), int(b_transposed),
+                                    raw_stream(a.device))
+    if r:
+        nv.check(r, "dfcclGemmBf16Ex")
     return out
 
 
