@@ -9,7 +9,9 @@
 // One launch takes all buckets of a step (a grid of one bucket after the other leaves a ramp up and down of the GPU per
 // bucket, and a host call), and clears the buckets' gradients on the way: they sit in arrays of their own that nobody needs
 // after the all-reduce, and a fill of its own would be one more launch per bucket.
-// Bound: HBM.  22 (SGD) or 30 (AdamW) bytes per element with bf16 parameters, 2 more for the gradient.
+// Bound: HBM.  22 (SGD) or 30 (AdamW) bytes per element with bf16 parameters, 2 more for the gradient.  What only this kernel
+// touches (master weights, moments, the cleared gradients) streams through L2 first to be evicted, so that the reduced gradients the
+// all-reduce has just written are still there: ResNet-50's three buckets, all-reduce and SGD, 168.5 -> 165.5 us, with blocks that come up early 163.5.
 // No counterpart in the reference, which has no optimizer (it is a collective library); this kernel exists so that the
 // gradient path of the benchmarks never leaves flat, heap-resident buffers.
 #include <cuda_bf16.h>
@@ -18,6 +20,7 @@
 #include <stdint.h>
 #include "dfccl.h"
 #include "dfccl_ops.h"
+#include "../gemm/tc_common.h"
 
 namespace {
 
@@ -69,10 +72,10 @@ __device__ __forceinline__ void updateBlock(const OptimArgs& a, const dfcclOptim
   for (int u = 0; u < UNROLL; ++u) {
     const size_t i = i0 + u * THREADS * 4;
     if (i >= nFull) continue;
-    w[u] = *(const float4*)(master + i);
+    w[u] = __ldcs((const float4*)(master + i));
     g[u] = *(const float4*)(grad + i);
-    m[u] = fresh ? zero : *(const float4*)(m1 + i);
-    if (ADAMW) v[u] = *(const float4*)(m2 + i);
+    m[u] = fresh ? zero : __ldcs((const float4*)(m1 + i));
+    if (ADAMW) v[u] = __ldcs((const float4*)(m2 + i));
   }
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) {
@@ -83,19 +86,19 @@ __device__ __forceinline__ void updateBlock(const OptimArgs& a, const dfcclOptim
       adamwOne(w[u].y, g[u].y, m[u].y, v[u].y, a.b1, a.b2, a.eps, decay, a.stepSize, a.invBias2Sqrt);
       adamwOne(w[u].z, g[u].z, m[u].z, v[u].z, a.b1, a.b2, a.eps, decay, a.stepSize, a.invBias2Sqrt);
       adamwOne(w[u].w, g[u].w, m[u].w, v[u].w, a.b1, a.b2, a.eps, decay, a.stepSize, a.invBias2Sqrt);
-      *(float4*)(m2 + i) = v[u];
+      __stcs((float4*)(m2 + i), v[u]);
     } else {
       sgdOne(w[u].x, g[u].x, m[u].x, a.b1, a.lr, a.wd);
       sgdOne(w[u].y, g[u].y, m[u].y, a.b1, a.lr, a.wd);
       sgdOne(w[u].z, g[u].z, m[u].z, a.b1, a.lr, a.wd);
       sgdOne(w[u].w, g[u].w, m[u].w, a.b1, a.lr, a.wd);
     }
-    *(float4*)(master + i) = w[u];
-    *(float4*)(m1 + i) = m[u];
+    __stcs((float4*)(master + i), w[u]);
+    __stcs((float4*)(m1 + i), m[u]);
     if (sizeof(P) == 2) {
       const __nv_bfloat162 lo = __floats2bfloat162_rn(w[u].x, w[u].y), hi = __floats2bfloat162_rn(w[u].z, w[u].w);
       *(uint2*)(param + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-      if (clear) *(uint2*)(clear + i) = make_uint2(0u, 0u);
+      if (clear) __stcs((uint2*)(clear + i), make_uint2(0u, 0u));
     } else {
       *(float4*)(param + i) = w[u];
       if (clear) *(float4*)(clear + i) = zero;
@@ -118,6 +121,8 @@ __device__ __forceinline__ void updateBlock(const OptimArgs& a, const dfcclOptim
 
 template <bool ADAMW>
 __global__ void __launch_bounds__(THREADS) optimKernel(const __grid_constant__ OptimArgs a) {
+  dfccl::tc::grid_dependency_wait();                     // the blocks come up while the kernel in front drains
+  dfccl::tc::grid_launch_dependents();
   int j = 0;
   while (j + 1 < a.n && blockIdx.x >= a.firstBlock[j + 1]) ++j;
   const dfcclOptimBucket& k = a.b[j];
@@ -149,7 +154,13 @@ ncclResult_t run(OptimArgs& a, const dfcclOptimBucket* buckets, int n, cudaStrea
       a.firstBlock[a.n++] = (uint32_t)blocks;
       blocks += more;
     }
-    if (a.n) optimKernel<ADAMW><<<(unsigned)blocks, THREADS, 0, stream>>>(a);
+    if (!a.n) continue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks); cfg.blockDim = dim3(THREADS); cfg.stream = stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, optimKernel<ADAMW>, a) != cudaSuccess) { (void)cudaGetLastError(); return ncclUnhandledCudaError; }
   }
   return cudaGetLastError() == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
 }
