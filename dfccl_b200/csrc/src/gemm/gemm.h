@@ -39,20 +39,20 @@ struct FusedArgs {
 // stored with the contraction index slow (A as [K, M], B as [K, N], row-major) and read by the tensor cores as it is.
 ncclResult_t gemmLaunch(const void* A, const void* B, void* C, int M, int N, int K, const FusedArgs* f, cudaStream_t stream,
                         int aMn = 0, int bMn = 0);
-// Plain GEMMs: what runs them.  tn = 0: the persistent CTA-pair kernel (cta_group::2, tiles of 256 x 256); otherwise one tile of
-// 128 or (pair) 256 rows x tn columns, or one of `split` slices of its contraction, per CTA or CTA pair.
-struct GemmTilePlan { bool pair; int tn, split; };
-GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs);
+// Plain GEMMs: what runs them.  width > 0: the persistent CTA-pair kernel (cta_group::2) with tiles of 256 x width; otherwise one
+// tile of 128 or (pair) 256 rows x tn columns, or one of `split` slices of its contraction, per CTA or CTA pair.
+struct GemmTilePlan { bool pair; int tn, split, width; };
+GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs, bool bMn, bool epilogue);
 ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream,
                             int aMn, int bMn, uint32_t* errDev, uint32_t* errHost);
 int gemmPairResident();
 struct GemmEpilogue;
-ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
+ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
                             uint32_t* errDev, uint32_t* errHost, const GemmEpilogue* e);
 // The same pass over a finished bf16 product C [M, N], in place (csrc/src/ops/block.cu).
 ncclResult_t applyEpilogue(const GemmEpilogue& e, void* C, int M, int N, cudaStream_t stream);
-// Cached tensor map of a row-major bf16 matrix [rows, cols] cut into boxes of boxRows x 64 columns, 128-byte swizzle.
-ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows);
+// Cached tensor map of a row-major bf16 matrix [rows, cols] cut into boxes of boxRows x 64 columns (128-byte swizzle) or x 32 (64-byte).
+ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows, uint32_t boxCols = 64);
 // The same for whole operands of a stage in one load: a K-major matrix [rows, k] as (64, rows, k / 64) with boxes of
 // 64 x boxRows x boxK / 64, an MN-major one ([k, rows] as stored) as (64, k, rows / 64) with boxes of 64 x boxK x boxRows / 64.
 ncclResult_t gemmMakeMap3(CUtensorMap* m, const void* base, uint64_t rows, uint64_t k, int mnMajor, uint32_t boxRows, uint32_t boxK);

@@ -76,6 +76,22 @@ __device__ __forceinline__ void tma_load_2d(void* smemDst, const CUtensorMap* ma
       ::"r"(smem_u32(smemDst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
+// Tile load of a 3-D map: x always 0, one instruction for a whole operand of a stage.
+__device__ __forceinline__ void tma_load_3d(void* smemDst, const CUtensorMap* map, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smemDst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(y), "r"(z)
+      : "memory");
+}
+// Tile store shared -> global, counted in the issuing thread's bulk groups; what lies outside the matrix is not written.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smemSrc, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(map), "r"(smem_u32(smemSrc)), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+// Shared memory written by ordinary stores, before a bulk copy reads it.
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -170,6 +186,12 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smemDst, const CUtensorMa
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(smemDst)), "l"(map), "r"(barClusterAddr), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* smemDst, const CUtensorMap* map, int y, int z, uint32_t barClusterAddr) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smemDst)), "l"(map), "r"(barClusterAddr), "r"(0), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smemResult, uint32_t ncols) {       // one full warp in EACH CTA of the pair

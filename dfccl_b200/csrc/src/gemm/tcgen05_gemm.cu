@@ -433,9 +433,9 @@ EncodeTiled encodeFn() {
 struct MapKey {
   const void* base;
   uint64_t d1, d2, s1;               // extents above the innermost one and the byte stride of the second dimension
-  uint32_t d0, b1, b2;               // innermost extent; box above the innermost 64 columns (b2 = 0: a 2-D map)
+  uint32_t d0, b0, b1, b2;           // innermost extent; box (b0: 64 columns, swizzled over 128 bytes, or 32 over 64; b2 = 0: a 2-D map)
   bool operator<(const MapKey& o) const {
-    return std::tie(base, d0, d1, d2, s1, b1, b2) < std::tie(o.base, o.d0, o.d1, o.d2, o.s1, o.b1, o.b2);
+    return std::tie(base, d0, d1, d2, s1, b0, b1, b2) < std::tie(o.base, o.d0, o.d1, o.d2, o.s1, o.b0, o.b1, o.b2);
   }
 };
 
@@ -444,10 +444,10 @@ ncclResult_t encodeMap(CUtensorMap* m, const MapKey& k) {
   if (!fn) { DF_WARN("cuTensorMapEncodeTiled is not available"); return ncclSystemError; }
   cuuint64_t dims[3] = {k.d0, k.d1, k.d2};
   cuuint64_t strides[2] = {k.s1, 128};
-  cuuint32_t box[3] = {BK, k.b1, k.b2};
+  cuuint32_t box[3] = {k.b0, k.b1, k.b2};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k.b2 ? 3 : 2, (void*)k.base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  k.b0 == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     DF_WARN("cuTensorMapEncodeTiled failed (%d) for %llu x %llu at %p", (int)r, (unsigned long long)k.d1, (unsigned long long)(k.d2 ? k.d2 * 64 : k.d0), k.base);
     return ncclInvalidArgument;
@@ -470,9 +470,9 @@ ncclResult_t cachedMap(CUtensorMap* m, const MapKey& k) {
   return ncclSuccess;
 }
 
-// rows x cols bf16, row-major (cols contiguous), tiles of boxRows x 64 columns, 128-byte swizzle
-ncclResult_t makeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows) {
-  return cachedMap(m, MapKey{base, rows, 0, cols * 2, (uint32_t)cols, boxRows, 0});
+// rows x cols bf16, row-major (cols contiguous), tiles of boxRows x 64 columns (128-byte swizzle) or 32 (64-byte swizzle)
+ncclResult_t makeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows, uint32_t boxCols = BK) {
+  return cachedMap(m, MapKey{base, rows, 0, cols * 2, (uint32_t)cols, boxCols, boxRows, 0});
 }
 
 std::atomic<int> g_reservedSms{0};
@@ -508,8 +508,8 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!f || f->mode == 0 || f->nranks <= 1) {
-    const GemmTilePlan p = gemmTilePlan(M, N, K, sms, paramI64("GEMM_PAIR", 1) != 0);
-    if (p.tn == 0) return gemmPairLaunch(A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host, e);
+    const GemmTilePlan p = gemmTilePlan(M, N, K, sms, paramI64("GEMM_PAIR", 1) != 0, bMn != 0, e && e->kind);
+    if (p.width) return gemmPairLaunch(p.width, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host, e);
     DFCHECK(gemmTileLaunch(p, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host));
     return e && e->kind ? applyEpilogue(*e, C, M, N, stream) : ncclSuccess;
   }
@@ -535,9 +535,9 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
 
 }  // namespace
 
-ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows) { return makeMap(m, base, rows, cols, boxRows); }
+ncclResult_t gemmMakeMap(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t boxRows, uint32_t boxCols) { return makeMap(m, base, rows, cols, boxRows, boxCols); }
 ncclResult_t gemmMakeMap3(CUtensorMap* m, const void* base, uint64_t rows, uint64_t k, int mnMajor, uint32_t boxRows, uint32_t boxK) {
-  return cachedMap(m, mnMajor ? MapKey{base, k, rows / 64, rows * 2, 64, boxK, boxRows / 64} : MapKey{base, rows, k / 64, k * 2, 64, boxRows, boxK / 64});
+  return cachedMap(m, mnMajor ? MapKey{base, k, rows / 64, rows * 2, 64, 64, boxK, boxRows / 64} : MapKey{base, rows, k / 64, k * 2, 64, 64, boxRows, boxK / 64});
 }
 ncclResult_t gemmLaunch(const void* A, const void* B, void* C, int M, int N, int K, const FusedArgs* f, cudaStream_t stream, int aMn, int bMn) {
   return launch(A, B, C, M, N, K, f, stream, aMn, bMn);

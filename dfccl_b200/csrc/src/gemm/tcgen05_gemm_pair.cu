@@ -1,15 +1,19 @@
 // bf16 GEMM on CTA pairs (tcgen05 cta_group::2), hand-written for sm_100a:
-//     C[M,N] = A[M,K] * B[N,K]^T,  tiles of 256 x 256, one tile per pair of CTAs (a cluster of two SMs).  Rows of the last
-//     row tile beyond M (M is a multiple of 128) are loaded as zeros and not stored.
-// Each CTA of a pair loads 128 rows of A and 128 rows of B per 64-wide K block (32 KB per stage instead of the 48 KB
-// of the one-CTA form, so six stages fit), the leader's single MMA thread issues 256 x 256 x 16 instructions that read
-// both CTAs' shared memory, and each CTA ends up with its 128 rows of the accumulator in its own tensor memory.
-// The tensor cores of an SM thus see every B row once per pair instead of once per CTA: half the shared-memory
-// operand traffic per FLOP, which is what bounds the one-CTA kernel.
+//     C[M,N] = A[M,K] * B[N,K]^T,  tiles of 256 x tn (tn a multiple of 32, chosen per product), one tile per pair of CTAs (a
+// cluster of two SMs) at a time.  Rows and columns of the last tiles beyond M (a multiple of 128) and N are loaded as zeros
+// and not stored.
+// Each CTA of a pair loads 128 rows of A and tn / 2 rows of B per stage (64 or 128 of the contraction), the leader's single MMA thread issues
+// 256 x tn x 16 instructions that read both CTAs' shared memory, and each CTA ends up with its 128 rows of the accumulator
+// in its own tensor memory.  The tensor cores of an SM thus see every B row once per pair instead of once per CTA: half the
+// shared-memory operand traffic per FLOP, which is what bounds a one-CTA kernel.
+// The width of a tile is what fits the number of tiles to the number of pairs: 3072 x 1024 outputs are 48 tiles of 256 x 256
+// on 74 pairs, or 72 of 256 x 192.
 //
 // Roles per CTA: warp 0 = TMA producer (one elected thread; completion of both CTAs' loads is counted on the
-// LEADER's barrier), warp 1 = tensor-memory owner, and in the leader the MMA issuer; warps 2-9 = epilogue over the
-// CTA's own accumulator half.  Stages are released and accumulators handed over with tcgen05.commit to both CTAs;
+// LEADER's barrier), warp 1 = tensor-memory owner, and in the leader the MMA issuer; the other warps = epilogue over the
+// CTA's own accumulator half, 32 rows x 32 columns at a time: tensor memory -> registers -> global memory, through boxes in
+// shared memory and TMA stores where the epilogue is what a tile waits for (gemmPairLaunch).
+// Stages are released and accumulators handed over with tcgen05.commit to both CTAs;
 // the epilogues of both CTAs arrive on the leader's accumulator-empty barrier.  No TMA load uses cluster multicast.
 // Every wait is bounded and ends in the error word of the device.
 //
@@ -29,46 +33,58 @@ namespace {
 
 using namespace tc;
 
-constexpr int PM = 256, PN = 256, BK = 64, HALF = 128, STAGES = 6, UMMA_K = 16;
-constexpr int A_BYTES = HALF * BK * 2, B_BYTES = HALF * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;   // per CTA
-constexpr int MN_BLOCK_BYTES = 64 * BK * 2;
-constexpr int TMEM_COLS = 512;                       // two accumulators of 256 fp32 columns (128 lanes each, per CTA)
-constexpr int NUM_THREADS = 320;                     // 10 warps
-constexpr int EPI_WARPS = 8;                         // two per 32 accumulator rows: the last tile's epilogue is not overlapped with anything
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+constexpr int PM = 256, HALF = 128, MAX_STAGES = 6, UMMA_K = 16;
+constexpr int SMEM_LIMIT = 227 * 1024, BAR_BYTES = 256, ALIGN_SLACK = 1024;
+constexpr int BOX_BYTES = 32 * 64;                   // a staged box of the epilogue: 32 rows x 32 columns
+constexpr int EPI_BOXES = 16, EPI_BYTES = EPI_BOXES * BOX_BYTES;
 constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on another GPU: seconds mean a lost partner
 
+// Epilogue warps: two per 32 accumulator rows, four where an element costs more than its rounding (8192 x 4096 x 1024 with bias and
+// residual 63 -> 59.7 us, with GELU 63.3 -> 60.3, with its gradient 71 -> 67.9; plain small products lose 0.3 - 0.5 us with four).
+__host__ __device__ constexpr int epiWarps(int epi) { return epi == EPI_NONE || epi == EPI_BIAS ? 8 : 16; }
+__host__ __device__ constexpr int pairThreads(int epi) { return 64 + 32 * epiWarps(epi); }
+
 struct PairArgs {
-  __nv_bfloat16* C;
   int M, N, K, ldc;
   int aMn, bMn;
+  int tn;                           // columns of a tile
+  int kStep;                        // blocks of 64 of the contraction in a stage: 1 or 2
+  int stages, stageBytes;
+  int tmemCols;                     // 512: two accumulators at columns 0 and 256; less: one, and no pair has a second tile
   int groupM;                       // row tiles per rasterisation group
   uint32_t* err;
   uint32_t* errHost;
+  __nv_bfloat16* C;
   GemmEpilogue e;
-  bool wide;                        // C, aux and pre start on 32-byte boundaries
+  int epiBytes;                     // boxes of the epilogue, or 0: straight from the registers
+  bool wide, wideC;                 // aux, and C and pre, start on a 32-byte boundary
 };
 
 template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
-dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const PairArgs g) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pairThreads(EPI), 1)
+dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapC,
+                    const __grid_constant__ CUtensorMap mapPre, const PairArgs g) {
+  constexpr int EPI_WARPS = epiWarps(EPI), PARTS = EPI_WARPS / 4, BUFS = EPI_BOXES / EPI_WARPS;
   extern __shared__ uint8_t smemRaw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  uint64_t* fullBar = (uint64_t*)(smem + STAGES * STAGE_BYTES);     // used in the leader only
-  uint64_t* emptyBar = fullBar + STAGES;                             // in both CTAs (commit to both)
-  uint64_t* accFull = emptyBar + STAGES;                             // [2] in both CTAs
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);       // the same offset in both CTAs
+  uint8_t* stg = smem + g.stages * g.stageBytes;
+  uint64_t* fullBar = (uint64_t*)(stg + g.epiBytes);                  // used in the leader only
+  uint64_t* emptyBar = fullBar + MAX_STAGES;                         // in both CTAs (commit to both)
+  uint64_t* accFull = emptyBar + MAX_STAGES;                         // [2] in both CTAs
   uint64_t* accEmpty = accFull + 2;                                  // [2] used in the leader only: the epilogue warps of both CTAs arrive
   uint32_t* tmemBaseSlot = (uint32_t*)(accEmpty + 2);
   volatile uint32_t* giveUp = tmemBaseSlot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t cr = cluster_ctarank();             // 0 = leader
-  const int mTiles = (g.M + PM - 1) / PM, nTiles = g.N / PN, kBlocks = g.K / BK;
+  const int mTiles = (g.M + PM - 1) / PM, nTiles = (g.N + g.tn - 1) / g.tn, kb64 = g.K / 64;
   const int numTiles = mTiles * nTiles;
   const int pair = blockIdx.x >> 1, numPairs = gridDim.x >> 1;
+  const int bHalf = g.tn / 2;
+  const int aBytes = HALF * 128 * g.kStep, mnBlock = 64 * 128 * g.kStep;      // MN-major operand: blocks of 64 MN-columns x K-rows; K-major: 64 K-columns x rows
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&fullBar[s], 1); mbar_init(&emptyBar[s], 1); }
+    for (int s = 0; s < g.stages; ++s) { mbar_init(&fullBar[s], 1); mbar_init(&emptyBar[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&accFull[a], 1); mbar_init(&accEmpty[a], 2 * EPI_WARPS); }
     // (not the device's error word: read here, beside the kernel in front, it could differ between the two CTAs, and one would
     // wait for a partner that does nothing.  After a kernel has given up the host refuses launches.)
@@ -76,8 +92,9 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
     tma_prefetch_desc(&mapB);
+    tma_prefetch_desc(&mapC);
   }
-  if (warp == 1) tmem_alloc_pair(tmemBaseSlot, TMEM_COLS);
+  if (warp == 1) tmem_alloc_pair(tmemBaseSlot, g.tmemCols);
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();                                // the partner's barriers exist before anything arrives on them
@@ -89,23 +106,28 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs; bytes counted in the leader)
     if (elect_one()) {
+      // One load per operand and stage where it is cut into whole blocks of 64 columns or rows: K-major operand [rows, K] as
+      // (64 K, rows, K / 64), boxes of 64 x rows x kStep; MN-major operand [K, cols] as (64 cols, K, cols / 64), boxes of
+      // 64 x 64 kStep x (cols / 64).  An MN-major B whose tiles are not whole blocks is loaded block by block, from any multiple
+      // of 16 columns.  The second half of the last stage may lie outside (zeros): it is loaded and not multiplied.
+      const uint32_t bar0 = mapa_u32(smem_u32(fullBar), 0);
+      const bool bLoose = g.bMn && bHalf % 64 != 0;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int t = pair; t < numTiles && ok; t += numPairs) {
         int mt, nt;
         raster_tile(t, mTiles, nTiles, g.groupM, mt, nt);
-        const int rowA = mt * PM + (int)cr * HALF, rowB = nt * PN + (int)cr * HALF;
-        for (int kb = 0; kb < kBlocks; ++kb) {
+        const int rowA = mt * PM + (int)cr * HALF, rowB = nt * g.tn + (int)cr * bHalf;
+        for (int k = 0; k < kb64; k += g.kStep) {
           if (!mbar_wait(&emptyBar[stage], phase ^ 1, giveUp, WAIT_NS)) { ok = false; break; }
-          if (cr == 0) mbar_expect_tx(&fullBar[stage], 2 * STAGE_BYTES);        // my bytes and the partner's
-          const uint32_t bar = mapa_u32(smem_u32(&fullBar[stage]), 0);
-          uint8_t* sa = smem + stage * STAGE_BYTES;
-          if (!g.aMn) tma_load_2d_pair(sa, &mapA, kb * BK, rowA, bar);
-          else for (int i = 0; i < HALF / 64; ++i) tma_load_2d_pair(sa + i * MN_BLOCK_BYTES, &mapA, rowA + 64 * i, kb * BK, bar);
-          if (!g.bMn) tma_load_2d_pair(sa + A_BYTES, &mapB, kb * BK, rowB, bar);
-          else for (int i = 0; i < HALF / 64; ++i) tma_load_2d_pair(sa + A_BYTES + i * MN_BLOCK_BYTES, &mapB, rowB + 64 * i, kb * BK, bar);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (cr == 0) mbar_expect_tx(&fullBar[stage], 2 * g.stageBytes);       // my bytes and the partner's
+          uint8_t* sa = smem + stage * g.stageBytes;
+          const uint32_t bar = bar0 + stage * 8;
+          tma_load_3d_pair(sa, &mapA, g.aMn ? k * 64 : rowA, g.aMn ? rowA / 64 : k, bar);
+          if (!bLoose) tma_load_3d_pair(sa + aBytes, &mapB, g.bMn ? k * 64 : rowB, g.bMn ? rowB / 64 : k, bar);
+          else for (int i = 0; i * 64 < bHalf; ++i) tma_load_2d_pair(sa + aBytes + i * mnBlock, &mapB, rowB + 64 * i, k * 64, bar);
+          if (++stage == g.stages) { stage = 0; phase ^= 1; }
         }
       }
       if (!ok) for (int i = 0; i < 20000; ++i) __nanosleep(200);     // copies already issued land before the CTA goes away
@@ -113,8 +135,11 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
     if (cr == 0 && elect_one()) {
-      const uint32_t idesc = umma_idesc_bf16(PM, PN, g.aMn, g.bMn);
+      const uint32_t idesc = umma_idesc_bf16(PM, g.tn, g.aMn, g.bMn);
+      // per instruction (16 K): K-major 32 bytes along the row; MN-major two groups of 8 K-rows.  Per 64 K: the next block of
+      // [rows] x 64 K-columns, or 64 K-rows further down the same blocks.
       const uint32_t stepA = g.aMn ? 128u : 2u, stepB = g.bMn ? 128u : 2u;
+      const uint32_t hopA = g.aMn ? 512u : HALF * 128 / 16, hopB = g.bMn ? 512u : (uint32_t)bHalf * 128 / 16;
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -123,57 +148,84 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
         const int ab = it & 1;
         if (!mbar_wait(&accEmpty[ab], ((it >> 1) & 1) ^ 1, giveUp, WAIT_NS)) break;
         tc_fence_after();
-        const uint32_t d = tmemBase + ab * PN;
-        for (int kb = 0; kb < kBlocks; ++kb) {
+        const uint32_t d = tmemBase + ab * 256;
+        for (int kb = 0; kb < kb64; kb += g.kStep) {
           if (!mbar_wait(&fullBar[stage], phase, giveUp, WAIT_NS)) { ok = false; break; }
           tc_fence_after();
-          const uint8_t* pa = smem + stage * STAGE_BYTES;
-          const uint64_t da = g.aMn ? umma_smem_desc_mn_sw128(pa, MN_BLOCK_BYTES) : umma_smem_desc_sw128(pa);
-          const uint64_t db = g.bMn ? umma_smem_desc_mn_sw128(pa + A_BYTES, MN_BLOCK_BYTES) : umma_smem_desc_sw128(pa + A_BYTES);
+          const uint8_t* pa = smem + stage * g.stageBytes;
+          const uint64_t da = g.aMn ? umma_smem_desc_mn_sw128(pa, mnBlock) : umma_smem_desc_sw128(pa);
+          const uint64_t db = g.bMn ? umma_smem_desc_mn_sw128(pa + aBytes, mnBlock) : umma_smem_desc_sw128(pa + aBytes);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16_pair(d, da + stepA * k, db + stepB * k, idesc, (kb | k) != 0);
+          for (int h = 0; h < 2; ++h) {
+            if (h == 1 && (g.kStep == 1 || kb + 1 == kb64)) break;
+#pragma unroll
+            for (int k = 0; k < 64 / UMMA_K; ++k)
+              umma_bf16_pair(d, da + hopA * h + stepA * k, db + hopB * h + stepB * k, idesc, (kb | h | k) != 0);
+          }
           umma_commit_pair(&emptyBar[stage]);         // both CTAs' stage is free once these MMAs have read it
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++stage == g.stages) { stage = 0; phase ^= 1; }
         }
         if (ok) umma_commit_pair(&accFull[ab]);       // both halves of the accumulator complete
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue: my 128 rows, TMEM -> bf16 -> global
-    const int quarter = warp & 3, colHalf = (warp - 2) >> 2;
+    // ------------------------------------------------------------ epilogue: my 128 rows, TMEM -> bf16 -> boxes -> global
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
     const uint32_t accEmptyLeader0 = mapa_u32(smem_u32(&accEmpty[0]), 0), accEmptyLeader1 = mapa_u32(smem_u32(&accEmpty[1]), 0);
+    // A box is stored with the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r / 2 % 4), so that eight lanes
+    // (rows) that write the same chunk meet eight different groups of four banks.
+    uint8_t* box0 = stg + (warp - 2) * BUFS * BOX_BYTES;
+    const uint32_t rowOff = lane * 64, swz = (lane >> 1) & 3;
+    int turn = 0;
+    auto store = [&](const CUtensorMap* map, __nv_bfloat16* base, const uint4 (&o)[4], int x, int y) {
+      if (EPI == EPI_GELU_GRAD || ((EPI == EPI_NONE || EPI == EPI_BIAS) && g.epiBytes == 0)) {      // 64 bytes of its row per lane, in whole sectors
+        __nv_bfloat16* p = base + (size_t)(y + lane) * g.ldc + x;
+        st_global32(p, o, g.wideC);
+        st_global32(p + 16, o + 2, g.wideC);
+        return;
+      }
+      uint8_t* box = box0 + turn * BOX_BYTES;
+      if (lane == 0) bulk_wait_read<BUFS - 1>();       // the store that read this buffer last has done so
+      __syncwarp();
+#pragma unroll
+      for (int v = 0; v < 4; ++v) *(uint4*)(box + rowOff + ((v ^ swz) << 4)) = o[v];
+      fence_async_shared();
+      __syncwarp();
+      if (lane == 0) { tma_store_2d(map, box, x, y); bulk_commit(); }
+      if (++turn == BUFS) turn = 0;
+    };
     int it = 0;
     for (int t = pair; t < numTiles; t += numPairs, ++it) {
       int mt, nt;
       raster_tile(t, mTiles, nTiles, g.groupM, mt, nt);
       const int ab = it & 1;
-      const bool mine = mt * PM + (int)cr * HALF < g.M;               // the last row tile may have only its upper half
-      const size_t tileOff = (size_t)(mt * PM + (int)cr * HALF + quarter * 32) * g.ldc + nt * PN;   // row 0 of this warp's 32 rows
-      const int beg = colHalf * (PN / 2);
-      // 32 columns of its row per lane and step, 32 bytes (a whole sector) per access: no staging rows, whose way through
-      // shared memory the operands need (8192 x 4096 x 1024 with GELU's gradient: 105 -> 70 - 79 us, by run)
+      const int row0 = mt * PM + (int)cr * HALF + quarter * 32, col0 = nt * g.tn;      // of this warp's 32 rows
+      const bool mine = row0 < g.M;                                   // the last row tile may have only its upper half
+      const int steps = min(g.tn, g.N - col0) / 32;
       constexpr bool AUX = EPI == EPI_BIAS_RES || EPI == EPI_GELU_GRAD;
-      constexpr int STEPS = PN / 2 / 32;
-      const size_t mineOff = tileOff + (size_t)lane * g.ldc + beg;
+      const __nv_bfloat16* aux = g.e.aux + (size_t)(row0 + lane) * g.ldc + col0;
+      uint4 own[4];
+      auto loadAux = [&](int i) {
+        if (!AUX || !mine || i >= steps) return;
+        ld_global32(aux + i * 32, own, g.wide);
+        ld_global32(aux + i * 32 + 16, own + 2, g.wide);
+      };
+      constexpr bool AHEAD = EPI == EPI_BIAS_RES;      // (GELU's gradient needs the registers)
+      if (AHEAD) loadAux(part);                        // on its way while the accumulator is computed
       if (!mbar_wait(&accFull[ab], (it >> 1) & 1, giveUp, WAIT_NS)) break;
       tc_fence_after();
 #pragma unroll 1
-      for (int i = 0; i < STEPS; ++i) {
+      for (int i = part; i < steps; i += PARTS) {
         if (!mine) break;
-        const int c = beg + i * 32;
+        const int c = i * 32;
         uint32_t r[32];
-        tmem_ld32(tmemBase + ((uint32_t)(quarter * 32) << 16) + ab * PN + c, r);
-        uint4 own[4];
-        if (AUX) {
-          ld_global32(g.e.aux + mineOff + i * 32, own, g.wide);
-          ld_global32(g.e.aux + mineOff + i * 32 + 16, own + 2, g.wide);
-        }
+        tmem_ld32(tmemBase + ((uint32_t)(quarter * 32) << 16) + ab * 256 + c, r);
+        if (!AHEAD) loadAux(i);
         tmem_ld_wait();
         if (EPI == EPI_BIAS || EPI == EPI_BIAS_RES || EPI == EPI_BIAS_GELU) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            const uint4 bv = ((const uint4*)(g.e.bias + nt * PN + c))[v];
+            const uint4 bv = ((const uint4*)(g.e.bias + col0 + c))[v];
             const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
@@ -194,6 +246,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
               r[8 * v + 2 * w] = __float_as_uint(lo); r[8 * v + 2 * w + 1] = __float_as_uint(hi);
             }
           }
+          if (AHEAD) loadAux(i + PARTS);
         }
         uint4 o[4];
 #pragma unroll
@@ -204,10 +257,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
           o[v].w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
         }
         if (EPI == EPI_BIAS_GELU) {
-          if (g.e.pre) {
-            st_global32(g.e.pre + mineOff + i * 32, o, g.wide);
-            st_global32(g.e.pre + mineOff + i * 32 + 16, o + 2, g.wide);
-          }
+          if (g.e.pre) store(&mapPre, g.e.pre, o, col0 + c, row0);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {                // of the rounded value: what the backward pass differentiates at
             uint32_t* ow = (uint32_t*)&o[v];
@@ -215,13 +265,13 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             for (int w = 0; w < 4; ++w) ow[w] = pack_bf16x2(geluTanh(bf16Lo(ow[w])), geluTanh(bf16Hi(ow[w])));
           }
         }
-        st_global32(g.C + mineOff + i * 32, o, g.wide);
-        st_global32(g.C + mineOff + i * 32 + 16, o + 2, g.wide);
+        store(&mapC, g.C, o, col0 + c, row0);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(ab ? accEmptyLeader1 : accEmptyLeader0);   // the pair's epilogue warps release the accumulator
     }
+    if (lane == 0) bulk_wait_read<0>();                // the boxes have been read before the CTA's shared memory goes away
   }
 
   // ---------------------------------------------------------------- leave: nothing of the pair may still use my shared or tensor memory
@@ -229,14 +279,14 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   __syncthreads();
   cluster_sync_all();
   tc_fence_after();
-  if (warp == 1) tmem_dealloc_pair(tmemBase, TMEM_COLS);
+  if (warp == 1) tmem_dealloc_pair(tmemBase, g.tmemCols);
   if (threadIdx.x == 0 && *giveUp) { atomicExch(g.err, 1u); *(volatile uint32_t*)g.errHost = 1u; __threadfence_system(); }
 }
 
 }  // namespace
 
 namespace {
-typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const PairArgs);
+typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const PairArgs);
 PairKernel pairKernel(int epi) {
   static const PairKernel k[] = {dfcclGemmPairKernel<EPI_NONE>, dfcclGemmPairKernel<EPI_BIAS>, dfcclGemmPairKernel<EPI_BIAS_RES>,
                                  dfcclGemmPairKernel<EPI_BIAS_GELU>, dfcclGemmPairKernel<EPI_GELU_GRAD>};
@@ -245,7 +295,7 @@ PairKernel pairKernel(int epi) {
 cudaError_t allowPairs() {
   return oncePerDevice([] {
     cudaError_t r = cudaSuccess;
-    for (int e = EPI_NONE; e <= EPI_GELU_GRAD && r == cudaSuccess; ++e) r = allowSharedMemory(pairKernel(e), SMEM_BYTES);
+    for (int e = EPI_NONE; e <= EPI_GELU_GRAD && r == cudaSuccess; ++e) r = allowSharedMemory(pairKernel(e), SMEM_LIMIT);
     return r;
   });
 }
@@ -258,7 +308,7 @@ int maxResidentPairs(int dev, int sms) {
     (void)allowPairs();                                // (the launch reports it)
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(sms & ~1); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.gridDim = dim3(sms & ~1); cfg.blockDim = dim3(pairThreads(EPI_NONE)); cfg.dynamicSmemBytes = SMEM_LIMIT;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, pairKernel(EPI_NONE), &cfg) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = sms / 2; }
     maxPairs[dev & 63] = std::min(n, sms / 2);
@@ -274,31 +324,56 @@ int gemmPairResident() {
   return maxResidentPairs(dev, sms);
 }
 
-ncclResult_t gemmPairLaunch(const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
+ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
                             uint32_t* errDev, uint32_t* errHost, const GemmEpilogue* e) {
-  CUtensorMap ma, mb;
-  if (!aMn) DFCHECK(gemmMakeMap(&ma, A, (uint64_t)M, (uint64_t)K, HALF)); else DFCHECK(gemmMakeMap(&ma, A, (uint64_t)K, (uint64_t)M, BK));
-  if (!bMn) DFCHECK(gemmMakeMap(&mb, B, (uint64_t)N, (uint64_t)K, HALF)); else DFCHECK(gemmMakeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
   CUDACHECK(allowPairs());
+  // 64 of the contraction in a stage keep more loads in flight beside wide tiles (8192 x 4096 x 1024 and its gradients 179 -> 176
+  // us); for narrower ones the tensor cores are through with such a stage before its two loads are issued (460 clocks)
+  const int kStep = width >= 224 ? 1 : 2, BK = 64 * kStep;
+  const int bHalf = width / 2, bBytes = bMn ? (bHalf + 63) / 64 * 64 * BK * 2 : bHalf * BK * 2;
+  CUtensorMap ma, mb, mc, mp;
+  DFCHECK(gemmMakeMap3(&ma, A, (uint64_t)M, (uint64_t)K, aMn, HALF, BK));
+  if (bMn && bHalf % 64) DFCHECK(gemmMakeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
+  else DFCHECK(gemmMakeMap3(&mb, B, (uint64_t)N, (uint64_t)K, bMn, bHalf, BK));
+  DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
+  mp = mc;
   PairArgs g;
   memset(&g, 0, sizeof(g));
-  g.C = (__nv_bfloat16*)C; g.M = M; g.N = N; g.K = K; g.ldc = N; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0;
+  g.M = M; g.N = N; g.K = K; g.ldc = N; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0; g.tn = width;
   g.err = errDev; g.errHost = errHost;
   if (e) g.e = *e;
-  g.wide = (((uintptr_t)C | (uintptr_t)g.e.aux | (uintptr_t)g.e.pre) & 31) == 0;
+  if (g.e.kind == EPI_BIAS_GELU && g.e.pre) DFCHECK(gemmMakeMap(&mp, g.e.pre, (uint64_t)M, (uint64_t)N, 32, 32));
+  g.C = (__nv_bfloat16*)C;
+  g.wide = ((uintptr_t)g.e.aux & 31) == 0;
+  g.wideC = (((uintptr_t)C | (uintptr_t)g.e.pre) & 31) == 0;
+  // Boxes and TMA stores drain a tile faster, straight stores leave the loads' engine and 32 KB of stages to the operands.  us,
+  // boxes / straight: plain 2560 x 3840 x 128 9.7 / 10.5, 5376 x 4096 x 256 16.8 / 19.5, 1920 x 1280 x 768 7.2 / 7.3, 8192 x 4096 x
+  // 1024 49.2 / 48.6, 2176 x 2304 x 2048 18.2 / 17.5, 8192^3 715 / 701; with bias and residual 8192 x 4096 x 1024 59.5 / 64.5, with
+  // GELU 60.6 / 63.8, 8192 x 1024 x 1024 17.6 / 20.0; with GELU's gradient, bound by its arithmetic, 69.9 / 67.9.
+  const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && K >= 896);
+  g.epiBytes = straight ? 0 : EPI_BYTES;
   { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int tiles = (M + PM - 1) / PM * (N / PN);
+  const int tiles = (M + PM - 1) / PM * ((N + width - 1) / width);
   const int pairs = std::min(tiles, maxResidentPairs(dev, sms));
+  g.kStep = kStep;
+  g.stageBytes = HALF * BK * 2 + bBytes;
+  const int room = SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK - g.epiBytes;
+  const int want = tiles > pairs ? MAX_STAGES : (K + BK - 1) / BK;
+  g.stages = std::min(std::min(MAX_STAGES, room / g.stageBytes), want);
+  g.tmemCols = tiles > pairs ? 512 : width <= 32 ? 32 : width <= 64 ? 64 : width <= 128 ? 128 : 256;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(NUM_THREADS); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = stream;
+  cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(pairThreads(g.e.kind)); cfg.stream = stream;
+  // at least the SM's shared memory times the share of its tensor memory: CTAs that are resident together, of this launch, of
+  // the next one or of another stream, then never wait for tensor memory
+  cfg.dynamicSmemBytes = std::max(g.stages * g.stageBytes + g.epiBytes + BAR_BYTES + ALIGN_SLACK, 228 * 1024 * g.tmemCols / 512 - 1024);
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
-  CUDACHECK(cudaLaunchKernelEx(&cfg, pairKernel(g.e.kind), ma, mb, g));
+  CUDACHECK(cudaLaunchKernelEx(&cfg, pairKernel(g.e.kind), ma, mb, mc, mp, g));
   return ncclSuccess;
 }
 

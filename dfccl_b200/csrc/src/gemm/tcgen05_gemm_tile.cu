@@ -4,7 +4,7 @@
 // What bounds such a product is how few SMs a handful of tiles occupies, the issue of loads and MMAs in a CTA (about 80 clocks
 // per MMA of 16 K however narrow the tile, 230 per load instruction: hence 128 K and one load per operand in a stage),
 // and the fixed cost of a launch.
-//   * Tiles of 128 x {64, 128} on one CTA (cta_group::1) or 256 x {128, 256} on a pair (cta_group::2, each CTA loads
+//   * Tiles of 128 x {64, 128} on one CTA (cta_group::1) or 256 x 128 on a pair (cta_group::2, each CTA loads
 //     half of B: fewer operand bytes per FLOP); the last row tile may stick out of M (TMA fills zeros, rows are not stored).
 //   * The contraction of a tile is cut into up to 4 slices on the CTAs of one cluster.  Every CTA of the cluster owns
 //     a slice of the tile's columns: the others write their fp32 partial sums of those columns into the owner's shared
@@ -57,19 +57,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
         "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
-      : "memory");
-}
-// Tile load of a 3-D map: x always 0, one instruction for a whole operand of a stage.
-__device__ __forceinline__ void tma_load_3d(void* smemDst, const CUtensorMap* map, int y, int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smemDst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(y), "r"(z)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(void* smemDst, const CUtensorMap* map, int y, int z, uint32_t barClusterAddr) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smemDst)), "l"(map), "r"(barClusterAddr), "r"(0), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void st_cluster16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -266,7 +253,7 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 
 typedef void (*TileKernel)(const CUtensorMap, const CUtensorMap, const TileArgs);
 TileKernel kernelOf(bool pair, int tn) {
-  if (pair) return tn == 128 ? dfcclGemmTileKernel<true, 128> : dfcclGemmTileKernel<true, 256>;
+  if (pair) return dfcclGemmTileKernel<true, 128>;
   return tn == 64 ? dfcclGemmTileKernel<false, 64> : dfcclGemmTileKernel<false, 128>;
 }
 
@@ -278,7 +265,7 @@ TileKernel kernelOf(bool pair, int tn) {
 struct Form { bool pair; int tn, split; double block, fixed; };
 constexpr Form FORMS[] = {
   {false, 64, 1, 0.150, 2.4}, {false, 64, 2, 0.150, 3.3}, {false, 64, 4, 0.150, 3.6}, {false, 128, 1, 0.172, 2.8},
-  {true, 128, 1, 0.140, 3.1}, {true, 128, 2, 0.140, 5.5}, {true, 256, 1, 0.280, 3.95},
+  {true, 128, 1, 0.140, 3.1}, {true, 128, 2, 0.140, 5.5},
 };
 
 int stagesOf(bool pair, int tn, int split, int kBlocks) {
@@ -289,39 +276,77 @@ int stagesOf(bool pair, int tn, int split, int kBlocks) {
 
 }  // namespace
 
-// The form with the least expected time.  The choice depends on the sizes alone (not on how the operands are stored, nor
-// on `pairs` as far as the number of slices goes), so that the same product is always summed in the same order.
-// The persistent kernel (tn = 0) overlaps a tile's epilogue with the next tile's loads, the others start anew for every
-// wave.  Measured, us (M x N x K: best form here / persistent kernel with one or two CTAs per tile before):
-//   128x512x512 3.6 / 7.0, 512x512x128 2.8 / 6.2, 1024x1024x1024 5.2 / 10.2, 1280x768x1920 7.4 / 14.1,
-//   896x2304x3072 11.8 / 18.7, 4096x512x4096 14.1 / 24.0, 2048x2048x2048 14.6 / 15.7, 128x256x8192 8.4 / 40.4;
-//   8192x1024x1024 persistent 15.4, best form 19.7.
-GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs) {
+// What the whole GPU takes for 64 of the contraction of that many tiles, however they are spread: power, or L2's bandwidth.
+double gpuUs(int rows, int tn, int tiles, int sms) { return 0.00156 * tn * tiles * rows / (128.0 * sms); }
+
+// The form with the least expected time: one of those above, or the persistent kernel with tiles of 256 x width.  Whether a
+// contraction is cut, and into how many slices, depends on the sizes and the epilogue alone (not on how the operands are stored,
+// nor on `pairs`), so that the same product is always summed in the same order; the width of a tile does not change a sum.
+// The persistent kernel: 3.2 us, and per wave of tiles 0.8 us + per 64 of the contraction what the tensor cores take for
+// the width, at least what a CTA's loads take (128 rows of A whatever the width), more when B is stored MN-major
+// in blocks of 64 columns that the tiles cut through, and when every SM works; at least what the whole GPU takes for the
+// FLOPs.  Fitted to some 500 products of all storage orders at widths of 32 to 256, 5 % rms.
+// It overlaps a tile's epilogue with the next tile's loads, the others start anew for every wave, but a wave of them is 0.7 us
+// cheaper (smaller blocks, no boxes to drain).  Measured, us (M x N x K: now / the better of these forms and width 256):
+//   2176x2304x2048 17.9 / 25.8 (width 160), 1280x3840x2560 21.2 / 29.4 (160), 896x6400x1536 16.9 / 20.1 (192),
+//   3072x1024x8192 42.6 / 47.5 (192), 1920x1280x768 7.1 / 8.5 (160), 3072x1792x6528 55.9 / 62.8 (160);
+//   a form of one wave: 128x512x512 3.6 (persistent 4.4), 1024x2048x1024 6.8 (7.3), 128x256x8192 8.4 in four slices
+//   (whole 21.3).
+double pairUs(int M, int N, int kb, int width, int sms, bool bMn) {
+  const int pairs = std::max(1, sms / 2), tiles = (M + 255) / 256 * ((N + width - 1) / width), waves = (tiles + pairs - 1) / pairs;
+  const double loads = bMn ? 0.13 : 0.092, loose = bMn && width / 2 % 64 ? 0.03 : 0.0;
+  const double busy = std::min(1.0, (double)tiles / pairs);
+  return 3.2 + waves * 0.8 + kb * std::max(waves * (std::max(loads, 0.00107 * width) + loose + 0.045 * busy), gpuUs(256, width, tiles, sms));
+}
+
+static GemmTilePlan choosePlan(int M, int N, int K, int sms, bool pairs, bool bMn, bool epilogue) {
   const int kb = K / 64;
   auto waves = [&](int clusters, int size) {          // clusters of 4 leave SMs of a GPC unused: 36 did not fit
     const int room = size == 1 ? sms : size == 2 ? sms / 2 : sms * 7 / 8 / size;
     return (clusters + std::max(room, 1) - 1) / std::max(room, 1);
   };
+  // an epilogue is a pass of its own behind these forms, which reads and writes the product (2048 x 1024: 2.8 us)
+  const double pass = epilogue ? 2.3 + 4.0 * M * N / 5e6 : 0.0;
   auto busy = [&](int ctas) { return 1.0 + 0.2 * std::min(1.0, (double)ctas / sms); };
   auto expect = [&](const Form& f) {
     const int size = (f.pair ? 2 : 1) * f.split, rows = f.pair ? 2 * TM : TM;
     const int tiles = (M + rows - 1) / rows * (N / f.tn);
-    return waves(tiles, size) * ((kb + f.split - 1) / f.split * f.block * busy(tiles * size) + f.fixed);
+    const int w = waves(tiles, size);
+    return w * f.fixed + std::max(w * ((kb + f.split - 1) / f.split * f.block * busy(tiles * size)), kb * gpuUs(rows, f.tn, tiles, sms)) + pass;
   };
-  const int big = (M + 255) / 256 * (N / 256);
-  GemmTilePlan p{true, 0, 1};
-  double best = waves(big, 2) * (kb * 0.28 * busy(2 * big)) + 4.65;
-  for (const Form& f : FORMS) {
-    if (f.split > kb) continue;
-    const double t = expect(f);
-    if (t < best) { best = t; p = GemmTilePlan{f.pair, f.tn, f.split}; }
-  }
-  if (!pairs && p.pair) {                              // one CTA per tile by request: the same slices
-    best = 1e30;
+  auto best = [&](bool mn, bool whole) {               // `whole`: contractions that are not cut
+    GemmTilePlan p{true, 0, 1, 256};
+    double us = pairUs(M, N, kb, 256, sms, mn);
+    for (int w = 32; w < 256; w += 32) {
+      const double t = pairUs(M, N, kb, w, sms, mn);
+      if (t < us) { us = t; p.width = w; }
+    }
+    for (const Form& f : FORMS) {
+      if (f.split > kb || (whole && f.split > 1)) continue;
+      const double t = expect(f);
+      if (t < us) { us = t; p = GemmTilePlan{f.pair, f.tn, f.split, 0}; }
+    }
+    return p;
+  };
+  GemmTilePlan p = best(false, false);
+  if (p.split == 1 && bMn) p = best(true, true);
+  if (!pairs && (p.pair || p.width)) {                 // one CTA per tile by request: the same slices
+    double us = 1e30;
+    const int split = p.split;
     for (const Form& f : FORMS)
-      if (!f.pair && f.split == p.split && expect(f) < best) { best = expect(f); p = GemmTilePlan{f.pair, f.tn, f.split}; }
+      if (!f.pair && f.split == split && expect(f) < us) { us = expect(f); p = GemmTilePlan{f.pair, f.tn, f.split, 0}; }
   }
   return p;
+}
+
+// (a product's sizes come back every step: the last few choices of the thread are kept, 0.15 us of a launch)
+GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs, bool bMn, bool epilogue) {
+  struct Kept { int M, N, K, key; GemmTilePlan p; };
+  static thread_local Kept kept[64];
+  const int key = 1 + sms * 8 + pairs * 4 + bMn * 2 + epilogue;
+  Kept& k = kept[((uint32_t)M * 31u + (uint32_t)N * 17u + (uint32_t)K * 7u + (uint32_t)key * 0x9E3779B1u) >> 7 & 63u];
+  if (k.key != key || k.M != M || k.N != N || k.K != K) k = Kept{M, N, K, key, choosePlan(M, N, K, sms, pairs, bMn, epilogue)};
+  return k.p;
 }
 
 ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream,
