@@ -622,23 +622,22 @@ __host__ __device__ bool reduce_dispatch(int inType, int outType, int op, const 
 #endif
 
 #ifdef DF_DATAPATH_SMALL_IMPL
+// (comparisons, the gradients' types first, and not a jump table: see nextPhase)
 __host__ __device__ bool reduce_small(int inType, int outType, int op, const DataArgs* a) {
   if (inType == outType) {
-    switch (inType) {
+    if (inType == ncclBfloat16) return reduceSmall<__nv_bfloat16, __nv_bfloat16>(a, op);
+    if (inType == ncclFloat32) return reduceSmall<float, float>(a, op);
 #ifndef DF_FAST_BUILD
-      case ncclInt8: return reduceSmall<int8_t, int8_t>(a, op);
-      case ncclUint8: return reduceSmall<uint8_t, uint8_t>(a, op);
-      case ncclInt32: return reduceSmall<int32_t, int32_t>(a, op);
-      case ncclUint32: return reduceSmall<uint32_t, uint32_t>(a, op);
-      case ncclInt64: return reduceSmall<int64_t, int64_t>(a, op);
-      case ncclUint64: return reduceSmall<uint64_t, uint64_t>(a, op);
-      case ncclFloat16: return reduceSmall<__half, __half>(a, op);
-      case ncclFloat64: return reduceSmall<double, double>(a, op);
+    if (inType == ncclFloat16) return reduceSmall<__half, __half>(a, op);
+    if (inType == ncclInt32) return reduceSmall<int32_t, int32_t>(a, op);
+    if (inType == ncclInt8) return reduceSmall<int8_t, int8_t>(a, op);
+    if (inType == ncclUint8) return reduceSmall<uint8_t, uint8_t>(a, op);
+    if (inType == ncclUint32) return reduceSmall<uint32_t, uint32_t>(a, op);
+    if (inType == ncclInt64) return reduceSmall<int64_t, int64_t>(a, op);
+    if (inType == ncclUint64) return reduceSmall<uint64_t, uint64_t>(a, op);
+    if (inType == ncclFloat64) return reduceSmall<double, double>(a, op);
 #endif
-      case ncclFloat32: return reduceSmall<float, float>(a, op);
-      case ncclBfloat16: return reduceSmall<__nv_bfloat16, __nv_bfloat16>(a, op);
-      default: return false;
-    }
+    return false;
   }
   if (op != OP_SUM) return false;
   if (inType == ncclBfloat16 && outType == ncclFloat32) return reduceSmall<__nv_bfloat16, float>(a, op);
@@ -653,8 +652,8 @@ __host__ __device__ bool reduce_small(int inType, int outType, int op, const Dat
 
 #define DF_SMALL_TRIPS 4       // calls of at most this many packs per thread and source go through the small bodies
 // What the step engine calls.
-DF_HD bool reduce_block(int inType, int outType, int op, const DataArgs* a) {
-  const bool small = a->n * (uint64_t)dtypeSize(inType) <= (uint64_t)df_nthreads() * 16u * DF_SMALL_TRIPS;
+DF_HD bool reduce_block(int inType, int outType, int esIn, int op, const DataArgs* a) {
+  const bool small = a->n * (uint64_t)esIn <= (uint64_t)df_nthreads() * 16u * DF_SMALL_TRIPS;
   if (small && reduce_small(inType, outType, op, a)) return true;
   return reduce_dispatch(inType, outType, op, a);
 }

@@ -507,7 +507,7 @@ DF_HD bool dataPhase(BlockShared* sh, RankDev* rd, int b) {
   if (sh->args.n != 0 && sh->args.ndst != 0) {
     const int how = sh->ctl1;
     bool known = true;
-    if (how == 1) known = reduce_block(c->inType, c->outType, c->op, &sh->args);
+    if (how == 1) known = reduce_block(c->inType, c->outType, c->esIn, c->op, &sh->args);
     else if (how == 0) copy_block(&sh->args);
     else known = moveMultimem(sh);
     if (!known && df_tid() == 0) sh->dyn.status = ST_BAD_ARG;
@@ -555,16 +555,20 @@ static DF_HD_NOINLINE void stageCopy(BlockShared* sh, int b, bool in) {
 }
 
 // ---- completion: count blocks; the last one publishes the device flag and the CQE
-// `idx`: the place of the host's entry, asked for before the fences so that it is on its way meanwhile.
-DF_HD void publishCompletion(BlockShared* sh, unsigned long long idx, int coll, uint32_t st, uint32_t epoch) {
+// `idx`: the place of the host's entry, asked for before the fences so that it is on its way meanwhile.  `early`: a stream may be
+// parked on the device flag.
+DF_HD void publishCompletion(BlockShared* sh, unsigned long long idx, int coll, uint32_t st, uint32_t epoch, bool early) {
   // The device flag releases a stream of THIS GPU (its wait is a stream memory operation, the consumers are kernels
   // launched behind it): everything the blocks wrote here is ordered before it by a fence of GPU scope, a quarter
   // of the cost of a system-scope one.  (What the blocks wrote into peers' memory was ordered by the fence before
   // their done flags, and this rank's result was complete when every peer's done flag had arrived.)
-  fence_acq_rel_gpu();
-  st_relaxed_sys_u64(&sh->k.doneEpoch[coll], ((uint64_t)st << 56) | epoch);
+  if (early) {
+    fence_acq_rel_gpu();
+    st_relaxed_sys_u64(&sh->k.doneEpoch[coll], ((uint64_t)st << 56) | epoch);
+  }
   // the host's entry: a host thread may read the result right after the callback, so the data is ordered system-wide
   fence_acq_rel_sys();
+  if (!early) st_relaxed_sys_u64(&sh->k.doneEpoch[coll], ((uint64_t)st << 56) | epoch);
   const uint32_t cap = sh->k.cqCap, gen = (uint32_t)(idx >> log2Of(cap)) + 1u;
   st_relaxed_sys_u64(&sh->k.hostCq[idx & (cap - 1)], cqeEncode(gen, st, (uint32_t)coll));
 }
@@ -593,33 +597,23 @@ DF_HD void completeColl(BlockShared* sh, RankDev* rd, int b) {
   if (last) {
     const unsigned long long idx = atomic_add_u64((unsigned long long*)&rd->devCqTail, 1ull);
     if (sh->cs.nBlocks > 1) atomic_exch_u32(&sh->k.doneCount[coll], 0u);
-    publishCompletion(sh, idx, coll, st, sh->dyn.epoch);
+    publishCompletion(sh, idx, coll, st, sh->dyn.epoch, (sh->dyn.sqeFlags & SQE_TRIGGERED) != 0);
   }
   trace(sh, rd, b, TR_DONE, coll);
 }
 
 // The first phase from `phase` on that has something to do for the loaded submission (a phase change costs two
 // block-wide barriers, a small collective would otherwise spend more time changing phases than moving data).
+// (Comparisons in the order of the phases: a jump table is a load from constant memory that a block meets cold.)
 DF_HD int nextPhase(const BlockShared* sh, int phase) {
   const CollStatic* c = &sh->cs;
   const int n = c->nranks, me = c->rank;
-  for (;; ++phase) {
-    switch (phase) {
-      case PH_COPY_IN:
-        if ((sh->dyn.sqeFlags & SQE_SEND_STAGED) && !rawSend(c) && !(c->kind == dfcclCollBroadcast && me != c->root)) return phase;
-        break;
-      case PH_POST_ARRIVE: case PH_WAIT_ARRIVE:
-        if (n > 1) return phase;
-        break;
-      case PH_POST_DONE: case PH_WAIT_DONE:
-        if (n > 1 && c->algo != dfcclAlgoPush) return phase;
-        break;
-      case PH_COPY_OUT:
-        if ((sh->dyn.sqeFlags & SQE_RECV_STAGED) && !rawRecv(c) && !(c->kind == dfcclCollReduce && me != c->root)) return phase;
-        break;
-      default: return phase;          // PH_DATA, PH_COMPLETE (PH_TRIGGER is never skipped to)
-    }
-  }
+  if (phase <= PH_COPY_IN && (sh->dyn.sqeFlags & SQE_SEND_STAGED) && !rawSend(c) && !(c->kind == dfcclCollBroadcast && me != c->root)) return PH_COPY_IN;
+  if (phase <= PH_WAIT_ARRIVE && n > 1) return phase < PH_POST_ARRIVE ? PH_POST_ARRIVE : phase;
+  if (phase <= PH_DATA) return PH_DATA;
+  if (phase <= PH_WAIT_DONE && n > 1 && c->algo != dfcclAlgoPush) return phase;
+  if (phase <= PH_COPY_OUT && (sh->dyn.sqeFlags & SQE_RECV_STAGED) && !rawRecv(c) && !(c->kind == dfcclCollReduce && me != c->root)) return PH_COPY_OUT;
+  return PH_COMPLETE;
 }
 
 // A wait of the loaded collective with its adaptive budget.  The budget is what the scheduler grants or, if larger,
@@ -653,6 +647,8 @@ DF_HD bool patientWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
 // the barrier that ends the wait, small bodies (datapath.h), one fence less in front of the completion.  25 MiB bf16 -> fp32 among
 // four 97.5 -> 85.9, a ragged reduce-scatter and all-gather 88.6 -> 76.5, 24 mixed collectives in four orders 297 -> 249; one
 // atomic for the blocks' count and verdicts, and an idle block that looks at its ring alone: 22.4, 83.5, 73.3, 247.
+// Comparisons instead of jump tables, phases one behind the other, one fence less for a completion that no stream waits for: with
+// the calls out of ctypes 21.1 -> 20.2, 83.5 -> 81.3, 69 -> 65.8, 220 -> 211.
 DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget, bool* moved) {
   if (!sh->standalone) loadColl(sh, rd, b, coll);
   const CollStatic* c = &sh->cs;
@@ -665,116 +661,109 @@ DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget
   bool listed = false;                                       // the pointer lists are up to date
   bool fetch = phase == PH_DATA && needsOffsets(c);          // resumed between two slices: another collective's offsets may stand here
   int rc = -1;
-  while (rc < 0) {
-    if (phase != entryPhase) *moved = true;
-    switch (phase) {
-      case PH_TRIGGER:
-        // (the daemon releases stream-ordered submissions from its trigger list and enters at PH_COPY_IN; this
-        // phase serves entries that were parked here by an earlier instance)
-        if (sh->dyn.sqeFlags & SQE_TRIGGERED) {
-          if (!boundedWait(sh, rd, rb, 2, sh->standalone ? budget : 1u)) {
-            if (noteStall(sh, rd)) { phase = PH_COMPLETE; break; }
-            rc = RC_STALLED;
-            break;
-          }
-          if (tid == 0) sh->dyn.stallSinceNs = 0;
-        }
-        if (tid == 0) trace(sh, rd, b, TR_START, coll);
+  // each phase that is due leads to a later one, or (a slice of the data) stays
+  do {
+    if (phase == PH_TRIGGER) {
+      // (the daemon releases stream-ordered submissions from its trigger list and enters at PH_COPY_IN; this
+      // phase serves entries that were parked here by an earlier instance)
+      if ((sh->dyn.sqeFlags & SQE_TRIGGERED) && !boundedWait(sh, rd, rb, 2, sh->standalone ? budget : 1u)) {
+        if (!noteStall(sh, rd)) { rc = RC_STALLED; break; }
+        phase = PH_COMPLETE;
+      } else {
+        if (tid == 0) { sh->dyn.stallSinceNs = 0; trace(sh, rd, b, TR_START, coll); }
         phase = nextPhase(sh, PH_COPY_IN);
-        break;
-      case PH_COPY_IN:
-        if ((sh->dyn.sqeFlags & SQE_SEND_STAGED) && !rawSend(c)) {
-          bool needed = !(c->kind == dfcclCollBroadcast && me != c->root);
-          if (needed) stageCopy(sh, rb, true);
-        }
-        phase = nextPhase(sh, PH_POST_ARRIVE);
-        break;
-      case PH_POST_ARRIVE: {
-        const bool pushed = c->algo == dfcclAlgoPush && n > 1;
-        if (pushed) pushOut(sh, rb);                         // the payload travels ahead of the arrival flag: stores, a fence, the flag
-        if (warp0) {
-          if (pushed || (sh->dyn.sqeFlags & SQE_SEND_STAGED)) fence_members(c);      // what the block has stored, a barrier ago
-          const uint32_t epoch = sh->dyn.epoch;
-          const uint64_t so = offTagged(mySendOff(sh), epoch), ro = offTagged(myRecvOff(sh), epoch);
-          for (int j = tid; j < n; j += df_warpsize()) {
-            if (j == me) continue;
-            FlagSlot* s = c->peerFlags[j] + (uint64_t)rb * n + me;
-            if (!pushed) { st_relaxed_sys_u64(&s->sendOff, so); st_relaxed_sys_u64(&s->recvOff, ro); }      // (not used by the push schedule)
-            if (c->oneDevice || pushed) st_relaxed_sys_u64(&s->arrive, epoch); else st_release_sys_u64(&s->arrive, epoch);
-          }
-        }
-        phase = PH_WAIT_ARRIVE;                              // the warp that posted is the one that polls
-        break;
       }
-      case PH_WAIT_ARRIVE:
-        if (n > 1 && !patientWait(sh, rd, rb, 0, budget)) {
-          if (noteStall(sh, rd)) { phase = PH_COMPLETE; break; }
+    }
+    if (phase == PH_COPY_IN) {
+      if ((sh->dyn.sqeFlags & SQE_SEND_STAGED) && !rawSend(c) && !(c->kind == dfcclCollBroadcast && me != c->root)) stageCopy(sh, rb, true);
+      phase = nextPhase(sh, PH_POST_ARRIVE);
+    }
+    if (phase == PH_POST_ARRIVE) {
+      const bool pushed = c->algo == dfcclAlgoPush && n > 1;
+      if (pushed) pushOut(sh, rb);                           // the payload travels ahead of the arrival flag: stores, a fence, the flag
+      if (warp0) {
+        if (pushed || (sh->dyn.sqeFlags & SQE_SEND_STAGED)) fence_members(c);        // what the block has stored, a barrier ago
+        const uint32_t epoch = sh->dyn.epoch;
+        const uint64_t so = offTagged(mySendOff(sh), epoch), ro = offTagged(myRecvOff(sh), epoch);
+        for (int j = tid; j < n; j += df_warpsize()) {
+          if (j == me) continue;
+          FlagSlot* s = c->peerFlags[j] + (uint64_t)rb * n + me;
+          if (!pushed) { st_relaxed_sys_u64(&s->sendOff, so); st_relaxed_sys_u64(&s->recvOff, ro); }        // (not used by the push schedule)
+          if (c->oneDevice || pushed) st_relaxed_sys_u64(&s->arrive, epoch); else st_release_sys_u64(&s->arrive, epoch);
+        }
+      }
+      phase = PH_WAIT_ARRIVE;                                // the warp that posted is the one that polls
+    }
+    if (phase == PH_WAIT_ARRIVE) {
+      if (n > 1 && !patientWait(sh, rd, rb, 0, budget)) {
+        if (!noteStall(sh, rd)) {
           if (tid == 0) trace(sh, rd, b, TR_STALL, coll);
           rc = RC_STALLED;
           break;
         }
+        phase = PH_COMPLETE;
+      } else {
         listed = n > 1;
         if (tid == 0) trace(sh, rd, b, TR_ARRIVED, coll);
         phase = PH_DATA;
-        break;
-      case PH_DATA: {
-        if (!listed) {
-          if (warp0 && fetch) fetchPeerOffsets(sh, rb);
-          fetch = false;
-          if (warp0) buildArgs(sh, rb);
-          df_sync();
-        }
-        listed = false;
-        if (tid == 0) trace(sh, rd, b, TR_DATA_BEGIN, coll);
-        const bool more = dataPhase(sh, rd, rb);             // ends with a barrier
-        if (tid == 0) trace(sh, rd, b, TR_DATA_END, coll);
-        if (more) {                                          // the cursor is saved; the phase stays PH_DATA
-          *moved = true;
-          if (sh->ctl0) {
-            if (tid == 0) { sh->stats.yields++; trace(sh, rd, b, TR_YIELD, coll); }
-            rc = RC_YIELD;
-          }
-          break;
-        }
-        // (push schedule: no done handshake - nobody reads my buffers and my slots are not reused before the
-        // peers' next-but-one call)
-        phase = nextPhase(sh, PH_POST_DONE);
-        break;
       }
-      case PH_POST_DONE:
-        if (n > 1 && warp0) {
-          // all payload stores of this block were issued before the barrier at the end of the data phase; a fence of
-          // the lanes that post makes them visible to the members before any done flag is
-          fence_members(c);
-          const uint64_t epoch = sh->dyn.epoch;
-          for (int j = tid; j < n; j += df_warpsize())
-            if (j != me) st_relaxed_sys_u64(&(c->peerFlags[j] + (uint64_t)rb * n + me)->done, epoch);
+    }
+    if (phase == PH_DATA) {
+      if (phase != entryPhase) *moved = true;
+      if (!listed) {
+        if (warp0 && fetch) fetchPeerOffsets(sh, rb);
+        fetch = false;
+        if (warp0) buildArgs(sh, rb);
+        df_sync();
+      }
+      listed = false;
+      if (tid == 0) trace(sh, rd, b, TR_DATA_BEGIN, coll);
+      const bool more = dataPhase(sh, rd, rb);               // ends with a barrier
+      if (tid == 0) trace(sh, rd, b, TR_DATA_END, coll);
+      if (more) {                                            // the cursor is saved; the phase stays PH_DATA
+        *moved = true;
+        if (sh->ctl0) {
+          if (tid == 0) { sh->stats.yields++; trace(sh, rd, b, TR_YIELD, coll); }
+          rc = RC_YIELD;
         }
-        phase = PH_WAIT_DONE;
-        break;
-      case PH_WAIT_DONE:
-        if (n > 1 && !patientWait(sh, rd, rb, 1, budget)) {
-          if (noteStall(sh, rd)) { phase = PH_COMPLETE; break; }
+        continue;
+      }
+      // (push schedule: no done handshake - nobody reads my buffers and my slots are not reused before the
+      // peers' next-but-one call)
+      phase = nextPhase(sh, PH_POST_DONE);
+    }
+    if (phase == PH_POST_DONE) {
+      if (n > 1 && warp0) {
+        // all payload stores of this block were issued before the barrier at the end of the data phase; a fence of
+        // the lanes that post makes them visible to the members before any done flag is
+        fence_members(c);
+        const uint64_t epoch = sh->dyn.epoch;
+        for (int j = tid; j < n; j += df_warpsize())
+          if (j != me) st_relaxed_sys_u64(&(c->peerFlags[j] + (uint64_t)rb * n + me)->done, epoch);
+      }
+      phase = PH_WAIT_DONE;
+    }
+    if (phase == PH_WAIT_DONE) {
+      if (n > 1 && !patientWait(sh, rd, rb, 1, budget)) {
+        if (!noteStall(sh, rd)) {
           if (tid == 0) trace(sh, rd, b, TR_STALL, coll);
           rc = RC_STALLED;
           break;
         }
+        phase = PH_COMPLETE;
+      } else {
         if (tid == 0) trace(sh, rd, b, TR_PEERS_DONE, coll);
         phase = nextPhase(sh, PH_COPY_OUT);
-        break;
-      case PH_COPY_OUT:
-        if ((sh->dyn.sqeFlags & SQE_RECV_STAGED) && !rawRecv(c)) {
-          bool needed = !(c->kind == dfcclCollReduce && me != c->root);
-          if (needed) stageCopy(sh, rb, false);
-        }
-        phase = PH_COMPLETE;
-        break;
-      default:  // PH_COMPLETE
-        completeColl(sh, rd, b);
-        rc = RC_DONE;
-        break;
+      }
     }
-  }
+    if (phase == PH_COPY_OUT) {
+      if ((sh->dyn.sqeFlags & SQE_RECV_STAGED) && !rawRecv(c) && !(c->kind == dfcclCollReduce && me != c->root)) stageCopy(sh, rb, false);
+      phase = PH_COMPLETE;
+    }
+    completeColl(sh, rd, b);
+    rc = RC_DONE;
+  } while (rc < 0);
+  if (phase != entryPhase) *moved = true;
   if (tid == 0) { sh->dyn.phase = phase; sh->dynDirty = 1; }
   return rc;
 }
