@@ -76,12 +76,17 @@ _lock = threading.Lock()
 _entries: Dict[str, Callable[..., int]] = {}
 
 
-def _load_hostcall():
-    path = _build.HOSTCALL if _build.HOSTCALL.exists() else _build.build_hostcall()
-    loader = importlib.machinery.ExtensionFileLoader("dfccl_hostcall", str(path))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("dfccl_hostcall", loader))
-    loader.exec_module(module)
-    return module
+@functools.lru_cache(maxsize=None)
+def _hostcall():
+    """The extension's ``call``, or None where it is missing and cannot be compiled (no compiler, no interpreter headers)."""
+    try:
+        path = _build.HOSTCALL if _build.HOSTCALL.exists() else _build.build_hostcall()
+        loader = importlib.machinery.ExtensionFileLoader("dfccl_hostcall", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("dfccl_hostcall", loader))
+        loader.exec_module(module)
+        return module.call
+    except (ImportError, OSError, RuntimeError):
+        return None
 
 
 def entry(name: str) -> Callable[..., int]:
@@ -89,7 +94,12 @@ def entry(name: str) -> Callable[..., int]:
     a ctypes call.  Other argument types are a ``TypeError``; ``lib()`` still takes them."""
     f = _entries.get(name)
     if f is None:
-        f = _entries[name] = functools.partial(_load_hostcall().call, C.cast(getattr(lib(), name), C.c_void_p).value)
+        slow, call = getattr(lib(), name), _hostcall()
+        if call is not None:
+            f = functools.partial(call, C.cast(slow, C.c_void_p).value)
+        else:
+            f = lambda *a: slow(*(NO_CALLBACK if t is CALLBACK and x is None else x for x, t in zip(a, slow.argtypes)))        # noqa: E731
+        _entries[name] = f
     return f
 
 

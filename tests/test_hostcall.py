@@ -41,3 +41,10 @@ def test_submissions_take_what_ctypes_takes():
         comm.destroy()
     finally:
         nv.set_backend(old)
+
+
+def test_without_the_extension(monkeypatch):
+    """No compiler and no built extension: the same calls through ctypes."""
+    monkeypatch.setattr(nv, "_hostcall", lambda: None)
+    monkeypatch.setattr(nv, "_entries", {})
+    test_submissions_take_what_ctypes_takes()
