@@ -396,25 +396,25 @@ DF_HD void copyOne(const char* src, char* dst, uint64_t n) {
   const int tid = df_tid(), nt = df_nthreads();
   const uint32_t head = (uint32_t)umin64((16u - (uint32_t)((uintptr_t)dst & 15)) & 15u, n);
   const uint32_t shift = (uint32_t)(((uintptr_t)src + head) & 15);
-  const uint32_t nPacks = (uint32_t)((n - head) / 16);
+  const uint64_t nPacks = (n - head) / 16;             // (a piece is as long as the limit of the push schedule is set: bytes take 64 bits)
   const char* s = src + head - shift;
 #pragma unroll 1
-  for (uint32_t p0 = (uint32_t)tid; p0 < nPacks; p0 += 4u * (uint32_t)nt) {
+  for (uint64_t p0 = (uint64_t)tid; p0 < nPacks; p0 += 4u * (uint32_t)nt) {
     uint4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const uint32_t p = p0 + (uint32_t)(u * nt);
+      const uint64_t p = p0 + (uint32_t)(u * nt);
       if (p >= nPacks) continue;
-      v[u] = ld16(s + p * 16u);
-      if (shift) v[u] = shiftPack(v[u], ld16(s + p * 16u + 16), shift);
+      v[u] = ld16(s + p * 16);
+      if (shift) v[u] = shiftPack(v[u], ld16(s + p * 16 + 16), shift);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const uint32_t p = p0 + (uint32_t)(u * nt);
-      if (p < nPacks) st16(dst + head + p * 16u, v[u]);
+      const uint64_t p = p0 + (uint32_t)(u * nt);
+      if (p < nPacks) st16(dst + head + p * 16, v[u]);
     }
   }
-  const uint64_t tail0 = head + (uint64_t)nPacks * 16;
+  const uint64_t tail0 = head + nPacks * 16;
 #pragma unroll 1
   for (uint64_t i = (uint64_t)(nt - 1 - tid); i < head + (n - tail0); i += nt) {
     const uint64_t e = i < head ? i : tail0 + (i - head);
