@@ -585,14 +585,13 @@ DF_HD void completeColl(BlockShared* sh, RankDev* rd, int b) {
   // the cached copy stays authoritative while the collective is loaded; it reaches global memory when another
   // collective is loaded, when the block parks, or when the next submission of this id is consumed
   sh->stats.collsDone++;
-  uint32_t st = status > 255 ? (uint32_t)ST_TIMEOUT : status;
+  uint32_t st = status <= ST_BAD_ARG ? status : (uint32_t)ST_TIMEOUT;
   bool last = true;
   if (sh->cs.nBlocks > 1) {                       // one word counts the blocks and carries their verdicts
     fence_acq_rel_gpu();
-    const uint32_t mine = 1u | (st != ST_OK ? 1u << 8 | st << 16 : 0u);
-    const uint32_t all = atomic_add_u32(&sh->k.doneCount[coll], mine) + mine;
+    const uint32_t mine = doneWord(st), all = atomic_add_u32(&sh->k.doneCount[coll], mine) + mine;
     last = (all & 0xffu) == (uint32_t)sh->cs.nBlocks;
-    st = (all >> 8) & 0xffu ? (all >> 16) / ((all >> 8) & 0xffu) : ST_OK;      // all failing blocks report the same cause
+    st = doneVerdict(all);
   }
   if (last) {
     const unsigned long long idx = atomic_add_u64((unsigned long long*)&rd->devCqTail, 1ull);

@@ -110,6 +110,12 @@ enum Phase : int32_t {
 };
 
 enum CollStatus : uint32_t { ST_OK = 0, ST_TIMEOUT = 1, ST_ABORTED = 2, ST_BAD_ARG = 3 };
+// The word in which the blocks of a collective count themselves and leave their verdicts: [7:0] how many are done, and of those
+// [15:8] how many timed out, [23:16] were aborted, [31:24] met a bad argument (DF_MAX_BLOCKS of each at most).
+static __host__ __device__ inline uint32_t doneWord(uint32_t status) { return 1u | (status != ST_OK ? 1u << (8u * (status <= ST_BAD_ARG ? status : ST_TIMEOUT)) : 0u); }
+// The collective's status where the causes differ: one that a block has reported.  (A wait that ran out is the cause of an
+// abort that follows it.)
+static __host__ __device__ inline uint32_t doneVerdict(uint32_t w) { return w >> 24 ? ST_BAD_ARG : w >> 8 & 0xffu ? ST_TIMEOUT : w >> 16 & 0xffu ? ST_ABORTED : ST_OK; }
 
 // ---- immutable description of a registered collective (one per collId per rank)
 struct alignas(16) CollStatic {
@@ -252,9 +258,8 @@ struct RankConst {
   uint32_t* meta;                  // [maxColls] what a block needs to know to take or skip an entry: nBlocks | blockBase << 8 |
                                    // DF_META_VALID; never written after finalize
   CollDyn* dyn;                    // [nBlocks][maxColls]
-  uint32_t* doneCount;             // [maxColls] blocks that finished the current submission: [7:0] how many, [15:8] of those, how many
-                                   // with an error, [31:16] the sum of their statuses (a collective that runs in its stream
-                                   // counts its kernel's blocks here)
+  uint32_t* doneCount;             // [maxColls] blocks that finished the current submission and their verdicts (doneWord; a collective
+                                   // that runs in its stream counts its kernel's blocks here)
   volatile uint64_t* doneEpoch;    // [maxColls] device flag: epoch of the last finished submission
   volatile uint64_t* trigger;      // [maxColls] device flag written by stream memory operations
   BlockSaved* saved;               // [nBlocks]

@@ -50,3 +50,35 @@ int main() {
 }
 """.replace("SKEW", str(skew)))
     assert out == "ok\n"
+
+
+def test_verdict_of_blocks_that_fail_for_different_causes(tmp_path):
+    """A cause that a block reported, never one between two (1 timed out, 2 aborted, 3 bad argument): a bad argument before a wait
+    that ran out before an abort, whatever the order; the word the blocks share is clear afterwards."""
+    out = run_on_host(tmp_path, r"""
+#include <memory>
+#include <vector>
+static int verdict(const std::vector<uint32_t>& status) {
+  uint32_t done = 0;
+  uint64_t flag = 0, ring[4] = {};
+  RankDev rd;
+  memset(&rd, 0, sizeof(rd));
+  rd.doneCount = &done; rd.doneEpoch = &flag; rd.hostCq = ring; rd.cqCap = 4;
+  std::unique_ptr<BlockShared> sh(new BlockShared);
+  memset((void*)sh.get(), 0, sizeof(BlockShared));
+  sh->k = rd;
+  for (size_t b = 0; b < status.size(); ++b) {
+    sh->cs.nBlocks = (int)status.size(); sh->loadedColl = 0; sh->dyn.epoch = 7; sh->dyn.status = status[b];
+    completeColl(sh.get(), &rd, (int)b);
+    if ((rd.devCqTail != 0) != (b + 1 == status.size())) return -1;
+  }
+  if (done != 0 || flag != ((uint64_t)cqeStatus(ring[0]) << 56 | 7)) return -2;
+  return (int)cqeStatus(ring[0]);
+}
+int main() {
+  for (auto& s : std::vector<std::vector<uint32_t>>{{0, 0}, {0, 1}, {2, 0, 0}, {3}, {1, 2}, {2, 1, 2, 2}, {1, 3}, {3, 1}, {2, 3, 2}, {1, 2, 3}}) printf("%d ", verdict(s));
+  for (uint32_t s = 0; s < 4; ++s) printf("%d ", verdict(std::vector<uint32_t>(DF_MAX_BLOCKS, s)));
+  return 0;
+}
+""")
+    assert out.split() == "0 1 2 3 1 1 3 3 3 3 0 1 2 3".split()
