@@ -79,13 +79,15 @@ _entries: Dict[str, Callable[..., int]] = {}
 @functools.lru_cache(maxsize=None)
 def _hostcall():
     """The extension's ``call``, or None where it is missing and cannot be compiled (no compiler, no interpreter headers)."""
+    path = _build.try_hostcall()
+    if path is None:
+        return None
     try:
-        path = _build.HOSTCALL if _build.HOSTCALL.exists() else _build.build_hostcall()
         loader = importlib.machinery.ExtensionFileLoader("dfccl_hostcall", str(path))
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("dfccl_hostcall", loader))
         loader.exec_module(module)
         return module.call
-    except (ImportError, OSError, RuntimeError):
+    except (ImportError, OSError):
         return None
 
 

@@ -1,13 +1,19 @@
 """Entry points called without ctypes: argument conversion, and what only ctypes converts."""
 import ctypes as C
+import os
+import subprocess
+import warnings
 
 import numpy as np
 import pytest
 
+from dfccl_b200 import _build
 from dfccl_b200 import native as nv
 
 
 def test_arguments():
+    if nv._hostcall() is None:
+        pytest.skip("no compiler or no interpreter headers: the entry points go through ctypes")
     f = nv.entry("dfcclGetBackend")
     v = C.c_int(-1)
     assert f(C.addressof(v)) == nv.SUCCESS and v.value in (nv.BACKEND_CUDA, nv.BACKEND_HOST)
@@ -43,8 +49,42 @@ def test_submissions_take_what_ctypes_takes():
         nv.set_backend(old)
 
 
-def test_without_the_extension(monkeypatch):
-    """No compiler and no built extension: the same calls through ctypes."""
-    monkeypatch.setattr(nv, "_hostcall", lambda: None)
+@pytest.mark.parametrize("gcc", ["missing", "failing"])
+def test_without_the_extension(monkeypatch, tmp_path, gcc):
+    """No compiler, or none that finds the interpreter's headers, and no built extension: the library is compiled and linked
+    all the same, and the same calls go through ctypes."""
+    obj = tmp_path / "x.o"
+    obj.touch()
+
+    def run(cmd, **kw):
+        if cmd[0] == _build.nvcc():
+            (tmp_path / "libdfccl.so").touch()
+        elif gcc == "missing":
+            raise FileNotFoundError(cmd[0])
+        return subprocess.CompletedProcess(cmd, 0 if cmd[0] == _build.nvcc() else 1, "", "no such header")
+
+    monkeypatch.setattr(_build, "LIB", tmp_path / "libdfccl.so")
+    monkeypatch.setattr(_build, "LIBDIR", tmp_path)
+    monkeypatch.setattr(_build, "HOSTCALL", tmp_path / "dfccl_hostcall.so")
+    monkeypatch.setattr(_build, "_compile", lambda *a: obj)
+    monkeypatch.setattr(_build.subprocess, "run", run)
+    monkeypatch.setattr(nv, "_hostcall", nv._hostcall.__wrapped__)
     monkeypatch.setattr(nv, "_entries", {})
-    test_submissions_take_what_ctypes_takes()
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        assert _build.build().exists()
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        assert nv._hostcall() is None
+        test_submissions_take_what_ctypes_takes()
+
+
+def test_a_stale_extension_is_built_again(monkeypatch, tmp_path):
+    if nv._hostcall() is None:
+        pytest.skip("no compiler or no interpreter headers")
+    so = tmp_path / "dfccl_hostcall.so"
+    monkeypatch.setattr(_build, "HOSTCALL", so)
+    monkeypatch.setattr(_build, "LIBDIR", tmp_path)
+    so.write_bytes(b"of another time")
+    os.utime(so, (1, 1))
+    assert nv._hostcall.__wrapped__() is not None
+    assert so.stat().st_size > 1000
