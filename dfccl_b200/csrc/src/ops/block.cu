@@ -2,8 +2,8 @@
 // forward and backward, column sums (bias gradients), and the GEMM epilogues as passes of their own.
 // All of it streams activations once, so HBM (or L2) bounds it: 16 bytes per load, every row in registers between its two
 // passes, and enough warps to keep 148 SMs loading.  The measured times stand at the kernels.
-// They are short and follow one another: each is launched as a dependent of the kernel in front, so that its blocks are up when
-// that one ends.  With that and one kernel for a column sum instead of two, three GPT-2 blocks of 1024 (forward to AdamW) took
+// They are short and follow one another: each (but the epilogue pass) is launched as a dependent of the kernel in front, so that its
+// blocks are up when that one ends.  With that and one kernel for a column sum instead of two, three GPT-2 blocks of 1024 (forward to AdamW) took
 // 2856 us instead of 2916.
 // The reference has no counterpart (it is a collective library); the GPT-2 workload uses these.
 #include <cuda_bf16.h>
@@ -195,19 +195,11 @@ __global__ void __launch_bounds__(1024) sumLinesKernel(const float* __restrict__
   }
 }
 
-// Column sums in one launch: a cluster of SUM_CTAS blocks takes 64 columns, a stretch of the rows each; a warp reads four rows
-// of 128 bytes at a time, eight such loads in flight, the block adds its warps up through shared memory, and the cluster's blocks
-// write 64 / SUM_CTAS columns each from one another's shared memory.  No scratch in global memory, no second kernel, a
-// fixed order of the sums.  Bound: one read of the matrix.
-constexpr int SUM_CTAS = 8;
-__global__ void __cluster_dims__(SUM_CTAS, 1, 1) __launch_bounds__(256) columnSumKernel(const __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ out, int rows, int n) {
-  __shared__ float part[8][4][64 + 4];
-  __shared__ float sums[64];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = blockIdx.x % SUM_CTAS;
-  const int c0 = blockIdx.x / SUM_CTAS * 64, c = c0 + (lane & 7) * 8;
-  const int per = (rows + SUM_CTAS - 1) / SUM_CTAS, beg = rank * per, end = min(rows, beg + per);
-  tc::grid_dependency_wait();
-  tc::grid_launch_dependents();
+// Sums of 64 columns from c0 on over rows [beg, end) by a block of 256 threads, in `sums`: a warp reads four rows of 128 bytes at a
+// time, eight such loads in flight, the block adds its warps up through shared memory in a fixed order.
+struct ColumnShared { float part[8][4][64 + 4], sums[64]; };
+__device__ __forceinline__ void sumColumns(ColumnShared& sh, const __nv_bfloat16* __restrict__ g, int beg, int end, int n, int c0) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = c0 + (lane & 7) * 8;
   float a[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) a[e] = 0.f;
@@ -221,17 +213,30 @@ __global__ void __cluster_dims__(SUM_CTAS, 1, 1) __launch_bounds__(256) columnSu
     }
   }
 #pragma unroll
-  for (int e = 0; e < 8; ++e) part[warp][lane >> 3][(lane & 7) * 8 + e] = a[e];
+  for (int e = 0; e < 8; ++e) sh.part[warp][lane >> 3][(lane & 7) * 8 + e] = a[e];
   __syncthreads();
   if (threadIdx.x < 64) {
     float s = 0.f;
 #pragma unroll
     for (int w = 0; w < 8; ++w)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) s += part[w][q][threadIdx.x];
-    sums[threadIdx.x] = s;
+      for (int q = 0; q < 4; ++q) s += sh.part[w][q][threadIdx.x];
+    sh.sums[threadIdx.x] = s;
   }
   __syncthreads();
+}
+
+// Column sums in one launch: a cluster of SUM_CTAS blocks takes 64 columns, a stretch of the rows each, and the cluster's blocks
+// write 64 / SUM_CTAS columns each from one another's shared memory.  No scratch in global memory, no second kernel, a
+// fixed order of the sums.  Bound: one read of the matrix.
+constexpr int SUM_CTAS = 8;
+__global__ void __cluster_dims__(SUM_CTAS, 1, 1) __launch_bounds__(256) columnSumKernel(const __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ out, int rows, int n) {
+  __shared__ ColumnShared sh;
+  const int rank = blockIdx.x % SUM_CTAS, c0 = blockIdx.x / SUM_CTAS * 64;
+  const int per = (rows + SUM_CTAS - 1) / SUM_CTAS, beg = rank * per, end = min(rows, beg + per);
+  tc::grid_dependency_wait();
+  tc::grid_launch_dependents();
+  sumColumns(sh, g, beg, end, n, c0);
   tc::cluster_sync_all();                                // every block's sums are there
   if (threadIdx.x < 64 / SUM_CTAS) {
     const int k = rank * (64 / SUM_CTAS) + threadIdx.x;
@@ -239,12 +244,23 @@ __global__ void __cluster_dims__(SUM_CTAS, 1, 1) __launch_bounds__(256) columnSu
 #pragma unroll
     for (int b = 0; b < SUM_CTAS; ++b) {
       float v;
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(tc::mapa_u32(tc::smem_u32(&sums[k]), b)) : "memory");
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(tc::mapa_u32(tc::smem_u32(&sh.sums[k]), b)) : "memory");
       s += v;
     }
     if (c0 + k < n) out[c0 + k] = __float2bfloat16_rn(s);
   }
   tc::cluster_sync_all();                                // nobody reads this block's shared memory any more
+}
+
+// The same for matrices too narrow for their height (sumStretches): gridDim.y stretches of rows, a line of fp32 sums in `work`
+// each, which sumLinesKernel adds up.
+__global__ void __launch_bounds__(256) columnLinesKernel(const __nv_bfloat16* __restrict__ g, float* __restrict__ work, int rows, int n) {
+  __shared__ ColumnShared sh;
+  const int per = (rows + gridDim.y - 1) / gridDim.y, beg = blockIdx.y * per, end = min(rows, beg + per), c = blockIdx.x * 64 + threadIdx.x;
+  tc::grid_dependency_wait();
+  tc::grid_launch_dependents();
+  sumColumns(sh, g, beg, end, n, blockIdx.x * 64);
+  if (threadIdx.x < 64 && c < n) work[(size_t)blockIdx.y * n + c] = sh.sums[threadIdx.x];
 }
 
 template <int EPI>
@@ -284,11 +300,21 @@ bool aligned(const void* a, const void* b = nullptr, const void* c = nullptr, co
   return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e) & 15) == 0;
 }
 int lnBlocks(int rows, int sms) { return std::max(1, std::min((rows + 7) / 8, sms)); }
+// Stretches of rows of a column sum; 0: one launch of clusters.  A block of a cluster sums an eighth of the rows however many there
+// are, and a narrow matrix has few clusters: from 16384 rows on and below 2048 columns (fewer than 256 blocks of clusters) the rows
+// are cut into what gives every SM two blocks.  us behind a kernel that rewrites the matrix, clusters / stretches: 8192 x 1024 4.8 / 5.8,
+// 16384 x 256 6.7 / 5.7, 16384 x 1024 7.8 / 7.0, 16384 x 1536 8.0 / 7.8, 65536 x 256 18.6 / 6.7, 32768 x 768 11.0 / 7.7, 65536 x 1536
+// 41.4 / 34.9, 16384 x 2048 8.8 / 8.7, 24576 x 2048 15.9 / 16.7, 16384 x 3072 13.4 / 17.0; four or eight blocks an SM are slower.
+int sumStretches(int rows, int n, int sms) {
+  const int groups = (n + 63) / 64;
+  if (rows < 16384 || groups * SUM_CTAS >= 256) return 0;
+  return std::max(1, std::min(2 * sms / groups, rows / 128));
+}
 // Launched so that the blocks may come up while the kernel in front still drains (tc_common.h: grid_dependency_wait).
 template <typename... P, typename... A>
-cudaError_t launchBehind(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t stream, A... args) {
+cudaError_t launchBehind(void (*kernel)(P...), dim3 grid, int block, int smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
@@ -338,9 +364,9 @@ DF_API ncclResult_t dfcclLayerNormForward(const void* x, const void* gamma, cons
   return e == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
 }
 
-// fp32 words of scratch memory a backward pass needs on the current device (a column sum: none).
+// fp32 words of scratch memory a backward pass / a column sum needs on the current device.
 DF_API size_t dfcclLayerNormWork(int rows, int d) { return (size_t)lnBlocks(rows, smCount()) * 2 * d; }
-DF_API size_t dfcclColumnSumWork(int, int) { return 0; }
+DF_API size_t dfcclColumnSumWork(int rows, int n) { return rows <= 0 || n <= 0 ? 0 : (size_t)sumStretches(rows, n, smCount()) * n; }
 
 // Gradients of x (plus `pass`, the gradient that reaches x by another way, where given), gamma and beta.
 DF_API ncclResult_t dfcclLayerNormBackward(const void* gy, const void* x, const void* gamma, const void* mean, const void* rstd, const void* pass,
@@ -354,9 +380,16 @@ DF_API ncclResult_t dfcclLayerNormBackward(const void* gy, const void* x, const 
   return e == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
 }
 
-// out[n] = sum over rows of g [rows, n], added up in fp32.
-DF_API ncclResult_t dfcclColumnSum(const void* g, void* out, void*, int rows, int n, cudaStream_t stream) {
+// out[n] = sum over rows of g [rows, n], added up in fp32.  `work`: dfcclColumnSumWork words (null: in one launch whatever the shape).
+DF_API ncclResult_t dfcclColumnSum(const void* g, void* out, void* work, int rows, int n, cudaStream_t stream) {
   if (rows <= 0 || n <= 0 || n % 8 || !g || !out || !aligned(g)) return ncclInvalidArgument;
-  const cudaError_t e = launchBehind(columnSumKernel, (n + 63) / 64 * SUM_CTAS, 256, 0, stream, (const __nv_bfloat16*)g, (__nv_bfloat16*)out, rows, n);
+  const int groups = (n + 63) / 64, stretches = work ? sumStretches(rows, n, smCount()) : 0;
+  cudaError_t e;
+  if (stretches) {
+    e = launchBehind(columnLinesKernel, dim3(groups, stretches), 256, 0, stream, (const __nv_bfloat16*)g, (float*)work, rows, n);
+    if (e == cudaSuccess) e = launchBehind(sumLinesKernel, (n + 31) / 32, 1024, 0, stream, (const float*)work, stretches, n, (__nv_bfloat16*)out, (__nv_bfloat16*)out, n);
+  } else {
+    e = launchBehind(columnSumKernel, groups * SUM_CTAS, 256, 0, stream, (const __nv_bfloat16*)g, (__nv_bfloat16*)out, rows, n);
+  }
   return e == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
 }

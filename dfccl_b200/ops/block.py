@@ -73,7 +73,9 @@ def column_sum(g: torch.Tensor) -> torch.Tensor:
     rows, n = g.shape
     out = torch.empty(n, dtype=torch.bfloat16, device=g.device)
     with on_device(g.device):
-        nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), None, rows, n, raw_stream(g.device)), "dfcclColumnSum")
+        words = nv.lib().dfcclColumnSumWork(rows, n)
+        work = torch.empty(words, dtype=torch.float32, device=g.device) if words else None
+        nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), _ptr(work), rows, n, raw_stream(g.device)), "dfcclColumnSum")
     return out
 
 

@@ -106,6 +106,20 @@ def test_column_sum(native, rows, n):
     assert _rel(block.column_sum(g), g.double().sum(0)) < HALF_ULP
 
 
+@pytest.mark.parametrize("rows,n", [(16383, 200), (16384, 8), (16387, 200), (65536, 64), (65539, 264), (131072, 128), (16385, 1984), (16400, 2048)])
+def test_column_sum_of_tall_matrices(native, rows, n):
+    """In stretches of rows with scratch memory, and in one launch without."""
+    from dfccl_b200.ops import block
+    torch.manual_seed(rows + n)
+    g = torch.randn(rows, n, device="cuda").to(torch.bfloat16)
+    want, out = g.double().sum(0), torch.empty(n, device="cuda", dtype=torch.bfloat16)
+    got = block.column_sum(g)
+    assert _rel(got, want) < HALF_ULP
+    assert torch.equal(got, block.column_sum(g))
+    native.check(native.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), None, rows, n, torch.cuda.current_stream().cuda_stream), "dfcclColumnSum")
+    assert _rel(out, want) < HALF_ULP
+
+
 @pytest.mark.parametrize("tokens,d,hooked", [(256, 256, False), (8192, 512, False), (256, 256, True)])
 def test_block_against_torch_operators(native, tokens, d, hooked):
     """Output and every gradient of a one-rank block; modules with hooks are called as modules."""
