@@ -31,6 +31,9 @@ size_t dfcclGemmFusedArgsSize(void);
 ncclResult_t dfcclGemmCheck(int* failed);
 // CTA pairs of the cta_group::2 GEMM kernel that can be resident together on the current device.
 ncclResult_t dfcclGemmPairResident(int* pairs);
+/* What runs a plain product on a GPU of `sms` SMs: {CTA pairs, columns of a tile of the tile kernel or 0, slices of the contraction,
+ * columns of a tile of the persistent kernel or 0}. */
+ncclResult_t dfcclGemmPlan(int M, int N, int K, int bTransposed, int epilogue, int sms, int plan[4]);
 /* SMs the fused launches leave free for a persistent kernel that runs beside them (the daemon's blocks). */
 ncclResult_t dfcclGemmReserveSms(int n);
 

@@ -593,6 +593,15 @@ DF_API ncclResult_t dfcclGemmPairResident(int* pairs) {
   return ncclSuccess;
 }
 
+// What runs a plain product on a GPU of that many SMs: plan = {CTA pairs, columns of a tile of the tile kernel or 0, slices of the
+// contraction, columns of a tile of the persistent kernel or 0}.
+DF_API ncclResult_t dfcclGemmPlan(int M, int N, int K, int bTransposed, int epilogue, int sms, int plan[4]) {
+  if (!plan || M <= 0 || N <= 0 || K <= 0 || M % BM || N % BN || K % BK || sms <= 0) return ncclInvalidArgument;
+  const GemmTilePlan p = gemmTilePlan(M, N, K, sms, paramI64("GEMM_PAIR", 1) != 0, bTransposed != 0, epilogue != EPI_NONE);
+  plan[0] = p.pair; plan[1] = p.width ? 0 : p.tn; plan[2] = p.split; plan[3] = p.width;
+  return ncclSuccess;
+}
+
 // SMs the fused launches leave free for a persistent kernel that runs beside them (e.g. the daemon's blocks).
 DF_API ncclResult_t dfcclGemmReserveSms(int n) {
   if (n < 0 || n > 128) return ncclInvalidArgument;

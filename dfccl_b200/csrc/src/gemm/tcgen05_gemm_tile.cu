@@ -4,7 +4,7 @@
 // What bounds such a product is how few SMs a handful of tiles occupies, the issue of loads and MMAs in a CTA (about 80 clocks
 // per MMA of 16 K however narrow the tile, 230 per load instruction: hence 128 K and one load per operand in a stage),
 // and the fixed cost of a launch.
-//   * Tiles of 128 x {64, 128} on one CTA (cta_group::1) or 256 x 128 on a pair (cta_group::2, each CTA loads
+//   * Tiles of 128 x {64, 128} on one CTA (cta_group::1) or 256 x {128, 256} on a pair (cta_group::2, each CTA loads
 //     half of B: fewer operand bytes per FLOP); the last row tile may stick out of M (TMA fills zeros, rows are not stored).
 //   * The contraction of a tile is cut into up to 4 slices on the CTAs of one cluster.  Every CTA of the cluster owns
 //     a slice of the tile's columns: the others write their fp32 partial sums of those columns into the owner's shared
@@ -253,7 +253,7 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 
 typedef void (*TileKernel)(const CUtensorMap, const CUtensorMap, const TileArgs);
 TileKernel kernelOf(bool pair, int tn) {
-  if (pair) return dfcclGemmTileKernel<true, 128>;
+  if (pair) return tn == 128 ? dfcclGemmTileKernel<true, 128> : dfcclGemmTileKernel<true, 256>;
   return tn == 64 ? dfcclGemmTileKernel<false, 64> : dfcclGemmTileKernel<false, 128>;
 }
 
@@ -330,6 +330,12 @@ static GemmTilePlan choosePlan(int M, int N, int K, int sms, bool pairs, bool bM
   };
   GemmTilePlan p = best(false, false);
   if (p.split == 1 && bMn) p = best(true, true);
+  // One wave of plain tiles of 256 x 256 gains nothing from the persistent kernel's overlap, and the form with the same tile has
+  // stages of 128 of the contraction and a geometry that the compiler knows.  us, persistent / form: 4096 x 1024 x 8192 58.5 / 56.9,
+  // x 2048 16.8 / 15.8, x 1024 10.8 / 10.0, x 512 7.9 / 7.6, 1024 x 4096 x 8192 59.2 / 57.1, 7168 x 512 x 960 11.9 / 11.3, 3328 x 1024 x
+  // 4032 24.4 / 23.8; but 640 x 5120 x 448 7.2 / 7.3, 4096 x 1024 x 128 5.3 / 5.8, and with one or two row tiles, whose operands hardly
+  // meet in L2, 512 x 7168 x 4992 29.4 / 31.4, 384 x 7680 x 5248 33.5 / 34.9.
+  if (pairs && !epilogue && p.width == 256 && (M + 255) / 256 * (N / 256) <= sms / 2 && K >= 512 && M > 512) p = GemmTilePlan{true, 256, 1, 0};
   if (!pairs && (p.pair || p.width)) {                 // one CTA per tile by request: the same slices
     double us = 1e30;
     const int split = p.split;
@@ -357,7 +363,7 @@ ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B,
   CUDACHECK(oncePerDevice([] {
     cudaError_t r = cudaSuccess;
     for (const Form& f : FORMS) if (r == cudaSuccess) r = allowSharedMemory(kernelOf(f.pair, f.tn), SMEM_LIMIT);
-    return r;
+    return r == cudaSuccess ? allowSharedMemory(kernelOf(true, 256), SMEM_LIMIT) : r;
   }));
   TileArgs g;
   memset(&g, 0, sizeof(g));

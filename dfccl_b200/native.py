@@ -176,7 +176,7 @@ def lib() -> C.CDLL:
             "dfcclLayerNormForward": [vp, vp, vp, vp, vp, vp, i, i, C.c_float, vp],
             "dfcclLayerNormBackward": [vp] * 10 + [i, i, vp], "dfcclLayerNormWork": [i, i], "dfcclLayerNormMaxWidth": [],
             "dfcclGemmCheck": [C.POINTER(i)],
-            "dfcclGemmPairResident": [C.POINTER(i)],
+            "dfcclGemmPairResident": [C.POINTER(i)], "dfcclGemmPlan": [i, i, i, i, i, i, C.POINTER(i)],
             "dfcclGemmFused": [vp, vp, vp, i, i, i, vp, sz, vp],
             "dfcclHeapPeerBase": [vp, i, C.POINTER(vp)],
             "dfcclCommTransport": [vp, C.POINTER(i)],

@@ -16,3 +16,22 @@ def test_tall_column_sums_fill_the_gpu(rows, n):
 @pytest.mark.parametrize("rows,n", [(1, 8), (8192, 1024), (16383, 64), (65536, 2048), (131072, 4096)])
 def test_other_column_sums_are_one_launch(rows, n):
     assert nv.lib().dfcclColumnSumWork(rows, n) == 0
+
+
+def gemm_plan(m, n, k, b_transposed=False, epilogue=0, sms=148):
+    """(pairs, tile columns, slices, width of a persistent tile)"""
+    import ctypes as C
+    plan = (C.c_int * 4)()
+    nv.check(nv.lib().dfcclGemmPlan(m, n, k, int(b_transposed), epilogue, sms, plan), "dfcclGemmPlan")
+    return tuple(plan)
+
+
+@pytest.mark.parametrize("m,n,k", [(4096, 1024, 8192), (1024, 4096, 8192), (4096, 1024, 1024), (2304, 2048, 8192), (9472, 512, 8192)])
+def test_one_wave_of_the_widest_tiles(m, n, k):
+    """Plain products of at most a tile per pair of SMs run on the tile kernel, whatever the storage order; with an epilogue, with
+    more tiles than pairs, with a short contraction or less than three row tiles on the persistent one."""
+    for bt in (False, True):
+        assert gemm_plan(m, n, k, bt) == (1, 256, 1, 0)
+    assert gemm_plan(m, n, k, False, 1)[3] == 256
+    assert gemm_plan(2 * m, n, k)[3] == gemm_plan(2 * m, n, k, True)[3] == 256
+    assert gemm_plan(m, n, 448)[1] != 256 and gemm_plan(512, 7168, k)[1] != 256

@@ -1,24 +1,35 @@
 """Persistent tiles of 256 x width: widths that cut the last column tile, an MN-major operand whose blocks of 64 columns the tiles
-cut through, odd numbers of 64-wide contraction blocks, a half empty last row tile, more tiles than pairs and fewer."""
+cut through, odd numbers of 64-wide contraction blocks, a half empty last row tile, more tiles than pairs and fewer; the tile form of
+256 x 256 at the edges of its range."""
 import pytest
 import torch
 
+from test_dispatch_rules import gemm_plan
+
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(512, 1280, 2304), (1408, 512, 2368),            # width 64
-          (128, 4864, 3840), (2432, 512, 4544),            # 96, the last tile 64 columns
-          (6528, 1024, 2496),                              # 128
-          (2432, 1024, 256), (4096, 1280, 2368),           # 160, the last tile 64 columns / whole tiles
-          (4864, 512, 256), (1536, 2304, 320),             # 192
-          (3072, 1024, 2112), (384, 7936, 256),            # 224 K-major and 192 MN-major; one wave of 256
-          (896, 4096, 256), (1152, 3328, 2624)]            # 256
+# (m, n, k), width with B stored K-major and MN-major (0: a tile form runs it; T: the one of 256 x 256)
+T = "tile"
+SHAPES = [((512, 1280, 2304), 64, 0), ((1408, 512, 2368), 64, 0),
+          ((128, 4864, 3840), 96, 0), ((2432, 512, 4544), 96, 0),                         # the last tile 64 columns
+          ((6528, 1024, 2496), 128, 128), ((2560, 2816, 1728), 224, 128),
+          ((2432, 1024, 256), 160, 160), ((4096, 1280, 2368), 160, 160),                  # the last tile 64 columns / whole tiles
+          ((2816, 1792, 2240), 160, 160),                                                 # 32 columns
+          ((4864, 512, 256), 192, 192), ((1536, 2304, 320), 192, 192),
+          ((3072, 1024, 2112), 224, 192), ((1152, 5632, 512), 224, 224), ((2688, 2560, 320), 224, 224),        # 128, 32, 96 columns
+          ((384, 7936, 256), 256, 256), ((896, 4096, 256), 256, 256), ((2304, 3584, 576), 256, 256),
+          ((1152, 3328, 2624), T, T), ((640, 5120, 512), T, T), ((4096, 1024, 576), T, T)]
 
 
-@pytest.mark.parametrize("m,n,k", SHAPES)
-def test_widths_at_their_edges(m, n, k):
+@pytest.mark.parametrize("shape,k_major,mn_major", SHAPES)
+def test_widths_at_their_edges(shape, k_major, mn_major):
     """The error against 64 bits is that of one rounding to bf16 (2**-8 of a value at most, 2**-9 in the 2-norm over many), the
     same bits for every storage order, and nothing outside the result is written."""
     from dfccl_b200.ops import gemm
+    m, n, k = shape
+    for b_t, want in ((False, k_major), (True, mn_major)):
+        _, tile, _, width = gemm_plan(m, n, k, b_t)
+        assert (tile == 256) if want == T else width == want
     torch.manual_seed(m + 3 * n + 5 * k)
     a = torch.randn(m, k, device="cuda", dtype=torch.bfloat16)
     b = torch.randn(n, k, device="cuda", dtype=torch.bfloat16)
