@@ -37,6 +37,7 @@ constexpr int PM = 256, HALF = 128, MAX_STAGES = 6, UMMA_K = 16;
 constexpr int SMEM_LIMIT = 227 * 1024, BAR_BYTES = 256, ALIGN_SLACK = 1024;
 constexpr int BOX_BYTES = 32 * 64;                   // a staged box of the epilogue: 32 rows x 32 columns
 constexpr int EPI_BOXES = 16, EPI_BYTES = EPI_BOXES * BOX_BYTES;
+constexpr int WIDE_STAGE = (HALF + 128) * 64 * 2;    // a stage of the widest tile, per CTA
 constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on another GPU: seconds mean a lost partner
 
 // Epilogue warps: two per 32 accumulator rows, four where an element costs more than its rounding (8192 x 4096 x 1024 with bias and
@@ -60,14 +61,17 @@ struct PairArgs {
   bool wide, wideC;                 // aux, and C and pre, start on a 32-byte boundary
 };
 
-template <int EPI>
+// WIDE: tiles of 256 x 256 in stages of 64, known to the compiler: the loops that issue loads and MMAs keep no geometry.  us:
+// 8192 x 4096 x 1024 56.0 -> 55.6, its data gradient 56.2 -> 55.7, 4096 x 4096 x 1024 and its gradients 94.0 -> 93.8.
+template <int EPI, bool WIDE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pairThreads(EPI), 1)
 dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapC,
                     const __grid_constant__ CUtensorMap mapPre, const PairArgs g) {
+  const int tn = WIDE ? 256 : g.tn, kStep = WIDE ? 1 : g.kStep, stageBytes = WIDE ? WIDE_STAGE : g.stageBytes;
   constexpr int EPI_WARPS = epiWarps(EPI), PARTS = EPI_WARPS / 4, BUFS = EPI_BOXES / EPI_WARPS;
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);       // the same offset in both CTAs
-  uint8_t* stg = smem + g.stages * g.stageBytes;
+  uint8_t* stg = smem + g.stages * stageBytes;
   uint64_t* fullBar = (uint64_t*)(stg + g.epiBytes);                  // used in the leader only
   uint64_t* emptyBar = fullBar + MAX_STAGES;                         // in both CTAs (commit to both)
   uint64_t* accFull = emptyBar + MAX_STAGES;                         // [2] in both CTAs
@@ -77,11 +81,11 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t cr = cluster_ctarank();             // 0 = leader
-  const int mTiles = (g.M + PM - 1) / PM, nTiles = (g.N + g.tn - 1) / g.tn, kb64 = g.K / 64;
+  const int mTiles = (g.M + PM - 1) / PM, nTiles = (g.N + tn - 1) / tn, kb64 = g.K / 64;
   const int numTiles = mTiles * nTiles;
   const int pair = blockIdx.x >> 1, numPairs = gridDim.x >> 1;
-  const int bHalf = g.tn / 2;
-  const int aBytes = HALF * 128 * g.kStep, mnBlock = 64 * 128 * g.kStep;      // MN-major operand: blocks of 64 MN-columns x K-rows; K-major: 64 K-columns x rows
+  const int bHalf = tn / 2;
+  const int aBytes = HALF * 128 * kStep, mnBlock = 64 * 128 * kStep;      // MN-major operand: blocks of 64 MN-columns x K-rows; K-major: 64 K-columns x rows
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < g.stages; ++s) { mbar_init(&fullBar[s], 1); mbar_init(&emptyBar[s], 1); }
@@ -111,18 +115,18 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       // 64 x 64 kStep x (cols / 64).  An MN-major B whose tiles are not whole blocks is loaded block by block, from any multiple
       // of 16 columns.  The second half of the last stage may lie outside (zeros): it is loaded and not multiplied.
       const uint32_t bar0 = mapa_u32(smem_u32(fullBar), 0);
-      const bool bLoose = g.bMn && bHalf % 64 != 0;
+      const bool bLoose = !WIDE && g.bMn && bHalf % 64 != 0;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int t = pair; t < numTiles && ok; t += numPairs) {
         int mt, nt;
         raster_tile(t, mTiles, nTiles, g.groupM, mt, nt);
-        const int rowA = mt * PM + (int)cr * HALF, rowB = nt * g.tn + (int)cr * bHalf;
-        for (int k = 0; k < kb64; k += g.kStep) {
+        const int rowA = mt * PM + (int)cr * HALF, rowB = nt * tn + (int)cr * bHalf;
+        for (int k = 0; k < kb64; k += kStep) {
           if (!mbar_wait(&emptyBar[stage], phase ^ 1, giveUp, WAIT_NS)) { ok = false; break; }
-          if (cr == 0) mbar_expect_tx(&fullBar[stage], 2 * g.stageBytes);       // my bytes and the partner's
-          uint8_t* sa = smem + stage * g.stageBytes;
+          if (cr == 0) mbar_expect_tx(&fullBar[stage], 2 * stageBytes);       // my bytes and the partner's
+          uint8_t* sa = smem + stage * stageBytes;
           const uint32_t bar = bar0 + stage * 8;
           tma_load_3d_pair(sa, &mapA, g.aMn ? k * 64 : rowA, g.aMn ? rowA / 64 : k, bar);
           if (!bLoose) tma_load_3d_pair(sa + aBytes, &mapB, g.bMn ? k * 64 : rowB, g.bMn ? rowB / 64 : k, bar);
@@ -135,7 +139,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
     if (cr == 0 && elect_one()) {
-      const uint32_t idesc = umma_idesc_bf16(PM, g.tn, g.aMn, g.bMn);
+      const uint32_t idesc = umma_idesc_bf16(PM, tn, g.aMn, g.bMn);
       // per instruction (16 K): K-major 32 bytes along the row; MN-major two groups of 8 K-rows.  Per 64 K: the next block of
       // [rows] x 64 K-columns, or 64 K-rows further down the same blocks.
       const uint32_t stepA = g.aMn ? 128u : 2u, stepB = g.bMn ? 128u : 2u;
@@ -149,15 +153,15 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
         if (!mbar_wait(&accEmpty[ab], ((it >> 1) & 1) ^ 1, giveUp, WAIT_NS)) break;
         tc_fence_after();
         const uint32_t d = tmemBase + ab * 256;
-        for (int kb = 0; kb < kb64; kb += g.kStep) {
+        for (int kb = 0; kb < kb64; kb += kStep) {
           if (!mbar_wait(&fullBar[stage], phase, giveUp, WAIT_NS)) { ok = false; break; }
           tc_fence_after();
-          const uint8_t* pa = smem + stage * g.stageBytes;
+          const uint8_t* pa = smem + stage * stageBytes;
           const uint64_t da = g.aMn ? umma_smem_desc_mn_sw128(pa, mnBlock) : umma_smem_desc_sw128(pa);
           const uint64_t db = g.bMn ? umma_smem_desc_mn_sw128(pa + aBytes, mnBlock) : umma_smem_desc_sw128(pa + aBytes);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            if (h == 1 && (g.kStep == 1 || kb + 1 == kb64)) break;
+            if (h == 1 && (kStep == 1 || kb + 1 == kb64)) break;
 #pragma unroll
             for (int k = 0; k < 64 / UMMA_K; ++k)
               umma_bf16_pair(d, da + hopA * h + stepA * k, db + hopB * h + stepB * k, idesc, (kb | h | k) != 0);
@@ -199,9 +203,9 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       int mt, nt;
       raster_tile(t, mTiles, nTiles, g.groupM, mt, nt);
       const int ab = it & 1;
-      const int row0 = mt * PM + (int)cr * HALF + quarter * 32, col0 = nt * g.tn;      // of this warp's 32 rows
+      const int row0 = mt * PM + (int)cr * HALF + quarter * 32, col0 = nt * tn;      // of this warp's 32 rows
       const bool mine = row0 < g.M;                                   // the last row tile may have only its upper half
-      const int steps = min(g.tn, g.N - col0) / 32;
+      const int steps = min(tn, g.N - col0) / 32;
       constexpr bool AUX = EPI == EPI_BIAS_RES || EPI == EPI_GELU_GRAD;
       const __nv_bfloat16* aux = g.e.aux + (size_t)(row0 + lane) * g.ldc + col0;
       uint4 own[4];
@@ -287,15 +291,18 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 
 namespace {
 typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const PairArgs);
-PairKernel pairKernel(int epi) {
-  static const PairKernel k[] = {dfcclGemmPairKernel<EPI_NONE>, dfcclGemmPairKernel<EPI_BIAS>, dfcclGemmPairKernel<EPI_BIAS_RES>,
-                                 dfcclGemmPairKernel<EPI_BIAS_GELU>, dfcclGemmPairKernel<EPI_GELU_GRAD>};
+template <bool WIDE>
+PairKernel pairKernelOf(int epi) {
+  static const PairKernel k[] = {dfcclGemmPairKernel<EPI_NONE, WIDE>, dfcclGemmPairKernel<EPI_BIAS, WIDE>, dfcclGemmPairKernel<EPI_BIAS_RES, WIDE>,
+                                 dfcclGemmPairKernel<EPI_BIAS_GELU, WIDE>, dfcclGemmPairKernel<EPI_GELU_GRAD, WIDE>};
   return k[epi];
 }
+PairKernel pairKernel(int epi, bool wide) { return wide ? pairKernelOf<true>(epi) : pairKernelOf<false>(epi); }
 cudaError_t allowPairs() {
   return oncePerDevice([] {
     cudaError_t r = cudaSuccess;
-    for (int e = EPI_NONE; e <= EPI_GELU_GRAD && r == cudaSuccess; ++e) r = allowSharedMemory(pairKernel(e), SMEM_LIMIT);
+    for (int e = EPI_NONE; e <= EPI_GELU_GRAD; ++e)
+      for (int w = 0; w < 2 && r == cudaSuccess; ++w) r = allowSharedMemory(pairKernel(e, w != 0), SMEM_LIMIT);
     return r;
   });
 }
@@ -310,7 +317,7 @@ int maxResidentPairs(int dev, int sms) {
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(sms & ~1); cfg.blockDim = dim3(pairThreads(EPI_NONE)); cfg.dynamicSmemBytes = SMEM_LIMIT;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, pairKernel(EPI_NONE), &cfg) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = sms / 2; }
+    if (cudaOccupancyMaxActiveClusters(&n, pairKernel(EPI_NONE, true), &cfg) != cudaSuccess || n <= 0) { (void)cudaGetLastError(); n = sms / 2; }
     maxPairs[dev & 63] = std::min(n, sms / 2);
   }
   return maxPairs[dev & 63];
@@ -359,7 +366,7 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   const int tiles = (M + PM - 1) / PM * ((N + width - 1) / width);
   const int pairs = std::min(tiles, maxResidentPairs(dev, sms));
   g.kStep = kStep;
-  g.stageBytes = HALF * BK * 2 + bBytes;
+  g.stageBytes = HALF * BK * 2 + bBytes;               // width 256: WIDE_STAGE, however B is stored
   const int room = SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK - g.epiBytes;
   const int want = tiles > pairs ? MAX_STAGES : (K + BK - 1) / BK;
   g.stages = std::min(std::min(MAX_STAGES, room / g.stageBytes), want);
@@ -373,7 +380,7 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at; cfg.numAttrs = 1;
-  CUDACHECK(cudaLaunchKernelEx(&cfg, pairKernel(g.e.kind), ma, mb, mc, mp, g));
+  CUDACHECK(cudaLaunchKernelEx(&cfg, pairKernel(g.e.kind, width == 256), ma, mb, mc, mp, g));
   return ncclSuccess;
 }
 
