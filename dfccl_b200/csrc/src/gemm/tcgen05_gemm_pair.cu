@@ -96,7 +96,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
     tma_prefetch_desc(&mapB);
-    tma_prefetch_desc(&mapC);
+    if (g.epiBytes) tma_prefetch_desc(&mapC);
   }
   if (warp == 1) tmem_alloc_pair(tmemBaseSlot, g.tmemCols);
   tc_fence_before();
@@ -342,14 +342,11 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   DFCHECK(gemmMakeMap3(&ma, A, (uint64_t)M, (uint64_t)K, aMn, HALF, BK));
   if (bMn && bHalf % 64) DFCHECK(gemmMakeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
   else DFCHECK(gemmMakeMap3(&mb, B, (uint64_t)N, (uint64_t)K, bMn, bHalf, BK));
-  DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
-  mp = mc;
   PairArgs g;
   memset(&g, 0, sizeof(g));
   g.M = M; g.N = N; g.K = K; g.ldc = N; g.aMn = aMn ? 1 : 0; g.bMn = bMn ? 1 : 0; g.tn = width;
   g.err = errDev; g.errHost = errHost;
   if (e) g.e = *e;
-  if (g.e.kind == EPI_BIAS_GELU && g.e.pre) DFCHECK(gemmMakeMap(&mp, g.e.pre, (uint64_t)M, (uint64_t)N, 32, 32));
   g.C = (__nv_bfloat16*)C;
   g.wide = ((uintptr_t)g.e.aux & 31) == 0;
   g.wideC = (((uintptr_t)C | (uintptr_t)g.e.pre) & 31) == 0;
@@ -359,6 +356,10 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   // GELU 60.6 / 63.8, 8192 x 1024 x 1024 17.6 / 20.0; with GELU's gradient, bound by its arithmetic, 69.9 / 67.9.
   const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && K >= 896);
   g.epiBytes = straight ? 0 : EPI_BYTES;
+  mc = ma;                                             // (straight stores take no map: none is made, or kept, per output)
+  if (!straight) DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
+  mp = mc;
+  if (g.e.kind == EPI_BIAS_GELU && g.e.pre) DFCHECK(gemmMakeMap(&mp, g.e.pre, (uint64_t)M, (uint64_t)N, 32, 32));
   { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
