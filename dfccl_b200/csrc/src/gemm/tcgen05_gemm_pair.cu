@@ -1,7 +1,7 @@
 // bf16 GEMM on CTA pairs (tcgen05 cta_group::2), hand-written for sm_100a:
-//     C[M,N] = A[M,K] * B[N,K]^T,  tiles of 256 x tn (tn a multiple of 32, chosen per product), one tile per pair of CTAs (a
-// cluster of two SMs) at a time.  Rows and columns of the last tiles beyond M (a multiple of 128) and N are loaded as zeros
-// and not stored.
+//     C[M,N] = A[M,K] * B[N,K]^T,  tiles of 256 x tn, one tile per pair of CTAs (a cluster of two SMs) at a time; tn is chosen per
+// product, 64 to 256 in steps of 32, from 128 on where B is stored MN-major.  Rows and columns of the last tiles beyond M (a
+// multiple of 128) and N are loaded as zeros and not stored.
 // Each CTA of a pair loads 128 rows of A and tn / 2 rows of B per stage (64 or 128 of the contraction), the leader's single MMA thread issues
 // 256 x tn x 16 instructions that read both CTAs' shared memory, and each CTA ends up with its 128 rows of the accumulator
 // in its own tensor memory.  The tensor cores of an SM thus see every B row once per pair instead of once per CTA: half the
@@ -371,7 +371,7 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   const int room = SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK - g.epiBytes;
   const int want = tiles > pairs ? MAX_STAGES : (K + BK - 1) / BK;
   g.stages = std::min(std::min(MAX_STAGES, room / g.stageBytes), want);
-  g.tmemCols = tiles > pairs ? 512 : width <= 32 ? 32 : width <= 64 ? 64 : width <= 128 ? 128 : 256;
+  g.tmemCols = tiles > pairs ? 512 : width <= 64 ? 64 : width <= 128 ? 128 : 256;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(pairThreads(g.e.kind)); cfg.stream = stream;

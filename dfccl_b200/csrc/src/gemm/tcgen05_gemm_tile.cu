@@ -317,7 +317,7 @@ static GemmTilePlan choosePlan(int M, int N, int K, int sms, bool pairs, bool bM
   auto best = [&](bool mn, bool whole) {               // `whole`: contractions that are not cut
     GemmTilePlan p{true, 0, 1, 256};
     double us = pairUs(M, N, kb, 256, sms, mn);
-    for (int w = 32; w < 256; w += 32) {
+    for (int w = mn ? 128 : 64; w < 256; w += 32) {      // (narrower ones never were the least: 780 000 products, 132 and 148 SMs)
       const double t = pairUs(M, N, kb, w, sms, mn);
       if (t < us) { us = t; p.width = w; }
     }

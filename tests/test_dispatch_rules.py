@@ -35,3 +35,10 @@ def test_one_wave_of_the_widest_tiles(m, n, k):
     assert gemm_plan(m, n, k, False, 1)[3] == 256
     assert gemm_plan(2 * m, n, k)[3] == gemm_plan(2 * m, n, k, True)[3] == 256
     assert gemm_plan(m, n, 448)[1] != 256 and gemm_plan(512, 7168, k)[1] != 256
+
+
+def test_widths_of_the_persistent_kernel():
+    """What its tiles can be: 64 columns and more, 128 and more where B is stored MN-major (what its tests run is all of it)."""
+    seen = {bt: {gemm_plan(128 * m, 256 * n, 64 * k, bt, e)[3] for m in range(1, 33) for n in range(1, 33) for k in (1, 2, 3, 5, 8, 16, 36, 60, 128) for e in (0, 1)}
+            for bt in (False, True)}
+    assert seen[False] - {0} == {64, 96, 128, 160, 192, 224, 256} and seen[True] - {0} == {128, 160, 192, 224, 256}
