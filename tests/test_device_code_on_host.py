@@ -82,3 +82,49 @@ int main() {
 }
 """)
     assert out.split() == "0 1 2 3 1 1 3 3 3 3 0 1 2 3".split()
+
+
+def test_offsets_are_those_of_the_epoch(tmp_path):
+    """Members on one device: whatever order the words of a slot arrive in, a wait succeeds with the offsets of its own epoch, also
+    where the tag's 16 bits come round, and never with those of a peer that has gone on without it."""
+    out = run_on_host(tmp_path, r"""
+#include <memory>
+static bool arrived(FlagSlot* f, uint32_t epoch, uint64_t* send, uint64_t* recv) {
+  static DaemonCtl ctl;
+  RankDev rd;
+  memset((void*)&rd, 0, sizeof(rd));
+  rd.ctl = &ctl;
+  std::unique_ptr<BlockShared> sh(new BlockShared);
+  memset((void*)sh.get(), 0, sizeof(BlockShared));
+  sh->k = rd;
+  CollStatic* c = &sh->cs;
+  c->kind = dfcclCollBroadcast; c->inType = c->outType = ncclInt8; c->nranks = 2; c->root = 1; c->nBlocks = 1; c->count = 64;
+  c->algo = dfcclAlgoOneShot; c->oneDevice = 1; c->myFlags = f; c->scale = 1.0;
+  planColl(c, 0);
+  sh->dyn.epoch = epoch;
+  const bool ok = boundedWait(sh.get(), &rd, 0, 0, 4);
+  *send = sh->peerSend[1]; *recv = sh->peerRecv[1];
+  return ok;
+}
+int main() {
+  for (uint32_t epoch : {1u, 2u, 0xffffu, 0x10000u, 0x10001u, 0x20000u, 0xffff0000u}) {
+    for (int seen = 0; seen < 8; ++seen) {               // bit by bit: the arrival, the send offset, the receive offset are there
+      FlagSlot f[2];
+      memset((void*)f, 0, sizeof(f));
+      f[1].arrive = seen & 1 ? epoch : epoch - 1;
+      f[1].sendOff = seen & 2 ? offTagged(4096, epoch) : epoch > 1 ? offTagged(512, epoch - 1) : 0;
+      f[1].recvOff = seen & 4 ? offTagged(8192, epoch) : epoch > 1 ? offTagged(1024, epoch - 1) : 0;
+      uint64_t s, r;
+      const bool ok = arrived(f, epoch, &s, &r);
+      if (ok != (seen == 7)) { printf("epoch %u words %d: %d\n", epoch, seen, ok); return 1; }
+      if (ok && (s != 4096 || r != 8192)) return 2;
+      f[1].arrive = epoch + 1;                           // the peer has gone on
+      f[1].sendOff = offTagged(512, epoch + 1);
+      if (arrived(f, epoch, &s, &r)) return 3;
+    }
+  }
+  puts("ok");
+  return 0;
+}
+""")
+    assert out == "ok\n"
