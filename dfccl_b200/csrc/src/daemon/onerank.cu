@@ -5,12 +5,9 @@
 // Bound: HBM (or L2 for what fits there).  A block of 256 threads takes 1024 consecutive 16-byte packs, four per
 // thread and all four loads before the first store, so that 5 resident blocks (48 registers a thread) keep 80 KB per SM in
 // flight; calls too small to give every SM such a block take one pack per thread instead (more blocks, shorter chains).
-// Measured: all-reduce of 8388611 fp32 values in ordinary tensors 13.4 us = 5.0 TB/s read + write; the collective kernel
-// that stages such buffers into the heap and out again on 64 blocks took 64.7 us; 11.3 with blocks that come up behind the
-// kernel in front (below).  Eight calls of 64 KB one behind the other in a stream, submitted and awaited: 61.0 us, with one
-// cluster a call and early blocks 41.6.  bf16 -> fp32 packs are stored as whole
-// 32-byte sectors: with that (and the shorter publication) three gradient buckets of 51 MB and their SGD step went from 186
-// to 172 us, 25 MiB among four ranks through the daemon's data path, which stores alike, from 112 to 106.
+// The blocks come up while the kernel in front of them in the stream drains.  bf16 -> fp32 packs are stored as whole 32-byte sectors.
+// Measured: all-reduce of 8388611 fp32 values in ordinary tensors 11.4 us = 5.9 TB/s read + write (13.9 without early blocks; the
+// collective kernel, which stages such buffers into the heap and out again on 64 blocks, 64.7).
 #include "../device/engine.h"
 #include "../device/launch.h"
 #include "../gemm/tc_common.h"
@@ -52,7 +49,9 @@ __device__ __forceinline__ void publishDone(const OneRankDone& done) {
 }
 
 // SHORT: the whole call is one cluster of blocks, which meet at the cluster's barrier before one thread publishes, instead of
-// counting themselves in global memory (a fence and an atomic, two round trips to L2 at the end of a kernel that moves 64 KB).
+// counting themselves in global memory (a fence and an atomic, two round trips to L2 at the end of a kernel that moves 64 KB).  Up
+// to what a cluster holds with four packs a thread in flight; eight calls behind one another in a stream, blocks that count
+// themselves / one cluster, us: 8 KB 38.8 / 35.5, 64 KB 45.8 / 36.3, 128 KB (the limit) 47.4 / 37.2.
 // The blocks may come up while the kernel in front of them in the stream still runs, and wait for its end before they read.
 template <typename Tin, typename Tout, bool COPY, int U, bool SHORT>
 __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs a) {

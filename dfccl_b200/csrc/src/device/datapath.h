@@ -650,7 +650,10 @@ __host__ __device__ bool reduce_small(int inType, int outType, int op, const Dat
 __host__ __device__ bool reduce_small(int inType, int outType, int op, const DataArgs* a);
 #endif
 
-#define DF_SMALL_TRIPS 4       // calls of at most this many packs per thread and source go through the small bodies
+// Calls of at most this many packs per thread and source go through the small bodies.  bf16 -> fp32 among four ranks, us, limit
+// 2 / 4 / 8: 0.9 M values 24.2 / 24.1 / 24.2, 1.3 M 28.6 / 26.7 / 26.7, 1.9 M 32.2 / 30.7 / 30.2, 2.6 M 35.9 / 36 / 34.4, 3.7 M 42.1 / 42.2 /
+// 40.3: the small body is the better one at this limit, and a little beyond it.
+#define DF_SMALL_TRIPS 4
 // What the step engine calls.
 DF_HD bool reduce_block(int inType, int outType, int esIn, int op, const DataArgs* a) {
   const bool small = a->n * (uint64_t)esIn <= (uint64_t)df_nthreads() * 16u * DF_SMALL_TRIPS;

@@ -640,14 +640,12 @@ DF_HD bool patientWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
 // `*moved` is set when at least one phase (or slice) was left behind during this visit.
 // The phase lives in a register of every thread: a visit reads it when it begins, and thread 0 writes it back when it ends
 // (every way out has met a barrier since the read), so that a change of phase costs no barrier of its own.
-// What bounds a small collective here is instructions, barriers and round trips to L2 one behind the other, in one block.  509 bf16
-// among four ranks of a device, submitted and awaited on the host, 33.4 us -> 23.7 with: the phase in a register, the rank's
-// constants in shared memory, the partition worked out at registration, the pointer lists built by one lane per member in front of
-// the barrier that ends the wait, small bodies (datapath.h), one fence less in front of the completion.  25 MiB bf16 -> fp32 among
-// four 97.5 -> 85.9, a ragged reduce-scatter and all-gather 88.6 -> 76.5, 24 mixed collectives in four orders 297 -> 249; one
-// atomic for the blocks' count and verdicts, and an idle block that looks at its ring alone: 22.4, 83.5, 73.3, 247.
-// Comparisons instead of jump tables, phases one behind the other, one fence less for a completion that no stream waits for: with
-// the calls out of ctypes 21.1 -> 20.2, 83.5 -> 81.3, 69 -> 65.8, 220 -> 211.
+// What bounds a small collective here is instructions, barriers and round trips to L2 one behind the other, in one block.  Hence
+// the phase in a register, the rank's constants in shared memory, the partition worked out at registration, the pointer lists built
+// by one lane per member in front of the barrier that ends the wait, small bodies (datapath.h), one atomic for the blocks' count and
+// verdicts, comparisons instead of jump tables, and no fence that nobody waits for.  Among four ranks of a device, submitted and
+// awaited on the host, before / with all of these and calls that do not go through ctypes, us: 509 bf16 33.9 / 19.8, 25 MiB
+// bf16 -> fp32 97.9 / 81.2, a ragged reduce-scatter and all-gather 90.7 / 66.5, 24 mixed collectives in four orders 295 / 203 - 214.
 DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget, bool* moved) {
   if (!sh->standalone) loadColl(sh, rd, b, coll);
   const CollStatic* c = &sh->cs;

@@ -334,8 +334,9 @@ int gemmPairResident() {
 ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream, int aMn, int bMn,
                             uint32_t* errDev, uint32_t* errHost, const GemmEpilogue* e) {
   CUDACHECK(allowPairs());
-  // 64 of the contraction in a stage keep more loads in flight beside wide tiles (8192 x 4096 x 1024 and its gradients 179 -> 176
-  // us); for narrower ones the tensor cores are through with such a stage before its two loads are issued (460 clocks)
+  // 64 of the contraction in a stage keep more loads in flight beside wide tiles (stages of 128: 8192 x 4096 x 1024 and its
+  // gradients 0.3 - 0.5 % slower, 4096 x 1024 x 8192 the same); for narrower ones the tensor cores are through with such a stage
+  // before its two loads are issued (460 clocks)
   const int kStep = width >= 224 ? 1 : 2, BK = 64 * kStep;
   const int bHalf = width / 2, bBytes = bMn ? (bHalf + 63) / 64 * 64 * BK * 2 : bHalf * BK * 2;
   CUtensorMap ma, mb, mc, mp;
@@ -350,10 +351,13 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   g.C = (__nv_bfloat16*)C;
   g.wide = ((uintptr_t)g.e.aux & 31) == 0;
   g.wideC = (((uintptr_t)C | (uintptr_t)g.e.pre) & 31) == 0;
-  // Boxes and TMA stores drain a tile faster, straight stores leave the loads' engine and 32 KB of stages to the operands.  us,
-  // boxes / straight: plain 2560 x 3840 x 128 9.7 / 10.5, 5376 x 4096 x 256 16.8 / 19.5, 1920 x 1280 x 768 7.2 / 7.3, 8192 x 4096 x
-  // 1024 49.2 / 48.6, 2176 x 2304 x 2048 18.2 / 17.5, 8192^3 715 / 701; with bias and residual 8192 x 4096 x 1024 59.5 / 64.5, with
-  // GELU 60.6 / 63.8, 8192 x 1024 x 1024 17.6 / 20.0; with GELU's gradient, bound by its arithmetic, 69.9 / 67.9.
+  // Boxes and TMA stores drain a tile faster, straight stores leave the loads' engine and 32 KB of stages to the operands.  The
+  // lines of plain products cross between contractions of 768 and 1024.  us, boxes / straight: 8192 x 4096 x 256 25.8 / 30.5, x 512 32.6 /
+  // 35.6, x 768 44.2 / 45.3, x 896 48.7 / 49.0, x 1024 57.7 / 55.5, x 1536 84.0 / 80.7; 2560 x 3840 x 768 14.9 / 15.0, x 896 16.6 / 16.3;
+  // 2176 x 2304 x 768 10.3 / 10.5, x 896 11.1 / 10.7; 1920 x 1280 x 512 6.4 / 6.6, x 1024 8.0 / 8.1, x 1536 9.7 / 9.6; 8192^3 715 / 701.
+  // (With a bias wide ones cross later: 8192 x 4096 x 1024 57.3 / 61.3, x 1280 73.2 / 72.5, 5376 x 4096 x 1024 38.3 / 39.8; narrow
+  // ones do not: 1920 x 1280 x 1024 8.6 / 8.5.)  With bias and residual 8192 x 4096 x 1024 59.5 / 64.5, with GELU 60.6 / 63.8, 8192 x
+  // 1024 x 1024 17.6 / 20.0; with GELU's gradient, bound by its arithmetic, 69.9 / 67.9.
   const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && K >= 896);
   g.epiBytes = straight ? 0 : EPI_BYTES;
   mc = ma;                                             // (straight stores take no map: none is made, or kept, per output)

@@ -280,8 +280,10 @@ int stagesOf(bool pair, int tn, int split, int kBlocks) {
 double gpuUs(int rows, int tn, int tiles, int sms) { return 0.00156 * tn * tiles * rows / (128.0 * sms); }
 
 // The form with the least expected time: one of those above, or the persistent kernel with tiles of 256 x width.  Whether a
-// contraction is cut, and into how many slices, depends on the sizes and the epilogue alone (not on how the operands are stored,
-// nor on `pairs`), so that the same product is always summed in the same order; the width of a tile does not change a sum.
+// contraction is cut, and into how many slices, depends on the sizes and on whether there is an epilogue (not on how the operands
+// are stored, nor on `pairs`), so that the same product is always summed in the same order; the width of a tile does not change a
+// sum.  An epilogue makes whole contractions more frequent (512 x 256 x 1024: four slices without): inside the persistent kernel it
+// is applied to the fp32 sum and the result rounded once, behind a cut product to its rounded value.
 // The persistent kernel: 3.2 us, and per wave of tiles 0.8 us + per 64 of the contraction what the tensor cores take for
 // the width, at least what a CTA's loads take (128 rows of A whatever the width), more when B is stored MN-major
 // in blocks of 64 columns that the tiles cut through, and when every SM works; at least what the whole GPU takes for the
