@@ -147,6 +147,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
+      int loads = (numTiles - pair + numPairs - 1) / numPairs * ((kb64 + kStep - 1) / kStep) - g.stages;     // that wait for a stage
       bool ok = true;
       for (int t = pair; t < numTiles && ok; t += numPairs, ++it) {
         const int ab = it & 1;
@@ -166,7 +167,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             for (int k = 0; k < 64 / UMMA_K; ++k)
               umma_bf16_pair(d, da + hopA * h + stepA * k, db + hopB * h + stepB * k, idesc, (kb | h | k) != 0);
           }
-          umma_commit_pair(&emptyBar[stage]);         // both CTAs' stage is free once these MMAs have read it
+          if (loads-- > 0) umma_commit_pair(&emptyBar[stage]);      // both CTAs' stage is free once these MMAs have read it
           if (++stage == g.stages) { stage = 0; phase ^= 1; }
         }
         if (ok) umma_commit_pair(&accFull[ab]);       // both halves of the accumulator complete
@@ -271,17 +272,22 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
         }
         store(&mapC, g.C, o, col0 + c, row0);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(ab ? accEmptyLeader1 : accEmptyLeader0);   // the pair's epilogue warps release the accumulator
+      if (t + 2 * numPairs < numTiles) {               // the pair's epilogue warps release the accumulator to the tile after the next
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(ab ? accEmptyLeader1 : accEmptyLeader0);
+      }
     }
     if (lane == 0) bulk_wait_read<0>();                // the boxes have been read before the CTA's shared memory goes away
   }
 
   // ---------------------------------------------------------------- leave: nothing of the pair may still use my shared or tensor memory
+  // (Every arrival between the CTAs is one that somebody has waited for, so that none is on its way any more; and none of them, nor the
+  // barrier, waits for the epilogue's stores, which the end of the kernel does anyway.  With releasing arrivals, one for every accumulator,
+  // a CTA left 1.3 us after its last store.)
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();
+  cluster_sync_relaxed();
   tc_fence_after();
   if (warp == 1) tmem_dealloc_pair(tmemBase, g.tmemCols);
   if (threadIdx.x == 0 && *giveUp) { atomicExch(g.err, 1u); *(volatile uint32_t*)g.errHost = 1u; __threadfence_system(); }

@@ -159,7 +159,9 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             else umma_bf16(tmemBase, dai, dbi, idesc, (k > k0) | (h | i));
           }
         }
-        if (PAIR) umma_commit_pair(&emptyBar[stage], mask); else umma_commit(&emptyBar[stage]);
+        if (k + 2 * g.stages < k1) {                  // (a load waits for the stage)
+          if (PAIR) umma_commit_pair(&emptyBar[stage], mask); else umma_commit(&emptyBar[stage]);
+        }
         if (++stage == g.stages) { stage = 0; phase ^= 1; }
       }
       if (ok) { if (PAIR) umma_commit_pair(accFull, mask); else umma_commit(accFull); }
@@ -245,7 +247,7 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();
+  if (PAIR) cluster_sync_relaxed();                  // (the end of the kernel waits for the stores, the partner need not)
   tc_fence_after();
   if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmemBase, TN); else tmem_dealloc(tmemBase, TN); }
   if (threadIdx.x == 0 && *giveUp) { atomicExch(g.err, 1u); *(volatile uint32_t*)g.errHost = 1u; __threadfence_system(); }

@@ -72,6 +72,25 @@ def test_cta_pair_kernel_agrees_with_the_one_cta_kernel(m, n, k, a_t, b_t, monke
     assert torch.equal(c_pair, c_one)
 
 
+@pytest.mark.parametrize("m,n,k", [(8192, 4096, 64), (8192, 4096, 192), (2432, 4096, 256), (4864, 4096, 448), (2432, 2560, 1088), (4736, 4096, 576)])
+def test_gemm_with_several_tiles_per_pair(m, n, k):
+    """Two to seven tiles per pair, fewer and more steps of the contraction than there are stages: accumulators and stages are
+    released only where somebody takes them again."""
+    from dfccl_b200.ops import gemm
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(n, k, device="cuda", dtype=torch.bfloat16)
+    c = gemm.matmul_nt(a, b)
+    again = [gemm.matmul_nt(a, b) for _ in range(4)]
+    torch.cuda.synchronize()
+    assert gemm.check_kernels()
+    assert all(torch.equal(c, d) for d in again)
+    ref = a.double() @ b.double().t()
+    # one rounding to bf16 (8 significant bits: 2^-8 of the value at most) of an fp32 sum: k roundings of 2^-24 of partial sums below |a| |b|^T
+    bound = ref.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * (k * 2.0 ** -24) + 1e-30
+    assert bool(((c.double() - ref).abs() <= bound * 1.01).all())
+
+
 def test_gemm_rejects_shapes_it_cannot_tile():
     from dfccl_b200.ops import gemm
     a = torch.randn(100, 64, device="cuda", dtype=torch.bfloat16)
