@@ -36,7 +36,7 @@ using namespace tc;
 constexpr int PM = 256, HALF = 128, MAX_STAGES = 6, UMMA_K = 16;
 constexpr int SMEM_LIMIT = 227 * 1024, BAR_BYTES = 256, ALIGN_SLACK = 1024;
 constexpr int BOX_BYTES = 32 * 64;                   // a staged box of the epilogue: 32 rows x 32 columns
-constexpr int EPI_BOXES = 16, EPI_BYTES = EPI_BOXES * BOX_BYTES;
+constexpr int EPI_BOXES = 16, EPI_BYTES = EPI_BOXES * BOX_BYTES;      // boxes of their own, where a pair has several tiles
 constexpr int WIDE_STAGE = (HALF + 128) * 64 * 2;    // a stage of the widest tile, per CTA
 constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on another GPU: seconds mean a lost partner
 
@@ -57,7 +57,9 @@ struct PairArgs {
   uint32_t* errHost;
   __nv_bfloat16* C;
   GemmEpilogue e;
-  int epiBytes;                     // boxes of the epilogue, or 0: straight from the registers
+  bool boxes;                       // results go through boxes (the kinds without a choice: GELU_GRAD never, others always)
+  int once;                         // a pair has one tile: the boxes of one of its warps, in the operands' stages; 0: several, boxes of their own
+  int epiBytes;                     // of those
   bool wide, wideC;                 // aux, and C and pre, start on a 32-byte boundary
 };
 
@@ -96,7 +98,7 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
     tma_prefetch_desc(&mapB);
-    if (g.epiBytes) tma_prefetch_desc(&mapC);
+    if (g.boxes) tma_prefetch_desc(&mapC);
   }
   if (warp == 1) tmem_alloc_pair(tmemBaseSlot, g.tmemCols);
   tc_fence_before();
@@ -179,25 +181,28 @@ dfcclGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     const uint32_t accEmptyLeader0 = mapa_u32(smem_u32(&accEmpty[0]), 0), accEmptyLeader1 = mapa_u32(smem_u32(&accEmpty[1]), 0);
     // A box is stored with the 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r / 2 % 4), so that eight lanes
     // (rows) that write the same chunk meet eight different groups of four banks.
-    uint8_t* box0 = stg + (warp - 2) * BUFS * BOX_BYTES;
+    // A pair's only tile finds the operands' stages free, with a box for every store: none waits for another one's.
+    uint8_t* const box0 = g.once ? smem + (warp - 2) * g.once * BOX_BYTES : stg + (warp - 2) * BUFS * BOX_BYTES;
     const uint32_t rowOff = lane * 64, swz = (lane >> 1) & 3;
     int turn = 0;
     auto store = [&](const CUtensorMap* map, __nv_bfloat16* base, const uint4 (&o)[4], int x, int y) {
-      if (EPI == EPI_GELU_GRAD || ((EPI == EPI_NONE || EPI == EPI_BIAS) && g.epiBytes == 0)) {      // 64 bytes of its row per lane, in whole sectors
+      if (EPI == EPI_GELU_GRAD || ((EPI == EPI_NONE || EPI == EPI_BIAS) && !g.boxes)) {      // 64 bytes of its row per lane, in whole sectors
         __nv_bfloat16* p = base + (size_t)(y + lane) * g.ldc + x;
         st_global32(p, o, g.wideC);
         st_global32(p + 16, o + 2, g.wideC);
         return;
       }
       uint8_t* box = box0 + turn * BOX_BYTES;
-      if (lane == 0) bulk_wait_read<BUFS - 1>();       // the store that read this buffer last has done so
-      __syncwarp();
+      if (!g.once) {
+        if (lane == 0) bulk_wait_read<BUFS - 1>();     // the store that read this buffer last has done so
+        __syncwarp();
+      }
 #pragma unroll
       for (int v = 0; v < 4; ++v) *(uint4*)(box + rowOff + ((v ^ swz) << 4)) = o[v];
       fence_async_shared();
       __syncwarp();
       if (lane == 0) { tma_store_2d(map, box, x, y); bulk_commit(); }
-      if (++turn == BUFS) turn = 0;
+      if (++turn == BUFS && !g.once) turn = 0;
     };
     int it = 0;
     for (int t = pair; t < numTiles; t += numPairs, ++it) {
@@ -357,30 +362,32 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   g.C = (__nv_bfloat16*)C;
   g.wide = ((uintptr_t)g.e.aux & 31) == 0;
   g.wideC = (((uintptr_t)C | (uintptr_t)g.e.pre) & 31) == 0;
-  // Boxes and TMA stores drain a tile faster, straight stores leave the loads' engine and 32 KB of stages to the operands.  The
-  // lines of plain products cross between contractions of 768 and 1024.  us, boxes / straight: 8192 x 4096 x 256 25.8 / 30.5, x 512 32.6 /
-  // 35.6, x 768 44.2 / 45.3, x 896 48.7 / 49.0, x 1024 57.7 / 55.5, x 1536 84.0 / 80.7; 2560 x 3840 x 768 14.9 / 15.0, x 896 16.6 / 16.3;
-  // 2176 x 2304 x 768 10.3 / 10.5, x 896 11.1 / 10.7; 1920 x 1280 x 512 6.4 / 6.6, x 1024 8.0 / 8.1, x 1536 9.7 / 9.6; 8192^3 715 / 701.
-  // (With a bias wide ones cross later: 8192 x 4096 x 1024 57.3 / 61.3, x 1280 73.2 / 72.5, 5376 x 4096 x 1024 38.3 / 39.8; narrow
-  // ones do not: 1920 x 1280 x 1024 8.6 / 8.5.)  With bias and residual 8192 x 4096 x 1024 59.5 / 64.5, with GELU 60.6 / 63.8, 8192 x
-  // 1024 x 1024 17.6 / 20.0; with GELU's gradient, bound by its arithmetic, 69.9 / 67.9.
-  const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && K >= 896);
-  g.epiBytes = straight ? 0 : EPI_BYTES;
-  mc = ma;                                             // (straight stores take no map: none is made, or kept, per output)
-  if (!straight) DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
-  mp = mc;
-  if (g.e.kind == EPI_BIAS_GELU && g.e.pre) DFCHECK(gemmMakeMap(&mp, g.e.pre, (uint64_t)M, (uint64_t)N, 32, 32));
-  { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int tiles = (M + PM - 1) / PM * ((N + width - 1) / width);
   const int pairs = std::min(tiles, maxResidentPairs(dev, sms));
+  // Boxes and TMA stores drain a tile faster, straight stores leave the loads' engine and 32 KB of stages to the operands of the tiles
+  // that follow: a pair's only tile, whose boxes lie in the stages it no longer needs, goes through them, others with short
+  // contractions.  us, boxes / straight: 1920 x 1792 x 3072 18.0 / 18.6, 3200 x 768 x 1088 11.4 / 11.7; several tiles, widths from 224 on: up to
+  // K = 256 14 % less with boxes, 512 4 %, 768 the same, 1024 1 % more, 1536 2 %; narrower ones 8 %, 0, 2 % more, 3 %, 4 % (230 and 800
+  // products of all storage orders).
+  const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && tiles > pairs && K >= 768);
+  const int parts = epiWarps(g.e.kind) / 4, stored = g.e.kind == EPI_BIAS_GELU && g.e.pre ? 2 : 1;
+  g.boxes = !straight;
+  g.once = tiles > pairs ? 0 : (width / 32 + parts - 1) / parts * stored;
+  g.epiBytes = g.boxes && !g.once ? EPI_BYTES : 0;
+  mc = ma;                                             // (straight stores take no map: none is made, or kept, per output)
+  if (!straight) DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
+  mp = mc;
+  if (g.e.kind == EPI_BIAS_GELU && g.e.pre) DFCHECK(gemmMakeMap(&mp, g.e.pre, (uint64_t)M, (uint64_t)N, 32, 32));
+  { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   g.kStep = kStep;
   g.stageBytes = HALF * BK * 2 + bBytes;               // width 256: WIDE_STAGE, however B is stored
   const int room = SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK - g.epiBytes;
   const int want = tiles > pairs ? MAX_STAGES : (K + BK - 1) / BK;
   g.stages = std::min(std::min(MAX_STAGES, room / g.stageBytes), want);
+  if (g.boxes) while (g.stages * g.stageBytes < epiWarps(g.e.kind) * g.once * BOX_BYTES) ++g.stages;       // (four of 32 KB at most)
   g.tmemCols = tiles > pairs ? 512 : width <= 64 ? 64 : width <= 128 ? 128 : 256;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));

@@ -34,6 +34,7 @@ constexpr int MN_BLOCK_BYTES = 64 * BK * 2;          // MN-major operand: 64 MN-
 constexpr int NUM_THREADS = 320;                     // 10 warps
 constexpr int EPI_ROW_BYTES = 64 * 2 + 16;           // a staged row of the epilogue: rows start in different banks
 constexpr int EPI_BYTES = 8 * 32 * EPI_ROW_BYTES;    // one buffer of 32 rows per epilogue warp, in the operands' stages once those are done
+constexpr int BOX_BYTES = 32 * 64;                   // whole contractions: boxes of 32 rows x 32 columns, in the same place
 constexpr int SMEM_LIMIT = 227 * 1024, BAR_BYTES = 256, ALIGN_SLACK = 1024;
 constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on another GPU: seconds mean a lost partner
 
@@ -49,6 +50,10 @@ struct TileArgs {
 
 __host__ __device__ constexpr int bRows(bool pair, int tn) { return pair ? tn / 2 : tn; }                    // rows of B a CTA loads per K block
 __host__ __device__ constexpr int stageBytes(bool pair, int tn) { return A_BYTES + bRows(pair, tn) * BK * 2; }
+// Whole contractions leave through boxes and TMA stores where a warp has two blocks of 32 columns or more.  us, row segments / boxes:
+// 4096 x 1024 x 1024 (tiles of 256 x 256) 10.4 / 9.9, 1920 x 1792 x 3072 19.8 / 19.4, 512 x 4096 x 768 (256 x 128) 6.15 / 6.04, 2944 x 512 x
+// 256 (128 x 128) 5.84 / 5.73; but 768 x 1024 x 512 (128 x 64) 4.81 / 4.92.
+__host__ __device__ constexpr bool boxed(int tn) { return tn >= 128; }
 __host__ __device__ constexpr int exchangeBytes(int tn, int split) { return split > 1 ? (split - 1) * TM * (tn / split) * 4 : 0; }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -65,8 +70,10 @@ __device__ __forceinline__ void st_cluster16(uint32_t addr, uint32_t a, uint32_t
 
 template <bool PAIR, int TN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const TileArgs g) {
+dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapC,
+                    const TileArgs g) {
   constexpr int STAGE_BYTES = stageBytes(PAIR, TN), BROWS = bRows(PAIR, TN);
+  constexpr bool BOXED = boxed(TN);
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);       // the same offset in every CTA of the cluster
   uint8_t* exch = smem + max(g.stages * STAGE_BYTES, EPI_BYTES);                                // [split - 1][columns / 4][128 rows] of 16 bytes
@@ -95,6 +102,7 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     mbar_fence_init();
     tma_prefetch_desc(&mapA);
     tma_prefetch_desc(&mapB);
+    if (BOXED && g.split == 1) tma_prefetch_desc(&mapC);
   }
   if (warp == 1) { if (PAIR) tmem_alloc_pair(tmemBaseSlot, TN); else tmem_alloc(tmemBaseSlot, TN); }
   tc_fence_before();
@@ -178,6 +186,36 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     accOk = __all_sync(0xffffffffu, mbar_wait(accFull, 0, giveUp, WAIT_NS));
     tc_fence_after();
   }
+  if (BOXED && g.split == 1) {
+    // 32 rows x 32 columns at a time: tensor memory -> a box in the operands' stages, which are done with -> a TMA store.  In a box,
+    // 16-byte chunk c of row r sits at chunk c ^ (r / 2 % 4) (the 64-byte swizzle): eight lanes that write the same chunk meet
+    // eight different groups of four banks.
+    if (warp >= 2 && accOk && rowBase < g.M) {
+      constexpr int BOXES = TN / 64;
+      const uint32_t swz = (lane >> 1) & 3;
+#pragma unroll 1
+      for (int i = 0; i < BOXES; ++i) {
+        const int c = colHalf * (TN / 2) + i * 32;
+        uint8_t* box = smem + ((warp - 2) * BOXES + i) * BOX_BYTES;
+        uint32_t r[32];
+        tmem_ld32(tRow + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          uint4 o;
+          o.x = pack_bf16x2(__uint_as_float(r[8 * v]), __uint_as_float(r[8 * v + 1]));
+          o.y = pack_bf16x2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
+          o.z = pack_bf16x2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
+          o.w = pack_bf16x2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
+          *(uint4*)(box + lane * 64 + ((v ^ swz) << 4)) = o;
+        }
+        fence_async_shared();
+        __syncwarp();
+        if (lane == 0) { tma_store_2d(&mapC, box, nt * TN + c, rowBase + quarter * 32); bulk_commit(); }
+      }
+      if (lane == 0) bulk_wait_read<0>();              // the boxes have been read before the CTA's shared memory goes away
+    }
+  }
   if (g.split > 1) {
     if (warp >= 2 && accOk) {
       for (int c = colHalf * 32; c < TN; c += 64) {
@@ -201,7 +239,7 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     __syncwarp();
     cluster_sync_all();                                              // every partial sum is in its owner's shared memory
   }
-  if (warp >= 2 && accOk && rowBase + row < g.M) {                   // (whole CTAs only: M and the tiles are multiples of 128)
+  if (!(BOXED && g.split == 1) && warp >= 2 && accOk && rowBase < g.M) {          // (whole CTAs only: M and the tiles are multiples of 128)
     // up to 64 columns at a time: tensor memory (+ the partners' sums) -> staging rows -> whole row segments to global memory
     uint8_t* stg = smem + (warp - 2) * 32 * EPI_ROW_BYTES;
     const int cols = max(W / 2, 16), beg = colHalf * cols, step = min(cols, 64), lanesPerRow = step / 8, shift = 31 - __clz(lanesPerRow);
@@ -253,7 +291,7 @@ dfcclGemmTileKernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   if (threadIdx.x == 0 && *giveUp) { atomicExch(g.err, 1u); *(volatile uint32_t*)g.errHost = 1u; __threadfence_system(); }
 }
 
-typedef void (*TileKernel)(const CUtensorMap, const CUtensorMap, const TileArgs);
+typedef void (*TileKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const TileArgs);
 TileKernel kernelOf(bool pair, int tn) {
   if (pair) return tn == 128 ? dfcclGemmTileKernel<true, 128> : dfcclGemmTileKernel<true, 256>;
   return tn == 64 ? dfcclGemmTileKernel<false, 64> : dfcclGemmTileKernel<false, 128>;
@@ -361,9 +399,11 @@ GemmTilePlan gemmTilePlan(int M, int N, int K, int sms, bool pairs, bool bMn, bo
 
 ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B, void* C, int M, int N, int K, cudaStream_t stream,
                             int aMn, int bMn, uint32_t* errDev, uint32_t* errHost) {
-  CUtensorMap ma, mb;
+  CUtensorMap ma, mb, mc;
   DFCHECK(gemmMakeMap3(&ma, A, (uint64_t)M, (uint64_t)K, aMn, TM, BK));
   DFCHECK(gemmMakeMap3(&mb, B, (uint64_t)N, (uint64_t)K, bMn, bRows(p.pair, p.tn), BK));
+  mc = ma;
+  if (boxed(p.tn) && p.split == 1) DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
   CUDACHECK(oncePerDevice([] {
     cudaError_t r = cudaSuccess;
     for (const Form& f : FORMS) if (r == cudaSuccess) r = allowSharedMemory(kernelOf(f.pair, f.tn), SMEM_LIMIT);
@@ -387,7 +427,7 @@ ncclResult_t gemmTileLaunch(const GemmTilePlan& p, const void* A, const void* B,
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
   at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = clusterSize; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = clusterSize > 1 ? 2 : 1;
-  CUDACHECK(cudaLaunchKernelEx(&cfg, kernelOf(p.pair, p.tn), ma, mb, g));
+  CUDACHECK(cudaLaunchKernelEx(&cfg, kernelOf(p.pair, p.tn), ma, mb, mc, g));
   return ncclSuccess;
 }
 
