@@ -40,10 +40,11 @@ __device__ __forceinline__ void oneElem(const OneRankArgs& a, uint64_t e) {
   *((Tout*)a.dst + e) = Elem<Tout>::down(finish<Tin, Tout>(acc, a.scale, a.postDiv));
 }
 
-__device__ __forceinline__ void publishDone(const OneRankDone& done) {
+// The place of the host's entry in its ring.
+__device__ __forceinline__ unsigned long long takePlace(const OneRankDone& done) { return atomic_add_u64((unsigned long long*)&done.rd->devCqTail, 1ull); }
+__device__ __forceinline__ void publishDone(const OneRankDone& done, unsigned long long idx) {
   RankDev* rd = done.rd;
-  const unsigned long long idx = atomic_add_u64((unsigned long long*)&rd->devCqTail, 1ull);
-  fence_sys();
+  fence_acq_rel_sys();
   st_relaxed_sys_u64(&rd->doneEpoch[done.coll], ((uint64_t)ST_OK << 56) | done.epoch);
   st_relaxed_sys_u64(&rd->hostCq[idx & (rd->cqCap - 1)], cqeEncode((uint32_t)(idx / rd->cqCap) + 1u, ST_OK, (uint32_t)done.coll));
 }
@@ -66,6 +67,9 @@ __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs 
   char* d = a.dst + a.head * sizeof(Tout);
   tc::grid_dependency_wait();
   tc::grid_launch_dependents();
+  // (a place taken now keeps the places behind it waiting until this call is done: a matter of microseconds where it is SHORT)
+  unsigned long long place = 0;
+  if (SHORT && blockIdx.x == 0 && threadIdx.x == 0) place = takePlace(a.done);
   uint4 v[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) if (p0 + u * STEP < a.nPacks) v[u] = s[p0 + u * STEP];
@@ -101,7 +105,7 @@ __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs 
   }
   if (SHORT) {
     tc::cluster_sync_all();
-    if (blockIdx.x == 0 && threadIdx.x == 0) publishDone(a.done);
+    if (blockIdx.x == 0 && threadIdx.x == 0) publishDone(a.done, place);
     return;
   }
   if (a.done.rd == nullptr) return;
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs 
       if (atomic_add_u32(count, 1u) + 1u != gridDim.x) return;
       *(volatile uint32_t*)count = 0u;
     }
-    publishDone(a.done);
+    publishDone(a.done, takePlace(a.done));
   }
 }
 
@@ -132,7 +136,7 @@ __global__ void dfcclOneRankTraceKernel(const OneRankDone done, bool end) {
   }
   trace(done.rd, 0, TR_DATA_END, done.coll);
   trace(done.rd, 0, TR_DONE, done.coll);
-  publishDone(done);
+  publishDone(done, takePlace(done));
 }
 
 template <typename Tin, typename Tout, bool COPY>
