@@ -508,7 +508,9 @@ ncclResult_t launch(const void* A, const void* B, void* C, int M, int N, int K, 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!f || f->mode == 0 || f->nranks <= 1) {
-    const GemmTilePlan p = gemmTilePlan(M, N, K, sms, paramI64("GEMM_PAIR", 1) != 0, bMn != 0, e && e->kind);
+    // (the setting is looked up, 0.4 us of a launch, only for products it could change)
+    GemmTilePlan p = gemmTilePlan(M, N, K, sms, true, bMn != 0, e && e->kind);
+    if ((p.pair || p.width) && paramI64("GEMM_PAIR", 1) == 0) p = gemmTilePlan(M, N, K, sms, false, bMn != 0, e && e->kind);
     if (p.width) return gemmPairLaunch(p.width, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host, e);
     DFCHECK(gemmTileLaunch(p, A, B, C, M, N, K, stream, aMn, bMn, ew.dev, (uint32_t*)ew.host));
     return e && e->kind ? applyEpilogue(*e, C, M, N, stream) : ncclSuccess;

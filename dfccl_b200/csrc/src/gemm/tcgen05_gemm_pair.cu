@@ -381,7 +381,8 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   if (!straight) DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
   mp = mc;
   if (g.e.kind == EPI_BIAS_GELU && g.e.pre) DFCHECK(gemmMakeMap(&mp, g.e.pre, (uint64_t)M, (uint64_t)N, 32, 32));
-  { int64_t gm = paramI64("GEMM_RASTER_GROUP", 8); g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
+  // (where every pair has one tile the order decides nothing)
+  { int64_t gm = tiles > pairs ? paramI64("GEMM_RASTER_GROUP", 8) : 8; g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   g.kStep = kStep;
   g.stageBytes = HALF * BK * 2 + bBytes;               // width 256: WIDE_STAGE, however B is stored
   const int room = SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK - g.epiBytes;

@@ -2,6 +2,7 @@
 column sums (bias gradients), and what a GEMM does with its product before storing it (``csrc/src/gemm/epilogue.h``)."""
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 from typing import Optional
 
@@ -10,7 +11,7 @@ import torch.nn as nn
 from torch.autograd.function import once_differentiable
 
 from .. import native as nv
-from ..utils.tensors import on_device, raw_stream
+from ..utils.tensors import on_device, raw_stream, stream_of
 
 NONE, BIAS, BIAS_RES, BIAS_GELU, GELU_GRAD = range(5)
 
@@ -27,7 +28,7 @@ class Epilogue:
     def args(self):
         for t in (self.bias, self.aux, self.pre):
             assert t is None or (t.dtype == torch.bfloat16 and t.is_cuda and t.is_contiguous())
-        return (self.kind, _ptr(self.bias), _ptr(self.aux), _ptr(self.pre))
+        return self.kind, _ptr(self.bias), _ptr(self.aux), _ptr(self.pre)
 
     def args_for(self, m: int, n: int):
         """The same for a product of [m, n]; the kernels read and write by address alone."""
@@ -68,14 +69,25 @@ def apply_epilogue_(product: torch.Tensor, epi: Epilogue) -> torch.Tensor:
     return product
 
 
+@functools.lru_cache(maxsize=1024)
+def _work_words(entry: str, device: int, rows: int, n: int) -> int:
+    """fp32 words of scratch memory: a function of the sizes and of the device, which is the current one."""
+    return getattr(nv.lib(), entry)(rows, n)
+
+
+@functools.lru_cache(maxsize=1)
+def _max_width() -> int:
+    return nv.lib().dfcclLayerNormMaxWidth()
+
+
 def column_sum(g: torch.Tensor) -> torch.Tensor:
     """Sum over the rows of a contiguous bf16 matrix, in fp32, rounded once."""
     rows, n = g.shape
     out = torch.empty(n, dtype=torch.bfloat16, device=g.device)
     with on_device(g.device):
-        words = nv.lib().dfcclColumnSumWork(rows, n)
+        words = _work_words("dfcclColumnSumWork", g.get_device(), rows, n)
         work = torch.empty(words, dtype=torch.float32, device=g.device) if words else None
-        nv.check(nv.lib().dfcclColumnSum(g.data_ptr(), out.data_ptr(), _ptr(work), rows, n, raw_stream(g.device)), "dfcclColumnSum")
+        nv.check(nv.entry("dfcclColumnSum")(g.data_ptr(), out.data_ptr(), _ptr(work), rows, n, stream_of(g)), "dfcclColumnSum")
     return out
 
 
@@ -89,8 +101,9 @@ class _NormFn(torch.autograd.Function):
         y = torch.empty_like(x)
         stats = torch.empty(2, rows, dtype=torch.float32, device=x.device)
         with on_device(x.device):
-            nv.check(nv.lib().dfcclLayerNormForward(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), stats.data_ptr(), stats[1].data_ptr(),
-                                                    rows, d, eps, raw_stream(x.device)), "dfcclLayerNormForward")
+            mean = stats.data_ptr()
+            nv.check(nv.lib().dfcclLayerNormForward(x.data_ptr(), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mean, mean + 4 * rows,
+                                                    rows, d, eps, stream_of(x)), "dfcclLayerNormForward")
         ctx.save_for_backward(x, gamma, stats)
         ctx.set_materialize_grads(False)
         return x, y
@@ -105,9 +118,10 @@ class _NormFn(torch.autograd.Function):
         gy, gpass = packed(gy), packed(gpass)
         gx, gg, gb = torch.empty_like(x), torch.empty_like(gamma), torch.empty_like(gamma)
         with on_device(x.device):
-            work = torch.empty(nv.lib().dfcclLayerNormWork(rows, d), dtype=torch.float32, device=x.device)
-            nv.check(nv.lib().dfcclLayerNormBackward(gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), stats.data_ptr(), stats[1].data_ptr(), _ptr(gpass),
-                                                     gx.data_ptr(), gg.data_ptr(), gb.data_ptr(), work.data_ptr(), rows, d, raw_stream(x.device)),
+            work = torch.empty(_work_words("dfcclLayerNormWork", x.get_device(), rows, d), dtype=torch.float32, device=x.device)
+            mean = stats.data_ptr()
+            nv.check(nv.entry("dfcclLayerNormBackward")(gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), mean, mean + 4 * stats.stride(0), _ptr(gpass),
+                                                        gx.data_ptr(), gg.data_ptr(), gb.data_ptr(), work.data_ptr(), rows, d, stream_of(x)),
                      "dfcclLayerNormBackward")
         return gx, gg, gb, None
 
@@ -122,7 +136,7 @@ def norm_residual(ln: nn.LayerNorm, x: torch.Tensor):
     """``(x, ln(x))``.  The hand-written kernels for contiguous bf16 rows on a GPU (widths a multiple of 8 up to the
     kernels' limit); anything else goes through the module."""
     ok = (unhooked(ln, nn.LayerNorm) and x.is_cuda and x.dim() == 2 and x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[0] > 0
-          and tuple(ln.normalized_shape) == (x.shape[1],) and x.shape[1] % 8 == 0 and x.shape[1] <= nv.lib().dfcclLayerNormMaxWidth()
+          and tuple(ln.normalized_shape) == (x.shape[1],) and x.shape[1] % 8 == 0 and x.shape[1] <= _max_width()
           and all(p is not None and p.dtype == torch.bfloat16 and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0
                   for p in (ln.weight, ln.bias))
           and x.data_ptr() % 16 == 0 and not torch.is_autocast_enabled("cuda"))

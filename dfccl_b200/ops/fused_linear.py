@@ -24,7 +24,7 @@ import torch
 import torch.distributed as dist
 
 from .. import native as nv
-from ..utils.tensors import raw_stream, tensor_from_ptr
+from ..utils.tensors import raw_stream, stream_of, tensor_from_ptr
 from .block import Epilogue, NO_EPILOGUE, packed
 from .gemm import BM, BN, BK
 
@@ -96,22 +96,26 @@ class _Local:
     def operand(self, x: torch.Tensor) -> torch.Tensor:
         """``x`` as the GEMM reads it, [M, K] bf16 on the 16-byte grid: cast, and spread over the rows, as copying it into an
         operand does."""
+        if x.dtype == torch.bfloat16 and x.shape == (self.m, self.k) and x.device == self.tp.device and x.is_contiguous() and x.data_ptr() % 16 == 0:
+            return x
         if x.shape != (self.m, self.k):
             x = x.reshape(self.m, self.k) if x.numel() == self.m * self.k and x.shape[-1] == self.k else x.expand(self.m, self.k)
         return packed(x.to(self.tp.device, torch.bfloat16))
 
     def local(self, x: torch.Tensor, w: torch.Tensor, w_transposed: bool = False, epi: Epilogue = NO_EPILOGUE) -> torch.Tensor:
         assert self.tp.n == 1
-        x, w = self.operand(x), w.to(self.tp.device, torch.bfloat16).contiguous()
+        x = self.operand(x)
+        if not (w.dtype == torch.bfloat16 and w.device == self.tp.device and w.is_contiguous()):
+            w = w.to(self.tp.device, torch.bfloat16).contiguous()
         if w.shape != ((self.k, self.n_out) if w_transposed else (self.n_out, self.k)):
             raise ValueError(f"weight of {tuple(w.shape)} for an operator of {self.n_out} outputs and {self.k} inputs")
         out = torch.empty(self.m, self.n_out, dtype=torch.bfloat16, device=self.tp.device)
         epilogue = epi.args_for(self.m, self.n_out)
-        ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), raw_stream(self.tp.device)
+        ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), stream_of(out)
         if self.coll_id is not None:
-            nv.check(nv.lib().dfcclRunFusedGemmLocal(self.coll_id, *ptrs, int(w_transposed), *epilogue, st, self.tp.ctx.handle), "dfcclRunFusedGemmLocal")
+            nv.check(nv.entry("dfcclRunFusedGemmLocal")(self.coll_id, *ptrs, int(w_transposed), *epilogue, st, self.tp.ctx.handle.value), "dfcclRunFusedGemmLocal")
         else:
-            nv.check(nv.lib().dfcclGemmBf16Epilogue(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epilogue, st), "dfcclGemmBf16Epilogue")
+            nv.check(nv.entry("dfcclGemmBf16Epilogue")(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epilogue, st), "dfcclGemmBf16Epilogue")
         return out
 
 

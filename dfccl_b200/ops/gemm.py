@@ -6,7 +6,7 @@ import ctypes as C
 import torch
 
 from .. import native as nv
-from ..utils.tensors import raw_stream
+from ..utils.tensors import stream_of
 
 BM, BN, BK = 128, 256, 64
 
@@ -20,15 +20,15 @@ def matmul_nt(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None)
     the library's own tensor-core kernel: TMA-fed shared-memory stages, ``tcgen05.mma`` into tensor
     memory, fp32 accumulation, bf16 result."""
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.is_cuda and b.is_cuda
-    assert a.dim() == 2 and b.dim() == 2 and a.shape[1] == b.shape[1]
+    assert a.dim() == 2 and b.dim() == 2
+    (m, k), (n, kb) = a.shape, b.shape
+    assert k == kb
     a, b = a.contiguous(), b.contiguous()
-    m, k = a.shape
-    n = b.shape[0]
     if not gemm_supported(m, n, k):
         raise ValueError(f"tcgen05 GEMM needs M % {BM} == 0, N % {BN} == 0, K % {BK} == 0, got {m} x {n} x {k}")
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
-    r = nv.entry("dfcclGemmBf16")(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, raw_stream(a.device))
+    r = nv.entry("dfcclGemmBf16")(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, stream_of(a))
     if r:
         nv.check(r, "dfcclGemmBf16")
     return out
@@ -50,7 +50,7 @@ def matmul(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, *,
     if out is None:
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     r = nv.entry("dfcclGemmBf16Ex")(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, int(a_transposed), int(b_transposed),
-                                    raw_stream(a.device))
+                                    stream_of(a))
     if r:
         nv.check(r, "dfcclGemmBf16Ex")
     return out

@@ -30,6 +30,11 @@ def raw_stream(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
+def stream_of(t: torch.Tensor) -> int:
+    """The same for the device that holds ``t``, a GPU."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
 _HERE = contextlib.nullcontext()
 
 
