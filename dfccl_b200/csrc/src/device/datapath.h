@@ -196,6 +196,14 @@ DF_HD uint4 shiftPack(const uint4& lo, const uint4& hi, uint32_t shift) {
 #endif
 }
 
+#if DF_DEVICE_CODE
+// the neighbour lane's pack (the last lane gets its own back); the whole warp calls it
+__device__ __forceinline__ uint4 nextLane(const uint4& v) {
+  return make_uint4(__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1), __shfl_down_sync(0xffffffffu, v.z, 1),
+                    __shfl_down_sync(0xffffffffu, v.w, 1));
+}
+#endif
+
 // U logical packs of one source for this thread; pack u starts `u * strideB` bytes after `s`, `shift` = s & 15.
 // SHIFT = false: s is aligned.  FULL: every thread of the block loads all of its U packs (warp shuffles are safe).
 template <bool FULL, bool SHIFT, int U>
@@ -206,20 +214,26 @@ DF_HD void loadPacks(uint4* out, const char* s, uint32_t strideB, uint32_t shift
     return;
   }
   const char* a = s - shift;                       // aligned; every aligned pack touched holds at least one wanted byte
+#if DF_DEVICE_CODE
+  if (FULL) {                                      // every load before the first shuffle, which waits for its pack
+    uint4 last[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      out[u] = ld16(a + (uint64_t)u * strideB);
+      if ((threadIdx.x & 31) == 31) last[u] = ld16(a + (uint64_t)u * strideB + 16);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint4 hi = nextLane(out[u]);
+      out[u] = shiftPack(out[u], (threadIdx.x & 31) == 31 ? last[u] : hi, shift);
+    }
+    return;
+  }
+#endif
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (!(FULL || p0 + (uint64_t)u * stride < nPacks)) continue;
-    const uint4 lo = ld16(a + (uint64_t)u * strideB);
-    uint4 hi;
-#if DF_DEVICE_CODE
-    if (FULL) {
-      hi.x = __shfl_down_sync(0xffffffffu, lo.x, 1); hi.y = __shfl_down_sync(0xffffffffu, lo.y, 1);
-      hi.z = __shfl_down_sync(0xffffffffu, lo.z, 1); hi.w = __shfl_down_sync(0xffffffffu, lo.w, 1);
-      if ((threadIdx.x & 31) == 31) hi = ld16(a + (uint64_t)u * strideB + 16);
-    } else
-#endif
-      hi = ld16(a + (uint64_t)u * strideB + 16);
-    out[u] = shiftPack(lo, hi, shift);
+    out[u] = shiftPack(ld16(a + (uint64_t)u * strideB), ld16(a + (uint64_t)u * strideB + 16), shift);
   }
 }
 
@@ -331,7 +345,7 @@ DF_HD void reduceTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t 
 template <typename Tin, typename Tout, int OP, bool SHIFT>
 DF_HD void reduceTrips(const DataArgs* a, uint64_t nPacks, int nsrc, int ndst, typename Elem<Tin>::Acc mul, bool doMul, int postDiv,
                        double scale, uint64_t srcOff, uint64_t dstOff, uint32_t shift) {
-  constexpr int U = OP == OP_SUM ? 4 : 2;     // the sum carries the traffic; the rarer operators trade speed for code size
+  constexpr int U = OP == OP_SUM && !SHIFT ? 4 : 2;     // the sum carries the traffic; the rarer operators trade speed for code size, shifting takes registers
   const int tid = df_tid(), nt = df_nthreads();
   // Software-pipelined over the sources inside a trip: the U loads of source j+1 are issued before
   // the U packs of source j are consumed, so up to 2*U 16-byte loads are in flight per thread.
@@ -354,52 +368,65 @@ DF_HD void reduceTrips(const DataArgs* a, uint64_t nPacks, int nsrc, int ndst, t
 // 4 ranks 41.9 / 38.3, 13.1 M fp32 106.5 / 97.2; 16.8 M fp32 8 ranks 231 / 210; below 1 M the same.  Results twice as wide as their
 // operands are mostly stores: among four ranks one pack a source does better than two (13.1 M 80.7 / 76.2, two 79.4), among eight the
 // trips stay (170 / 169 - 174).  Copies gain nothing from loads ahead, shorter ones lose 1 - 2 %.
-template <typename Tin, typename Tout, int N>
+// SHIFT: the sources are `shift` bytes off the 16-byte grid.  The 32 aligned packs that a warp loads make 31 logical ones, each from a
+// lane's and its neighbour's (31 of 32 of the traffic is wanted, and no lane has a second load to keep registers for).
+// In the trips a shuffle per pack stood between its load and the next one's.  us, reduce-scatter of fp32 and all-gather of bf16 among
+// four ranks, pieces off the grid, before / now: 20 003 values 65 / 56, 250 003 66.8 / 54.3, 1 000 003 121 / 76, 2 000 003 194 / 101 (2 000 000,
+// on the grid, 93); two ranks 2 000 003 118 / 66.5.
+template <typename Tin, typename Tout, int N, bool SHIFT>
 DF_HD void reduceAhead(const DataArgs* a, uint64_t nPacks, int ndst, typename Elem<Tin>::Acc mul, bool doMul, int postDiv, double scale,
-                       uint64_t srcOff, uint64_t dstOff) {
+                       uint64_t srcOff, uint64_t dstOff, uint32_t shift) {
   typedef typename Elem<Tin>::Acc A;
   constexpr int V = 16 / (int)sizeof(Tin), OUTB = V * (int)sizeof(Tout), NW = (OUTB + 15) / 16;
   constexpr int U = N == 4 && NW == 2 ? 1 : 8 / N;
-  const uint32_t nt = (uint32_t)df_nthreads();
+  const uint32_t tid = (uint32_t)df_tid(), nt = (uint32_t)df_nthreads(), lane = SHIFT ? tid & 31u : 0u;
+  const uint32_t step = SHIFT ? nt / 32u * 31u : nt;       // from one of a thread's packs to its next
   const char* src[N];
 #pragma unroll
-  for (int j = 0; j < N; ++j) src[j] = a->src[j] + srcOff;
+  for (int j = 0; j < N; ++j) src[j] = a->src[j] + srcOff - (SHIFT ? shift : 0);
   uint4 in[U][N];
   auto load = [&](uint64_t p) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (p + (uint32_t)u * nt >= nPacks) continue;
+      const uint64_t q = p + (uint32_t)u * step;
+      if (SHIFT ? q - lane >= nPacks || q > nPacks : q >= nPacks) continue;        // (aligned pack nPacks holds the end of the last logical one)
 #pragma unroll
-      for (int j = 0; j < N; ++j) in[u][j] = ld16(src[j] + (p + (uint32_t)u * nt) * 16);
+      for (int j = 0; j < N; ++j) in[u][j] = ld16(src[j] + q * 16);
     }
   };
-  uint64_t p = (uint64_t)df_tid();
+  uint64_t p = SHIFT ? (uint64_t)(tid / 32u * 31u + lane) : tid;
   load(p);
 #pragma unroll 1
-  while (p < nPacks) {
+  while (p - lane < nPacks) {                              // (SHIFT: the same for a warp's lanes)
     uint4 ow[U][NW];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (p + (uint32_t)u * nt >= nPacks) continue;
+      if (p + (uint32_t)u * step - lane >= nPacks) continue;
       A acc[V];
 #pragma unroll
-      for (int j = 0; j < N; ++j)
+      for (int j = 0; j < N; ++j) {
+        uint4 v = in[u][j];
+#if DF_DEVICE_CODE
+        if (SHIFT) v = shiftPack(v, nextLane(v), shift);
+#endif
 #pragma unroll
         for (int k = 0; k < V; ++k) {
-          const A e = (A)Lane<Tin>::get(in[u][j], k);
+          const A e = (A)Lane<Tin>::get(v, k);
           acc[k] = j == 0 ? e : red<OP_SUM>(acc[k], e);
         }
+      }
       finishPack<Tin, Tout>(ow[u], acc, mul, doMul, postDiv, scale);
     }
     const uint64_t q = p;
-    p += U * nt;
+    p += U * step;
     load(p);
+    if (SHIFT && lane == 31u) continue;
 #pragma unroll 1
     for (int d = 0; d < ndst; ++d) {
       char* o = a->dst[d] + dstOff + q * OUTB;
       const bool wide = OUTB == 32 && ((uintptr_t)o & 31) == 0;
 #pragma unroll
-      for (int u = 0; u < U; ++u) if (q + (uint32_t)u * nt < nPacks) storePack<OUTB>(o + (uint64_t)u * nt * OUTB, ow[u], wide);
+      for (int u = 0; u < U; ++u) if (q + (uint32_t)u * step < nPacks) storePack<OUTB>(o + (uint64_t)u * step * OUTB, ow[u], wide);
     }
   }
 }
@@ -497,6 +524,14 @@ DF_HD_NOINLINE bool reduceSmall(const DataArgs* a, int op) {
   return true;
 }
 
+template <typename Tin, typename Tout, bool SHIFT>
+DF_HD void reduceAheadOf(const DataArgs* a, uint64_t nPacks, int nsrc, int ndst, typename Elem<Tin>::Acc mul, bool doMul, int postDiv, double scale,
+                         uint64_t srcOff, uint64_t dstOff, uint32_t shift) {
+  if (nsrc == 2) reduceAhead<Tin, Tout, 2, SHIFT>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
+  else if (nsrc == 4) reduceAhead<Tin, Tout, 4, SHIFT>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
+  else reduceAhead<Tin, Tout, 8, SHIFT>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
+}
+
 template <typename Tin, typename Tout, int OP>
 DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   typedef typename Elem<Tin>::Acc A;
@@ -513,9 +548,11 @@ DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   const uint32_t shift = l.shift;
   const uint64_t srcOff = head * sizeof(Tin), dstOff = head * sizeof(Tout);
   if (nPacks) {
-    if (OP == OP_SUM && shift == 0 && nsrc == 2) reduceAhead<Tin, Tout, 2>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff);
-    else if (OP == OP_SUM && shift == 0 && nsrc == 4) reduceAhead<Tin, Tout, 4>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff);
-    else if (OP == OP_SUM && shift == 0 && nsrc == 8 && sizeof(Tout) <= sizeof(Tin)) reduceAhead<Tin, Tout, 8>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff);
+    const bool ahead = OP == OP_SUM && (nsrc == 2 || nsrc == 4 || (nsrc == 8 && sizeof(Tout) <= sizeof(Tin)));
+    if (ahead && shift == 0) reduceAheadOf<Tin, Tout, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
+#if DF_DEVICE_CODE
+    else if (ahead) reduceAheadOf<Tin, Tout, true>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
+#endif
     else if (shift == 0) reduceTrips<Tin, Tout, OP, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
     else reduceTrips<Tin, Tout, OP, true>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
   }
@@ -559,6 +596,31 @@ DF_HD void copyTrips(const DataArgs* a, uint64_t nPacks, int ndst, uint64_t off,
   const uint64_t step = (uint64_t)nt * U;
   const uint32_t strideB = (uint32_t)nt * 16u;
   uint64_t base = 0;
+#if DF_DEVICE_CODE
+  if (SHIFT) {                                             // 31 packs from the 32 that a warp loads (reduceAhead)
+    const uint32_t lane = (uint32_t)tid & 31u, hop = (uint32_t)nt / 32u * 31u;
+    const char* s = a->src[0] + off - shift;
+#pragma unroll 1
+    for (uint64_t p = (uint32_t)tid / 32u * 31u + lane; p - lane < nPacks; p += U * hop) {
+      uint4 raw[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint64_t q = p + (uint32_t)u * hop;
+        if (q - lane < nPacks && q <= nPacks) raw[u] = ld16(s + q * 16);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) raw[u] = shiftPack(raw[u], nextLane(raw[u]), shift);
+      if (lane == 31u) continue;
+#pragma unroll 1
+      for (int d = 0; d < ndst; ++d) {
+        char* o = a->dst[d] + off + p * 16;
+#pragma unroll
+        for (int u = 0; u < U; ++u) if (p + (uint32_t)u * hop < nPacks) st16(o + (uint64_t)u * hop * 16, raw[u]);
+      }
+    }
+    return;
+  }
+#endif
   for (; base + step <= nPacks; base += step) copyTrip<true, SHIFT, U>(a, base + tid, nPacks, strideB, ndst, off, shift);
   for (; base + nt <= nPacks; base += nt) copyTrip<true, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);
   if (base + tid < nPacks) copyTrip<false, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);

@@ -1,5 +1,6 @@
 """Long sums of two, four and eight aligned sources, whose loads run ahead of the stores: whole trips of a block, one pack more and
-less, ragged ends, every element size, results wider and narrower than the operands."""
+less, ragged ends, every element size, results wider and narrower than the operands; and sums and copies of pieces that start off
+the 16-byte grid, where a warp's 32 aligned packs make 31."""
 import pytest
 
 from test_gpu_daemon import _loopback_case, nv  # noqa: F401
@@ -19,3 +20,16 @@ def test_sums_with_loads_ahead(nv, kind, nranks, count, dtype, out, op):  # noqa
     if kind == "reducescatter":
         count = (count + 15) // 16 * 16                    # chunks on the 16-byte grid; others take the shifted path
     _loopback_case(nv, kind, nranks, count, dtype, op=op, out_name=out, blocks=1)
+
+
+# 465 packs of 16 bytes are what a block's 15 warps make of one load each
+SHIFTED = [("reducescatter", 2, 4 * 465 * 40 + 1, "FLOAT32", None), ("reducescatter", 4, 4 * 465 * 38 + 3, "FLOAT32", None), ("reducescatter", 4, 4 * 465 + 3, "FLOAT32", None),
+           ("reducescatter", 8, 8 * 465 * 36 + 1, "BFLOAT16", None), ("reducescatter", 4, 8 * 465 * 37 - 3, "BFLOAT16", "FLOAT32"), ("reducescatter", 3, 4 * 465 * 40 + 3, "FLOAT32", None),
+           ("reducescatter", 2, 4 * 465 * 41 - 1, "FLOAT32", "BFLOAT16"), ("reducescatter", 8, 8 * 465 * 35 + 9, "FLOAT16", "FLOAT32"), ("reducescatter", 4, 16 * 465 * 36 + 5, "UINT8", None),
+           ("allgather", 4, 8 * 465 * 40 + 7, "BFLOAT16", None), ("allgather", 2, 16 * 465 * 8 * 5 + 3, "UINT8", None), ("allgather", 2, 4 * 465 * 8 * 5 + 1, "FLOAT32", None), ("allgather", 8, 8 * 31 + 5, "BFLOAT16", None)]
+
+
+@pytest.mark.parametrize("kind,nranks,count,dtype,out", SHIFTED)
+def test_pieces_off_the_grid(nv, kind, nranks, count, dtype, out):  # noqa: F811
+    for blocks in (1, 3):
+        _loopback_case(nv, kind, nranks, count, dtype, out_name=out, blocks=blocks)
