@@ -337,8 +337,17 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
     FlagSlot* mine = sh->cs.myFlags + (uint64_t)b * n;
     uint32_t spins = 0;
     bool ok;
+    // At every fourth poll the last lane looks at the ring too, its load on its way with theirs: a wait with a lot of patience ends when
+    // there is something else to do.  (At every sixteenth where all peers are in the collective already: they are done soon, and another
+    // collective's context costs more than that.)
+    const uint32_t often = which == 1 ? 15u : 3u;
     for (;;) {
       bool laneOk = true;
+      uint64_t entry = 0, tag = 1;
+      if ((spins & often) == often && lane == ws - 1 && !sh->standalone && sh->k.devSq != nullptr) {
+        entry = ld_relaxed_sys_u64(sh->k.devSq[sh->frontier & (sh->k.sqCap - 1)].w);
+        tag = sqTag(sh->frontier, sh->k.sqCap);
+      }
       if (which == 2) {
         if (lane == 0) laneOk = (int32_t)((uint32_t)ld_relaxed_sys_u64(&sh->k.trigger[sh->loadedColl]) - (uint32_t)sh->dyn.trigger) >= 0;
       } else {
@@ -357,6 +366,7 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
       }
       bool laneStop = false;
       if ((spins & 255) == 255 && lane == 0) laneStop = abortRequested(&sh->k);
+      if (entry >> 57 == tag) laneStop = true;
       ok = df_warp_all(laneOk);
       const bool stop = !df_warp_all(!laneStop);      // uniform: every lane leaves the loop together
       ++spins;
@@ -615,12 +625,13 @@ DF_HD int nextPhase(const BlockShared* sh, int phase) {
   return PH_COMPLETE;
 }
 
-// A wait of the loaded collective with its adaptive budget.  The budget is what the scheduler grants or, if larger,
-// the patience this submission has earned: after a wait succeeded within s polls the next waits of the same
+// A wait of the loaded collective with its adaptive budget.  The budget is what the scheduler grants or, if larger and nothing else
+// is queued, the patience this submission has earned: after a wait succeeded within s polls the next waits of the same
 // submission may spend factor x s polls (capped), because a collective whose peers are demonstrably in it is worth
 // staying with (reference: RECV_SUCCESS_FACTOR, src/collectives_ofccl/device/ofccl_prims_simple.h:79-88,143-151).
 DF_HD bool patientWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t budget) {
-  const uint32_t eff = budget > sh->dyn.patience ? budget : sh->dyn.patience;
+  const bool alone = sh->standalone || sh->nActive <= 1;
+  const uint32_t eff = alone && sh->dyn.patience > budget ? sh->dyn.patience : budget;
   const bool ok = boundedWait(sh, rd, b, which, eff);
   if (ok && df_tid() == 0) {
     sh->dyn.stallSinceNs = 0;

@@ -24,7 +24,7 @@ import torch
 import torch.distributed as dist
 
 from .. import native as nv
-from ..utils.tensors import raw_stream, stream_of, tensor_from_ptr
+from ..utils.tensors import raw_stream, tensor_from_ptr
 from .block import Epilogue, NO_EPILOGUE, packed
 from .gemm import BM, BN, BK
 
@@ -111,11 +111,11 @@ class _Local:
             raise ValueError(f"weight of {tuple(w.shape)} for an operator of {self.n_out} outputs and {self.k} inputs")
         out = torch.empty(self.m, self.n_out, dtype=torch.bfloat16, device=self.tp.device)
         epilogue = epi.args_for(self.m, self.n_out)
-        ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), stream_of(out)
+        ptrs, st = (x.data_ptr(), w.data_ptr(), out.data_ptr()), raw_stream(self.tp.device)
         if self.coll_id is not None:
             nv.check(nv.entry("dfcclRunFusedGemmLocal")(self.coll_id, *ptrs, int(w_transposed), *epilogue, st, self.tp.ctx.handle.value), "dfcclRunFusedGemmLocal")
         else:
-            nv.check(nv.entry("dfcclGemmBf16Epilogue")(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epilogue, st), "dfcclGemmBf16Epilogue")
+            nv.check(nv.lib().dfcclGemmBf16Epilogue(*ptrs, self.m, self.n_out, self.k, 0, int(w_transposed), *epilogue, st), "dfcclGemmBf16Epilogue")
         return out
 
 
