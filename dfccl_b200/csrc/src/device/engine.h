@@ -656,7 +656,8 @@ DF_HD bool patientWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
 // by one lane per member in front of the barrier that ends the wait, small bodies (datapath.h), one atomic for the blocks' count and
 // verdicts, comparisons instead of jump tables, and no fence that nobody waits for.  Among four ranks of a device, submitted and
 // awaited on the host, before / with all of these and calls that do not go through ctypes, us: 509 bf16 33.9 / 19.8, 25 MiB
-// bf16 -> fp32 97.9 / 81.2, a ragged reduce-scatter and all-gather 90.7 / 66.5, 24 mixed collectives in four orders 295 / 203 - 214.
+// bf16 -> fp32 97.9 / 81.2, a ragged reduce-scatter and all-gather 90.7 / 66.5, 24 mixed collectives in four orders 295 / 211; since, with
+// other bodies of the sums (datapath.h) and shorter waits (daemon_impl.h), 76.2, 54.3 and 147.
 DF_HD int runColl(BlockShared* sh, RankDev* rd, int b, int coll, uint32_t budget, bool* moved) {
   if (!sh->standalone) loadColl(sh, rd, b, coll);
   const CollStatic* c = &sh->cs;

@@ -374,9 +374,10 @@ static GemmTilePlan choosePlan(int M, int N, int K, int sms, bool pairs, bool bM
   if (p.split == 1 && bMn) p = best(true, true);
   // One wave of plain tiles of 256 x 256 gains nothing from the persistent kernel's overlap, and the form with the same tile has
   // stages of 128 of the contraction and a geometry that the compiler knows.  us, persistent / form: 4096 x 1024 x 8192 58.5 / 56.9,
-  // x 2048 16.8 / 15.8, x 1024 10.8 / 10.0, x 512 7.9 / 7.6, 1024 x 4096 x 8192 59.2 / 57.1, 7168 x 512 x 960 11.9 / 11.3, 3328 x 1024 x
-  // 4032 24.4 / 23.8; but 640 x 5120 x 448 7.2 / 7.3, 4096 x 1024 x 128 5.3 / 5.8, and with one or two row tiles, whose operands hardly
-  // meet in L2, 512 x 7168 x 4992 29.4 / 31.4, 384 x 7680 x 5248 33.5 / 34.9.
+  // x 2048 16.8 / 15.8, 1024 x 4096 x 8192 59.2 / 57.1, 7168 x 512 x 960 11.9 / 11.3, 3328 x 1024 x 4032 24.4 / 23.8; but 640 x 5120 x 448
+  // 7.2 / 7.3, 4096 x 1024 x 128 5.3 / 5.8, and with one or two row tiles, whose operands hardly meet in L2, 512 x 7168 x 4992 29.4 /
+  // 31.4, 384 x 7680 x 5248 33.5 / 34.9.  (Before results of either went through boxes in the operands' stages, which brought 4096 x 1024 x
+  // 1024 from 10.4 to 9.9 on the form.)
   if (pairs && !epilogue && p.width == 256 && (M + 255) / 256 * (N / 256) <= sms / 2 && K >= 512 && M > 512) p = GemmTilePlan{true, 256, 1, 0};
   if (!pairs && (p.pair || p.width)) {                 // one CTA per tile by request: the same slices
     double us = 1e30;
