@@ -196,13 +196,30 @@ DF_HD uint4 shiftPack(const uint4& lo, const uint4& hi, uint32_t shift) {
 #endif
 }
 
+// The neighbour lane's pack (the last lane gets its own back); the whole warp calls it.  `at`: where this lane's pack was read.
+DF_HD uint4 nextLane(const uint4& v, const char* at) {
 #if DF_DEVICE_CODE
-// the neighbour lane's pack (the last lane gets its own back); the whole warp calls it
-__device__ __forceinline__ uint4 nextLane(const uint4& v) {
   return make_uint4(__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1), __shfl_down_sync(0xffffffffu, v.z, 1),
                     __shfl_down_sync(0xffffffffu, v.w, 1));
-}
+#else
+  return ld16(at + 16);
 #endif
+}
+
+// Shifted packs without a second load: the aligned packs that a warp of `ws` lanes loads make ws - 1 logical ones, each from a lane's and its
+// neighbour's.  (A host thread is a warp of one lane, which reads its neighbour's itself.)  A thread's packs are `first`, first + step, ...
+struct ShiftedWalk { uint32_t lane, step; uint64_t first; };
+DF_HD ShiftedWalk shiftedWalk(uint32_t tid, uint32_t nt, uint32_t ws) {
+  const uint32_t makes = ws > 1 ? ws - 1 : 1, lane = tid % ws;
+  ShiftedWalk w;
+  w.lane = lane; w.step = nt / ws * makes; w.first = (uint64_t)(tid / ws * makes + lane);
+  return w;
+}
+// The warp whose lane `lane` is at pack q has something to do (the same for its lanes); this lane loads aligned pack q (number nPacks holds
+// the end of the last logical one); this lane makes packs of its own.
+DF_HD bool shiftedWarpAt(uint64_t q, uint32_t lane, uint64_t nPacks) { return q - lane < nPacks; }
+DF_HD bool shiftedLoads(uint64_t q, uint32_t lane, uint64_t nPacks) { return shiftedWarpAt(q, lane, nPacks) && q <= nPacks; }
+DF_HD bool shiftedMakes(uint32_t lane, uint32_t ws) { return ws == 1 || lane != ws - 1; }
 
 // U logical packs of one source for this thread; pack u starts `u * strideB` bytes after `s`, `shift` = s & 15.
 // SHIFT = false: s is aligned.  FULL: every thread of the block loads all of its U packs (warp shuffles are safe).
@@ -224,7 +241,7 @@ DF_HD void loadPacks(uint4* out, const char* s, uint32_t strideB, uint32_t shift
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint4 hi = nextLane(out[u]);
+      const uint4 hi = nextLane(out[u], nullptr);
       out[u] = shiftPack(out[u], (threadIdx.x & 31) == 31 ? last[u] : hi, shift);
     }
     return;
@@ -379,8 +396,10 @@ DF_HD void reduceAhead(const DataArgs* a, uint64_t nPacks, int ndst, typename El
   typedef typename Elem<Tin>::Acc A;
   constexpr int V = 16 / (int)sizeof(Tin), OUTB = V * (int)sizeof(Tout), NW = (OUTB + 15) / 16;
   constexpr int U = N == 4 && NW == 2 ? 1 : 8 / N;
-  const uint32_t tid = (uint32_t)df_tid(), nt = (uint32_t)df_nthreads(), lane = SHIFT ? tid & 31u : 0u;
-  const uint32_t step = SHIFT ? nt / 32u * 31u : nt;       // from one of a thread's packs to its next
+  const uint32_t tid = (uint32_t)df_tid(), nt = (uint32_t)df_nthreads(), ws = (uint32_t)df_warpsize();
+  ShiftedWalk w = {0u, nt, tid};
+  if (SHIFT) w = shiftedWalk(tid, nt, ws);
+  const uint32_t lane = w.lane, step = w.step;             // (from one of a thread's packs to its next)
   const char* src[N];
 #pragma unroll
   for (int j = 0; j < N; ++j) src[j] = a->src[j] + srcOff - (SHIFT ? shift : 0);
@@ -389,26 +408,25 @@ DF_HD void reduceAhead(const DataArgs* a, uint64_t nPacks, int ndst, typename El
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const uint64_t q = p + (uint32_t)u * step;
-      if (SHIFT ? q - lane >= nPacks || q > nPacks : q >= nPacks) continue;        // (aligned pack nPacks holds the end of the last logical one)
+      if (!(SHIFT ? shiftedLoads(q, lane, nPacks) : q < nPacks)) continue;
 #pragma unroll
       for (int j = 0; j < N; ++j) in[u][j] = ld16(src[j] + q * 16);
     }
   };
-  uint64_t p = SHIFT ? (uint64_t)(tid / 32u * 31u + lane) : tid;
+  uint64_t p = w.first;
   load(p);
 #pragma unroll 1
-  while (p - lane < nPacks) {                              // (SHIFT: the same for a warp's lanes)
+  while (shiftedWarpAt(p, lane, nPacks)) {
     uint4 ow[U][NW];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (p + (uint32_t)u * step - lane >= nPacks) continue;
+      const uint64_t q = p + (uint32_t)u * step;
+      if (!shiftedWarpAt(q, lane, nPacks)) continue;
       A acc[V];
 #pragma unroll
       for (int j = 0; j < N; ++j) {
         uint4 v = in[u][j];
-#if DF_DEVICE_CODE
-        if (SHIFT) v = shiftPack(v, nextLane(v), shift);
-#endif
+        if (SHIFT) v = shiftPack(v, nextLane(v, src[j] + q * 16), shift);
 #pragma unroll
         for (int k = 0; k < V; ++k) {
           const A e = (A)Lane<Tin>::get(v, k);
@@ -420,7 +438,7 @@ DF_HD void reduceAhead(const DataArgs* a, uint64_t nPacks, int ndst, typename El
     const uint64_t q = p;
     p += U * step;
     load(p);
-    if (SHIFT && lane == 31u) continue;
+    if (SHIFT && !shiftedMakes(lane, ws)) continue;
 #pragma unroll 1
     for (int d = 0; d < ndst; ++d) {
       char* o = a->dst[d] + dstOff + q * OUTB;
@@ -550,9 +568,7 @@ DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   if (nPacks) {
     const bool ahead = OP == OP_SUM && (nsrc == 2 || nsrc == 4 || (nsrc == 8 && sizeof(Tout) <= sizeof(Tin)));
     if (ahead && shift == 0) reduceAheadOf<Tin, Tout, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
-#if DF_DEVICE_CODE
     else if (ahead) reduceAheadOf<Tin, Tout, true>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
-#endif
     else if (shift == 0) reduceTrips<Tin, Tout, OP, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
     else reduceTrips<Tin, Tout, OP, true>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
   }
@@ -596,31 +612,33 @@ DF_HD void copyTrips(const DataArgs* a, uint64_t nPacks, int ndst, uint64_t off,
   const uint64_t step = (uint64_t)nt * U;
   const uint32_t strideB = (uint32_t)nt * 16u;
   uint64_t base = 0;
-#if DF_DEVICE_CODE
-  if (SHIFT) {                                             // 31 packs from the 32 that a warp loads (reduceAhead)
-    const uint32_t lane = (uint32_t)tid & 31u, hop = (uint32_t)nt / 32u * 31u;
+  if (SHIFT) {                                             // (see shiftedWalk)
+    const uint32_t ws = (uint32_t)df_warpsize();
+    const ShiftedWalk w = shiftedWalk((uint32_t)df_tid(), (uint32_t)df_nthreads(), ws);
     const char* s = a->src[0] + off - shift;
 #pragma unroll 1
-    for (uint64_t p = (uint32_t)tid / 32u * 31u + lane; p - lane < nPacks; p += U * hop) {
+    for (uint64_t p = w.first; shiftedWarpAt(p, w.lane, nPacks); p += U * w.step) {
       uint4 raw[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const uint64_t q = p + (uint32_t)u * hop;
-        if (q - lane < nPacks && q <= nPacks) raw[u] = ld16(s + q * 16);
+        const uint64_t q = p + (uint32_t)u * w.step;
+        if (shiftedLoads(q, w.lane, nPacks)) raw[u] = ld16(s + q * 16);
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) raw[u] = shiftPack(raw[u], nextLane(raw[u]), shift);
-      if (lane == 31u) continue;
+      for (int u = 0; u < U; ++u) {
+        const uint64_t q = p + (uint32_t)u * w.step;
+        if (ws > 1 || shiftedWarpAt(q, w.lane, nPacks)) raw[u] = shiftPack(raw[u], nextLane(raw[u], s + q * 16), shift);
+      }
+      if (!shiftedMakes(w.lane, ws)) continue;
 #pragma unroll 1
       for (int d = 0; d < ndst; ++d) {
         char* o = a->dst[d] + off + p * 16;
 #pragma unroll
-        for (int u = 0; u < U; ++u) if (p + (uint32_t)u * hop < nPacks) st16(o + (uint64_t)u * hop * 16, raw[u]);
+        for (int u = 0; u < U; ++u) if (p + (uint32_t)u * w.step < nPacks) st16(o + (uint64_t)u * w.step * 16, raw[u]);
       }
     }
     return;
   }
-#endif
   for (; base + step <= nPacks; base += step) copyTrip<true, SHIFT, U>(a, base + tid, nPacks, strideB, ndst, off, shift);
   for (; base + nt <= nPacks; base += nt) copyTrip<true, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);
   if (base + tid < nPacks) copyTrip<false, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);

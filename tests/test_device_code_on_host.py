@@ -7,11 +7,11 @@ import pytest
 from dfccl_b200 import _build
 
 
-def run_on_host(tmp_path, body: str) -> str:
+def run_on_host(tmp_path, body: str, defines=()) -> str:
     """Compile ``body`` behind the step engine's header, run it, return what it printed."""
     src, exe = tmp_path / "case.cu", tmp_path / "case"
     src.write_text('#include "device/engine.h"\n#include <stdio.h>\n#include <string.h>\nusing namespace dfccl;\n' + body)
-    cmd = [_build.nvcc(), "-std=c++17", "-O2", "-DDF_FAST_BUILD", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(_build.CSRC / "src"),
+    cmd = [_build.nvcc(), "-std=c++17", "-O2", "-DDF_FAST_BUILD", *(f"-D{d}" for d in defines), "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(_build.CSRC / "src"),
            "-I", str(_build.CSRC / "include"), str(src), "-o", str(exe)]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
@@ -127,4 +127,88 @@ int main() {
   return 0;
 }
 """)
+    assert out == "ok\n"
+
+
+def test_shifted_packs_are_made_once_each(tmp_path):
+    """Warps of 32 lanes: every logical pack is made by one lane, whose neighbour has loaded the pack behind it; nothing is loaded
+    beyond aligned pack nPacks; the lanes of a warp go round together."""
+    out = run_on_host(tmp_path, r"""
+#include <vector>
+int main() {
+  for (uint32_t nt : {32u, 64u, 480u})
+    for (uint32_t unroll : {1u, 2u, 4u, 8u})
+      for (uint64_t nPacks : {1ull, 2ull, 30ull, 31ull, 32ull, 62ull, 63ull, 464ull, 465ull, 466ull, 929ull, 930ull, 3719ull, 3720ull, 3721ull, 10007ull}) {
+        std::vector<int> made(nPacks, 0);
+        for (uint32_t warp = 0; warp < nt / 32; ++warp) {
+          ShiftedWalk w[32];
+          for (uint32_t l = 0; l < 32; ++l) w[l] = shiftedWalk(warp * 32 + l, nt, 32);
+          for (uint64_t trip = 0;; ++trip) {
+            const uint64_t hop = trip * unroll * w[0].step;
+            const bool go = shiftedWarpAt(w[0].first + hop, w[0].lane, nPacks);
+            for (uint32_t l = 0; l < 32; ++l) if (shiftedWarpAt(w[l].first + hop, w[l].lane, nPacks) != go) return 1;
+            if (!go) break;
+            for (uint32_t u = 0; u < unroll; ++u)
+              for (uint32_t l = 0; l < 32; ++l) {
+                const uint64_t q = w[l].first + hop + (uint64_t)u * w[l].step;
+                if (w[l].lane != l || (shiftedLoads(q, l, nPacks) && q > nPacks)) return 2;
+                if (!shiftedMakes(l, 32) || q >= nPacks) continue;
+                if (!shiftedLoads(q, l, nPacks) || !shiftedLoads(q + 1, l + 1, nPacks) || w[l + 1].first != w[l].first + 1) return 3;
+                ++made[q];
+              }
+          }
+        }
+        for (int m : made) if (m != 1) { printf("%u threads, %u, %llu packs: one made %d times\n", nt, unroll, (unsigned long long)nPacks, m); return 4; }
+      }
+  puts("ok");
+  return 0;
+}
+""")
+    assert out == "ok\n"
+
+
+def test_shifted_sums_and_copies_stay_in_their_buffers(tmp_path):
+    """Sums of one to nine sources and copies of pieces off the 16-byte grid, whose last wanted byte is the last of a page with nothing
+    behind it and whose first is the first of one with nothing in front of it."""
+    out = run_on_host(tmp_path, r"""
+#include <sys/mman.h>
+#include <vector>
+#include <memory>
+static const size_t PAGE = 4096, SPAN = 4 * PAGE;
+static char* page() {                                  // SPAN bytes between two pages that cannot be touched
+  char* p = (char*)mmap(nullptr, SPAN + 2 * PAGE, PROT_NONE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  return mprotect(p + PAGE, SPAN, PROT_READ | PROT_WRITE) ? nullptr : p + PAGE;
+}
+int main() {
+  std::unique_ptr<DataArgs> a(new DataArgs);
+  std::vector<char*> in;
+  for (int j = 0; j < 9; ++j) in.push_back(page());
+  std::vector<char> out(SPAN + 128);
+  for (int atEnd = 0; atEnd < 2; ++atEnd)
+    for (int nsrc = 0; nsrc <= 9; ++nsrc)              // 0: a copy
+      for (uint32_t bytes : {20u, 36u, 64u, 516u, 1028u, 2052u, 8188u, 16380u})
+        for (uint32_t skew : {0u, 4u, 8u, 12u}) {      // of the destination, against sources whose ends or beginnings lie on the grid
+          const uint32_t n = bytes / 4;
+          memset((void*)a.get(), 0, sizeof(DataArgs));
+          char* dst = (char*)(((uintptr_t)out.data() + 32) & ~(uintptr_t)31) + 32 + skew;
+          memset(out.data(), 7, out.size());
+          const size_t at = atEnd ? SPAN - bytes : 0;
+          for (int j = 0; j < (nsrc ? nsrc : 1); ++j) {
+            a->src[j] = in[j] + at;
+            for (uint32_t i = 0; i < n; ++i) ((float*)a->src[j])[i] = (float)((i * 37 + j * 101) % 1009) + 0.25f * j;
+          }
+          a->dst[0] = dst; a->nsrc = nsrc ? nsrc : 1; a->ndst = 1; a->scale = 1.0; a->postDiv = 0;
+          if (nsrc) { a->n = n; if (!reduce_dispatch(ncclFloat32, ncclFloat32, OP_SUM, a.get())) return 2; }
+          else { a->n = bytes; copy_multi(a.get()); }
+          for (uint32_t i = 0; i < n; ++i) {
+            float s = ((const float*)a->src[0])[i];
+            for (int j = 1; j < nsrc; ++j) s += ((const float*)a->src[j])[i];
+            if (((const float*)dst)[i] != s) { printf("%d sources, %u bytes, skew %u: element %u\n", nsrc, bytes, skew, i); return 3; }
+          }
+          if (dst[-1] != 7 || dst[bytes] != 7) return 4;
+        }
+  puts("ok");
+  return 0;
+}
+""", defines=("DF_DATAPATH_IMPL",))
     assert out == "ok\n"
