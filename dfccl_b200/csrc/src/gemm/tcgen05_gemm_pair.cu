@@ -45,6 +45,28 @@ constexpr uint64_t WAIT_NS = 4000000000ull;          // nothing here waits on an
 __host__ __device__ constexpr int epiWarps(int epi) { return epi == EPI_NONE || epi == EPI_BIAS ? 8 : 16; }
 __host__ __device__ constexpr int pairThreads(int epi) { return 64 + 32 * epiWarps(epi); }
 
+// A stage: `kSteps` blocks of 64 of the contraction (gemmPairLaunch), HALF rows of A and half the tile's columns of B.
+constexpr int kSteps(int width) { return width >= 224 ? 1 : 2; }
+constexpr int bBytesOf(int width, bool bMn) { return (bMn ? (width / 2 + 63) / 64 * 64 : width / 2) * 64 * kSteps(width) * 2; }
+constexpr int stageBytesOf(int width, bool bMn) { return HALF * 64 * kSteps(width) * 2 + bBytesOf(width, bMn); }
+// Boxes of one epilogue warp where a pair has one tile, and the stages that hold all of them.
+constexpr int boxesOnce(int epi, int width, bool stored) { return (width / 32 + epiWarps(epi) / 4 - 1) / (epiWarps(epi) / 4) * (stored ? 2 : 1); }
+constexpr int stagesOnce(int epi, int width, bool bMn, bool stored) {
+  return (epiWarps(epi) * boxesOnce(epi, width, stored) * BOX_BYTES + stageBytesOf(width, bMn) - 1) / stageBytesOf(width, bMn);
+}
+// They have a barrier each and fit in front of the barriers: five stages (150 KB) at width 224 and three of 56 KB at 192, with GELU and
+// its pre-activation stored, are the most.
+constexpr bool boxesFit() {
+  for (int epi = EPI_NONE; epi <= EPI_GELU_GRAD; ++epi)
+    for (int width = 64; width <= 256; width += 32)
+      for (int i = 0; i < 4; ++i) {
+        const int stages = stagesOnce(epi, width, (i & 1) != 0, i >= 2 && epi == EPI_BIAS_GELU);
+        if (stages > MAX_STAGES || stages * stageBytesOf(width, (i & 1) != 0) > SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK) return false;
+      }
+  return true;
+}
+static_assert(boxesFit(), "the boxes of a pair's only tile do not fit its operands' stages");
+
 struct PairArgs {
   int M, N, K, ldc;
   int aMn, bMn;
@@ -348,8 +370,7 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   // 64 of the contraction in a stage keep more loads in flight beside wide tiles (stages of 128: 8192 x 4096 x 1024 and its
   // gradients 0.3 - 0.5 % slower, 4096 x 1024 x 8192 the same); for narrower ones the tensor cores are through with such a stage
   // before its two loads are issued (460 clocks)
-  const int kStep = width >= 224 ? 1 : 2, BK = 64 * kStep;
-  const int bHalf = width / 2, bBytes = bMn ? (bHalf + 63) / 64 * 64 * BK * 2 : bHalf * BK * 2;
+  const int kStep = kSteps(width), BK = 64 * kStep, bHalf = width / 2;
   CUtensorMap ma, mb, mc, mp;
   DFCHECK(gemmMakeMap3(&ma, A, (uint64_t)M, (uint64_t)K, aMn, HALF, BK));
   if (bMn && bHalf % 64) DFCHECK(gemmMakeMap(&mb, B, (uint64_t)K, (uint64_t)N, BK));
@@ -373,9 +394,9 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   // K = 256 14 % less with boxes, 512 4 %, 768 the same, 1024 1 % more, 1536 2 %; narrower ones 8 %, 0, 2 % more, 3 %, 4 % (230 and 800
   // products of all storage orders).
   const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && tiles > pairs && K >= 768);
-  const int parts = epiWarps(g.e.kind) / 4, stored = g.e.kind == EPI_BIAS_GELU && g.e.pre ? 2 : 1;
+  const bool stored = g.e.kind == EPI_BIAS_GELU && g.e.pre;
   g.boxes = !straight;
-  g.once = tiles > pairs ? 0 : (width / 32 + parts - 1) / parts * stored;
+  g.once = tiles > pairs ? 0 : boxesOnce(g.e.kind, width, stored);
   g.epiBytes = g.boxes && !g.once ? EPI_BYTES : 0;
   mc = ma;                                             // (straight stores take no map: none is made, or kept, per output)
   if (!straight) DFCHECK(gemmMakeMap(&mc, C, (uint64_t)M, (uint64_t)N, 32, 32));
@@ -384,11 +405,12 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   // (where every pair has one tile the order decides nothing)
   { int64_t gm = tiles > pairs ? paramI64("GEMM_RASTER_GROUP", 8) : 8; g.groupM = (int)(gm < 1 ? 1 : gm > 64 ? 64 : gm); }
   g.kStep = kStep;
-  g.stageBytes = HALF * BK * 2 + bBytes;               // width 256: WIDE_STAGE, however B is stored
+  g.stageBytes = stageBytesOf(width, bMn != 0);        // width 256: WIDE_STAGE, however B is stored
   const int room = SMEM_LIMIT - BAR_BYTES - ALIGN_SLACK - g.epiBytes;
   const int want = tiles > pairs ? MAX_STAGES : (K + BK - 1) / BK;
   g.stages = std::min(std::min(MAX_STAGES, room / g.stageBytes), want);
-  if (g.boxes) while (g.stages * g.stageBytes < epiWarps(g.e.kind) * g.once * BOX_BYTES) ++g.stages;       // (four of 32 KB at most)
+  if (g.boxes && g.once) g.stages = std::max(g.stages, stagesOnce(g.e.kind, width, bMn != 0, stored));        // (boxesFit)
+  if (g.stages > MAX_STAGES || g.stages * g.stageBytes > room) return ncclInternalError;
   g.tmemCols = tiles > pairs ? 512 : width <= 64 ? 64 : width <= 128 ? 128 : 256;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
