@@ -392,8 +392,12 @@ ncclResult_t gemmPairLaunch(int width, const void* A, const void* B, void* C, in
   // that follow: a pair's only tile, whose boxes lie in the stages it no longer needs, goes through them, others with short
   // contractions.  us, boxes / straight: 1920 x 1792 x 3072 18.0 / 18.6, 3200 x 768 x 1088 11.4 / 11.7; several tiles, widths from 224 on: up to
   // K = 256 14 % less with boxes, 512 4 %, 768 the same, 1024 1 % more, 1536 2 %; narrower ones 8 %, 0, 2 % more, 3 %, 4 % (230 and 800
-  // products of all storage orders).
-  const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && tiles > pairs && K >= 768);
+  // products of all storage orders).  A bias, added between tensor memory and the store, moves the line of the wide ones: 8192 x 4096 x
+  // 768 44.9 / 47.9, x 832 46.1 / 47.8, x 896 48.7 / 49.5, x 1024 56.5 / 57.2, 5376 x 4096 x 768 29.4 / 30.9, x 896 35.3 / 36.1, 4096 x 3072 x 768 17.8 /
+  // 18.7, x 896 22.1 / 22.3, x 1024 23.9 / 23.8, 16384 x 768 x 768 19.6 / 20.2, x 896 23.4 / 23.7, x 1024 25.7 / 25.6, 3840 x 1792 x 896 14.2 / 14.0; not that of
+  // narrower ones: 2560 x 3840 x 512 13.5 / 13.7, x 768 16.6 / 15.2, 2176 x 2304 x 768 11.9 / 10.7, x 1024 13.2 / 12.0.
+  const int line = g.e.kind == EPI_BIAS && width >= 224 ? 1024 : 768;
+  const bool straight = g.e.kind == EPI_GELU_GRAD || ((g.e.kind == EPI_NONE || g.e.kind == EPI_BIAS) && tiles > pairs && K >= line);
   const bool stored = g.e.kind == EPI_BIAS_GELU && g.e.pre;
   g.boxes = !straight;
   g.once = tiles > pairs ? 0 : boxesOnce(g.e.kind, width, stored);

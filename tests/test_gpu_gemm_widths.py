@@ -74,3 +74,22 @@ def test_epilogues_inside_ragged_tiles(m, n, k):
         else:
             ref = want[kind]
         assert ((out.double() - ref).norm() / ref.norm()).item() < 2 ** -9
+
+
+@pytest.mark.parametrize("m,n,k", [(4096, 3072, 704), (4096, 3072, 768), (4096, 3072, 1024), (3840, 1792, 960), (2176, 2304, 704), (2176, 2304, 832)])
+def test_bias_on_either_side_of_the_line(m, n, k):
+    """Several tiles per pair, results through boxes and straight from the registers: one rounding, nothing behind the result."""
+    from dfccl_b200 import native as nv
+    from dfccl_b200.ops import block
+    assert gemm_plan(m, n, k, False, 1)[3] >= 160
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(n, k, device="cuda") * k ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(n, device="cuda").to(torch.bfloat16)
+    out = torch.full((m + 128, n), 7.0, device="cuda", dtype=torch.bfloat16)
+    nv.check(nv.lib().dfcclGemmBf16Epilogue(a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, 0, 0, *block.Epilogue(block.BIAS, bias).args(),
+                                            torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    ref = a.double() @ b.double().t() + bias.double()
+    assert ((out[:m].double() - ref).norm() / ref.norm()).item() < 2 ** -9
+    assert bool((out[m:] == 7.0).all())
