@@ -74,8 +74,8 @@ DF_HD int consumeSubmissions(BlockShared* sh, RankDev* rd, int b, SqSlot slot, S
       // A stream-ordered caller may publish the next submission of a collective while this block
       // still runs the previous one.  The entry is never dropped: consumption stops here and
       // resumes once the running submission has completed.
-      if (sh->busy[coll >> 5] & (1u << (coll & 31))) break;
-      if ((q.flags & SQE_TRIGGERED) ? sh->nTrig >= DF_MAX_ACTIVE : sh->nActive >= DF_MAX_ACTIVE) break;   // (cannot happen: one outstanding submission per id)
+      const bool full = (q.flags & SQE_TRIGGERED) ? sh->nTrig >= DF_MAX_ACTIVE : sh->nActive >= DF_MAX_ACTIVE;   // (cannot happen: one outstanding submission per id)
+      if (full || (sh->busy[coll >> 5] & (1u << (coll & 31)))) { sh->stuckAt = sh->frontier; break; }
     }
     ++sh->frontier;
     ++got;
@@ -176,7 +176,7 @@ DF_HD void blockRestore(BlockShared* sh, RankDev* rd, int b) {
   BlockSaved* sv = &rd->saved[b];
   if (tid == 0) {
     sh->k = *rd;
-    sh->nParked = 0; sh->nReady = 0; sh->frontierSeen = sv->frontier;
+    sh->nParked = 0; sh->nReady = 0; sh->frontierSeen = sv->frontier; sh->stuckAt = ~0ull;
     sh->loadedColl = -1; sh->standalone = 0; sh->dynDirty = 0; sh->quit = 0; sh->abortSeen = 0; sh->ctl1Full = 0;
     sh->frontier = sv->frontier; sh->nActive = sv->nActive; sh->nTrig = sv->nTrig;
     DevStats z = {};
@@ -315,7 +315,8 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
       // once one block of this rank has left voluntarily the others take no new work and follow as
       // soon as they cannot progress: a collective needs all its blocks, so the relaunch comes sooner
       winding = left;
-      if (!winding && have && consumeSubmissions(sh, rd, b, slot, next, haveNext) > 0) progressed = true;
+      if (have && winding) sh->stuckAt = sh->frontier;
+      else if (have && consumeSubmissions(sh, rd, b, slot, next, haveNext) > 0) progressed = true;
       reportFrontier(sh, b, !progressed);
       if (sh->abortSeen) sh->quit = 3;
       else if (sh->k.maxLifetimeNs && now - bornNs > sh->k.maxLifetimeNs && !sh->quit) {

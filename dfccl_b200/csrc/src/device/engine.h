@@ -48,6 +48,7 @@ struct BlockShared {
   DevStats stats;
   uint64_t frontier;
   uint64_t frontierSeen;         // as last reported to the host
+  uint64_t stuckAt;              // an entry that the block has met and cannot take yet (~0: none): no reason to end a wait
   uint32_t nParked;              // entries of the task queue with a wait mark, as of the end of the last pass
   uint32_t nActive;
   uint32_t quit;                 // 1 = voluntary, 2 = final, 3 = abort
@@ -338,13 +339,13 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
     uint32_t spins = 0;
     bool ok;
     // At every fourth poll the last lane looks at the ring too, its load on its way with theirs: a wait with a lot of patience ends when
-    // there is something else to do.  (At every sixteenth where all peers are in the collective already: they are done soon, and another
+    // there is something else to do, which an entry is not that the block has met and cannot take.  (At every sixteenth where all peers are in the collective already: they are done soon, and another
     // collective's context costs more than that.)
     const uint32_t often = which == 1 ? 15u : 3u;
     for (;;) {
       bool laneOk = true;
       uint64_t entry = 0, tag = 1;
-      if ((spins & often) == often && lane == ws - 1 && !sh->standalone && sh->k.devSq != nullptr) {
+      if ((spins & often) == often && lane == ws - 1 && !sh->standalone && sh->k.devSq != nullptr && sh->frontier != sh->stuckAt) {
         entry = ld_relaxed_sys_u64(sh->k.devSq[sh->frontier & (sh->k.sqCap - 1)].w);
         tag = sqTag(sh->frontier, sh->k.sqCap);
       }

@@ -212,3 +212,64 @@ int main() {
 }
 """, defines=("DF_DATAPATH_IMPL",))
     assert out == "ok\n"
+
+
+def test_an_entry_that_cannot_be_taken_ends_no_wait(tmp_path):
+    """The next submission of a collective that still runs stays at the head of the ring: the wait that has nothing else to do keeps its
+    budget; an entry that can be taken ends it at the fourth poll (at the sixteenth where the peers have arrived)."""
+    out = run_on_host(tmp_path, r"""
+#include "device/daemon_impl.h"
+#include <memory>
+static DaemonCtl ctl;
+static RankDev rd;
+static SqSlot ring[8];
+static FlagSlot flags[2];
+static uint32_t meta[4];
+static CollDyn dyn[4];
+static uint64_t frontier;
+static std::unique_ptr<BlockShared> sh;
+static void put(uint64_t index, int coll) {
+  Sqe q;
+  memset((void*)&q, 0, sizeof(q));
+  q.collId = (decltype(q.collId))coll; q.epoch = 2;
+  ring[index & 7] = sqEncode(q, sqTag(index, 8));
+}
+static void say(int v) { printf("%d ", v); }
+static int take() {
+  SqSlot slot, next;
+  const bool haveNext = sqPeek(&sh->k, sh->frontier + 1, &next), have = sqPeek(&sh->k, sh->frontier, &slot);
+  return have ? consumeSubmissions(sh.get(), &rd, 0, slot, next, haveNext) : 0;
+}
+static int polls(int which) {
+  if (boundedWait(sh.get(), &rd, 0, which, 200)) return -1;
+  return (int)sh->waitSpins;
+}
+int main() {
+  memset((void*)&rd, 0, sizeof(rd)); memset((void*)ring, 0, sizeof(ring));
+  rd.ctl = &ctl; rd.devSq = ring; rd.sqCap = 8; rd.nBlocks = 1; rd.maxColls = 4; rd.meta = meta; rd.dyn = dyn; rd.hostFrontier = &frontier;
+  for (auto& m : meta) m = DF_META_VALID | 1u;
+  sh.reset(new BlockShared);
+  memset((void*)sh.get(), 0, sizeof(BlockShared));
+  BlockSaved sv;
+  memset((void*)&sv, 0, sizeof(sv));
+  rd.saved = &sv;
+  blockRestore(sh.get(), &rd, 0);
+  CollStatic* c = &sh->cs;
+  c->kind = dfcclCollBroadcast; c->inType = c->outType = ncclInt8; c->nranks = 2; c->root = 1; c->nBlocks = 1; c->count = 64;
+  c->algo = dfcclAlgoOneShot; c->oneDevice = 1; c->myFlags = flags; c->scale = 1.0;
+  planColl(c, 0);
+  put(0, 1);
+  say(take());                                         // collective 1 runs, its peer is not there
+  sh->dyn.epoch = 2;
+  say(polls(0)); say(polls(1));
+  put(1, 1);                                           // its next submission: stays where it is
+  say(polls(0)); say(take());                          // (the wait that meets it first ends)
+  say(polls(0)); say(polls(1));
+  sh->busy[0] = 0;                                     // collective 1 has completed
+  say(take());
+  put(2, 2);
+  say(polls(0)); say(polls(1)); say(take()); say(polls(0));
+  return 0;
+}
+""")
+    assert out.split() == "1 200 200 4 0 200 200 1 4 16 1 200".split()
