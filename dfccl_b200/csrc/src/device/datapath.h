@@ -362,7 +362,10 @@ DF_HD void reduceTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t 
 template <typename Tin, typename Tout, int OP, bool SHIFT>
 DF_HD void reduceTrips(const DataArgs* a, uint64_t nPacks, int nsrc, int ndst, typename Elem<Tin>::Acc mul, bool doMul, int postDiv,
                        double scale, uint64_t srcOff, uint64_t dstOff, uint32_t shift) {
-  constexpr int U = OP == OP_SUM && !SHIFT ? 4 : 2;     // the sum carries the traffic; the rarer operators trade speed for code size, shifting takes registers
+  // The sum carries the traffic; the rarer operators trade speed for code size, shifting takes registers.  (Shifted sums of as many sources
+  // as reduceAhead does not take, reduce-scatter of 1 000 003 fp32, four packs with a shuffle behind every load / two with all loads first, us:
+  // 3 ranks 45.0 / 36.3, 5 114 / 74, 7 197 / 119; 8 ranks bf16 -> fp32 141 / 91; shorter ones 3 - 20 % less too.)
+  constexpr int U = OP == OP_SUM && !SHIFT ? 4 : 2;
   const int tid = df_tid(), nt = df_nthreads();
   // Software-pipelined over the sources inside a trip: the U loads of source j+1 are issued before
   // the U packs of source j are consumed, so up to 2*U 16-byte loads are in flight per thread.
@@ -453,6 +456,13 @@ DF_HD void reduceAhead(const DataArgs* a, uint64_t nPacks, int ndst, typename El
 // misalignment (true for equal offsets into symmetric buffers): `head` elements bring the destinations to their alignment, from
 // there on the sources are read as packs shifted by `shift` bytes.  Anything else goes element by element (no packs).
 struct Lineup { uint64_t head, nPacks; uint32_t shift; };
+// Where the sources of a call whose pointers line up stand against the grid of its destinations.
+DF_HD uint32_t shiftOf(const DataArgs* a, int esIn, int esOut) {
+  const int outB = 16 / esIn * esOut, DA = outB >= 16 ? 16 : outB;
+  const uint32_t sphase = (uint32_t)((uintptr_t)a->src[0] & 15), dphase = (uint32_t)((uintptr_t)a->dst[0] & (DA - 1));
+  const uint64_t head = ((DA - dphase) & (DA - 1)) / (uint32_t)esOut;
+  return (sphase + (uint32_t)(head > a->n ? a->n : head) * esIn) & 15;
+}
 DF_HD Lineup lineUp(const DataArgs* a, int nsrc, int ndst, uint64_t n, int esIn, int esOut) {
   const int V = 16 / esIn, outB = V * esOut, DA = outB >= 16 ? 16 : outB;          // alignment the vector stores need
   const uint32_t sphase = (uint32_t)((uintptr_t)a->src[0] & 15), dphase = (uint32_t)((uintptr_t)a->dst[0] & (DA - 1));
@@ -550,30 +560,13 @@ DF_HD void reduceAheadOf(const DataArgs* a, uint64_t nPacks, int nsrc, int ndst,
   else reduceAhead<Tin, Tout, 8, SHIFT>(a, nPacks, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
 }
 
+// The head, the ragged tail, or everything when the pointers do not line up: element by element.
 template <typename Tin, typename Tout, int OP>
-DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
+DF_HD void reduceLoose(const DataArgs* a, uint64_t head, uint64_t nPacks) {
   typedef typename Elem<Tin>::Acc A;
-  constexpr int V = 16 / (int)sizeof(Tin);
-  const int tid = df_tid(), nt = df_nthreads();
-  const int nsrc = a->nsrc, ndst = a->ndst;
-  const uint64_t n = a->n;
+  const int tid = df_tid(), nt = df_nthreads(), nsrc = a->nsrc, ndst = a->ndst, postDiv = a->postDiv;
+  const uint64_t n = a->n, tail0 = head + nPacks * (16 / sizeof(Tin));
   const double scale = a->scale;
-  const int postDiv = a->postDiv;
-  const bool doMul = scale != 1.0;
-  const A mul = (A)scale;
-  const Lineup l = lineUp(a, nsrc, ndst, n, (int)sizeof(Tin), (int)sizeof(Tout));
-  const uint64_t head = l.head, nPacks = l.nPacks;
-  const uint32_t shift = l.shift;
-  const uint64_t srcOff = head * sizeof(Tin), dstOff = head * sizeof(Tout);
-  if (nPacks) {
-    const bool ahead = OP == OP_SUM && (nsrc == 2 || nsrc == 4 || (nsrc == 8 && sizeof(Tout) <= sizeof(Tin)));
-    if (ahead && shift == 0) reduceAheadOf<Tin, Tout, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
-    else if (ahead) reduceAheadOf<Tin, Tout, true>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
-    else if (shift == 0) reduceTrips<Tin, Tout, OP, false>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, 0);
-    else reduceTrips<Tin, Tout, OP, true>(a, nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, shift);
-  }
-  // the head, the ragged tail, or everything when the pointers do not line up: element by element
-  const uint64_t tail0 = head + nPacks * V;
   for (uint64_t i = looseStart(tid, nt, nPacks); i < head + (n - tail0); i += nt) {
     const uint64_t e = i < head ? i : tail0 + (i - head);
     A acc = A();
@@ -592,12 +585,39 @@ DF_HD_NOINLINE void reduce_copy(const DataArgs* a) {
   }
 }
 
+// One body for calls on the 16-byte grid and one for shifted sources: what a body uses of its caller's registers goes to local memory and
+// comes back behind fences that emptied L1, and shifting takes most of them.  Bytes of frame, both in one / on the grid: fp32 maximum 248 /
+// 16, bf16 maximum 248 / 64, fp32 sum 248 / 160, copies 136 / 16.  us for all-reduces from the host: maxima of fp32 2 ranks 1 M values 28.3 /
+// 26.9, 4 ranks 1 M 27.8 / 26.0, 4 M 59.5 / 56.5, fp64 4 ranks 1 M 32.6 / 29.4; broadcast of 2 M bf16 24.6 / 23.8; sums, and shifted sources, the
+// same.  (Each lines the pointers up by itself: handed over, the shifted loops took 3 - 7 % longer.)
+template <typename Tin, typename Tout, int OP, bool SHIFT>
+DF_HD_NOINLINE void reduceBody(const DataArgs* a) {
+  const int nsrc = a->nsrc, ndst = a->ndst, postDiv = a->postDiv;
+  const double scale = a->scale;
+  const bool doMul = scale != 1.0;
+  const typename Elem<Tin>::Acc mul = (typename Elem<Tin>::Acc)scale;
+  const Lineup l = lineUp(a, nsrc, ndst, a->n, (int)sizeof(Tin), (int)sizeof(Tout));
+  const uint64_t srcOff = l.head * sizeof(Tin), dstOff = l.head * sizeof(Tout);
+  if (l.nPacks) {
+    if (OP == OP_SUM && (nsrc == 2 || nsrc == 4 || (nsrc == 8 && sizeof(Tout) <= sizeof(Tin))))
+      reduceAheadOf<Tin, Tout, SHIFT>(a, l.nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, l.shift);
+    else reduceTrips<Tin, Tout, OP, SHIFT>(a, l.nPacks, nsrc, ndst, mul, doMul, postDiv, scale, srcOff, dstOff, l.shift);
+  }
+  reduceLoose<Tin, Tout, OP>(a, l.head, l.nPacks);
+}
+
+template <typename Tin, typename Tout, int OP>
+DF_HD void reduce_copy(const DataArgs* a) {
+  if (shiftOf(a, (int)sizeof(Tin), (int)sizeof(Tout))) reduceBody<Tin, Tout, OP, true>(a);
+  else reduceBody<Tin, Tout, OP, false>(a);
+}
+
 // Byte copy of one source to M destinations (AllGather, Broadcast, staging).
-template <bool FULL, bool SHIFT, int U>
-DF_HD void copyTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t strideB, int ndst, uint64_t off, uint32_t shift) {
+template <bool FULL, int U>
+DF_HD void copyTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t strideB, int ndst, uint64_t off) {
   const uint32_t stride = strideB >> 4;
   uint4 raw[U];
-  loadPacks<FULL, SHIFT, U>(raw, a->src[0] + off + p0 * 16, strideB, shift, p0, stride, nPacks);
+  loadPacks<FULL, false, U>(raw, a->src[0] + off + p0 * 16, strideB, 0, p0, stride, nPacks);
   for (int d = 0; d < ndst; ++d) {
     char* o = a->dst[d] + off + p0 * 16;
 #pragma unroll
@@ -605,43 +625,43 @@ DF_HD void copyTrip(const DataArgs* a, uint64_t p0, uint64_t nPacks, uint32_t st
   }
 }
 
-template <bool SHIFT>
-DF_HD void copyTrips(const DataArgs* a, uint64_t nPacks, int ndst, uint64_t off, uint32_t shift) {
+DF_HD void copyTrips(const DataArgs* a, uint64_t nPacks, int ndst, uint64_t off) {
   constexpr int U = 8;
   const int tid = df_tid(), nt = df_nthreads();
   const uint64_t step = (uint64_t)nt * U;
   const uint32_t strideB = (uint32_t)nt * 16u;
   uint64_t base = 0;
-  if (SHIFT) {                                             // (see shiftedWalk)
-    const uint32_t ws = (uint32_t)df_warpsize();
-    const ShiftedWalk w = shiftedWalk((uint32_t)df_tid(), (uint32_t)df_nthreads(), ws);
-    const char* s = a->src[0] + off - shift;
+  for (; base + step <= nPacks; base += step) copyTrip<true, U>(a, base + tid, nPacks, strideB, ndst, off);
+  for (; base + nt <= nPacks; base += nt) copyTrip<true, 1>(a, base + tid, nPacks, strideB, ndst, off);
+  if (base + tid < nPacks) copyTrip<false, 1>(a, base + tid, nPacks, strideB, ndst, off);
+}
+
+DF_HD void copyShifted(const DataArgs* a, uint64_t nPacks, int ndst, uint64_t off, uint32_t shift) {
+  constexpr int U = 8;
+  const uint32_t ws = (uint32_t)df_warpsize();
+  const ShiftedWalk w = shiftedWalk((uint32_t)df_tid(), (uint32_t)df_nthreads(), ws);
+  const char* s = a->src[0] + off - shift;
 #pragma unroll 1
-    for (uint64_t p = w.first; shiftedWarpAt(p, w.lane, nPacks); p += U * w.step) {
-      uint4 raw[U];
+  for (uint64_t p = w.first; shiftedWarpAt(p, w.lane, nPacks); p += U * w.step) {
+    uint4 raw[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint64_t q = p + (uint32_t)u * w.step;
-        if (shiftedLoads(q, w.lane, nPacks)) raw[u] = ld16(s + q * 16);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint64_t q = p + (uint32_t)u * w.step;
-        if (ws > 1 || shiftedWarpAt(q, w.lane, nPacks)) raw[u] = shiftPack(raw[u], nextLane(raw[u], s + q * 16), shift);
-      }
-      if (!shiftedMakes(w.lane, ws)) continue;
-#pragma unroll 1
-      for (int d = 0; d < ndst; ++d) {
-        char* o = a->dst[d] + off + p * 16;
-#pragma unroll
-        for (int u = 0; u < U; ++u) if (p + (uint32_t)u * w.step < nPacks) st16(o + (uint64_t)u * w.step * 16, raw[u]);
-      }
+    for (int u = 0; u < U; ++u) {
+      const uint64_t q = p + (uint32_t)u * w.step;
+      if (shiftedLoads(q, w.lane, nPacks)) raw[u] = ld16(s + q * 16);
     }
-    return;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t q = p + (uint32_t)u * w.step;
+      if (ws > 1 || shiftedWarpAt(q, w.lane, nPacks)) raw[u] = shiftPack(raw[u], nextLane(raw[u], s + q * 16), shift);
+    }
+    if (!shiftedMakes(w.lane, ws)) continue;
+#pragma unroll 1
+    for (int d = 0; d < ndst; ++d) {
+      char* o = a->dst[d] + off + p * 16;
+#pragma unroll
+      for (int u = 0; u < U; ++u) if (p + (uint32_t)u * w.step < nPacks) st16(o + (uint64_t)u * w.step * 16, raw[u]);
+    }
   }
-  for (; base + step <= nPacks; base += step) copyTrip<true, SHIFT, U>(a, base + tid, nPacks, strideB, ndst, off, shift);
-  for (; base + nt <= nPacks; base += nt) copyTrip<true, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);
-  if (base + tid < nPacks) copyTrip<false, SHIFT, 1>(a, base + tid, nPacks, strideB, ndst, off, shift);
 }
 
 // Small copies, in the body of the kernel.
@@ -668,33 +688,36 @@ DF_HD void copySmall(const DataArgs* a) {
 }
 
 #ifdef DF_DATAPATH_IMPL
-__host__ __device__ void copy_multi(const DataArgs* a) {
-  const int tid = df_tid(), nt = df_nthreads();
-  const int ndst = a->ndst;
-  const uint64_t nbytes = a->n;
-  // destinations at one misalignment: `head` bytes bring them to 16, from there the source is read as shifted packs
-  const uint32_t dphase = ndst ? (uint32_t)((uintptr_t)a->dst[0] & 15) : 0;
-  bool vec = ndst > 0;
-  for (int j = 1; j < ndst; ++j) vec &= ((uintptr_t)a->dst[j] & 15) == dphase;
-  uint64_t head = vec ? (16 - dphase) % 16 : 0;
-  if (head > nbytes) head = nbytes;
-  const uint32_t shift = (uint32_t)(((uintptr_t)a->src[0] + head) & 15);
-  const uint64_t nPacks = vec ? (nbytes - head) / 16 : 0;
-  if (nPacks) {
-    if (shift == 0) copyTrips<false>(a, nPacks, ndst, head, 0);
-    else copyTrips<true>(a, nPacks, ndst, head, shift);
-  }
-  const uint64_t tail0 = head + nPacks * 16;
-  for (uint64_t i = looseStart(tid, nt, nPacks); i < head + (nbytes - tail0); i += nt) {
+DF_HD void copyLoose(const DataArgs* a, uint64_t head, uint64_t nPacks) {
+  const int nt = df_nthreads(), ndst = a->ndst;
+  const uint64_t nbytes = a->n, tail0 = head + nPacks * 16;
+  for (uint64_t i = looseStart(df_tid(), nt, nPacks); i < head + (nbytes - tail0); i += nt) {
     const uint64_t e = i < head ? i : tail0 + (i - head);
     uint8_t b = ld_elem((const uint8_t*)a->src[0] + e);
     for (int d = 0; d < ndst; ++d) st_elem((uint8_t*)a->dst[d] + e, b);
   }
 }
-
+template <bool SHIFT>
+DF_HD void copyBody(const DataArgs* a) {
+  const int ndst = a->ndst;
+  Lineup l = {0, 0, 0};
+  if (ndst) l = lineUp(a, 1, ndst, a->n, 1, 1);
+  if (l.nPacks) {
+    if (SHIFT) copyShifted(a, l.nPacks, ndst, l.head, l.shift);
+    else copyTrips(a, l.nPacks, ndst, l.head);
+  }
+  copyLoose(a, l.head, l.nPacks);
+}
+__host__ __device__ void copy_on_grid(const DataArgs* a) { copyBody<false>(a); }
+__host__ __device__ void copy_shifted(const DataArgs* a) { copyBody<true>(a); }
 #else
-__host__ __device__ void copy_multi(const DataArgs* a);
+__host__ __device__ void copy_on_grid(const DataArgs* a);
+__host__ __device__ void copy_shifted(const DataArgs* a);
 #endif
+// (the caller chooses: a body between it and these would have a frame of its own, a round trip to L2 on the way back)
+DF_HD void copy_multi(const DataArgs* a) {
+  if (a->ndst && shiftOf(a, 1, 1)) copy_shifted(a); else copy_on_grid(a);
+}
 
 DF_HD int dtypeSize(int t) {
   switch (t) {
