@@ -264,18 +264,23 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
     // every entry is visited all the same, so that a wait that will never succeed reaches its time limit
     const uint32_t nAct = sh->nActive;
     if (nAct) {
-      if (sh->nParked && scanParked(sh, rd, b)) progressed = true;
+      const bool lone = nAct == 1;
+      if (!lone && sh->nParked && scanParked(sh, rd, b)) progressed = true;
       const bool fullPass = sh->ctl1Full != 0;
       for (uint32_t i = 0; i < nAct; ++i) {
         const int coll = sh->active[i];
         if (coll == 0xffff) continue;
-        if (sh->actWait[i] && !fullPass) continue;
-        // With nothing else queued there is nothing to switch to: polling longer is free, and a new submission ends it (boundedWait).
+        if (sh->actWait[i] && !fullPass && !lone) continue;
+        // With nothing else queued there is nothing to switch to: the block stays with the collective, whose wait ends when something else is
+        // submitted (boundedWait), or after a while beside submissions that a stream may release.
         // With other collectives queued a wait looks twice: the scan looks at the flags of all that are parked at once, and a block that
         // goes on posts the arrivals its peers wait for.  us, 24 mixed collectives of 1 K to 1 M values in four orders / 16 up to 256 K in
-        // two / 30 up to 64 K in four: 211 / 128 / 128 where the oldest had twenty polls, the others four, and a submission did not end a
-        // wait (of up to 110 us, alone); 147 / 73 / 102 now, with four polls 159 / 78 / 104, eight 172 / 83 / 105.
-        const uint32_t budget = nAct == 1 ? sh->k.spinBudget * sh->k.headTries : (sh->k.spinBudget + 15u) / 16u;
+        // two / 30 up to 64 K in four: 211 / 94 / 115 where the oldest had twenty polls, the others four, and a submission did not end a
+        // wait (of up to 110 us, alone); 147 / 90 / 100 now, with four polls 159 / 78 / 104 against 147 / 73 / 102, eight 172 / 83 / 105.
+        // What streams release comes in program order as a rule, the same on all ranks: there the oldest has its tries (2 ranks, 4 x 1 M bf16 ->
+        // fp32 by one stream 118 -> 112, published ahead 126 -> 120; more polls, the same).
+        const uint32_t crowd = (sh->k.spinBudget + 15u) / 16u;
+        const uint32_t budget = !lone ? crowd : sh->nTrig ? pollsBesideTriggers(&sh->k) : sh->k.spinBudget * sh->k.headTries;
         bool moved = false;
         int rc = runColl(sh, rd, b, coll, budget, &moved);
         if (rc == RC_DONE || rc == RC_YIELD || moved) progressed = true;

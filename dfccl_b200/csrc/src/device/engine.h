@@ -339,8 +339,11 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
     uint32_t spins = 0;
     bool ok;
     // At every fourth poll the last lane looks at the ring too, its load on its way with theirs: a wait with a lot of patience ends when
-    // there is something else to do, which an entry is not that the block has met and cannot take.  (At every sixteenth where all peers are in the collective already: they are done soon, and another
-    // collective's context costs more than that.)
+    // there is something else to do, which an entry is not that the block has met and cannot take, and hardly one that a stream has yet to
+    // release.  (At every sixteenth where all peers are in the collective already: they are done soon, and another collective's context
+    // costs more than that.)  us, all-reduces of bf16 -> fp32 that one stream releases in the same order on all ranks, no look / a look that any
+    // entry ends / now: 2 ranks 4 x 1 M 114 / 121 / 112, 4 ranks 141 / 158 / 145, 4 ranks 8 x 500 K 246 / 280 / 259; 2 ranks 8 x 1 M in two orders 279 /
+    // 230 / 234 (277 where these entries end no wait).
     const uint32_t often = which == 1 ? 15u : 3u;
     for (;;) {
       bool laneOk = true;
@@ -366,8 +369,8 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
         }
       }
       bool laneStop = false;
-      if ((spins & 255) == 255 && lane == 0) laneStop = abortRequested(&sh->k);
-      if (entry >> 57 == tag) laneStop = true;
+      if ((spins & 255) == 255 && lane == 0) laneStop = abortRequested(&sh->k) || (!sh->standalone && ld_relaxed_sys_u32(&rd->quitting) != 0);      // (the others have left: so does this block)
+      if (entry >> 57 == tag && (!((entry >> 48) & SQE_TRIGGERED) || spins + 1 >= pollsBesideTriggers(&sh->k))) laneStop = true;
       ok = df_warp_all(laneOk);
       const bool stop = !df_warp_all(!laneStop);      // uniform: every lane leaves the loop together
       ++spins;
@@ -627,12 +630,15 @@ DF_HD int nextPhase(const BlockShared* sh, int phase) {
 }
 
 // A wait of the loaded collective with its adaptive budget.  The budget is what the scheduler grants or, if larger and nothing else
-// is queued, the patience this submission has earned: after a wait succeeded within s polls the next waits of the same
+// is queued or may be released, the patience this submission has earned: after a wait succeeded within s polls the next waits of the same
 // submission may spend factor x s polls (capped), because a collective whose peers are demonstrably in it is worth
-// staying with (reference: RECV_SUCCESS_FACTOR, src/collectives_ofccl/device/ofccl_prims_simple.h:79-88,143-151).
+// staying with (reference: RECV_SUCCESS_FACTOR, src/collectives_ofccl/device/ofccl_prims_simple.h:79-88,143-151).  Beside others the
+// oldest of the queue has NUM_TRY_TASKQ_HEAD times the budget if a stream released it.
 DF_HD bool patientWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t budget) {
-  const bool alone = sh->standalone || sh->nActive <= 1;
-  const uint32_t eff = alone && sh->dyn.patience > budget ? sh->dyn.patience : budget;
+  uint32_t eff = budget;
+  if (sh->standalone || (sh->nActive <= 1 && sh->nTrig == 0)) {
+    if (sh->dyn.patience > eff) eff = sh->dyn.patience;
+  } else if (sh->nActive > 1 && (sh->dyn.sqeFlags & SQE_TRIGGERED) && sh->active[0] == sh->loadedColl) eff = budget * sh->k.headTries;
   const bool ok = boundedWait(sh, rd, b, which, eff);
   if (ok && df_tid() == 0) {
     sh->dyn.stallSinceNs = 0;

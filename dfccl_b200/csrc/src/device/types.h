@@ -279,6 +279,8 @@ struct RankConst {
   uint64_t maxLifetimeNs;          // one launch of the daemon leaves after this long regardless of its state (0 = never)
   uint64_t sliceBytes;             // PH_DATA yields after this many bytes when others are queued (0 = never)
 };
+// Polls of a wait beside submissions that a stream has not released yet: their trigger words are looked at in between.
+static __host__ __device__ inline uint32_t pollsBesideTriggers(const RankConst* k) { return (k->spinBudget + 7u) / 8u * k->headTries; }
 struct RankDev : RankConst {
   uint64_t svcHead;                // entries the service warp has copied
   uint64_t devCqTail;

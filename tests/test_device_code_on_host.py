@@ -216,7 +216,8 @@ int main() {
 
 def test_an_entry_that_cannot_be_taken_ends_no_wait(tmp_path):
     """The next submission of a collective that still runs stays at the head of the ring: the wait that has nothing else to do keeps its
-    budget; an entry that can be taken ends it at the fourth poll (at the sixteenth where the peers have arrived)."""
+    budget; an entry that can be taken ends it at the fourth poll (at the sixteenth where the peers have arrived), one that a stream
+    has yet to release at the twentieth (thirty-second)."""
     out = run_on_host(tmp_path, r"""
 #include "device/daemon_impl.h"
 #include <memory>
@@ -228,10 +229,10 @@ static uint32_t meta[4];
 static CollDyn dyn[4];
 static uint64_t frontier;
 static std::unique_ptr<BlockShared> sh;
-static void put(uint64_t index, int coll) {
+static void put(uint64_t index, int coll, uint32_t flags = 0) {
   Sqe q;
   memset((void*)&q, 0, sizeof(q));
-  q.collId = (decltype(q.collId))coll; q.epoch = 2;
+  q.collId = coll; q.epoch = 2; q.flags = flags;
   ring[index & 7] = sqEncode(q, sqTag(index, 8));
 }
 static void say(int v) { printf("%d ", v); }
@@ -246,7 +247,7 @@ static int polls(int which) {
 }
 int main() {
   memset((void*)&rd, 0, sizeof(rd)); memset((void*)ring, 0, sizeof(ring));
-  rd.ctl = &ctl; rd.devSq = ring; rd.sqCap = 8; rd.nBlocks = 1; rd.maxColls = 4; rd.meta = meta; rd.dyn = dyn; rd.hostFrontier = &frontier;
+  rd.ctl = &ctl; rd.spinBudget = 32; rd.headTries = 5; rd.devSq = ring; rd.sqCap = 8; rd.nBlocks = 1; rd.maxColls = 4; rd.meta = meta; rd.dyn = dyn; rd.hostFrontier = &frontier;
   for (auto& m : meta) m = DF_META_VALID | 1u;
   sh.reset(new BlockShared);
   memset((void*)sh.get(), 0, sizeof(BlockShared));
@@ -269,7 +270,45 @@ int main() {
   say(take());
   put(2, 2);
   say(polls(0)); say(polls(1)); say(take()); say(polls(0));
+  put(3, 3, SQE_TRIGGERED);                            // a stream has yet to release it
+  say(polls(0)); say(polls(1)); say(take()); say((int)sh->nTrig);
   return 0;
 }
 """)
-    assert out.split() == "1 200 200 4 0 200 200 1 4 16 1 200".split()
+    assert out.split() == "1 200 200 4 0 200 200 1 4 16 1 200 20 32 1 1".split()
+
+
+def test_how_long_a_wait_lasts(tmp_path):
+    """RECV_SUCCESS_FACTOR: a wait that succeeded at its first poll allows the next of the same submission `factor` polls, where that is
+    more than its budget and nothing else is queued or may be released.  NUM_TRY_TASKQ_HEAD: beside others the oldest of the queue has
+    that many budgets where a stream released it."""
+    out = run_on_host(tmp_path, r"""
+#include <memory>
+static DaemonCtl ctl;
+static uint32_t polls(uint32_t factor, uint32_t budget, uint32_t queued, uint32_t waiting = 0, uint32_t flags = 0, int place = 0) {
+  FlagSlot f[2];
+  memset((void*)f, 0, sizeof(f));
+  RankDev rd;
+  memset((void*)&rd, 0, sizeof(rd));
+  rd.ctl = &ctl; rd.recvSuccessFactor = factor; rd.spinBudget = 32; rd.headTries = 5;
+  std::unique_ptr<BlockShared> sh(new BlockShared);
+  memset((void*)sh.get(), 0, sizeof(BlockShared));
+  sh->k = rd; sh->nActive = queued; sh->nTrig = waiting; sh->loadedColl = 3;
+  for (uint32_t i = 0; i < queued; ++i) sh->active[i] = (int)i == place ? 3 : 7;
+  CollStatic* c = &sh->cs;
+  c->kind = dfcclCollBroadcast; c->inType = c->outType = ncclInt8; c->nranks = 2; c->root = 1; c->nBlocks = 1; c->count = 64;
+  c->algo = dfcclAlgoOneShot; c->oneDevice = 1; c->myFlags = f; c->scale = 1.0;
+  planColl(c, 0);
+  sh->dyn.epoch = 1; sh->dyn.sqeFlags = flags;
+  f[1].arrive = 1; f[1].sendOff = offTagged(64, 1); f[1].recvOff = offTagged(128, 1);
+  if (!patientWait(sh.get(), &rd, 0, 0, budget) || sh->waitSpins != 1) return 0;
+  if (patientWait(sh.get(), &rd, 0, 1, budget)) return 1;      // the peer is never done
+  return sh->waitSpins;
+}
+int main() {
+  printf("%u %u %u %u %u ", polls(0, 2, 1), polls(50, 2, 1), polls(50, 160, 1), polls(50, 2, 2), polls(1u << 30, 2, 1));
+  printf("%u %u %u %u %u\n", polls(50, 20, 1, 1), polls(0, 2, 2, 0, SQE_TRIGGERED), polls(0, 2, 2, 0, SQE_TRIGGERED, 1), polls(50, 2, 2, 3, SQE_TRIGGERED), polls(0, 160, 1, 0, SQE_TRIGGERED));
+  return 0;
+}
+""")
+    assert out.split() == ["2", "50", "160", "2", str(64 * 32), "20", "10", "2", "10", "160"]
