@@ -1,9 +1,10 @@
 """Long sums of two, four and eight aligned sources, whose loads run ahead of the stores: whole trips of a block, one pack more and
-less, ragged ends, every element size, results wider and narrower than the operands; and sums and copies of pieces that start off
-the 16-byte grid, where a warp's 32 aligned packs make 31."""
+less, ragged ends (all-reduces: the pieces of a reduce-scatter of odd length start off the grid), every element size, results wider and
+narrower than the operands, in place and not; and sums and copies of pieces that start off the 16-byte grid, where a warp's 32
+aligned packs make 31."""
 import pytest
 
-from test_gpu_daemon import _loopback_case, nv  # noqa: F401
+from test_gpu_daemon import TORCH_OF, _loopback_case, nv  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -18,7 +19,8 @@ CASES = [(2, 4 * 1920 * 3, "FLOAT32", None, "AVG"), (2, 8 * 1920 * 4 + 8, "BFLOA
 @pytest.mark.parametrize("nranks,count,dtype,out,op", CASES)
 def test_sums_with_loads_ahead(nv, kind, nranks, count, dtype, out, op):  # noqa: F811
     if kind == "reducescatter":
-        count = (count + 15) // 16 * 16                    # chunks on the 16-byte grid; others take the shifted path
+        pack = 16 // TORCH_OF[dtype].itemsize
+        count = (count + pack - 1) // pack * pack          # chunks on the 16-byte grid; others take the shifted path
     _loopback_case(nv, kind, nranks, count, dtype, op=op, out_name=out, blocks=1)
 
 
@@ -33,3 +35,15 @@ SHIFTED = [("reducescatter", 2, 4 * 465 * 40 + 1, "FLOAT32", None), ("reducescat
 def test_pieces_off_the_grid(nv, kind, nranks, count, dtype, out):  # noqa: F811
     for blocks in (1, 3):
         _loopback_case(nv, kind, nranks, count, dtype, out_name=out, blocks=blocks)
+
+
+# every source's next packs are loaded in front of the present ones' stores, which go to one of the sources
+IN_PLACE = [("allreduce", 2, 8 * 1920 * 7 + 5, "BFLOAT16", "SUM"), ("allreduce", 4, 4 * 960 * 4 * 5 + 3, "FLOAT32", "AVG"), ("allreduce", 8, 8 * 480 * 8 * 5 + 1, "BFLOAT16", "SUM"),
+            ("allreduce", 4, 300007, "INT32", "MAX"), ("reducescatter", 2, 4 * 1920 * 9 + 4, "FLOAT32", "SUM"), ("reducescatter", 4, 8 * 960 * 5 - 8, "BFLOAT16", "SUM"),
+            ("reducescatter", 8, 4 * 480 * 40 + 3, "FLOAT32", "SUM"), ("allgather", 4, 300007, "BFLOAT16", "SUM")]
+
+
+@pytest.mark.parametrize("kind,nranks,count,dtype,op", IN_PLACE)
+def test_long_calls_in_place(nv, kind, nranks, count, dtype, op):  # noqa: F811
+    for blocks in (1, 3):
+        _loopback_case(nv, kind, nranks, count, dtype, op=op, in_place=True, iters=3, blocks=blocks, algo=nv.ALGO_TWOSHOT if kind == "allreduce" else 0)

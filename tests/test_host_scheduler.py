@@ -136,9 +136,9 @@ def test_deferred_submission_runs_when_released(host_backend, trigger_first):
         c.destroy()
 
 
-def test_patience_grows_after_successful_waits(host_backend):
-    """With a tiny base budget and a large success factor, collectives still complete under disordered issue, and
-    fewer context switches are needed than with the factor switched off."""
+def test_disordered_issue_with_tiny_budgets(host_backend):
+    """With a budget of two polls a wait, with and without patience for collectives whose waits have succeeded, collectives issued in
+    different orders complete, by switching between them.  (What patience does to a wait: test_device_code_on_host.)"""
     nv = host_backend
     switches = {}
     for factor in (0, 50):
