@@ -12,7 +12,11 @@ where the two waits are *bounded*: after ``spin_budget`` unsuccessful polls
 the daemon parks the collective (its cursor is two integers) and visits the
 next entry of its queue — the behaviour of the reference's ``waitPeer`` budget
 (src/collectives_ofccl/device/ofccl_prims_simple.h:118-140) and task-queue
-traversal (src/collectives_ofccl/device/enqueue_ofccl_dev.cu:922-1023).  With
+traversal (src/collectives_ofccl/device/enqueue_ofccl_dev.cu:922-1023).  (That
+is the reference's rule.  The device scheduler of this library gives a wait
+beside other collectives a sixteenth of the threshold, the queue's head more only
+where a stream released it, and finds parked collectives again by a scan of their
+flags.)  With
 ``preemptive=False`` the same machine models a stream-ordered library: a wait
 never gives up, so incompatible issue orders hang, which the model reports
 together with the wait-for cycle that explains it.
