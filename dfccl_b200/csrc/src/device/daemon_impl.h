@@ -278,7 +278,7 @@ DF_HD void daemonBlockMain(RankDev* rd, int b, BlockShared* sh) {
         // two / 30 up to 64 K in four: 211 / 94 / 115 where the oldest had twenty polls, the others four, and a submission did not end a
         // wait (of up to 110 us, alone); 147 / 90 / 100 now, with four polls 159 / 78 / 104 against 147 / 73 / 102, eight 172 / 83 / 105.
         // What streams release comes in program order as a rule, the same on all ranks: there the oldest has its tries (2 ranks, 4 x 1 M bf16 ->
-        // fp32 by one stream 118 -> 112, published ahead 126 -> 120; more polls, the same).
+        // fp32 by one stream 117.6 -> 114.5, published ahead 126 -> 121; more polls, the same).
         const uint32_t crowd = (sh->k.spinBudget + 15u) / 16u;
         const uint32_t budget = !lone ? crowd : sh->nTrig ? pollsBesideTriggers(&sh->k) : sh->k.spinBudget * sh->k.headTries;
         bool moved = false;

@@ -342,8 +342,8 @@ DF_HD bool boundedWait(BlockShared* sh, RankDev* rd, int b, int which, uint32_t 
     // there is something else to do, which an entry is not that the block has met and cannot take, and hardly one that a stream has yet to
     // release.  (At every sixteenth where all peers are in the collective already: they are done soon, and another collective's context
     // costs more than that.)  us, all-reduces of bf16 -> fp32 that one stream releases in the same order on all ranks, no look / a look that any
-    // entry ends / now: 2 ranks 4 x 1 M 114 / 121 / 112, 4 ranks 141 / 158 / 145, 4 ranks 8 x 500 K 246 / 280 / 259; 2 ranks 8 x 1 M in two orders 279 /
-    // 230 / 234 (277 where these entries end no wait).
+    // entry ends / now: 2 ranks 4 x 1 M 115 / 123 / 114, 4 ranks 141 / 158 / 148, 4 ranks 8 x 500 K 249 / 279 / 264; 2 ranks 8 x 1 M in two orders 283 /
+    // 234 / 238 (277 where these entries end no wait, the others then 112, 142, 254).
     const uint32_t often = which == 1 ? 15u : 3u;
     for (;;) {
       bool laneOk = true;
