@@ -54,7 +54,8 @@ __device__ __forceinline__ void publishDone(const OneRankDone& done, unsigned lo
 // to what a cluster holds with four packs a thread in flight; eight calls behind one another in a stream, blocks that count
 // themselves / one cluster, us: 8 KB 38.8 / 35.5, 64 KB 45.8 / 36.3, 128 KB (the limit) 47.4 / 37.2.
 // What is left of such a call (4.5 us): 1.35 until the kernel in front is known to have ended, 0.6 for the data, 0.65 for the cluster's
-// barrier, 1.9 for the system-wide fence and the entry, whose place was asked for in front of the loads (eight of 64 KB 36.8 -> 36.2).
+// barrier, 1.9 for the system-wide fence and the entry, whose place was asked for in front of the loads (eight of
+// 64 KB 36.1 -> 35.5, of 128 KB as fp32 40.1 -> 38.5, of 16 KB and less the same).
 // The blocks may come up while the kernel in front of them in the stream still runs, and wait for its end before they read.
 template <typename Tin, typename Tout, bool COPY, int U, bool SHORT>
 __global__ void __launch_bounds__(THREADS) dfcclOneRankKernel(const OneRankArgs a) {
